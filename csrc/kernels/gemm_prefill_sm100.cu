@@ -63,7 +63,7 @@ struct PrefillParams {
   // row, rows, -} of num_group_tiles[0] tiles, and a group's weight rows start at group * group_w_rows
   int out_fp32;
   const int4* group_tiles; const int* num_group_tiles;
-  int group_w_rows;
+  int group_w_rows, group_rows;          // weight rows of a group, token rows of a tile of the table (128 or 256)
   BulkArParams ar;
 };
 
@@ -103,11 +103,14 @@ __device__ __forceinline__ void decode_item(const PrefillParams& p, int item, in
 }
 
 // mbarrier wait that also gives up as soon as another role of this CTA has raised the abort flag
+// (CLUSTER: the phase is completed by another CTA of the cluster too)
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, uint32_t parity, int* status, int code,
                                                    volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
+  auto done = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+  if (done()) return true;
   const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {
+  while (!done()) {
     if (*abort_flag) return false;
     if (clock64() - t0 > kWaitCycles) {
       if (status) atomicCAS(status, 0, code);
@@ -424,34 +427,49 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_kernel(const __grid_const
 
 // ------------------------------------------------------------------------------------------------------------------
 // Token-major form (one GPU, or the local product in front of a library collective).  Same pipeline, but the operands
-// trade places: the 128 rows of the MMA are 128 TOKENS (A = the activation tile) and its columns are BNF output features
+// trade places: the rows of the MMA are TOKENS (A = the activation tile) and its columns are output features
 // (B = the weight tile), so the accumulator is [token lane][feature column] — the layout of Y itself.  Each epilogue
-// thread owns one token row and handles 16 consecutive features per step: bias and residual arrive as 16-byte vectors
-// and the result leaves as two 16-byte stores, instead of one 2-byte store per element in the feature-major form, whose
+// thread owns one token row and handles 32 consecutive features per step: bias and residual arrive as 16-byte vectors
+// and the result leaves as 16-byte stores, instead of one 2-byte store per element in the feature-major form, whose
 // epilogue (a dependent chain per element on four warps) took ten times longer than the main loop of the short-K
-// row-parallel products.  Gated form: gate and up accumulators of 128 features each, act(gate) * up on the way out.
-template <int BNF, bool DUAL>
-__global__ void __launch_bounds__(192, 1) gemm_prefill_tm_kernel(const __grid_constant__ CUtensorMap tmX,
+// row-parallel products.  Gated form: gate and up accumulators side by side, act(gate) * up on the way out.
+//
+// CG = 2: the two CTAs of a cluster work on one tile of 256 tokens with `cta_group::2` MMAs issued by the first of them.
+// Each CTA keeps its 128 tokens (A, and their accumulator rows in its own TMEM) and HALF of the tile's weight rows, which
+// the tensor cores of both read: per MMA an SM then takes 128 + NCOL / 2 rows from shared memory instead of 128 + NCOL,
+// and as many fewer arrive by TMA.  With 128 x 256 tiles of single CTAs those reads and writes together (192 bytes per
+// cycle) were more than shared memory delivers.  In the gated form the first CTA holds the gate rows and the second the
+// up rows.  Both producers signal the first CTA's full barrier; a commit frees the stage in both.
+//
+// NCOL: accumulator columns of a tile (gated: half of them gate, half up).
+constexpr int kPrefillTmThreads = 320;      // producer, MMA, two epilogue warps per quarter of the accumulator's rows
+__host__ __device__ constexpr int prefill_tm_stages(int stage_bytes) { return 196 * 1024 / stage_bytes < kPrefillMaxStages ? 196 * 1024 / stage_bytes : kPrefillMaxStages; }
+
+template <int NCOL, bool DUAL, int CG>
+__global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(const __grid_constant__ CUtensorMap tmX,
                                                                  const __grid_constant__ CUtensorMap tmW,
                                                                  const PrefillParams p) {
-  constexpr int A_BYTES = 128 * 64 * 2;                  // 128 tokens x 64 k
-  constexpr int B_BYTES = BNF * 64 * 2;                  // BNF features x 64 k
-  constexpr int NACC = DUAL ? 2 : 1;
-  constexpr int STAGE_BYTES = A_BYTES + B_BYTES * NACC;
-  constexpr uint32_t TMEM_COLS = 2 * BNF * NACC;         // double-buffered accumulators
-  constexpr uint32_t IDESC = umma_idesc(128, BNF, 1, 1, 1);
-  static_assert((BNF == 256 && !DUAL) || (BNF == 128 && DUAL), "feature tile of the token-major kernel");
+  constexpr int FEAT = DUAL ? NCOL / 2 : NCOL;           // features of an output tile
+  constexpr int TOK = 128 * CG;                          // tokens of an output tile
+  constexpr int A_BYTES = 128 * 64 * 2;                  // this CTA's 128 tokens x 64 k
+  constexpr int B_BYTES = NCOL / CG * 64 * 2;            // this CTA's weight rows x 64 k
+  constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  constexpr int STAGES = prefill_tm_stages(STAGE_BYTES);
+  constexpr uint32_t TMEM_COLS = 2 * NCOL;               // double-buffered accumulators
+  constexpr uint32_t IDESC = umma_idesc(TOK, NCOL, 1, 1, 1);
+  static_assert((NCOL == 256 || NCOL == 128) && (CG == 1 || CG == 2), "tile of the token-major kernel");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t full_bar[kPrefillMaxStages], empty_bar[kPrefillMaxStages], tmem_full[2], tmem_empty[2];
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tmem_full[2], tmem_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_abort_mem;
   volatile int* s_abort = &s_abort_mem;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int stages = p.stages;
-  // n_tiles: feature tiles of BNF, t_tiles: token blocks of 128 (grouped: at most so many)
+  const int half = CG == 2 ? (int)cluster_ctarank() : 0;      // which 128 tokens of a tile are this CTA's
+  const int first = blockIdx.x / CG, step = gridDim.x / CG;
+  // n_tiles: feature tiles of FEAT, t_tiles: token blocks of TOK (grouped: at most so many)
   const int total = p.n_tiles * (p.group_tiles ? min(*p.num_group_tiles, p.t_tiles) : p.t_tiles);
   // an item's feature tile, first token row, number of rows and first weight row of its group
   struct Item { int nt, row0, rows, w0; };
@@ -463,21 +481,23 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_tm_kernel(const __grid_co
     } else {
       int blk;
       decode_item(p, item, r.nt, blk);
-      r.row0 = blk * 128;
+      r.row0 = blk * TOK;
       r.rows = p.T - r.row0;
       r.w0 = 0;
     }
+    r.row0 += half * 128;
+    r.rows -= half * 128;
     return r;
   };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
-      mbar_init(&tmem_empty[a], 4);
+      mbar_init(&tmem_empty[a], 8 * CG);
     }
     s_abort_mem = 0;
     fence_barrier_init();
@@ -486,101 +506,129 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_tm_kernel(const __grid_co
     tma_prefetch_desc(&tmX);
   }
   if (warp == 1) {
-    tmem_alloc(&tmem_base_s, TMEM_COLS);
-    tmem_relinquish();
+    if constexpr (CG == 2) {
+      tmem_alloc_pair(&tmem_base_s, TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(&tmem_base_s, TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tcgen05_fence_before();
   __syncthreads();
+  if constexpr (CG == 2) {              // both CTAs' barriers and accumulators exist before either touches the other's
+    cluster_arrive();
+    cluster_wait();
+  }
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_base_s;
 
+  // The two issuing threads are the kernel's critical path when a step's MMAs are short, so their loops carry stage, phase
+  // and descriptors along instead of dividing, and look at the abort flag only when a wait does not succeed at once.
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t hint = kEvictNormal;
-      int it = 0;
+      const uint32_t lead_bar = CG == 2 ? dsmem_addr(smem_u32(full_bar), 0) : 0;      // the first CTA's full barriers
+      int s = 0;
+      uint32_t ph = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < total && ok; item += gridDim.x) {
+      auto step_stage = [&] { if (++s == STAGES) { s = 0; ph ^= 1; } };
+      for (int item = first; item < total && ok; item += step) {
         const Item im = item_of(item);
-        for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
-          const int s = it % stages;
-          const uint32_t ph = (it / stages) & 1;
-          if (*s_abort || !mbar_wait_or_abort(&empty_bar[s], ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY, s_abort)) {
+        const int wrow = im.w0 + im.nt * FEAT + half * (DUAL ? p.dual_off : NCOL / 2);
+        for (int kb = 0; kb < p.num_kb; ++kb, step_stage()) {
+          if (!mbar_wait_or_abort<CG == 2>(&empty_bar[s], ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY, s_abort)) {
             ok = false;
             break;
           }
-          mbar_expect_tx(&full_bar[s], STAGE_BYTES);
           uint8_t* a = smem + s * STAGE_BYTES;
-          tma_load_2d(a, &tmX, &full_bar[s], kb * 64, im.row0, hint);
-          tma_load_2d(a + A_BYTES, &tmW, &full_bar[s], kb * 64, im.w0 + im.nt * BNF, hint);
-          if (DUAL) tma_load_2d(a + A_BYTES + B_BYTES, &tmW, &full_bar[s], kb * 64, im.w0 + p.dual_off + im.nt * BNF, hint);
+          if constexpr (CG == 2) {
+            if (half == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
+            tma_load_2d_pair(a, &tmX, lead_bar + 8 * s, kb * 64, im.row0, hint);
+            tma_load_2d_pair(a + A_BYTES, &tmW, lead_bar + 8 * s, kb * 64, wrow, hint);
+          } else {
+            mbar_expect_tx(&full_bar[s], STAGE_BYTES);
+            tma_load_2d(a, &tmX, &full_bar[s], kb * 64, im.row0, hint);
+            tma_load_2d(a + A_BYTES, &tmW, &full_bar[s], kb * 64, wrow, hint);
+            if (DUAL) tma_load_2d(a + A_BYTES + FEAT * 128, &tmW, &full_bar[s], kb * 64, wrow + p.dual_off, hint);
+          }
         }
       }
       if (!ok) {
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000LL) {}
+      } else if (CG == 2) {
+        // the first CTA's commits also arrive here: stay until every stage has been given back
+        for (int k = 0; k < STAGES; ++k, step_stage())
+          if (!mbar_wait_or_abort<true>(&empty_bar[s], ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY, s_abort)) break;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int it = 0, lt = 0;
+    if (half == 0 && elect_one()) {
+      const uint64_t adesc0 = umma_desc_k128(smem_u32(smem));                      // tokens
+      const uint64_t bdesc0 = umma_desc_k128(smem_u32(smem) + A_BYTES);            // features (gated: gate rows, then up rows)
+      int s = 0, lt = 0;
+      uint32_t ph = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < total && ok; item += gridDim.x, ++lt) {
+      for (int item = first; item < total && ok; item += step, ++lt) {
         const int a = lt & 1;
         const uint32_t aph = (lt >> 1) & 1;
-        if (*s_abort || !mbar_wait_or_abort(&tmem_empty[a], aph ^ 1, p.status, XFT_ERR_WAIT_TMEM, s_abort)) break;
+        if (!mbar_wait_or_abort<CG == 2>(&tmem_empty[a], aph ^ 1, p.status, XFT_ERR_WAIT_TMEM, s_abort)) break;
         tcgen05_fence_after();
-        const uint32_t acc = tmem_base + (uint32_t)(a * BNF * NACC);
-        for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
-          const int s = it % stages;
-          const uint32_t ph = (it / stages) & 1;
-          if (!mbar_wait_or_abort(&full_bar[s], ph, p.status, XFT_ERR_WAIT_FULL, s_abort)) {
+        const uint32_t acc = tmem_base + (uint32_t)(a * NCOL);
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          if (!mbar_wait_or_abort<CG == 2>(&full_bar[s], ph, p.status, XFT_ERR_WAIT_FULL, s_abort)) {
             ok = false;
             break;
           }
           tcgen05_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-          const uint64_t adesc = umma_desc_k128(a_addr);                      // tokens
-          const uint64_t bdesc = umma_desc_k128(a_addr + A_BYTES);            // features (gate)
+          const uint64_t off = (uint64_t)(s * (STAGE_BYTES / 16));
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            umma_bf16(acc, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > 0 || k > 0) ? 1u : 0u);
-            if (DUAL) {
-              const uint64_t b1desc = umma_desc_k128(a_addr + A_BYTES + B_BYTES);
-              umma_bf16(acc + BNF, adesc + 2 * k, b1desc + 2 * k, IDESC, (kb > 0 || k > 0) ? 1u : 0u);
-            }
+            const uint32_t acc_on = (kb > 0 || k > 0) ? 1u : 0u;
+            if constexpr (CG == 2) umma_bf16_pair(acc, adesc0 + off + 2 * k, bdesc0 + off + 2 * k, IDESC, acc_on);
+            else umma_bf16(acc, adesc0 + off + 2 * k, bdesc0 + off + 2 * k, IDESC, acc_on);
           }
-          tcgen05_commit(&empty_bar[s]);
+          if constexpr (CG == 2) tcgen05_commit_pair(&empty_bar[s]);
+          else tcgen05_commit(&empty_bar[s]);
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
-        if (ok) tcgen05_commit(&tmem_full[a]);
+        if (ok) {
+          if constexpr (CG == 2) tcgen05_commit_pair(&tmem_full[a]);
+          else tcgen05_commit(&tmem_full[a]);
+        }
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue: one token row per thread
+    // ------------------------------------------------------------------ epilogue: one token row and half the features per thread
     const int q = warp & 3;
+    const int c_begin = warp < 6 ? 0 : FEAT / 2, c_end = c_begin + FEAT / 2;
     const int row = q * 32 + lane;
     const bool vec = (p.N % 8 == 0) && (p.ldo % 8 == 0) && (!p.residual || p.ldr % 8 == 0);
+    // 32-byte rows' pieces: every store fills a whole sector
+    const bool vec32 = vec && p.ldo % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
     const bool bias16 = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
     int lt = 0;
-    for (int item = blockIdx.x; item < total; item += gridDim.x, ++lt) {
+    for (int item = first; item < total; item += step, ++lt) {
       const Item im = item_of(item);
       const int a = lt & 1;
       const uint32_t aph = (lt >> 1) & 1;
       mbar_wait_or_abort(&tmem_full[a], aph, p.status, XFT_ERR_WAIT_TMEM, s_abort);
-      if (named_bar_or(1, 128, *s_abort != 0)) break;
+      if (named_bar_or(1, 256, *s_abort != 0)) break;
       tcgen05_fence_after();
-      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + (uint32_t)(a * BNF * NACC);
+      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + (uint32_t)(a * NCOL);
       const int t = im.row0 + row;
       const bool t_ok = row < im.rows;
       __nv_bfloat16* orow = p.out + (size_t)t * p.ldo;
       const __nv_bfloat16* rrow = p.residual ? p.residual + (size_t)t * p.ldr : nullptr;
 #pragma unroll 1
-      for (int c = 0; c < BNF; c += 32) {
-        const int n0 = im.nt * BNF + c;
+      for (int c = c_begin; c < c_end; c += 32) {
+        const int n0 = im.nt * FEAT + c;
         const bool full = vec && n0 + 32 <= p.N;
         uint32_t v[32];
         uint32_t vu[DUAL ? 32 : 1];
         tmem_ld32(taddr + c, v);
-        if constexpr (DUAL) tmem_ld32(taddr + BNF + c, reinterpret_cast<uint32_t (&)[32]>(vu));
+        if constexpr (DUAL) tmem_ld32(taddr + FEAT + c, reinterpret_cast<uint32_t (&)[32]>(vu));
         uint4 res[4];
         const bool take = rrow && full && t_ok && !p.out_fp32;
         if (take) {
@@ -588,10 +636,13 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_tm_kernel(const __grid_co
           for (int j = 0; j < 4; ++j) res[j] = *reinterpret_cast<const uint4*>(rrow + n0 + 8 * j);
         }
         tmem_ld_wait();
-        if (c + 32 >= BNF) {
+        if (c + 32 >= c_end) {
           tcgen05_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&tmem_empty[a]);
+          if (lane == 0) {
+            if constexpr (CG == 2) mbar_arrive_cluster(dsmem_addr(smem_u32(&tmem_empty[a]), 0));
+            else mbar_arrive(&tmem_empty[a]);
+          }
         }
         if (!t_ok || n0 >= p.N) continue;
         float x[32];
@@ -671,15 +722,19 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_tm_kernel(const __grid_co
               }
             }
           }
+          uint32_t w[16];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t w[4];
+          for (int j = 0; j < 16; ++j) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
+            w[j] = *reinterpret_cast<const uint32_t*>(&b);
+          }
+          if (vec32) {
+            st_global_256(orow + n0, w);
+            st_global_256(orow + n0 + 16, w + 8);
+          } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const __nv_bfloat162 b = __floats2bfloat162_rn(x[8 * i + 2 * j], x[8 * i + 2 * j + 1]);
-              w[j] = *reinterpret_cast<const uint32_t*>(&b);
-            }
-            *reinterpret_cast<uint4*>(orow + n0 + 8 * i) = make_uint4(w[0], w[1], w[2], w[3]);
+            for (int i = 0; i < 4; ++i)
+              *reinterpret_cast<uint4*>(orow + n0 + 8 * i) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
           }
         } else {
 #pragma unroll
@@ -694,33 +749,54 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_tm_kernel(const __grid_co
       }
     }
   }
+  __syncwarp();
   tcgen05_fence_before();
   __syncthreads();
+  if constexpr (CG == 2) {              // neither CTA's shared memory or accumulator goes while the other may still use it
+    cluster_arrive();
+    cluster_wait();
+  }
   if (warp == 1) {
     tcgen05_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if constexpr (CG == 2) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
-template <int BNF, bool DUAL>
-static int launch_prefill_tm(const CUtensorMap& tmX, const CUtensorMap& tmW, PrefillParams& p, int num_ctas,
+template <int NCOL, bool DUAL, int CG>
+static int launch_prefill_tm(const void* X, int ldx, const void* W, int w_rows, int ldw, PrefillParams& p, int num_ctas,
                              cudaStream_t st) {
-  constexpr int STAGE_BYTES = 128 * 64 * 2 + BNF * 64 * 2 * (DUAL ? 2 : 1);
-  int stages = (196 * 1024) / STAGE_BYTES;
-  if (stages > kPrefillMaxStages) stages = kPrefillMaxStages;
-  p.stages = stages;
-  const size_t smem = (size_t)stages * STAGE_BYTES + 1024;
+  constexpr int STAGE_BYTES = 128 * 64 * 2 + NCOL / CG * 64 * 2;
+  constexpr int FEAT = DUAL ? NCOL / 2 : NCOL;
+  p.n_tiles = (p.N + FEAT - 1) / FEAT;
+  if (!p.group_tiles) p.t_tiles = (p.T + 128 * CG - 1) / (128 * CG);
+  CUtensorMap tmW, tmX;
+  int r = make_tensor_map(&tmW, W, (uint64_t)w_rows, (uint64_t)p.K, (uint64_t)ldw, (uint32_t)(DUAL ? FEAT : NCOL / CG), 2);
+  if (r) return 1000 - r;
+  r = make_tensor_map(&tmX, X, (uint64_t)p.T, (uint64_t)p.K, (uint64_t)ldx, 128, 2);
+  if (r) return 2000 - r;
+  const size_t smem = (size_t)prefill_tm_stages(STAGE_BYTES) * STAGE_BYTES + 1024;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_prefill_tm_kernel<BNF, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    if (cudaFuncSetAttribute(gemm_prefill_tm_kernel<NCOL, DUAL, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
       return 3000 + (int)cudaGetLastError();
     attr_set = true;
   }
-  const int total = p.n_tiles * p.t_tiles;
-  const int grid = total < num_ctas ? total : num_ctas;
-  gemm_prefill_tm_kernel<BNF, DUAL><<<grid, 192, smem, st>>>(tmX, tmW, p);
-  return (int)cudaGetLastError();
+  const int total = p.n_tiles * p.t_tiles, slots = num_ctas / CG > 0 ? num_ctas / CG : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((total < slots ? total : slots) * CG);
+  cfg.blockDim = dim3(kPrefillTmThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CG;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CG > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_prefill_tm_kernel<NCOL, DUAL, CG>, tmX, tmW, (const PrefillParams)p);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
 template <int BN, bool DUAL>
@@ -851,8 +927,6 @@ extern "C" int xft_bulk_ar_layout(long long* out, int n) {
 // res_scale * residual, bf16.  gated != 0: gate rows [0, N) and up rows [dual_off, dual_off + N) of W.
 static int prefill_tm(const void* X, int ldx, const void* W, int w_rows, int ldw, PrefillParams& p, int gated, int num_ctas,
                       cudaStream_t st) {
-  const int bnf = gated ? 128 : 256;
-  p.n_tiles = (p.N + bnf - 1) / bnf;
   p.num_kb = (p.K + 63) / 64;
   p.gn = 8;
   if (num_ctas <= 0) {
@@ -861,12 +935,25 @@ static int prefill_tm(const void* X, int ldx, const void* W, int w_rows, int ldw
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     num_ctas = sms > 0 ? sms : 148;
   }
-  CUtensorMap tmW, tmX;
-  int r = make_tensor_map(&tmW, W, (uint64_t)w_rows, (uint64_t)p.K, (uint64_t)ldw, (uint32_t)bnf, 2);
-  if (r) return 1000 - r;
-  r = make_tensor_map(&tmX, X, (uint64_t)p.T, (uint64_t)p.K, (uint64_t)ldx, 128, 2);
-  if (r) return 2000 - r;
-  return gated ? launch_prefill_tm<128, true>(tmX, tmW, p, num_ctas, st) : launch_prefill_tm<256, false>(tmX, tmW, p, num_ctas, st);
+#define XFT_TM(NCOL, CG)                                                                    \
+  (gated ? launch_prefill_tm<NCOL, true, CG>(X, ldx, W, w_rows, ldw, p, num_ctas, st)       \
+         : launch_prefill_tm<NCOL, false, CG>(X, ldx, W, w_rows, ldw, p, num_ctas, st))
+  if (p.group_tiles) return p.group_rows == 256 ? XFT_TM(256, 2) : XFT_TM(256, 1);
+  // Which tile: the number of rounds that the SMs need, times what a 64-deep step of one tile takes, plus what a launch costs
+  // beside its steps (accumulator on its way out, start of a cluster), all in steps of the largest tile (about 0.33 us).
+  // Fitted to a sweep of 25 shapes on B200.  T x N x K, us with 256 x 256 (pair) / 256 x 128 (pair) / 128 x 128 tiles:
+  // 8192 x 8192 x 8192: 757 / 953 / 1016; 2048 x 4096 x 4096: 59 / 66 / 70; 512 x 12288 x 4096: 49 / 48 / 52;
+  // 512 x 4096 x 11008: 66 / 43 / 47; 778 x 2560 x 2048: 31 / 23 / 21; 200 x 3072 x 1024: 19 / 14 / 12.
+  const int feats = gated ? 2 * p.N : p.N, pairs = num_ctas / 2 > 0 ? num_ctas / 2 : 1;
+  auto rounds = [&](int tok, int ncol, int slots) {
+    const long long tiles = (long long)((p.T + tok - 1) / tok) * ((feats + ncol - 1) / ncol);
+    return (float)((tiles + slots - 1) / slots) * (float)p.num_kb;
+  };
+  const float wide = rounds(256, 256, pairs) + 8.f, pair = 0.6f * rounds(256, 128, pairs) + 9.f,
+              single = 0.65f * rounds(128, 128, num_ctas) + 3.f;
+  if (wide <= pair && wide <= single) return XFT_TM(256, 2);
+  return pair < single ? XFT_TM(128, 2) : XFT_TM(128, 1);
+#undef XFT_TM
 }
 
 extern "C" int xft_gemm_bf16_prefill_tm(const void* X, int ldx, const void* W, int w_rows, int ldw, void* Y, int ldo, int T,
@@ -878,7 +965,6 @@ extern "C" int xft_gemm_bf16_prefill_tm(const void* X, int ldx, const void* W, i
   p.N = N; p.T = T; p.K = K; p.out = reinterpret_cast<__nv_bfloat16*>(Y); p.ldo = ldo; p.bias = bias;
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual); p.ldr = ldr; p.res_scale = res_scale; p.act = act;
   p.status = status; p.dual_off = dual_off;
-  p.t_tiles = (T + 127) / 128;
   return prefill_tm(X, ldx, W, w_rows, ldw, p, gated, num_ctas, st);
 }
 
@@ -890,21 +976,20 @@ extern "C" int xft_gemm_bf16_prefill_tm_f32(const void* X, int ldx, const void* 
   PrefillParams p{};
   p.N = N; p.T = T; p.K = K; p.out = reinterpret_cast<__nv_bfloat16*>(Y); p.ldo = ldo; p.bias = bias; p.res_scale = param; p.act = act;
   p.status = status; p.out_fp32 = 1;
-  p.t_tiles = (T + 127) / 128;
   return prefill_tm(X, ldx, W, w_rows, ldw, p, 0, 0, st);
 }
 
-// Rows sorted by group (experts at prompt sizes): token tiles of 128 rows from xft_moe_plan, W [groups * group_w_rows, K];
+// Rows sorted by group (experts at prompt sizes): token tiles of `tile_rows` (128 or 256) rows from xft_moe_plan, W [groups * group_w_rows, K];
 // gated: a group's rows are gate [0, N), up [dual_off, dual_off + N).  bf16 rows out.
 extern "C" int xft_gemm_bf16_grouped_tm(const void* X, int ldx, int x_rows, const void* W, int w_rows, int ldw, void* Y, int ldo,
                                         int N, int K, int gated, int dual_off, int group_w_rows, const void* group_tiles,
-                                        const int* num_group_tiles, int max_tiles, int act, int* status, cudaStream_t st) {
+                                        const int* num_group_tiles, int max_tiles, int tile_rows, int act, int* status, cudaStream_t st) {
   if (x_rows <= 0 || N <= 0 || K <= 0 || max_tiles <= 0) return 0;
-  if ((K & 7) || (ldx & 7) || (ldw & 7) || !group_tiles || !num_group_tiles) return -2;
+  if ((K & 7) || (ldx & 7) || (ldw & 7) || !group_tiles || !num_group_tiles || (tile_rows != 128 && tile_rows != 256)) return -2;
   PrefillParams p{};
   p.N = N; p.T = x_rows; p.K = K; p.out = reinterpret_cast<__nv_bfloat16*>(Y); p.ldo = ldo; p.res_scale = 1.f; p.act = act;
   p.status = status; p.dual_off = dual_off;
   p.group_tiles = reinterpret_cast<const int4*>(group_tiles); p.num_group_tiles = num_group_tiles; p.group_w_rows = group_w_rows;
-  p.t_tiles = max_tiles;
+  p.t_tiles = max_tiles; p.group_rows = tile_rows;
   return prefill_tm(X, ldx, W, w_rows, ldw, p, gated, 0, st);
 }

@@ -150,7 +150,9 @@ def moe_experts(x, idx, w, experts, act="silu", expert_offset=0, packed=None, ex
     ws = N.Workspace.get(dev)
     lib = _lib()
     avg = max(1, ((T * k if expected_pairs is None else min(int(expected_pairs), T * k)) + E - 1) // E)
-    bn = 16 if avg <= 16 else 32 if avg <= 32 else 64 if avg <= 64 else 128
+    # 256 rows: two CTAs share a tile (bf16 only).  A group's last tile is half empty on average, which eats the fifth that
+    # pairs gain below about 430 rows per expert
+    bn = 16 if avg <= 16 else 32 if avg <= 32 else 64 if avg <= 64 else 128 if avg < 512 or pk.get("fp8") else 256
     max_rows = T * k
     max_tiles = (max_rows + bn - 1) // bn + E
     idx32 = idx if idx.dtype == torch.int32 else idx.int()
@@ -179,14 +181,14 @@ def moe_experts(x, idx, w, experts, act="silu", expert_offset=0, packed=None, ex
                                  N._stream()), "moe_combine")
         ws.launches += 5
         return out
-    if bn == 128:
+    if bn >= 128:
         # prompt sizes: the token-major persistent kernel; rows stay bf16 until the weighted sum
         y16 = torch.empty(max_rows, H, dtype=torch.bfloat16, device=dev)
         fn = lib.xft_gemm_bf16_grouped_tm
         N._check(fn(N._p(xs), H, max_rows, N._p(pk["gu"]), E * up, H, N._p(h1), I, I, H, int(gated), I, up, N._p(tiles), N._p(meta),
-                    max_tiles, N._ACT[act], N._p(ws.status), N._stream()), "grouped gate_up")
+                    max_tiles, bn, N._ACT[act], N._p(ws.status), N._stream()), "grouped gate_up")
         N._check(fn(N._p(h1), I, max_rows, N._p(pk["dn"]), E * H, I, N._p(y16), H, H, I, 0, 0, H, N._p(tiles), N._p(meta), max_tiles,
-                    0, N._p(ws.status), N._stream()), "grouped down")
+                    bn, 0, N._p(ws.status), N._stream()), "grouped down")
         out = torch.empty(T, H, dtype=torch.float32, device=dev)
         fn = lib.xft_moe_combine_bf16
         N._check(fn(N._p(y16), N._p(pos), N._p(w.contiguous()), k, N._p(add32), N._p(add16), H, N._p(None), N._p(out), T, H,
