@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(160, (HD <= 128 ? 2 : 1)) attn_decode_tma_kern
       tma_load_2d(kt + TILE + h * KT * 64, &tmV, &full_bar[st], h * 64, row, kEvictFirst);
     }
   };
-  if (warp == 4 && lane == 0)
+  if (warp == 4 && elect_one())
     for (int n = 0; n < npre; ++n) issue_tile(n);
   grid_dep_wait();
   if (tid < 128) load_tile_bf16<HD, 128>(qs, p.q + ((size_t)tok * p.hq + h_lo) * HD, HD, 16, nq, tid);
@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(160, (HD <= 128 ? 2 : 1)) attn_decode_tma_kern
   WarpAttn<HD, KW, true, KT, EXT> wa;
   wa.init();
   if (warp == 4) {
-    if (lane == 0) {
+    if (elect_one()) {
       for (int n = npre; n < nloc; ++n) {
         const int st = n % STAGES;
         if (!mbar_wait(&empty_bar[st], ((n / STAGES) & 1) ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) { s_abort = 1; break; }

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_co
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&q_full, kPfTileBytes);
       // q is [T, hq * 128]: rows past the end of the tensor read as zero, rows of the next sequence are never stored
       tma_load_2d(sQ, &tmQ, &q_full, h * 128, q0 + row0, kEvictFirst);
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_co
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // S = Q K^T: both operands K-major, M = 128 query rows, N = 128 keys, K = 128 features in 8 steps of 16
       constexpr uint32_t IDESC_S = umma_idesc(128, 128, 1, 1, 1);
       // O = P V: A = P K-major (keys contiguous), B = V MN-major (bit 16), N = 128 features, K = 128 keys

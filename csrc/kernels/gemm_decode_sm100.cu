@@ -346,7 +346,7 @@ auto ar_reduce = [&]() {
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       // a weight byte is read once: stream it past L2; the token tile is re-read by every CTA: keep it
       const uint64_t hint_w = kEvictFirst, hint_x = kEvictLast;
       const int n_units = u1 - u0;
@@ -371,10 +371,10 @@ auto ar_reduce = [&]() {
           if (++kb2 == p.num_kb) { kb2 = 0; ++tile2; }
         }
       }
-      for (int it = pre; it < n_units; ++it) {
-        const int s = it % stages;
-        const uint32_t ph = (it / stages) & 1;
-        if (!mbar_wait(&empty_bar[s], ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
+      Ring r = {0, 1};                        // there is more to load only when the first round took every stage
+      for (int it = pre; it < n_units; ++it, r.next(stages)) {
+        const int s = r.s;
+        if (!mbar_wait(&empty_bar[s], r.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
         mbar_expect_tx(&full_bar[s], STAGE_BYTES);
         uint8_t* a = smem + s * STAGE_BYTES;
         tma_load_2d(a, &tmW, &full_bar[s], kb * 64, tile * 128, hint_w);
@@ -385,8 +385,10 @@ auto ar_reduce = [&]() {
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      int it = 0, seg = 0;
+    if (elect_one()) {
+      const uint64_t adesc0 = umma_desc_k128(smem_u32(smem)), bdesc0 = umma_desc_k128(smem_u32(smem) + A_BYTES * NACC);
+      int seg = 0;
+      Ring r = {0, 0};
       bool ok = true;
       for (int u = u0; u < u1 && ok; ++seg) {
         const int kb_begin = u % p.num_kb;
@@ -396,20 +398,17 @@ auto ar_reduce = [&]() {
         if (!mbar_wait(&tmem_empty[a], aph ^ 1, p.status, XFT_ERR_WAIT_TMEM)) break;
         tcgen05_fence_after();
         const uint32_t acc = tmem_base + (uint32_t)(a * ACC_COLS);
-        for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
-          const int s = it % stages;
-          const uint32_t ph = (it / stages) & 1;
-          if (!mbar_wait(&full_bar[s], ph, p.status, XFT_ERR_WAIT_FULL)) { ok = false; break; }
-          if (it == 0) SK_STAMP(3);
+        for (int kb = kb_begin; kb < kb_end; ++kb, r.next(stages)) {
+          const int s = r.s;
+          if (!mbar_wait(&full_bar[s], r.ph, p.status, XFT_ERR_WAIT_FULL)) { ok = false; break; }
+          if (kb == kb_begin && seg == 0) SK_STAMP(3);
           tcgen05_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-          const uint64_t adesc = umma_desc_k128(a_addr);
-          const uint64_t bdesc = umma_desc_k128(a_addr + A_BYTES * NACC);
+          const uint64_t adesc = adesc0 + (uint64_t)(s * (STAGE_BYTES / 16)), bdesc = bdesc0 + (uint64_t)(s * (STAGE_BYTES / 16));
 #pragma unroll
           for (int k = 0; k < 4; ++k) {          // 4 x (K = 16) per 64-wide k-block; +32 B = +2 in the address field
             umma_bf16(acc, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > kb_begin || k > 0) ? 1u : 0u);
             if (DUAL) {
-              const uint64_t a1desc = umma_desc_k128(a_addr + A_BYTES);
+              const uint64_t a1desc = adesc + A_BYTES / 16;
               umma_bf16(acc + BN, a1desc + 2 * k, bdesc + 2 * k, IDESC, (kb > kb_begin || k > 0) ? 1u : 0u);
             }
           }

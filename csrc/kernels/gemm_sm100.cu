@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(192) gemm_bf16_kernel(const __grid_constant__ 
   const int tn_stride = (DUAL && p.pair) ? 256 : 128;      // output features covered per CTA
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // a weight byte is read once when one token tile covers the batch (decode): stream it past
       // L2; the small activation tile is re-read by every feature tile: keep it
       const uint64_t hint_w = p.t_tiles == 1 ? kEvictFirst : kEvictNormal;
@@ -178,11 +178,10 @@ __global__ void __launch_bounds__(192) gemm_bf16_kernel(const __grid_constant__ 
       grid_dep_wait();
       for (int i = 0; i < pre; ++i)
         tma_load_2d(smem + i * STAGE_BYTES + A_BYTES * NACC, &tmX, &full_bar[i], x_col0 + (kb0 + i) * 64, x_row0, hint_x);
-      int it = pre;
-      for (int kb = kb0 + pre; kb < kend; ++kb, ++it) {
-        const int s = it % stages;
-        const uint32_t ph = (it / stages) & 1;
-        if (!mbar_wait(&empty_bar[s], ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
+      Ring r = {0, 1};                        // there is more to load only when the first round took every stage
+      for (int kb = kb0 + pre; kb < kend; ++kb, r.next(stages)) {
+        const int s = r.s;
+        if (!mbar_wait(&empty_bar[s], r.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
         mbar_expect_tx(&full_bar[s], STAGE_BYTES);
         uint8_t* a = smem + s * STAGE_BYTES;
         tma_load_2d(a, &tmW, &full_bar[s], kb * 64, w_row0 + tile_n * tn_stride, hint_w);
@@ -191,22 +190,20 @@ __global__ void __launch_bounds__(192) gemm_bf16_kernel(const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && active) {
-      int it = 0;
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        const int s = it % stages;
-        const uint32_t ph = (it / stages) & 1;
-        if (!mbar_wait(&full_bar[s], ph, p.status, XFT_ERR_WAIT_FULL)) break;
+    if (active && elect_one()) {
+      const uint64_t adesc0 = umma_desc_k128(smem_u32(smem)), bdesc0 = umma_desc_k128(smem_u32(smem) + A_BYTES * NACC);
+      Ring r = {0, 0};
+      for (int kb = kb0; kb < kb1; ++kb, r.next(stages)) {
+        const int s = r.s;
+        if (!mbar_wait(&full_bar[s], r.ph, p.status, XFT_ERR_WAIT_FULL)) break;
         tcgen05_fence_after();
-        const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-        const uint64_t adesc = umma_desc_k128(a_addr);
-        const uint64_t bdesc = umma_desc_k128(a_addr + A_BYTES * NACC);
+        const uint64_t adesc = adesc0 + (uint64_t)(s * (STAGE_BYTES / 16)), bdesc = bdesc0 + (uint64_t)(s * (STAGE_BYTES / 16));
 #pragma unroll
         for (int k = 0; k < 4; ++k) {       // 4 x (K = 16) per 64-wide k-block; +32 B = +2 in the address field
-          umma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, IDESC, (it > 0 || k > 0) ? 1u : 0u);
+          umma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
           if (DUAL) {
-            const uint64_t a1desc = umma_desc_k128(a_addr + A_BYTES);
-            umma_bf16(tmem_base + BN, a1desc + 2 * k, bdesc + 2 * k, IDESC, (it > 0 || k > 0) ? 1u : 0u);
+            const uint64_t a1desc = adesc + A_BYTES / 16;
+            umma_bf16(tmem_base + BN, a1desc + 2 * k, bdesc + 2 * k, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
           }
         }
         tcgen05_commit(&empty_bar[s]);       // frees the stage when these MMAs have read it

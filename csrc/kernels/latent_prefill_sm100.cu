@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(384, 1) attn_flat_tc_kernel(const __grid_const
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_expect_tx(&q_full, tiles_q * nq * kFlChunk);
         for (int i = 0; i < tiles_q; ++i)
           for (int c = 0; c < nq; ++c)
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(384, 1) attn_flat_tc_kernel(const __grid_const
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------------ MMA issuer
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t IDESC_S = umma_idesc(128, 128, 1, 1, 1);
         const uint32_t idesc_o = umma_idesc(128, 64, 1, 1, 1) + (p.nv > 1 ? (8u << 17) : 0u) | (1u << 16);   // N = 64 nv, B MN-major
         auto issue_s = [&](int i, int j) {

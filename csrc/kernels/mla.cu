@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(384, 1) mla_attn_kernel(const __grid_constant_
   if (warp >= 8) {
     // ------------------------------------------------------------------ TMA producer
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == 8 && lane == 0) {
+    if (warp == 8 && elect_one()) {
       const int* bt = p.block_table + (size_t)b * p.bt_stride;
       auto issue = [&](int n) {
         const int s = n % STAGES, key = t_begin * MKT + n * (MKT / 2);

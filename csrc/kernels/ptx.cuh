@@ -87,6 +87,14 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
+// Stage of a ring of buffers and the parity of its round, carried along: `it % stages` and `it / stages` of a run-time count
+// are two divisions on the issuing thread's critical path.
+struct Ring {
+  int s;
+  uint32_t ph;
+  __device__ __forceinline__ void next(int stages) { if (++s == stages) { s = 0; ph ^= 1; } }
+};
+
 // ---------------------------------------------------------------- TMA
 constexpr uint64_t kEvictNormal = 0x1000000000000000ull;
 constexpr uint64_t kEvictFirst = 0x12F0000000000000ull;

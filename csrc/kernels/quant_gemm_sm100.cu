@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(192) qgemm_kernel(const __grid_constant__ CUte
 
   // stage layout: [raw A (xNACC)] [bf16 A (xNACC)] [B]
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t hint_w = p.t_tiles == 1 ? kEvictFirst : kEvictNormal;
       const uint64_t hint_x = p.n_tiles > 1 ? kEvictLast : kEvictNormal;
       constexpr int KEL = (QT == Q_INT8 || QT == Q_FP8) ? 64 : 32;      // raw bytes per k-block row
@@ -243,11 +243,10 @@ __global__ void __launch_bounds__(192) qgemm_kernel(const __grid_constant__ CUte
       grid_dep_wait();
       for (int i = 0; i < pre; ++i)
         tma_load_2d(smem + i * STAGE_BYTES + (RAW_BYTES + A_BYTES) * NACC, &tmX, &raw_full[i], (kb0 + i) * 64, x_row0, hint_x);
-      int it = pre;
-      for (int kb = kb0 + pre; kb < kend; ++kb, ++it) {
-        const int s = it % stages;
-        const uint32_t ph = (it / stages) & 1;
-        if (!mbar_wait(&empty_bar[s], ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
+      Ring r = {0, 1};                        // there is more to load only when the first round took every stage
+      for (int kb = kb0 + pre; kb < kend; ++kb, r.next(stages)) {
+        const int s = r.s;
+        if (!mbar_wait(&empty_bar[s], r.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
         mbar_expect_tx(&raw_full[s], TX_BYTES);
         uint8_t* st = smem + s * STAGE_BYTES;
         tma_load_2d(st, &tmW, &raw_full[s], kb * KEL, w_row0 + tile_n * 128, hint_w);
@@ -256,22 +255,21 @@ __global__ void __launch_bounds__(192) qgemm_kernel(const __grid_constant__ CUte
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && active) {
-      int it = 0;
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        const int s = it % stages;
-        const uint32_t ph = (it / stages) & 1;
-        if (!mbar_wait(&a_ready[s], ph, p.status, XFT_ERR_WAIT_FULL)) break;
+    if (active && elect_one()) {
+      const uint64_t adesc0 = umma_desc_k128(smem_u32(smem) + RAW_BYTES * NACC);
+      const uint64_t bdesc0 = umma_desc_k128(smem_u32(smem) + (RAW_BYTES + A_BYTES) * NACC);
+      Ring r = {0, 0};
+      for (int kb = kb0; kb < kb1; ++kb, r.next(stages)) {
+        const int s = r.s;
+        if (!mbar_wait(&a_ready[s], r.ph, p.status, XFT_ERR_WAIT_FULL)) break;
         tcgen05_fence_after();
-        const uint32_t base = smem_u32(smem + s * STAGE_BYTES);
-        const uint64_t adesc = umma_desc_k128(base + RAW_BYTES * NACC);
-        const uint64_t bdesc = umma_desc_k128(base + (RAW_BYTES + A_BYTES) * NACC);
+        const uint64_t adesc = adesc0 + (uint64_t)(s * (STAGE_BYTES / 16)), bdesc = bdesc0 + (uint64_t)(s * (STAGE_BYTES / 16));
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          umma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, IDESC, (it > 0 || k > 0) ? 1u : 0u);
+          umma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
           if (DUAL) {
-            const uint64_t a1 = umma_desc_k128(base + RAW_BYTES * NACC + A_BYTES);
-            umma_bf16(tmem_base + BN, a1 + 2 * k, bdesc + 2 * k, IDESC, (it > 0 || k > 0) ? 1u : 0u);
+            const uint64_t a1 = adesc + A_BYTES / 16;
+            umma_bf16(tmem_base + BN, a1 + 2 * k, bdesc + 2 * k, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
           }
         }
         tcgen05_commit(&empty_bar[s]);
@@ -286,12 +284,11 @@ __global__ void __launch_bounds__(192) qgemm_kernel(const __grid_constant__ CUte
     const bool n_ok = n < p.N;
     const int et = threadIdx.x - 64;
     {
-      int it = 0;
+      Ring r = {0, 0};
       bool alive = true;
-      for (int kb = kb0; kb < kend; ++kb, ++it) {
-        const int s = it % stages;
-        const uint32_t ph = (it / stages) & 1;
-        if (alive && !mbar_wait(&raw_full[s], ph, p.status, XFT_ERR_WAIT_FULL)) alive = false;
+      for (int kb = kb0; kb < kend; ++kb, r.next(stages)) {
+        const int s = r.s;
+        if (alive && !mbar_wait(&raw_full[s], r.ph, p.status, XFT_ERR_WAIT_FULL)) alive = false;
         if (alive) {
           uint8_t* st = smem + s * STAGE_BYTES;
           float sc0 = 1.f, sc1 = 1.f;
@@ -440,32 +437,39 @@ __global__ void __launch_bounds__(192) w8a8_gemm_kernel(const __grid_constant__ 
   const uint32_t tmem_base = tmem_base_s;
   grid_dep_launch();
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
+      const uint64_t hint_w = p.t_tiles == 1 ? kEvictFirst : kEvictNormal;
+      // weights never depend on the previous kernel: the first `stages` tiles are requested before the grid dependency resolves
+      const int pre = min(stages, kb1 - kb0);
+      for (int i = 0; i < pre; ++i) {
+        mbar_expect_tx(&full_bar[i], STAGE_BYTES);
+        tma_load_2d(smem + i * STAGE_BYTES, &tmW, &full_bar[i], (kb0 + i) * 128, tile_n * 128, hint_w);
+      }
       grid_dep_wait();
-      int it = 0;
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        const int s = it % stages;
-        const uint32_t ph = (it / stages) & 1;
-        if (!mbar_wait(&empty_bar[s], ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
+      for (int i = 0; i < pre; ++i)
+        tma_load_2d(smem + i * STAGE_BYTES + A_BYTES, &tmX, &full_bar[i], (kb0 + i) * 128, tile_t * BN, kEvictLast);
+      Ring r = {0, 1};
+      for (int kb = kb0 + pre; kb < kb1; ++kb, r.next(stages)) {
+        const int s = r.s;
+        if (!mbar_wait(&empty_bar[s], r.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
         mbar_expect_tx(&full_bar[s], STAGE_BYTES);
         uint8_t* st = smem + s * STAGE_BYTES;
-        tma_load_2d(st, &tmW, &full_bar[s], kb * 128, tile_n * 128, p.t_tiles == 1 ? kEvictFirst : kEvictNormal);
+        tma_load_2d(st, &tmW, &full_bar[s], kb * 128, tile_n * 128, hint_w);
         tma_load_2d(st + A_BYTES, &tmX, &full_bar[s], kb * 128, tile_t * BN, kEvictLast);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int it = 0;
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        const int s = it % stages;
-        const uint32_t ph = (it / stages) & 1;
-        if (!mbar_wait(&full_bar[s], ph, p.status, XFT_ERR_WAIT_FULL)) break;
+    if (elect_one()) {
+      const uint64_t adesc0 = umma_desc_k128(smem_u32(smem)), bdesc0 = umma_desc_k128(smem_u32(smem) + A_BYTES);
+      Ring r = {0, 0};
+      for (int kb = kb0; kb < kb1; ++kb, r.next(stages)) {
+        const int s = r.s;
+        if (!mbar_wait(&full_bar[s], r.ph, p.status, XFT_ERR_WAIT_FULL)) break;
         tcgen05_fence_after();
-        const uint32_t base = smem_u32(smem + s * STAGE_BYTES);
-        const uint64_t adesc = umma_desc_k128(base), bdesc = umma_desc_k128(base + A_BYTES);
+        const uint64_t adesc = adesc0 + (uint64_t)(s * (STAGE_BYTES / 16)), bdesc = bdesc0 + (uint64_t)(s * (STAGE_BYTES / 16));
 #pragma unroll
         for (int k = 0; k < 4; ++k)       // 4 x (K = 32 int8 = 32 bytes)
-          umma_i8(tmem_base, adesc + 2 * k, bdesc + 2 * k, IDESC, (it > 0 || k > 0) ? 1u : 0u);
+          umma_i8(tmem_base, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
         tcgen05_commit(&empty_bar[s]);
       }
       tcgen05_commit(&tmem_full_bar);
