@@ -10,8 +10,9 @@ merge — is captured once and replayed.  Per step the host only
   2. fills ONE pinned int32 staging buffer [ids | positions | slots | kv_lens | state slots | block_table],
   3. issues one H2D copy, one graph launch, one D2H copy of the chosen tokens, and waits.
 
-Greedy decoding with no repetition penalty takes this path; anything else (sampling, beams,
-penalties, prefill, pipeline stages) runs the eager path in `engine.Model`.
+Greedy decoding with no repetition penalty takes this path, and so do the decode steps of `forward_cb`, which return logits
+(`step_logits`: nothing is read back, the caller's stream carries the step).  Anything else (sampling, beams, penalties,
+prefill, pipeline stages) runs the eager path in `engine.Model`.
 """
 from __future__ import annotations
 
@@ -33,7 +34,8 @@ def _capture(graph, stream):
     was = gc.isenabled()
     gc.disable()
     try:
-        with torch.cuda.graph(graph, stream=stream):
+        # thread_local: what other threads of the program do on the GPU meanwhile is no concern of this capture
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
             yield
     finally:
         if was:
@@ -41,7 +43,7 @@ def _capture(graph, stream):
 
 
 class _Graph:
-    __slots__ = ("graph", "B", "W", "host", "dev", "tok_dev", "tok_host", "batch", "version", "nsplit", "kernels")
+    __slots__ = ("graph", "B", "W", "host", "dev", "tok_dev", "tok_host", "batch", "version", "nsplit", "kernels", "logits", "ring", "turn")
 
 
 class CudaRunner:
@@ -58,6 +60,7 @@ class CudaRunner:
         self.timing = False               # record a CUDA-event pair around each step's launch
         self.step_events = []
         self._scratch_block = self._scratch_state = None
+        self._tail = None                 # end of the last logits step
         if self.enabled:
             # taken now, while the pools are empty: a block taken after a request reserved its blocks would leave that
             # request one block short and make the pools grow (and move) in the middle of its decode
@@ -126,10 +129,20 @@ class CudaRunner:
                 self._scratch_state = self.m.cache.take_state()
         return self._scratch_block
 
-    def worth_capturing(self, seqs: Sequence) -> bool:
+    def _logits_key(self, seqs: Sequence):
+        """Like `_key`, but the table is as wide as the contexts of this step, rounded up to a power of two (from 8 blocks on):
+        callers of `forward_cb` need not say how long their sequences get, and a step planned for the longest possible
+        context would cut short ones into too many parts."""
+        B, limit = self._key(seqs)
+        need, W = max(self.m.cache.blocks_for(s.past_len + 1) for s in seqs), 8
+        while W < need:
+            W *= 2
+        return B, max(min(W, limit), need), "logits"
+
+    def worth_capturing(self, seqs: Sequence, key=None) -> bool:
         """For callers whose batch composition changes from step to step (serving): a shape is captured only when
         it is requested twice in a row or already has a graph; a shape seen once runs eagerly."""
-        key = self._key(seqs)
+        key = key or self._key(seqs)
         hit = key in self.graphs or key == getattr(self, "_last_key", None)
         self._last_key = key
         if len(self.graphs) > 64 and key not in self.graphs:      # bound the memory held by captured shapes
@@ -191,11 +204,11 @@ class CudaRunner:
             slots.append(cache.append_slots(s.seq_id, 1)[0])
         return slots
 
-    def _fill(self, g: _Graph, seqs, slots: List[int]) -> None:
+    def _fill(self, g: _Graph, seqs, slots: List[int], h=None) -> None:
         m = self.m
         B, W = g.B, g.W
         o_ids, o_pos, o_slot, o_kv, o_st, o_cu, o_bt, total = self._layout(B, W)
-        h = g.host
+        h = g.host if h is None else h
         cache = m.cache
         slots = list(slots)
         ids = [s.pending[0] for s in seqs]
@@ -317,3 +330,50 @@ class CudaRunner:
         self.h2d_bytes += g.host.numel() * 4
         self.d2h_bytes += g.tok_host.numel() * 8
         return g.tok_host.tolist()[:n_real]
+
+    RING = 4          # staging buffers of a logits graph: the host may be that many steps ahead of the GPU
+
+    def step_logits(self, seqs: Sequence) -> torch.Tensor:
+        """One decode step of `seqs` -> this rank's fp32 logits [len(seqs), vocab slice], in a tensor of the caller's.  Runs on
+        the caller's stream and waits for nothing."""
+        m = self.m
+        n = len(seqs)
+        self._scratch()                                # both may grow the pools: before the version check below
+        slots = self._reserve_slots(seqs)
+        key = self._logits_key(seqs)
+        B, W = key[:2]
+        g = self.graphs.get(key)
+        if g is None or g.version != m.cache.version:
+            g = self._build(B, W, W * m.cache.block)
+            g.ring = [(g.host if i == 0 else g.host.clone().pin_memory(), torch.cuda.Event()) for i in range(self.RING)]
+            g.turn = 0
+            self.graphs[key] = g
+        host, copied = g.ring[g.turn]
+        g.turn = (g.turn + 1) % self.RING
+        copied.synchronize()                           # its last copy to the device is done
+        self._fill(g, seqs, slots, host)
+        cur = torch.cuda.current_stream()
+        if self._tail is not None:
+            cur.wait_event(self._tail)                 # buffers of the graphs are shared by the streams of all callers
+        with torch.no_grad():
+            g.dev.copy_(host, non_blocking=True)
+            copied.record()
+            if g.graph is None:
+                out = m.decoder.forward(g.batch, m.cache)[:n].clone()      # eagerly: allocates workspaces; then captured
+                from ..ops import native as N
+                ws = N.Workspace.get(self.dev)
+                torch.cuda.synchronize(self.dev)
+                n0 = ws.launches
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.stream(self.stream), _capture(graph, self.stream):
+                    g.logits = m.decoder.forward(g.batch, m.cache)
+                g.graph, g.kernels = graph, ws.launches - n0
+            else:
+                g.graph.replay()
+                out = g.logits[:n].clone()
+                self.graph_launches += 1
+        self._tail = self._tail or torch.cuda.Event()
+        self._tail.record()
+        self.kernel_launches += g.kernels
+        self.h2d_bytes += host.numel() * 4
+        return out
