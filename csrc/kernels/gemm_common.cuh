@@ -82,6 +82,16 @@ __device__ __forceinline__ float apply_gated(float g, float u, int act, float pa
   return act == kActClamped ? clamped_glu(g, u, param) : apply_act(g, act) * u;
 }
 
+// One W8A8 value from the integer sum `g`: per-token scale, zero point and sum of codes, per-feature scale, zero point and sum.  The
+// roundings are spelled out, the same in every kernel: the next product rounds these values to int8 codes, where a last bit
+// moves whole steps of later layers.
+__device__ __forceinline__ float w8a8_value(float g, float sa, float za, float qs, float sw, float zw, float wsum, int K, float bias) {
+  const float sums = __fmaf_rn(__fmul_rn(sa, zw), qs, __fmul_rn(__fmul_rn(sa, sw), g));
+  return __fadd_rn(__fmaf_rn(__fmul_rn((float)K, za), zw, __fmaf_rn(__fmul_rn(za, sw), wsum, sums)), bias);
+}
+// A gate or up value of a W8A8 pair, rounded as a product that stores it would
+__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
+
 // K-major matrix [rows, cols] with row stride `ld` elements; box = 128 bytes x box_rows, 128B swizzle (gemm_sm100.cu).
 int make_tensor_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
                     uint32_t esize);

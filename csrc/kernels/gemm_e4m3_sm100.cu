@@ -1,0 +1,612 @@
+// Products of weights that e4m3 holds exactly, on the fp8 tensor path without expanding them to bf16:
+//     Y[T, N] = epilogue( X[T, K] · dequant(W[N, K])^T ),  bf16 activations, W in
+//   * fp8 e4m3 with one fp32 scale per 128 x 128 block (plain and grouped by expert), or
+//   * uint4 codes with a scale and a zero point per output channel (a byte 0..15 read as e4m3 is the code times 2^-9:
+//     subnormals and the first binade are equally spaced).
+//
+// An activation becomes the sum of two e4m3 numbers: x / s_t = hi + lo / 16 with s_t a power of two per row.  A bf16 value has
+// eight significant bits, hi takes four and lo the other four, so the sum is x itself down to 2^-15 of the row's maximum and off
+// by at most 2^-23 of that maximum below.  Both halves are columns of one `kind::f8f6f4` MMA (N = 2 BN), sums are fp32.  The
+// expanding kernel (quant_gemm_sm100.cu, still used for int8 and nf4) rounds fp8 x scale to bf16 and spends about 100
+// instructions per weight byte row; here fp8 tiles go from TMA to the tensor core untouched, and uint4 costs one AND and half a
+// shift per four codes.  Block scales multiply the fp32 sums of 128 k: two TMEM accumulators in turn, the epilogue warps fetch
+// one and add it to registers while the next fills.
+//
+// The same pipeline carries W8A8 at decode sizes (int8 weights and activations, `kind::i8`, s32 sums; the parts of a cluster
+// are added as integers).
+//
+// B200, us before (expanding kernel; W8A8: its own kernel, parts through global scratch) / here, with the split of X:
+//   fp8 2 x 28672 x 8192, 16 rows 417 / 78 (6.0 TB/s); 4096 x 4096, 16 rows 21 / 8; uint4 2 x 28672 x 8192, 16 rows 165 / 82;
+//   12288 x 4096, 32 rows 29 / 19.  Error against 64 bits (12288 x 4096, relative): fp8 1.6e-3 / 1e-7, uint4 1.4e-5 / 3e-7.
+//
+// A CTA owns 128 features x BN tokens (BN = 16, 32, 64).  Small products are cut along K over a cluster: every CTA leaves its
+// part in its own shared memory and finishes BN / cluster tokens from all parts.
+#include "gemm_common.cuh"
+
+#include <cuda_fp8.h>
+
+namespace xft {
+
+enum { kSrcFp8 = 0, kSrcU4 = 1, kSrcI8 = 2 };
+
+struct E4Params {
+  int N, T, K;
+  int dual_off;
+  void* out; int ldo; int out_fp32;
+  const float* bias;
+  const __nv_bfloat16* residual; int ldr; float res_scale;
+  int act;
+  int num_kb, n_tiles, t_tiles, splits;      // blocks of 128 k; CTAs of a cluster that share them
+  int x_lo;                  // column of the lo halves in a row of split activations
+  const float* x_scale;      // [rows] s_t
+  const float* x_sum;        // [rows] sum over k (uint4)
+  const float* scale;        // fp8: [N / 128, K / 128] blocks, row pitch scale_ld; uint4: [N]
+  const float* zero;         // uint4: [N]
+  int scale_ld;
+  const int4* group_tiles; const int* num_group_tiles; int group_w_rows;      // see quant_gemm_sm100.cu
+  const float* col_scale;
+  const float* a_zero; const float* a_qsum; const float* w_sum;      // W8A8: [T], [T], [N]; x_scale, scale and zero as above
+  int* status;
+};
+
+constexpr int kE4Threads = 320;              // producer, MMA, eight warps that fetch accumulators (and expand codes)
+
+__device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
+      "}\n"
+      :
+      : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr));
+}
+template <int C>
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* v) {
+  if constexpr (C == 8) tmem_ld8(taddr, v);
+  else if constexpr (C == 16) tmem_ld16(taddr, *reinterpret_cast<uint32_t (*)[16]>(v));
+  else tmem_ld32(taddr, *reinterpret_cast<uint32_t (*)[32]>(v));
+}
+
+template <int BN, bool DUAL, int SRC>
+struct E4Layout {
+  static constexpr int NACC = DUAL ? 2 : 1;
+  static constexpr int A_BYTES = 128 * 128 * NACC, RAW_BYTES = SRC == kSrcU4 ? 128 * 64 * NACC : 0, B_BYTES = (SRC == kSrcI8 ? 1 : 2) * BN * 128;
+  static constexpr int STAGE = (SRC == kSrcU4 ? RAW_BYTES : A_BYTES) + B_BYTES;       // what TMA fills
+  static constexpr int A_RING = SRC == kSrcU4 ? 2 * A_BYTES : 0;                      // expanded codes, two buffers
+  // two CTAs per SM where registers allow: one CTA's last accumulators and stores hide behind the other's stream
+  static constexpr int CTAS = BN <= 32 && A_RING + 3 * STAGE <= 110 * 1024 ? 2 : 1;
+  static constexpr int FIT = ((CTAS == 2 ? 110 : 224) * 1024 - A_RING) / STAGE;
+  static constexpr int STAGES = FIT > 8 ? 8 : FIT;
+  static constexpr int SMEM = A_RING + STAGES * STAGE + 1024;
+  static_assert(STAGES >= 3 && BN * NACC * 512 <= A_RING + STAGES * STAGE, "ring, and room for this CTA's part of the sums");
+};
+
+template <int BN, bool DUAL, int SRC>
+__global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
+    gemm_e4m3_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const E4Params p) {
+  using L = E4Layout<BN, DUAL, SRC>;
+  constexpr int NACC = L::NACC, STAGES = L::STAGES;
+  constexpr int NB = SRC == kSrcI8 ? BN : 2 * BN;                      // columns of an accumulator: hi [BN], lo [BN]
+  constexpr int ACC = NB * NACC;
+  constexpr int BUFS = SRC == kSrcFp8 ? 2 : 1;
+  constexpr uint32_t TMEM_COLS = BUFS * ACC < 32 ? 32 : BUFS * ACC;
+  constexpr uint32_t IDESC = SRC == kSrcI8 ? umma_idesc(128, BN, 1, 1, 2) : umma_idesc(128, 2 * BN, 0, 0, 1);
+  constexpr int HB = BN / 2;                                           // tokens per thread: two warps share a row of the tile
+  constexpr int TILE_A = 128 * 128;
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tmem_full[2], tmem_empty[2], a_ready[2], a_empty[2];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int s_group[4];
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int tile_n, tile_t;
+  {
+    constexpr int GN = 16;                                             // feature tiles that walk the token tiles together
+    const int per = GN * p.t_tiles, g = blockIdx.x / per, r = blockIdx.x % per, gn = min(GN, p.n_tiles - g * GN);
+    tile_n = g * GN + r % gn;
+    tile_t = r / gn;
+  }
+  const int rank = blockIdx.y;
+  const int kb0 = rank * p.num_kb / p.splits, kb1 = (rank + 1) * p.num_kb / p.splits;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&tmem_full[a], 1);
+      mbar_init(&tmem_empty[a], 8);
+      mbar_init(&a_ready[a], 256);
+      mbar_init(&a_empty[a], 1);
+    }
+    fence_barrier_init();
+    fence_proxy_async();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) { tmem_alloc(&tmem_base_s, TMEM_COLS); tmem_relinquish(); }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = tmem_base_s;
+  grid_dep_launch();
+  const bool grouped = p.group_tiles != nullptr;
+  if (grouped) {
+    grid_dep_wait();          // the tile table comes from the routing plan kernel
+    if (threadIdx.x == 0) {
+      int4 e = make_int4(0, 0, 0, 0);
+      if (tile_t < *p.num_group_tiles) e = p.group_tiles[tile_t];
+      s_group[0] = e.x; s_group[1] = e.y; s_group[2] = e.z;
+    }
+    __syncthreads();
+  }
+  const int w_row0 = (grouped ? s_group[0] * p.group_w_rows : 0) + tile_n * 128;
+  const int x_row0 = grouped ? s_group[1] : tile_t * BN;
+  const int x_rows = grouped ? s_group[2] : min(BN, p.T - x_row0);
+  const int kend = x_rows > 0 ? kb1 : kb0;                             // nothing to do for a tile without rows
+
+  uint8_t* ring = smem + L::A_RING;
+  if (warp == 0) {
+    if (elect_one()) {
+      constexpr int W_COLS = SRC == kSrcU4 ? 64 : 128;                 // bytes of a weight row per block of 128 k
+      constexpr int W_TILE = 128 * W_COLS;
+      const uint64_t hint_w = p.t_tiles == 1 || grouped ? kEvictFirst : kEvictNormal;
+      auto load_w = [&](int s, int kb) {
+        mbar_expect_tx(&full_bar[s], L::STAGE);
+        uint8_t* st = ring + s * L::STAGE;
+        tma_load_2d(st, &tmW, &full_bar[s], kb * W_COLS, w_row0, hint_w);
+        if (DUAL) tma_load_2d(st + W_TILE, &tmW, &full_bar[s], kb * W_COLS, p.dual_off + w_row0, hint_w);
+      };
+      auto load_x = [&](int s, int kb) {
+        uint8_t* st = ring + s * L::STAGE + W_TILE * NACC;
+        tma_load_2d(st, &tmX, &full_bar[s], kb * 128, x_row0, kEvictLast);
+        if (SRC != kSrcI8) tma_load_2d(st + BN * 128, &tmX, &full_bar[s], p.x_lo + kb * 128, x_row0, kEvictLast);
+      };
+      // weights never depend on the previous kernel: the first round is requested before the grid dependency resolves
+      const int pre = min(STAGES, kend - kb0);
+      for (int i = 0; i < pre; ++i) load_w(i, kb0 + i);
+      grid_dep_wait();
+      for (int i = 0; i < pre; ++i) load_x(i, kb0 + i);
+      Ring r = {0, 1};
+      for (int kb = kb0 + pre; kb < kend; ++kb, r.next(STAGES)) {
+        if (!mbar_wait(&empty_bar[r.s], r.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
+        load_w(r.s, kb);
+        load_x(r.s, kb);
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint64_t stage0 = umma_desc_k128(smem_u32(ring));
+      const uint64_t bdesc0 = stage0 + (L::STAGE - L::B_BYTES) / 16;
+      const uint64_t a0 = SRC == kSrcU4 ? umma_desc_k128(smem_u32(smem)) : stage0;
+      Ring r = {0, 0}, b = {0, 0};                                     // stage; buffer of expanded codes or accumulator
+      bool ok = true;
+      for (int kb = kb0; kb < kend; ++kb, r.next(STAGES), b.next(2)) {
+        if (SRC == kSrcFp8) ok = mbar_wait(&tmem_empty[b.s], b.ph ^ 1, p.status, XFT_ERR_WAIT_TMEM);
+        ok = ok && mbar_wait(&full_bar[r.s], r.ph, p.status, XFT_ERR_WAIT_FULL);
+        if (SRC == kSrcU4) ok = ok && mbar_wait(&a_ready[b.s], b.ph, p.status, XFT_ERR_WAIT_FULL);
+        if (!ok) break;
+        tcgen05_fence_after();
+        const uint64_t bd = bdesc0 + (uint64_t)(r.s * (L::STAGE / 16));
+        const uint64_t ad = a0 + (uint64_t)(SRC == kSrcU4 ? b.s * (L::A_BYTES / 16) : r.s * (L::STAGE / 16));
+        const uint32_t acc = tmem_base + (SRC == kSrcFp8 ? b.s * ACC : 0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {                                  // 4 x 32 k
+          const uint32_t on = (SRC != kSrcFp8 && kb > kb0) || k > 0;
+          auto mma = [&](uint32_t d, uint64_t a) {
+            if constexpr (SRC == kSrcI8) umma_i8(d, a, bd + 2 * k, IDESC, on);
+            else umma_f8(d, a, bd + 2 * k, IDESC, on);
+          };
+          mma(acc, ad + 2 * k);
+          if (DUAL) mma(acc + NB, ad + TILE_A / 16 + 2 * k);
+        }
+        tcgen05_commit(&empty_bar[r.s]);
+        if (SRC == kSrcU4) tcgen05_commit(&a_empty[b.s]);
+        if (SRC == kSrcFp8) tcgen05_commit(&tmem_full[b.s]);
+      }
+      if (SRC != kSrcFp8 && kend > kb0 && ok) tcgen05_commit(&tmem_full[0]);
+    }
+  }
+
+  // ---- warps 2..9: row = feature of the tile, tokens [c0, c0 + HB) of it
+  const int q = warp & 3, row = q * 32 + lane, half = warp >= 6, c0 = half * HB;
+  const int n = tile_n * 128 + row;
+  const bool n_ok = n < p.N;
+  float g[NACC][HB];
+#pragma unroll
+  for (int i = 0; i < NACC; ++i)
+#pragma unroll
+    for (int j = 0; j < HB; ++j) g[i][j] = 0.f;
+  bool ok = x_rows > 0;
+  if (warp >= 2) {
+    const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + c0;
+    auto fetch = [&](uint32_t col, float* to, float factor) {          // to += factor * (hi + lo / 16)
+      uint32_t hi[HB], lo[HB];
+      tmem_ld_cols<HB>(taddr + col, hi);
+      tmem_ld_cols<HB>(taddr + col + BN, lo);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < HB; ++j)
+        to[j] = fmaf(factor, fmaf(__uint_as_float(lo[j]), 0.0625f, __uint_as_float(hi[j])), to[j]);
+    };
+    if constexpr (SRC == kSrcFp8) {
+      const float* sc = p.scale + (size_t)(w_row0 >> 7) * p.scale_ld;
+      const float* sc_up = sc + (size_t)(p.dual_off >> 7) * p.scale_ld;
+      Ring b = {0, 0};
+      for (int kb = kb0; kb < kend && ok; ++kb, b.next(2)) {
+        const float f0 = __ldg(sc + kb), f1 = DUAL ? __ldg(sc_up + kb) : 0.f;
+        ok = mbar_wait(&tmem_full[b.s], b.ph, p.status, XFT_ERR_WAIT_TMEM);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tcgen05_fence_after();
+        fetch(b.s * ACC, g[0], f0);
+        if constexpr (DUAL) fetch(b.s * ACC + NB, g[1], f1);
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tmem_empty[b.s]);
+      }
+    } else if constexpr (SRC == kSrcI8) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&tmem_full[0], 0, p.status, XFT_ERR_WAIT_TMEM));
+      tcgen05_fence_after();
+      if (ok) {                                                        // s32, kept as they are
+        tmem_ld_cols<HB>(taddr, reinterpret_cast<uint32_t*>(g[0]));
+        if constexpr (DUAL) tmem_ld_cols<HB>(taddr + NB, reinterpret_cast<uint32_t*>(g[1]));
+        tmem_ld_wait();
+      }
+    } else {
+      // codes to bytes: a 16-byte piece holds 32 of them; the even ones go to one swizzled 16-byte piece of the operand row,
+      // the odd ones to the next (the activations' k are in the same order)
+      const int e = threadIdx.x - 64;
+      Ring r = {0, 0}, b = {0, 0};
+      bool alive = true;
+      for (int kb = kb0; kb < kend; ++kb, r.next(STAGES), b.next(2)) {
+        alive = alive && mbar_wait(&full_bar[r.s], r.ph, p.status, XFT_ERR_WAIT_FULL) &&
+                mbar_wait(&a_empty[b.s], b.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY);
+        if (alive) {
+          const uint8_t* raw = ring + r.s * L::STAGE;
+          uint8_t* a = smem + b.s * L::A_BYTES;
+#pragma unroll
+          for (int i = 0; i < 2 * NACC; ++i) {
+            const int ci = e + 256 * i, tr = ci >> 2, part = ci & 3;   // row of the stacked tiles, 32 codes of it
+            const uint4 w = *reinterpret_cast<const uint4*>(raw + ci * 16);
+            constexpr uint32_t M = 0x0F0F0F0Fu;
+            uint8_t* dst = a + tr * 128;
+            *reinterpret_cast<uint4*>(dst + (((2 * part) ^ (tr & 7)) << 4)) = make_uint4(w.x & M, w.y & M, w.z & M, w.w & M);
+            *reinterpret_cast<uint4*>(dst + (((2 * part + 1) ^ (tr & 7)) << 4)) =
+                make_uint4((w.x >> 4) & M, (w.y >> 4) & M, (w.z >> 4) & M, (w.w >> 4) & M);
+          }
+          fence_proxy_async();
+        }
+        mbar_arrive(&a_ready[b.s]);
+      }
+      if (kend > kb0) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&tmem_full[0], 0, p.status, XFT_ERR_WAIT_TMEM));
+        tcgen05_fence_after();
+        if (ok) {
+          fetch(0, g[0], 512.f);
+          if constexpr (DUAL) fetch(NB, g[1], 512.f);
+        }
+      }
+    }
+  }
+  if (warp >= 2) grid_dep_wait();                                      // outputs, residual and the row scales belong to the stream order
+
+  auto finish = [&](int t, float x, float u) {                         // t: token row of X and Y
+    const float st = p.x_scale[t];
+    if constexpr (SRC == kSrcI8) {
+      const float za = p.a_zero[t], qs = p.a_qsum[t];
+      auto value = [&](float acc, int nn) {
+        return w8a8_value((float)__float_as_int(acc), st, za, qs, p.scale[nn], p.zero ? p.zero[nn] : 0.f, p.w_sum ? p.w_sum[nn] : 0.f,
+                          p.K, p.bias ? p.bias[nn] : 0.f);
+      };
+      if (DUAL) x = apply_act(bf16_round(value(x, n)), p.act) * bf16_round(value(u, p.dual_off + n));
+      else x = apply_act(value(x, n), p.act);
+      if (p.residual) x += p.res_scale * __bfloat162float(p.residual[(size_t)t * p.ldr + n]);
+      if (p.out_fp32) reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + n] = x;
+      else reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + n] = __float2bfloat16(x);
+      return;
+    }
+    float s0 = st, s1 = st, b0 = p.bias ? p.bias[n] : 0.f, b1 = DUAL && p.bias ? p.bias[p.dual_off + n] : 0.f;
+    if (SRC == kSrcU4) {
+      const float xs = p.x_sum[t];
+      s0 *= p.scale[n];
+      b0 += p.zero[n] * xs;
+      if (DUAL) { s1 *= p.scale[p.dual_off + n]; b1 += p.zero[p.dual_off + n] * xs; }
+    }
+    x = apply_act(fmaf(x, s0, b0), p.act);
+    if (DUAL) x *= fmaf(u, s1, b1);
+    if (p.col_scale) x *= p.col_scale[t];
+    if (p.residual) x += p.res_scale * __bfloat162float(p.residual[(size_t)t * p.ldr + n]);
+    if (p.out_fp32) reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + n] = x;
+    else reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + n] = __float2bfloat16(x);
+  };
+  if (p.splits == 1) {
+    if (warp >= 2 && ok && n_ok) {
+#pragma unroll
+      for (int j = 0; j < HB; ++j)
+        if (c0 + j < x_rows) finish(x_row0 + c0 + j, g[0][j], DUAL ? g[NACC - 1][j] : 0.f);
+    }
+  } else {
+    // every MMA has read its operands (the last accumulator is here), so the ring is free for this CTA's part: [column][128]
+    float* part = reinterpret_cast<float*>(smem);
+    named_bar_sync(1, kE4Threads);                                     // the slower half may still wait for its accumulator
+    if (warp >= 2) {
+#pragma unroll
+      for (int i = 0; i < NACC; ++i)
+#pragma unroll
+        for (int j = 0; j < HB; ++j) part[(i * BN + c0 + j) * 128 + row] = g[i][j];
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    const int per = BN / p.splits;                                     // tokens of this CTA, half of them per warp of a row
+    if (warp >= 2 && n_ok) {
+      const int lo = rank * per + (half ? (per + 1) / 2 : 0), hi = half ? (rank + 1) * per : rank * per + (per + 1) / 2;
+      for (int c = lo; c < hi && c < x_rows; ++c) {
+        float v[8], w[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          const uint32_t a = smem_u32(part + c * 128 + row);
+          v[s] = s < p.splits ? ld_dsmem(dsmem_addr(a, s)) : 0.f;
+          w[s] = DUAL && s < p.splits ? ld_dsmem(dsmem_addr(a + BN * 512, s)) : 0.f;
+        }
+        float x = 0.f, u = 0.f;
+        if constexpr (SRC == kSrcI8) {
+          int xi = 0, ui = 0;
+#pragma unroll
+          for (int s = 0; s < 8; ++s) { xi += __float_as_int(v[s]); ui += __float_as_int(w[s]); }
+          x = __int_as_float(xi); u = __int_as_float(ui);
+        } else {
+#pragma unroll
+          for (int s = 0; s < 8; ++s) { x += v[s]; u += w[s]; }
+        }
+        finish(x_row0 + c, x, u);
+      }
+    }
+    __syncwarp();
+    cluster_arrive();                                                  // nobody leaves while its part is being read
+    cluster_wait();
+  }
+  __syncwarp();
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) { tcgen05_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
+}
+
+// Row r of X (or row src[r]) -> [hi | lo] e4m3, its power-of-two scale and its sum.  `nibbles`: k in the order in which uint4
+// codes expand, 16 even ones and 16 odd ones of every 32.  Rows from *rows_used on are left alone.
+__global__ void __launch_bounds__(256) split_e4m3_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int* __restrict__ src,
+                                                         const int* __restrict__ rows_used, int K, int Kp, int nibbles,
+                                                         uint8_t* __restrict__ out, float* __restrict__ scale, float* __restrict__ sum) {
+  __shared__ float s_mx[8], s_sum[8];
+  grid_dep_launch();
+  grid_dep_wait();
+  const int r = blockIdx.x;
+  if (rows_used && r >= *rows_used) return;
+  const __nv_bfloat16* row = x + (size_t)(src ? src[r] : r) * ldx;
+  float mx = 0.f, sm = 0.f;
+  for (int k = threadIdx.x * 8; k < K; k += 2048) {
+    const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(h[i]);
+      sm += f.x + f.y;
+      const float a = fabsf(f.x), b = fabsf(f.y);
+      if (a <= 3.4e38f) mx = fmaxf(mx, a);                             // infinities and NaN have no part in the scale
+      if (b <= 3.4e38f) mx = fmaxf(mx, b);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    sm += __shfl_xor_sync(0xffffffffu, sm, o);
+  }
+  if ((threadIdx.x & 31) == 0) { s_mx[threadIdx.x >> 5] = mx; s_sum[threadIdx.x >> 5] = sm; }
+  __syncthreads();
+  mx = s_mx[0]; sm = s_sum[0];
+  for (int w = 1; w < 8; ++w) { mx = fmaxf(mx, s_mx[w]); sm += s_sum[w]; }
+  int e;
+  const float f = frexpf(mx, &e);                                      // mx = f 2^e, 0.5 <= f < 1: at most 448 = 0.875 * 2^9
+  e = mx == 0.f ? 0 : max(-100, e - 9 + (f > 0.875f));
+  const float inv = exp2f((float)-e);
+  if (threadIdx.x == 0) {
+    scale[r] = exp2f((float)e);
+    if (sum) sum[r] = sm;
+  }
+  uint8_t* hi_row = out + (size_t)r * 2 * Kp;
+  for (int k = threadIdx.x * 8; k < Kp; k += 2048) {
+    uint8_t hi[8], lo[8];
+    if (k < K) {
+      const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+      const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float y = __bfloat162float(b[i]) * inv;
+        const __nv_fp8_storage_t c = __nv_cvt_float_to_fp8(y, __NV_SATFINITE, __NV_E4M3);
+        const float back = __half2float(__half(__nv_cvt_fp8_to_halfraw(c, __NV_E4M3)));
+        hi[i] = fabsf(y) <= 3.4e38f ? c : 0x7F;                        // an infinity or NaN makes its row NaN
+        lo[i] = fabsf(y) <= 3.4e38f ? __nv_cvt_float_to_fp8((y - back) * 16.f, __NV_SATFINITE, __NV_E4M3) : 0;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) hi[i] = lo[i] = 0;                   // 0 x garbage of a padded column could be NaN
+    }
+    if (nibbles) {
+      const int at = (k & ~31) + (k & 31) / 2;
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+        *reinterpret_cast<uchar4*>(hi_row + at + 16 * o) = make_uchar4(hi[o], hi[2 + o], hi[4 + o], hi[6 + o]);
+        *reinterpret_cast<uchar4*>(hi_row + Kp + at + 16 * o) = make_uchar4(lo[o], lo[2 + o], lo[4 + o], lo[6 + o]);
+      }
+    } else {
+      uint2 a, c;
+      memcpy(&a, hi, 8);
+      memcpy(&c, lo, 8);
+      *reinterpret_cast<uint2*>(hi_row + k) = a;
+      *reinterpret_cast<uint2*>(hi_row + Kp + k) = c;
+    }
+  }
+}
+
+int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes, uint32_t box_rows,
+                  uint32_t box_bytes);                                 // quant_gemm_sm100.cu: unswizzled bytes
+
+// One round of CTAs (two per SM up to 32 tokens, see E4Layout), at least four blocks of 128 k in each.
+static int e4_splits(int tiles, int num_kb, int bn) {
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= (bn <= 32 ? 2 : 1) * 148 && num_kb / (2 * s) >= 4) s *= 2;
+  return s;
+}
+
+template <int BN, bool DUAL, int SRC>
+static int launch_e4(const CUtensorMap& tmW, const CUtensorMap& tmX, const E4Params& p, cudaStream_t st) {
+  using L = E4Layout<BN, DUAL, SRC>;
+  const auto kernel = gemm_e4m3_kernel<BN, DUAL, SRC>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM) != cudaSuccess)
+      return 3000 + (int)cudaGetLastError();
+    attr_set = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.n_tiles * p.t_tiles, p.splits);
+  cfg.blockDim = dim3(kE4Threads);
+  cfg.dynamicSmemBytes = L::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = attr[0].val.clusterDim.z = 1;
+  attr[0].val.clusterDim.y = p.splits;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g_xft_pdl ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tmW, tmX, p);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+}  // namespace xft
+
+using namespace xft;
+
+// Columns of a row of split activations: hi and lo halves are this many bytes each.
+extern "C" int xft_split_e4m3_cols(int K) { return (K + 31) / 32 * 32; }
+
+// X [.., ldx] bf16 -> out [rows, 2 * cols], scale [rows], sum [rows] (or null); K, ldx multiples of 8, 16-byte aligned rows.
+extern "C" int xft_split_e4m3(const void* x, int ldx, const int* src, const int* rows_used, int rows, int K, int nibbles, void* out,
+                              float* scale, float* sum, cudaStream_t st) {
+  if (rows <= 0) return 0;
+  if ((K & 7) || (ldx & 7) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15)) return -2;
+  const cudaError_t e = launch_pdl(split_e4m3_kernel, dim3(rows), dim3(256), 0, st, (const __nv_bfloat16*)x, ldx, src, rows_used, K,
+                                   xft_split_e4m3_cols(K), nibbles, (uint8_t*)out, scale, sum);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+// src: 0 = e4m3 weights [w_rows, K] with block scales, 1 = uint4 [w_rows, K / 2] with scale / zero per row.  xs, x_scale, x_sum
+// from xft_split_e4m3 (`nibbles` = src).  Grouped (fp8): tiles of `bn` rows as in xft_qgemm_grouped; plain: group_tiles null.
+extern "C" int xft_gemm_e4m3(const void* xs, int x_rows, const float* x_scale, const float* x_sum, const void* W, int w_rows,
+                             int ldw_bytes, int src, void* Y, int ldo, int out_fp32, int T, int N, int K, int gated, int dual_off,
+                             const float* scale, const float* zero, int scale_ld, const float* bias, const void* residual, int ldr,
+                             float res_scale, int act, const void* group_tiles, const int* num_group_tiles, int group_w_rows,
+                             int max_tiles, int bn, const float* col_scale, int* status, cudaStream_t st) {
+  if (T <= 0 || N <= 0 || K <= 0) return 0;
+  if (K & 7) return -2;
+  if (src == kSrcFp8 && ((gated && (dual_off & 127)) || (group_tiles && (group_w_rows & 127)))) return -4;
+  if (src == kSrcU4 && (group_tiles || !zero || !x_sum)) return -4;
+  E4Params p{};
+  p.N = N; p.T = T; p.K = K; p.dual_off = dual_off; p.out = Y; p.ldo = ldo; p.out_fp32 = out_fp32; p.bias = bias;
+  p.residual = (const __nv_bfloat16*)residual; p.ldr = ldr; p.res_scale = res_scale; p.act = act; p.x_scale = x_scale;
+  p.x_sum = x_sum; p.scale = scale; p.zero = zero; p.scale_ld = scale_ld; p.status = status; p.col_scale = col_scale;
+  p.group_tiles = reinterpret_cast<const int4*>(group_tiles); p.num_group_tiles = num_group_tiles; p.group_w_rows = group_w_rows;
+  p.x_lo = xft_split_e4m3_cols(K);
+  if (!group_tiles) bn = T <= 16 ? 16 : T <= 32 ? 32 : 64;
+  p.num_kb = (K + 127) / 128;
+  p.n_tiles = (N + 127) / 128;
+  p.t_tiles = group_tiles ? max_tiles : (T + bn - 1) / bn;
+  p.splits = 1;
+  if (!group_tiles) p.splits = e4_splits(p.n_tiles * p.t_tiles, p.num_kb, bn);
+  CUtensorMap tmW, tmX;
+  int r = src == kSrcU4 ? make_byte_map(&tmW, W, (uint64_t)w_rows, (uint64_t)K / 2, (uint64_t)ldw_bytes, 128, 64)
+                        : make_tensor_map(&tmW, W, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw_bytes, 128, 1);
+  if (r) return 1000 - r;
+  r = make_tensor_map(&tmX, xs, (uint64_t)x_rows, (uint64_t)2 * p.x_lo, (uint64_t)2 * p.x_lo, (uint32_t)bn, 1);
+  if (r) return 2000 - r;
+#define XFT_E4(BN_)                                                                                     \
+  case BN_:                                                                                             \
+    if (src == kSrcU4) return gated ? launch_e4<BN_, true, kSrcU4>(tmW, tmX, p, st) : launch_e4<BN_, false, kSrcU4>(tmW, tmX, p, st); \
+    return gated ? launch_e4<BN_, true, kSrcFp8>(tmW, tmX, p, st) : launch_e4<BN_, false, kSrcFp8>(tmW, tmX, p, st);
+  switch (bn) { XFT_E4(16) XFT_E4(32) XFT_E4(64) }
+#undef XFT_E4
+  return -1;
+}
+
+namespace xft {
+// W8A8 at decode sizes (T <= 64), see xft_w8a8_gemm; gated: act(gate) * up, gate rows [0, N) and up rows from dual_off on.
+int launch_w8a8_decode(const void* qx, int ldqx, const void* Wq, int w_rows, int ldw, void* Y, int ldo, int out_fp32, int T, int N, int K,
+                       int gated, int dual_off, const float* a_scale, const float* a_zero, const float* a_qsum, const float* w_scale,
+                       const float* w_zero, const float* w_sum, const float* bias, const void* residual, int ldr, float res_scale,
+                       int act, int* status, cudaStream_t st) {
+  E4Params p{};
+  p.N = N; p.T = T; p.K = K; p.dual_off = dual_off; p.out = Y; p.ldo = ldo; p.out_fp32 = out_fp32; p.bias = bias;
+  p.residual = (const __nv_bfloat16*)residual; p.ldr = ldr; p.res_scale = res_scale; p.act = act; p.x_scale = a_scale;
+  p.a_zero = a_zero; p.a_qsum = a_qsum; p.scale = w_scale; p.zero = w_zero; p.w_sum = w_sum; p.status = status;
+  const int bn = T <= 16 ? 16 : T <= 32 ? 32 : 64;
+  p.num_kb = (K + 127) / 128;
+  p.n_tiles = (N + 127) / 128;
+  p.t_tiles = (T + bn - 1) / bn;
+  p.splits = e4_splits(p.n_tiles * p.t_tiles, p.num_kb, bn);
+  CUtensorMap tmW, tmX;
+  int r = make_tensor_map(&tmW, Wq, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw, 128, 1);
+  if (r) return 1000 - r;
+  r = make_tensor_map(&tmX, qx, (uint64_t)T, (uint64_t)K, (uint64_t)ldqx, (uint32_t)bn, 1);
+  if (r) return 2000 - r;
+#define XFT_I8(BN_) \
+  case BN_: return gated ? launch_e4<BN_, true, kSrcI8>(tmW, tmX, p, st) : launch_e4<BN_, false, kSrcI8>(tmW, tmX, p, st);
+  switch (bn) { XFT_I8(16) XFT_I8(32) XFT_I8(64) }
+#undef XFT_I8
+  return -1;
+}
+
+int launch_w8a8_prompt(const void* qx, int ldqx, const void* Wq, int w_rows, int ldw, void* Y, int ldo, int out_fp32, int T, int N, int K,
+                       int gated, int dual_off, const float* a_scale, const float* a_zero, const float* a_qsum, const float* w_scale,
+                       const float* w_zero, const float* w_sum, const float* bias, const void* residual, int ldr, float res_scale,
+                       int act, int* status, cudaStream_t st);      // gemm_prefill_sm100.cu
+}  // namespace xft
+
+// Y = epi(dequant(qx) · dequant(Wq)^T): qx int8 [T, K] with a_scale/a_zero/a_qsum from xft_quant_act, one scale and zero point per
+// weight row; y = sa sw acc + sa zw sum(qx) + za sw sum(qw) + K za zw, then bias, activation, residual.  gated: act(gate) * up of
+// gate rows [0, N) and up rows [dual_off, dual_off + N).  Up to 64 tokens the kernel above, then the
+// token-major one of gemm_prefill_sm100.cu.
+static int w8a8(const void* qx, int ldqx, const void* Wq, int ldw, void* Y, int ldo, int out_fp32, int T, int N, int K, int gated,
+                int dual_off, const float* a_scale, const float* a_zero, const float* a_qsum, const float* w_scale, const float* w_zero,
+                const float* w_sum, const float* bias, const void* residual, int ldr, float res_scale, int act, int* status,
+                cudaStream_t st) {
+  if (T <= 0 || N <= 0 || K <= 0) return 0;
+  if (K % 16) return -4;
+  const int w_rows = gated ? dual_off + N : N;
+  return (T <= 64 ? launch_w8a8_decode : launch_w8a8_prompt)(qx, ldqx, Wq, w_rows, ldw, Y, ldo, out_fp32, T, N, K, gated, dual_off,
+                                                             a_scale, a_zero, a_qsum, w_scale, w_zero, w_sum, bias, residual, ldr,
+                                                             res_scale, act, status, st);
+}
+
+extern "C" int xft_w8a8_gemm(const void* qx, int ldqx, const void* Wq, int ldw, void* Y, int ldo, int out_fp32, int T, int N, int K,
+                             const float* a_scale, const float* a_zero, const float* a_qsum, const float* w_scale, const float* w_zero,
+                             const float* w_sum, const float* bias, const void* residual, int ldr, float res_scale, int act, float*,
+                             size_t, int*, int, int* status, cudaStream_t st) {
+  return w8a8(qx, ldqx, Wq, ldw, Y, ldo, out_fp32, T, N, K, 0, 0, a_scale, a_zero, a_qsum, w_scale, w_zero, w_sum, bias, residual, ldr,
+              res_scale, act, status, st);
+}
+
+extern "C" int xft_w8a8_gemm_gated(const void* qx, int ldqx, const void* Wq, int ldw, void* Y, int ldo, int T, int N, int K, int dual_off,
+                                   const float* a_scale, const float* a_zero, const float* a_qsum, const float* w_scale,
+                                   const float* w_zero, const float* w_sum, const float* bias, int act, int* status, cudaStream_t st) {
+  return w8a8(qx, ldqx, Wq, ldw, Y, ldo, 0, T, N, K, 1, dual_off, a_scale, a_zero, a_qsum, w_scale, w_zero, w_sum, bias, nullptr, 0, 1.f,
+              act, status, st);
+}

@@ -64,6 +64,9 @@ struct PrefillParams {
   int out_fp32;
   const int4* group_tiles; const int* num_group_tiles;
   int group_w_rows, group_rows;          // weight rows of a group, token rows of a tile of the table (128 or 256)
+  // W8A8: int8 X and W, see xft_w8a8_gemm (all per token or per weight row)
+  const float* a_scale; const float* a_zero; const float* a_qsum; const float* w_scale; const float* w_zero; const float* w_sum;
+  int dual_rows;                         // weight rows between a gate feature and its up feature (ungated: all)
   BulkArParams ar;
 };
 
@@ -445,7 +448,7 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_kernel(const __grid_const
 constexpr int kPrefillTmThreads = 320;      // producer, MMA, two epilogue warps per quarter of the accumulator's rows
 __host__ __device__ constexpr int prefill_tm_stages(int stage_bytes) { return 196 * 1024 / stage_bytes < kPrefillMaxStages ? 196 * 1024 / stage_bytes : kPrefillMaxStages; }
 
-template <int NCOL, bool DUAL, int CG>
+template <int NCOL, bool DUAL, int CG, bool I8 = false>
 __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(const __grid_constant__ CUtensorMap tmX,
                                                                  const __grid_constant__ CUtensorMap tmW,
                                                                  const PrefillParams p) {
@@ -456,7 +459,9 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int STAGES = prefill_tm_stages(STAGE_BYTES);
   constexpr uint32_t TMEM_COLS = 2 * NCOL;               // double-buffered accumulators
-  constexpr uint32_t IDESC = umma_idesc(TOK, NCOL, 1, 1, 1);
+  constexpr int KEL = I8 ? 128 : 64;                     // k of a step: 128 bytes of a row
+  constexpr uint32_t IDESC = umma_idesc(TOK, NCOL, 1, 1, I8 ? 2 : 1);
+  constexpr int CW = DUAL || I8 ? 16 : 32;               // columns of an epilogue step: registers for what it holds at once
   static_assert((NCOL == 256 || NCOL == 128) && (CG == 1 || CG == 2), "tile of the token-major kernel");
 
   extern __shared__ uint8_t smem_raw[];
@@ -544,13 +549,13 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
           uint8_t* a = smem + s * STAGE_BYTES;
           if constexpr (CG == 2) {
             if (half == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
-            tma_load_2d_pair(a, &tmX, lead_bar + 8 * s, kb * 64, im.row0, hint);
-            tma_load_2d_pair(a + A_BYTES, &tmW, lead_bar + 8 * s, kb * 64, wrow, hint);
+            tma_load_2d_pair(a, &tmX, lead_bar + 8 * s, kb * KEL, im.row0, hint);
+            tma_load_2d_pair(a + A_BYTES, &tmW, lead_bar + 8 * s, kb * KEL, wrow, hint);
           } else {
             mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-            tma_load_2d(a, &tmX, &full_bar[s], kb * 64, im.row0, hint);
-            tma_load_2d(a + A_BYTES, &tmW, &full_bar[s], kb * 64, wrow, hint);
-            if (DUAL) tma_load_2d(a + A_BYTES + FEAT * 128, &tmW, &full_bar[s], kb * 64, wrow + p.dual_off, hint);
+            tma_load_2d(a, &tmX, &full_bar[s], kb * KEL, im.row0, hint);
+            tma_load_2d(a + A_BYTES, &tmW, &full_bar[s], kb * KEL, wrow, hint);
+            if (DUAL) tma_load_2d(a + A_BYTES + FEAT * 128, &tmW, &full_bar[s], kb * KEL, wrow + p.dual_off, hint);
           }
         }
       }
@@ -586,7 +591,8 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const uint32_t acc_on = (kb > 0 || k > 0) ? 1u : 0u;
-            if constexpr (CG == 2) umma_bf16_pair(acc, adesc0 + off + 2 * k, bdesc0 + off + 2 * k, IDESC, acc_on);
+            if constexpr (CG == 2 && I8) umma_i8_pair(acc, adesc0 + off + 2 * k, bdesc0 + off + 2 * k, IDESC, acc_on);
+            else if constexpr (CG == 2) umma_bf16_pair(acc, adesc0 + off + 2 * k, bdesc0 + off + 2 * k, IDESC, acc_on);
             else umma_bf16(acc, adesc0 + off + 2 * k, bdesc0 + off + 2 * k, IDESC, acc_on);
           }
           if constexpr (CG == 2) tcgen05_commit_pair(&empty_bar[s]);
@@ -621,22 +627,40 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
       const bool t_ok = row < im.rows;
       __nv_bfloat16* orow = p.out + (size_t)t * p.ldo;
       const __nv_bfloat16* rrow = p.residual ? p.residual + (size_t)t * p.ldr : nullptr;
+      auto load_cols = [&](uint32_t at, uint32_t* to) {
+        if constexpr (CW == 16) tmem_ld16(at, *reinterpret_cast<uint32_t (*)[16]>(to));
+        else tmem_ld32(at, *reinterpret_cast<uint32_t (*)[32]>(to));
+      };
+      // W8A8: integer sums of 16 features from weight row nn on -> values
+      float sa = 0.f, za = 0.f, qs = 0.f;
+      if constexpr (I8) {
+        if (t_ok) { sa = __ldg(p.a_scale + t); za = __ldg(p.a_zero + t); qs = __ldg(p.a_qsum + t); }
+      }
+      auto dequant = [&](const uint32_t* acc, int nn, bool whole, float* to) {
+#pragma unroll
+        for (int j = 0; j < CW; ++j) {
+          const int m = whole || nn % p.dual_rows + j < p.N ? nn + j : nn;
+          const float y = w8a8_value((float)(int)acc[j], sa, za, qs, __ldg(p.w_scale + m), p.w_zero ? __ldg(p.w_zero + m) : 0.f,
+                                     p.w_sum ? __ldg(p.w_sum + m) : 0.f, p.K, p.bias ? __ldg(p.bias + m) : 0.f);
+          to[j] = DUAL ? bf16_round(y) : y;
+        }
+      };
 #pragma unroll 1
-      for (int c = c_begin; c < c_end; c += 32) {
+      for (int c = c_begin; c < c_end; c += CW) {
         const int n0 = im.nt * FEAT + c;
-        const bool full = vec && n0 + 32 <= p.N;
-        uint32_t v[32];
-        uint32_t vu[DUAL ? 32 : 1];
-        tmem_ld32(taddr + c, v);
-        if constexpr (DUAL) tmem_ld32(taddr + FEAT + c, reinterpret_cast<uint32_t (&)[32]>(vu));
-        uint4 res[4];
-        const bool take = rrow && full && t_ok && !p.out_fp32;
+        const bool full = vec && n0 + CW <= p.N;
+        uint32_t v[CW];
+        uint32_t vu[DUAL ? CW : 1];
+        load_cols(taddr + c, v);
+        if constexpr (DUAL) load_cols(taddr + FEAT + c, vu);
+        uint4 res[CW / 8];
+        const bool take = rrow && full && t_ok;
         if (take) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) res[j] = *reinterpret_cast<const uint4*>(rrow + n0 + 8 * j);
+          for (int j = 0; j < CW / 8; ++j) res[j] = *reinterpret_cast<const uint4*>(rrow + n0 + 8 * j);
         }
         tmem_ld_wait();
-        if (c + 32 >= c_end) {
+        if (c + CW >= c_end) {
           tcgen05_fence_before();
           __syncwarp();
           if (lane == 0) {
@@ -645,105 +669,117 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
           }
         }
         if (!t_ok || n0 >= p.N) continue;
-        float x[32];
+        float x[CW];
+        if constexpr (I8) {
+          dequant(v, n0, full, x);
+        } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]);
-        if (p.bias && full && bias16) {
+          for (int j = 0; j < CW; ++j) x[j] = __uint_as_float(v[j]);
+        }
+        if (I8) {                                  // the bias is in already
+        } else if (p.bias && full && bias16) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
+          for (int j = 0; j < CW / 4; ++j) {
             const float4 w = __ldg(reinterpret_cast<const float4*>(p.bias + n0) + j);
             x[4 * j] += w.x; x[4 * j + 1] += w.y; x[4 * j + 2] += w.z; x[4 * j + 3] += w.w;
           }
         } else if (p.bias) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) if (full || n0 + j < p.N) x[j] += __ldg(p.bias + n0 + j);
+          for (int j = 0; j < CW; ++j) if (full || n0 + j < p.N) x[j] += __ldg(p.bias + n0 + j);
         }
         // one branch for the whole row: a branch per element cost more than the arithmetic
         switch (p.act & (kPrefillTimes - 1)) {
           case 1:
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = apply_act(x[j], 1);
+            for (int j = 0; j < CW; ++j) x[j] = apply_act(x[j], 1);
             break;
           case 2:
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = apply_act(x[j], 2);
+            for (int j = 0; j < CW; ++j) x[j] = apply_act(x[j], 2);
             break;
           case 3:
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = apply_act(x[j], 3);
+            for (int j = 0; j < CW; ++j) x[j] = apply_act(x[j], 3);
             break;
           case 4:
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = apply_act(x[j], 4);
+            for (int j = 0; j < CW; ++j) x[j] = apply_act(x[j], 4);
             break;
           case kActGeluErf:
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = gelu_erf(x[j]);
+            for (int j = 0; j < CW; ++j) x[j] = gelu_erf(x[j]);
             break;
           case kActTanh:
           case kActSoftcap:
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = apply_act(x[j], p.act, p.res_scale);
+            for (int j = 0; j < CW; ++j) x[j] = apply_act(x[j], p.act, p.res_scale);
             break;
           default: break;
         }
         if constexpr (DUAL) {
+          float up[CW];
+          if constexpr (I8) {
+            dequant(vu, p.dual_off + n0, full, up);
+          } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            float u = __uint_as_float(vu[j]);
-            if (p.bias && (full || n0 + j < p.N)) u += __ldg(p.bias + p.dual_off + n0 + j);
+            for (int j = 0; j < CW; ++j) up[j] = __uint_as_float(vu[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < CW; ++j) {
+            float u = up[j];
+            if (!I8 && p.bias && (full || n0 + j < p.N)) u += __ldg(p.bias + p.dual_off + n0 + j);
             x[j] = p.act == kActClamped ? clamped_glu(x[j], u, p.res_scale) : x[j] * u;
           }
+        }
+        if (take) {
+          const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(res);
+          if (p.act & kPrefillTimes) {
+#pragma unroll
+            for (int j = 0; j < CW / 2; ++j) {
+              const float2 f = __bfloat1622float2(r2[j]);
+              x[2 * j] *= f.x; x[2 * j + 1] *= f.y;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < CW / 2; ++j) {
+              const float2 f = __bfloat1622float2(r2[j]);
+              x[2 * j] += p.res_scale * f.x; x[2 * j + 1] += p.res_scale * f.y;
+            }
+          }
+        } else if (rrow) {
+#pragma unroll
+          for (int j = 0; j < CW; ++j)
+            if (n0 + j < p.N) x[j] = prefill_residual(x[j], __bfloat162float(rrow[n0 + j]), p.res_scale, p.act);
         }
         if (p.out_fp32) {
           float* frow = reinterpret_cast<float*>(p.out) + (size_t)t * p.ldo + n0;
           if (full) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
+            for (int j = 0; j < CW / 4; ++j)
               reinterpret_cast<float4*>(frow)[j] = make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) if (n0 + j < p.N) frow[j] = x[j];
+            for (int j = 0; j < CW; ++j) if (n0 + j < p.N) frow[j] = x[j];
           }
         } else if (full) {
-          if (take) {
-            const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(res);
-            if (p.act & kPrefillTimes) {
+          uint32_t w[CW / 2];
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const float2 f = __bfloat1622float2(r2[j]);
-                x[2 * j] *= f.x; x[2 * j + 1] *= f.y;
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const float2 f = __bfloat1622float2(r2[j]);
-                x[2 * j] += p.res_scale * f.x; x[2 * j + 1] += p.res_scale * f.y;
-              }
-            }
-          }
-          uint32_t w[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
+          for (int j = 0; j < CW / 2; ++j) {
             const __nv_bfloat162 b = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
             w[j] = *reinterpret_cast<const uint32_t*>(&b);
           }
           if (vec32) {
-            st_global_256(orow + n0, w);
-            st_global_256(orow + n0 + 16, w + 8);
+#pragma unroll
+            for (int i = 0; i < CW / 16; ++i) st_global_256(orow + n0 + 16 * i, w + 8 * i);
           } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < CW / 8; ++i)
               *reinterpret_cast<uint4*>(orow + n0 + 8 * i) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (n0 + j < p.N) {
-              float y = x[j];
-              if (rrow) y = prefill_residual(y, __bfloat162float(rrow[n0 + j]), p.res_scale, p.act);
-              orow[n0 + j] = __float2bfloat16(y);
-            }
+          for (int j = 0; j < CW; ++j) {
+            if (n0 + j < p.N) orow[n0 + j] = __float2bfloat16(x[j]);
           }
         }
       }
@@ -763,7 +799,7 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
   }
 }
 
-template <int NCOL, bool DUAL, int CG>
+template <int NCOL, bool DUAL, int CG, bool I8 = false>
 static int launch_prefill_tm(const void* X, int ldx, const void* W, int w_rows, int ldw, PrefillParams& p, int num_ctas,
                              cudaStream_t st) {
   constexpr int STAGE_BYTES = 128 * 64 * 2 + NCOL / CG * 64 * 2;
@@ -771,14 +807,14 @@ static int launch_prefill_tm(const void* X, int ldx, const void* W, int w_rows, 
   p.n_tiles = (p.N + FEAT - 1) / FEAT;
   if (!p.group_tiles) p.t_tiles = (p.T + 128 * CG - 1) / (128 * CG);
   CUtensorMap tmW, tmX;
-  int r = make_tensor_map(&tmW, W, (uint64_t)w_rows, (uint64_t)p.K, (uint64_t)ldw, (uint32_t)(DUAL ? FEAT : NCOL / CG), 2);
+  int r = make_tensor_map(&tmW, W, (uint64_t)w_rows, (uint64_t)p.K, (uint64_t)ldw, (uint32_t)(DUAL ? FEAT : NCOL / CG), I8 ? 1 : 2);
   if (r) return 1000 - r;
-  r = make_tensor_map(&tmX, X, (uint64_t)p.T, (uint64_t)p.K, (uint64_t)ldx, 128, 2);
+  r = make_tensor_map(&tmX, X, (uint64_t)p.T, (uint64_t)p.K, (uint64_t)ldx, 128, I8 ? 1 : 2);
   if (r) return 2000 - r;
   const size_t smem = (size_t)prefill_tm_stages(STAGE_BYTES) * STAGE_BYTES + 1024;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_prefill_tm_kernel<NCOL, DUAL, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    if (cudaFuncSetAttribute(gemm_prefill_tm_kernel<NCOL, DUAL, CG, I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
       return 3000 + (int)cudaGetLastError();
     attr_set = true;
@@ -795,7 +831,7 @@ static int launch_prefill_tm(const void* X, int ldx, const void* W, int w_rows, 
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = CG > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_prefill_tm_kernel<NCOL, DUAL, CG>, tmX, tmW, (const PrefillParams)p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_prefill_tm_kernel<NCOL, DUAL, CG, I8>, tmX, tmW, (const PrefillParams)p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -927,7 +963,8 @@ extern "C" int xft_bulk_ar_layout(long long* out, int n) {
 // res_scale * residual, bf16.  gated != 0: gate rows [0, N) and up rows [dual_off, dual_off + N) of W.
 static int prefill_tm(const void* X, int ldx, const void* W, int w_rows, int ldw, PrefillParams& p, int gated, int num_ctas,
                       cudaStream_t st) {
-  p.num_kb = (p.K + 63) / 64;
+  const bool i8 = p.a_scale != nullptr;
+  p.num_kb = i8 ? (p.K + 127) / 128 : (p.K + 63) / 64;
   p.gn = 8;
   if (num_ctas <= 0) {
     int dev = 0, sms = 0;
@@ -951,6 +988,12 @@ static int prefill_tm(const void* X, int ldx, const void* W, int w_rows, int ldw
   };
   const float wide = rounds(256, 256, pairs) + 8.f, pair = 0.6f * rounds(256, 128, pairs) + 9.f,
               single = 0.65f * rounds(128, 128, num_ctas) + 3.f;
+  if (i8) {                          // pairs only: the same line between wide and narrow tiles
+    if (wide <= pair) return gated ? launch_prefill_tm<256, true, 2, true>(X, ldx, W, w_rows, ldw, p, num_ctas, st)
+                                   : launch_prefill_tm<256, false, 2, true>(X, ldx, W, w_rows, ldw, p, num_ctas, st);
+    return gated ? launch_prefill_tm<128, true, 2, true>(X, ldx, W, w_rows, ldw, p, num_ctas, st)
+                 : launch_prefill_tm<128, false, 2, true>(X, ldx, W, w_rows, ldw, p, num_ctas, st);
+  }
   if (wide <= pair && wide <= single) return XFT_TM(256, 2);
   return pair < single ? XFT_TM(128, 2) : XFT_TM(128, 1);
 #undef XFT_TM
@@ -993,3 +1036,18 @@ extern "C" int xft_gemm_bf16_grouped_tm(const void* X, int ldx, int x_rows, cons
   p.t_tiles = max_tiles; p.group_rows = tile_rows;
   return prefill_tm(X, ldx, W, w_rows, ldw, p, gated, 0, st);
 }
+
+// W8A8 above 64 tokens, see xft_w8a8_gemm (gemm_e4m3_sm100.cu)
+namespace xft {
+int launch_w8a8_prompt(const void* qx, int ldqx, const void* Wq, int w_rows, int ldw, void* Y, int ldo, int out_fp32, int T, int N, int K,
+                       int gated, int dual_off, const float* a_scale, const float* a_zero, const float* a_qsum, const float* w_scale,
+                       const float* w_zero, const float* w_sum, const float* bias, const void* residual, int ldr, float res_scale,
+                       int act, int* status, cudaStream_t st) {
+  PrefillParams p{};
+  p.N = N; p.T = T; p.K = K; p.out = reinterpret_cast<__nv_bfloat16*>(Y); p.ldo = ldo; p.out_fp32 = out_fp32; p.bias = bias;
+  p.residual = reinterpret_cast<const __nv_bfloat16*>(residual); p.ldr = ldr; p.res_scale = res_scale; p.act = act;
+  p.status = status; p.dual_off = dual_off; p.dual_rows = gated ? dual_off : 0x7fffffff;
+  p.a_scale = a_scale; p.a_zero = a_zero; p.a_qsum = a_qsum; p.w_scale = w_scale; p.w_zero = w_zero; p.w_sum = w_sum;
+  return prefill_tm(qx, ldqx, Wq, w_rows, ldw, p, gated, 0, st);
+}
+}  // namespace xft

@@ -10,11 +10,13 @@
 //     matching the reference's numerics), and the same tcgen05 / TMEM pipeline as the bf16 kernel runs on it.
 //     Per-channel scale and zero are applied on the accumulator: y = s[n]*acc + z[n]*sum_k x[t,k].
 //
-// (2) W8A8: per-row dynamic asymmetric int8 activations (zero = (min+max)/2, scale = max|x-zero|/127,
-//     matmul_helper.h:2813-2855) x int8 weights on the int8 tensor path (tcgen05 kind::i8, s32 accumulators in
-//     TMEM); epilogue  y = sa*sw*acc + sa*zw*sum(qx) + za*sw*sum(qw) + K*za*zw  (+ bias, act, residual).
+// (2) What W8A8 products need of their activations: per-row dynamic asymmetric int8 (zero = (min+max)/2, scale = max|x-zero|/127,
+//     matmul_helper.h:2813-2855).  The products themselves run on `kind::i8` in gemm_e4m3_sm100.cu (up to 64 tokens) and
+//     gemm_prefill_sm100.cu.
 //
-// Both kernels share the split-K scheme of gemm_sm100.cu (partials in fp32 scratch, last arriver reduces).
+// (The Python engine runs fp8 and uint4 through gemm_e4m3_sm100.cu, which does not expand them.)
+//
+// The split-K scheme is that of gemm_sm100.cu (partials in fp32 scratch, last arriver reduces).
 #include "ptx.cuh"
 
 #include <cuda_fp8.h>
@@ -26,7 +28,7 @@ int make_tensor_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t c
 void plan_splits(int tiles, int num_kb, int bn, int nacc, size_t ws_bytes, int max_tiles, int* splits, int* kb_per_split);
 int pick_bn(int T);
 
-enum { Q_INT8 = 0, Q_INT4 = 1, Q_NF4 = 2, Q_FP8 = 3, Q_INT4F = 4 };
+enum { Q_INT8 = 0, Q_INT4 = 1, Q_NF4 = 2, Q_FP8 = 3 };
 
 struct QGemmParams {
   int N, T, K;
@@ -42,9 +44,6 @@ struct QGemmParams {
   const float* zero;       // [N] or null
   const float* xsum;       // [T] sum_k x[t,k] (needed when zero != null)
   int scale_ld;            // fp8: blocks per scale row
-  // w8a8
-  const float* a_scale; const float* a_zero; const float* a_qsum;   // [T]
-  const float* w_sum;      // [N] sum_k qw
   // Grouped mode (MoE experts, fp8 block-scaled weights): token tile i is group_tiles[i] = {group, first row, rows, -};
   // the weight rows (and, /128, the scale rows) of group g start at g * group_w_rows.  No split-K.
   const int4* group_tiles;
@@ -104,10 +103,6 @@ __device__ __forceinline__ void expand_row(const uint8_t* raw_row, uint8_t* a_ti
 // loads are consecutive and the swizzled 16-byte stores of a quarter warp never share a bank.
 //   Q_INT8:  the byte u = q + 128 is dropped into the mantissa of 2^23 (one PRMT), 2^23 + 128 is subtracted (exact),
 //            and the upper halves of two such floats are one bf16 pair (one PRMT): no integer-to-float conversion.
-//   Q_INT4F: words are stored nibble-interleaved (nibble i = element 2i, nibble i + 4 = element 2i + 1), so
-//            (w >> 4i) & 0x000F000F | 0x43004300 IS the bf16 pair (128 + e_2i, 128 + e_2i+1): one shift and one
-//            logic op per two elements.  The constant 128 is removed in the epilogue through the activations' row
-//            sums (the caller passes zero - 128 * scale).
 template <int QT>
 __device__ __forceinline__ void expand_tile(const uint8_t* raw, uint8_t* a_tile, int et) {
   if (QT == Q_INT8) {
@@ -130,21 +125,6 @@ __device__ __forceinline__ void expand_tile(const uint8_t* raw, uint8_t* a_tile,
       *reinterpret_cast<uint4*>(dst + (((2 * part) ^ (row & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
       *reinterpret_cast<uint4*>(dst + (((2 * part + 1) ^ (row & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
     }
-  } else {   // Q_INT4F
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int ci = et + 128 * i, row = ci >> 1, part = ci & 1;
-      const uint4 w = *reinterpret_cast<const uint4*>(raw + ci * 16);
-      const uint32_t x[4] = {w.x, w.y, w.z, w.w};
-      uint8_t* dst = a_tile + row * 128;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t v = x[j];
-        *reinterpret_cast<uint4*>(dst + (((4 * part + j) ^ (row & 7)) << 4)) =
-            make_uint4((v & 0x000F000Fu) | 0x43004300u, ((v >> 4) & 0x000F000Fu) | 0x43004300u,
-                       ((v >> 8) & 0x000F000Fu) | 0x43004300u, ((v >> 12) & 0x000F000Fu) | 0x43004300u);
-      }
-    }
   }
 }
 
@@ -153,7 +133,7 @@ constexpr int kQMaxStages = 8;
 template <int BN, bool DUAL, int QT>
 __global__ void __launch_bounds__(192) qgemm_kernel(const __grid_constant__ CUtensorMap tmW,
                                                     const __grid_constant__ CUtensorMap tmX, const QGemmParams p) {
-  constexpr int RAW_BYTES = (QT == Q_INT8 || QT == Q_FP8) ? 128 * 64 : 128 * 32;      // Q_INT4F is packed like Q_INT4
+  constexpr int RAW_BYTES = (QT == Q_INT8 || QT == Q_FP8) ? 128 * 64 : 128 * 32;
   constexpr int RAW_ROW = RAW_BYTES / 128;
   constexpr int A_BYTES = 128 * 64 * 2;
   constexpr int B_BYTES = BN * 64 * 2;
@@ -296,7 +276,7 @@ __global__ void __launch_bounds__(192) qgemm_kernel(const __grid_constant__ CUte
             sc0 = p.scale[(size_t)((w_row0 >> 7) + tile_n) * p.scale_ld + (kb >> 1)];
             if (DUAL) sc1 = p.scale[(size_t)((w_row0 >> 7) + (p.dual_off >> 7) + tile_n) * p.scale_ld + (kb >> 1)];
           }
-          if (QT == Q_INT8 || QT == Q_INT4F) {
+          if (QT == Q_INT8) {
             expand_tile<QT>(st, st + RAW_BYTES * NACC, et);
             if (DUAL) expand_tile<QT>(st + RAW_BYTES, st + RAW_BYTES * NACC + A_BYTES, et);
           } else {
@@ -401,156 +381,6 @@ __global__ void __launch_bounds__(192) qgemm_kernel(const __grid_constant__ CUte
   }
 }
 
-// ------------------------------------------------------------------------------------------ W8A8
-// A = int8 weights [N,K] (128 K-elements per 128-byte swizzled row), B = int8 activations [T,K]; s32 accumulators.
-template <int BN>
-__global__ void __launch_bounds__(192) w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmW,
-                                                        const __grid_constant__ CUtensorMap tmX, const QGemmParams p) {
-  constexpr int A_BYTES = 128 * 128;
-  constexpr int B_BYTES = BN * 128;
-  constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  constexpr uint32_t TMEM_COLS = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
-  constexpr uint32_t IDESC = umma_idesc(128, BN, 1, 1, 2);      // signed int8 x signed int8 -> s32
-
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t full_bar[kQMaxStages], empty_bar[kQMaxStages], tmem_full_bar;
-  __shared__ uint32_t tmem_base_s;
-  __shared__ int s_last;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int stages = p.stages;
-  const int tile_n = blockIdx.x % p.n_tiles, tile_t = blockIdx.x / p.n_tiles;
-  const int split = blockIdx.y;
-  const int kb0 = split * p.kb_per_split;
-  const int kb1 = min(kb0 + p.kb_per_split, p.num_kb);
-  const int tile_id = tile_t * p.n_tiles + tile_n;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    mbar_init(&tmem_full_bar, 1);
-    fence_barrier_init();
-    fence_proxy_async();
-  }
-  if (warp == 1) { tmem_alloc(&tmem_base_s, TMEM_COLS); tmem_relinquish(); }
-  tcgen05_fence_before();
-  __syncthreads();
-  tcgen05_fence_after();
-  const uint32_t tmem_base = tmem_base_s;
-  grid_dep_launch();
-  if (warp == 0) {
-    if (elect_one()) {
-      const uint64_t hint_w = p.t_tiles == 1 ? kEvictFirst : kEvictNormal;
-      // weights never depend on the previous kernel: the first `stages` tiles are requested before the grid dependency resolves
-      const int pre = min(stages, kb1 - kb0);
-      for (int i = 0; i < pre; ++i) {
-        mbar_expect_tx(&full_bar[i], STAGE_BYTES);
-        tma_load_2d(smem + i * STAGE_BYTES, &tmW, &full_bar[i], (kb0 + i) * 128, tile_n * 128, hint_w);
-      }
-      grid_dep_wait();
-      for (int i = 0; i < pre; ++i)
-        tma_load_2d(smem + i * STAGE_BYTES + A_BYTES, &tmX, &full_bar[i], (kb0 + i) * 128, tile_t * BN, kEvictLast);
-      Ring r = {0, 1};
-      for (int kb = kb0 + pre; kb < kb1; ++kb, r.next(stages)) {
-        const int s = r.s;
-        if (!mbar_wait(&empty_bar[s], r.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) break;
-        mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-        uint8_t* st = smem + s * STAGE_BYTES;
-        tma_load_2d(st, &tmW, &full_bar[s], kb * 128, tile_n * 128, hint_w);
-        tma_load_2d(st + A_BYTES, &tmX, &full_bar[s], kb * 128, tile_t * BN, kEvictLast);
-      }
-    }
-  } else if (warp == 1) {
-    if (elect_one()) {
-      const uint64_t adesc0 = umma_desc_k128(smem_u32(smem)), bdesc0 = umma_desc_k128(smem_u32(smem) + A_BYTES);
-      Ring r = {0, 0};
-      for (int kb = kb0; kb < kb1; ++kb, r.next(stages)) {
-        const int s = r.s;
-        if (!mbar_wait(&full_bar[s], r.ph, p.status, XFT_ERR_WAIT_FULL)) break;
-        tcgen05_fence_after();
-        const uint64_t adesc = adesc0 + (uint64_t)(s * (STAGE_BYTES / 16)), bdesc = bdesc0 + (uint64_t)(s * (STAGE_BYTES / 16));
-#pragma unroll
-        for (int k = 0; k < 4; ++k)       // 4 x (K = 32 int8 = 32 bytes)
-          umma_i8(tmem_base, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > kb0 || k > 0) ? 1u : 0u);
-        tcgen05_commit(&empty_bar[s]);
-      }
-      tcgen05_commit(&tmem_full_bar);
-    }
-  } else {
-    const int q = warp & 3, row = q * 32 + lane, n = tile_n * 128 + row;
-    const bool n_ok = n < p.N;
-    const int et = threadIdx.x - 64;
-    grid_dep_wait();
-    bool ok = mbar_wait(&tmem_full_bar, 0, p.status, XFT_ERR_WAIT_TMEM);
-    tcgen05_fence_after();
-    const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16);
-    const int t0 = tile_t * BN;
-    bool last = true;
-    if (p.splits > 1) {
-      float* wsp = p.ws + ((size_t)split * (p.n_tiles * p.t_tiles) + tile_id) * (size_t)BN * 128;
-      if (ok) {
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 16) {
-          uint32_t v[16];
-          tmem_ld16(taddr + c, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) wsp[(size_t)(c + j) * 128 + row] = (float)(int)v[j];
-        }
-      }
-      __threadfence();
-      named_bar_sync(1, 128);
-      if (et == 0) {
-        int old = atomicAdd(&p.counters[tile_id], 1);
-        s_last = (old == p.splits - 1);
-        if (s_last) p.counters[tile_id] = 0;
-      }
-      named_bar_sync(1, 128);
-      last = s_last != 0;
-      if (last) __threadfence();
-    }
-    if (last && ok) {
-      const float sw = n_ok ? p.scale[n] : 0.f, zw = (n_ok && p.zero) ? p.zero[n] : 0.f;
-      const float wsum = (n_ok && p.w_sum) ? p.w_sum[n] : 0.f;
-      const float bias = (n_ok && p.bias) ? p.bias[n] : 0.f;
-      const float* ws_tile = p.ws + (size_t)tile_id * (size_t)BN * 128;
-      const size_t ws_split_stride = (size_t)(p.n_tiles * p.t_tiles) * (size_t)BN * 128;
-#pragma unroll 1
-      for (int c = 0; c < BN; c += 16) {
-        float g[16];
-        if (p.splits > 1) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) g[j] = 0.f;
-          for (int s = 0; s < p.splits; ++s)
-#pragma unroll
-            for (int j = 0; j < 16; ++j) g[j] += __ldcg(ws_tile + s * ws_split_stride + (size_t)(c + j) * 128 + row);
-        } else {
-          uint32_t v[16];
-          tmem_ld16(taddr + c, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) g[j] = (float)(int)v[j];
-        }
-        if (n_ok) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int t = t0 + c + j;
-            if (t < p.T) {
-              const float sa = p.a_scale[t], za = p.a_zero[t], qs = p.a_qsum[t];
-              float x = sa * sw * g[j] + sa * zw * qs + za * sw * wsum + (float)p.K * za * zw + bias;
-              x = q_act(x, p.act);
-              if (p.residual) x += p.res_scale * __bfloat162float(p.residual[(size_t)t * p.ldr + n]);
-              if (p.out_fp32) reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + n] = x;
-              else reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + n] = __float2bfloat16(x);
-            }
-          }
-        }
-      }
-    }
-  }
-  tcgen05_fence_before();
-  __syncthreads();
-  if (warp == 1) { tcgen05_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
-}
-
 // Per-row dynamic int8 quantisation of activations (+ the sums the W8A8 epilogue needs) and plain row sums.
 __global__ void __launch_bounds__(256) quant_act_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int8_t* __restrict__ q,
                                                         int ldq, float* __restrict__ scale, float* __restrict__ zero,
@@ -560,8 +390,23 @@ __global__ void __launch_bounds__(256) quant_act_kernel(const __nv_bfloat16* __r
   grid_dep_wait();
   const int t = blockIdx.x;
   const __nv_bfloat16* row = x + (size_t)t * ldx;
+  // 16-byte pieces where every row starts on one
+  const bool vec = K % 8 == 0 && ldx % 8 == 0 && ldq % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) & 15) | (reinterpret_cast<uintptr_t>(q) & 7)) == 0;
   float mx = -INFINITY, mn = INFINITY;
-  for (int i = threadIdx.x; i < K; i += 256) { float v = __bfloat162float(row[i]); mx = fmaxf(mx, v); mn = fminf(mn, v); }
+  if (vec) {
+    for (int i = threadIdx.x * 8; i < K; i += 2048) {
+      const uint4 v = *reinterpret_cast<const uint4*>(row + i);
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(h[j]);
+        mx = fmaxf(mx, fmaxf(f.x, f.y));
+        mn = fminf(mn, fminf(f.x, f.y));
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < K; i += 256) { float v = __bfloat162float(row[i]); mx = fmaxf(mx, v); mn = fminf(mn, v); }
+  }
   for (int o = 16; o > 0; o >>= 1) { mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o)); mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o)); }
   if ((threadIdx.x & 31) == 0) { smx[threadIdx.x >> 5] = mx; smn[threadIdx.x >> 5] = mn; }
   __syncthreads();
@@ -571,11 +416,24 @@ __global__ void __launch_bounds__(256) quant_act_kernel(const __nv_bfloat16* __r
   const float s = fmaxf(fmaxf(mx - z, z - mn) / 127.f, 1e-10f);
   const float inv = 1.f / s;
   float acc = 0.f;
-  for (int i = threadIdx.x; i < K; i += 256) {
-    float r = rintf((__bfloat162float(row[i]) - z) * inv);
-    r = fminf(fmaxf(r, -127.f), 127.f);
-    q[(size_t)t * ldq + i] = (int8_t)r;
+  auto code = [&](float v) {
+    const float r = fminf(fmaxf(rintf((v - z) * inv), -127.f), 127.f);
     acc += r;
+    return (int8_t)r;
+  };
+  if (vec) {
+    for (int i = threadIdx.x * 8; i < K; i += 2048) {
+      const uint4 v = *reinterpret_cast<const uint4*>(row + i);
+      const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(&v);
+      int8_t c[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) c[j] = code(__bfloat162float(b[j]));
+      uint2 w;
+      memcpy(&w, c, 8);
+      *reinterpret_cast<uint2*>(q + (size_t)t * ldq + i) = w;
+    }
+  } else {
+    for (int i = threadIdx.x; i < K; i += 256) q[(size_t)t * ldq + i] = code(__bfloat162float(row[i]));
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) ssum[threadIdx.x >> 5] = acc;
@@ -604,7 +462,7 @@ __global__ void __launch_bounds__(256) row_sum_kernel(const __nv_bfloat16* __res
 typedef CUresult (*EncFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                           const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                           CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static int make_raw_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes,
+int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes,
                         uint32_t box_rows, uint32_t box_bytes) {
   static EncFn enc = nullptr;
   if (!enc) {
@@ -647,7 +505,6 @@ static int launch_qt(int qt, const CUtensorMap& a, const CUtensorMap& b, QGemmPa
     case Q_INT4: return launch_q<BN, DUAL, Q_INT4>(a, b, p, st);
     case Q_NF4: return launch_q<BN, DUAL, Q_NF4>(a, b, p, st);
     case Q_FP8: return launch_q<BN, DUAL, Q_FP8>(a, b, p, st);
-    case Q_INT4F: return launch_q<BN, DUAL, Q_INT4F>(a, b, p, st);
   }
   return -1;
 }
@@ -656,9 +513,7 @@ static int launch_qt(int qt, const CUtensorMap& a, const CUtensorMap& b, QGemmPa
 
 using namespace xft;
 
-// qtype: 0 int8, 1 uint4, 2 nf4, 3 fp8-e4m3 (block 128x128), 4 uint4 with nibble-interleaved words (nibble i of a
-// 32-bit word = element 2i, nibble i + 4 = element 2i + 1; the kernel feeds 128 + q, so the caller passes
-// zero - 128 * scale and always the row sums).  Wq: [w_rows, K] int8/fp8 or [w_rows, K/2] packed.
+// qtype: 0 int8, 1 uint4, 2 nf4, 3 fp8-e4m3 (block 128x128).  Wq: [w_rows, K] int8/fp8 or [w_rows, K/2] packed.
 // scale/zero: see QGemmParams.  xsum: [T] row sums of X, required when zero != null.
 extern "C" int xft_qgemm(const void* X, int ldx, const void* Wq, int w_rows, int ldw_bytes, int qtype, void* Y, int ldo,
                          int out_fp32, int T, int N, int K, int gated, int dual_off, const float* scale, const float* zero,
@@ -679,7 +534,7 @@ extern "C" int xft_qgemm(const void* X, int ldx, const void* Wq, int w_rows, int
               &p.kb_per_split);
   CUtensorMap tmW, tmX;
   const bool byte_el = qtype == Q_INT8 || qtype == Q_FP8;
-  int r = make_raw_map(&tmW, Wq, (uint64_t)w_rows, byte_el ? (uint64_t)K : (uint64_t)K / 2, (uint64_t)ldw_bytes, 128,
+  int r = make_byte_map(&tmW, Wq, (uint64_t)w_rows, byte_el ? (uint64_t)K : (uint64_t)K / 2, (uint64_t)ldw_bytes, 128,
                        byte_el ? 64 : 32);
   if (r) return 1000 - r;
   r = make_tensor_map(&tmX, X, (uint64_t)T, (uint64_t)K, (uint64_t)ldx, (uint32_t)bn, 2);
@@ -711,7 +566,7 @@ extern "C" int xft_qgemm_grouped(const void* X, int ldx, int x_rows, const void*
   p.num_kb = (K + 63) / 64;
   p.splits = 1; p.kb_per_split = p.num_kb;
   CUtensorMap tmW, tmX;
-  int r = make_raw_map(&tmW, Wq, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw_bytes, 128, 64);
+  int r = make_byte_map(&tmW, Wq, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw_bytes, 128, 64);
   if (r) return 1000 - r;
   r = make_tensor_map(&tmX, X, (uint64_t)x_rows, (uint64_t)K, (uint64_t)ldx, (uint32_t)bn, 2);
   if (r) return 2000 - r;
@@ -732,47 +587,5 @@ extern "C" int xft_quant_act(const void* x, int ldx, void* q, int ldq, float* sc
 extern "C" int xft_row_sum(const void* x, int ldx, float* out, int T, int K, cudaStream_t st) {
   if (T <= 0) return 0;
   cudaError_t e = launch_pdl(row_sum_kernel, dim3(T), dim3(256), 0, st, (const __nv_bfloat16*)x, ldx, out, K);
-  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
-}
-
-// Y = epi(dequant(qx) · dequant(Wq)^T): qx int8 [T, K] with a_scale/a_zero/a_qsum from xft_quant_act.
-extern "C" int xft_w8a8_gemm(const void* qx, int ldqx, const void* Wq, int ldw, void* Y, int ldo, int out_fp32, int T, int N,
-                             int K, const float* a_scale, const float* a_zero, const float* a_qsum, const float* w_scale,
-                             const float* w_zero, const float* w_sum, const float* bias, const void* residual, int ldr,
-                             float res_scale, int act, float* ws, size_t ws_bytes, int* counters, int n_counters,
-                             int* status, cudaStream_t st) {
-  if (T <= 0 || N <= 0 || K <= 0) return 0;
-  if (K % 16) return -4;
-  QGemmParams p{};
-  p.N = N; p.T = T; p.K = K; p.out = Y; p.ldo = ldo; p.out_fp32 = out_fp32; p.bias = bias;
-  p.residual = (const __nv_bfloat16*)residual; p.ldr = ldr; p.res_scale = res_scale; p.act = act; p.ws = ws;
-  p.counters = counters; p.status = status; p.scale = w_scale; p.zero = w_zero; p.w_sum = w_sum; p.a_scale = a_scale;
-  p.a_zero = a_zero; p.a_qsum = a_qsum;
-  const int bn = pick_bn(T);
-  p.n_tiles = (N + 127) / 128;
-  p.t_tiles = (T + bn - 1) / bn;
-  p.num_kb = (K + 127) / 128;
-  plan_splits(p.n_tiles * p.t_tiles, p.num_kb, bn, 1, ws ? ws_bytes : 0, counters ? n_counters : 0, &p.splits, &p.kb_per_split);
-  CUtensorMap tmW, tmX;
-  int r = make_tensor_map(&tmW, Wq, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, 128, 1);
-  if (r) return 1000 - r;
-  r = make_tensor_map(&tmX, qx, (uint64_t)T, (uint64_t)K, (uint64_t)ldqx, (uint32_t)bn, 1);
-  if (r) return 2000 - r;
-  const int stage = 128 * 128 + bn * 128;
-  int budget = bn <= 64 ? 110 * 1024 : 220 * 1024;
-  int stages = budget / stage;
-  if (stages > kQMaxStages) stages = kQMaxStages;
-  if (stages < 2) stages = 2;
-  p.stages = stages;
-  const size_t smem = (size_t)stages * stage + 1024;
-  dim3 grid(p.n_tiles * p.t_tiles, p.splits);
-  cudaError_t e = cudaSuccess;
-#define XFT_W(BN_)                                                                                             \
-  case BN_:                                                                                                    \
-    cudaFuncSetAttribute(w8a8_gemm_kernel<BN_>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);      \
-    e = launch_pdl(w8a8_gemm_kernel<BN_>, grid, dim3(192), smem, st, tmW, tmX, p);                             \
-    break;
-  switch (bn) { XFT_W(16) XFT_W(32) XFT_W(64) XFT_W(128) XFT_W(256) default: return -1; }
-#undef XFT_W
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }

@@ -152,7 +152,7 @@ def moe_experts(x, idx, w, experts, act="silu", expert_offset=0, packed=None, ex
     avg = max(1, ((T * k if expected_pairs is None else min(int(expected_pairs), T * k)) + E - 1) // E)
     # 256 rows: two CTAs share a tile (bf16 only).  A group's last tile is half empty on average, which eats the fifth that
     # pairs gain below about 430 rows per expert
-    bn = 16 if avg <= 16 else 32 if avg <= 32 else 64 if avg <= 64 else 128 if avg < 512 or pk.get("fp8") else 256
+    bn = 16 if avg <= 16 else 32 if avg <= 32 else 64 if avg <= 64 or pk.get("fp8") else 128 if avg < 512 else 256
     max_rows = T * k
     max_tiles = (max_rows + bn - 1) // bn + E
     idx32 = idx if idx.dtype == torch.int32 else idx.int()
@@ -165,22 +165,21 @@ def moe_experts(x, idx, w, experts, act="silu", expert_offset=0, packed=None, ex
                               N._p(src), N._p(row_w), N._p(tiles), N._p(meta), max_tiles, max_rows, N._stream()),
              "moe_plan")
     add32, add16 = (add, None) if add is None or add.dtype == torch.float32 else (None, add)
-    xs = torch.empty(max_rows, H, dtype=torch.bfloat16, device=dev)
-    N._check(lib.xft_moe_gather(N._p(x2), ldx, N._p(src), N._p(meta), N._p(xs), max_rows, H, N._stream()), "moe_gather")
     h1 = torch.empty(max_rows, I, dtype=torch.bfloat16, device=dev)
     if pk.get("fp8"):
+        from . import native_quant as Q
         ys = torch.empty(max_rows, H, dtype=torch.float32, device=dev)
-        N._check(lib.xft_qgemm_grouped(N._p(xs), H, max_rows, N._p(pk["gu"]), E * 2 * I, H, N._p(h1), I, 0, I, H, 1, I, 2 * I,
-                                       N._p(pk["gus"]), pk["gus"].shape[1], N._p(tiles), N._p(meta), max_tiles, min(bn, 128),
-                                       N._p(None), N._ACT[act], N._p(ws.status), N._stream()), "grouped fp8 gate_up")
-        N._check(lib.xft_qgemm_grouped(N._p(h1), I, max_rows, N._p(pk["dn"]), E * H, I, N._p(ys), H, 1, H, I, 0, 0, H,
-                                       N._p(pk["dns"]), pk["dns"].shape[1], N._p(tiles), N._p(meta), max_tiles, min(bn, 128),
-                                       N._p(row_w), 0, N._p(ws.status), N._stream()), "grouped fp8 down")
+        Q.gemm_e4m3(Q.split_e4m3(x2, ldx, src=src, rows_used=meta[1:], rows=max_rows), pk["gu"], H, 0, h1, max_rows, I, H, True, I,
+                    pk["gus"], None, pk["gus"].shape[1], act=act, tiles=tiles, n_tiles=meta, group_rows=2 * I, max_tiles=max_tiles, bn=bn)
+        Q.gemm_e4m3(Q.split_e4m3(h1, I, rows_used=meta[1:]), pk["dn"], I, 0, ys, max_rows, H, I, False, 0, pk["dns"], None,
+                    pk["dns"].shape[1], tiles=tiles, n_tiles=meta, group_rows=H, max_tiles=max_tiles, bn=bn, col_scale=row_w)
         out = torch.empty(T, H, dtype=torch.float32, device=dev)
         N._check(lib.xft_moe_combine(N._p(ys), N._p(pos), k, N._p(add32), N._p(add16), H, N._p(None), N._p(out), T, H,
                                  N._stream()), "moe_combine")
-        ws.launches += 5
+        ws.launches += 2
         return out
+    xs = torch.empty(max_rows, H, dtype=torch.bfloat16, device=dev)
+    N._check(lib.xft_moe_gather(N._p(x2), ldx, N._p(src), N._p(meta), N._p(xs), max_rows, H, N._stream()), "moe_gather")
     if bn >= 128:
         # prompt sizes: the token-major persistent kernel; rows stay bf16 until the weighted sum
         y16 = torch.empty(max_rows, H, dtype=torch.bfloat16, device=dev)

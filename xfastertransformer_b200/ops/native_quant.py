@@ -1,5 +1,6 @@
-"""Bindings of the quantised GEMM kernels (csrc/kernels/quant_gemm_sm100.cu): weight-only int8 / uint4 / nf4 /
-fp8-e4m3 dequant-GEMM and W8A8 (dynamic int8 activations x int8 weights on the int8 tensor path)."""
+"""Bindings of the quantised GEMM kernels: weight-only int8 / nf4 dequant-GEMM and W8A8 (dynamic int8 activations x int8 weights
+on the int8 tensor path) in csrc/kernels/quant_gemm_sm100.cu, fp8-e4m3 and uint4 weights on the fp8 tensor path in
+csrc/kernels/gemm_e4m3_sm100.cu."""
 from __future__ import annotations
 
 import ctypes as C
@@ -8,7 +9,8 @@ import torch
 
 from . import native as N
 
-_QT = {"int8": 0, "int4": 1, "nf4": 2, "fp8": 3, "int4f": 4}
+_QT = {"int8": 0, "nf4": 2}
+_E4M3 = {"fp8": 0, "int4": 1}             # weights that e4m3 holds: csrc/kernels/gemm_e4m3_sm100.cu
 _ready = False
 
 
@@ -16,7 +18,8 @@ def _lib():
     global _ready
     lib = N.lib()
     if not _ready:
-        for fn in ("xft_qgemm", "xft_quant_act", "xft_row_sum", "xft_w8a8_gemm"):
+        for fn in ("xft_qgemm", "xft_quant_act", "xft_row_sum", "xft_w8a8_gemm", "xft_split_e4m3", "xft_split_e4m3_cols",
+                   "xft_gemm_e4m3", "xft_w8a8_gemm_gated"):
             getattr(lib, fn).restype = C.c_int
         _ready = True
     return lib
@@ -30,23 +33,29 @@ def _row_sums(x2, ldx):
     return out
 
 
-def _int4_fast(W, w):
-    """uint4 weights in the kernel's fast layout (cached on the weight): within every 32-bit word the eight codes
-    e0..e7 move from nibble order [e0 e1 ... e7] to [e0 e2 e4 e6 | e1 e3 e5 e7], which lets the kernel build a bf16
-    pair with one shift and one logic op; and the zero point absorbs the constant 128 the kernel adds to each code."""
-    c = W.cache.get("int4f")
-    if c is None:
-        w32 = w.contiguous().view(torch.int32).to(torch.int64) & 0xFFFFFFFF
-        out = torch.zeros_like(w32)
-        for i in range(4):
-            out |= ((w32 >> (8 * i)) & 0xF) << (4 * i)                 # e_{2i}   -> nibble i
-            out |= ((w32 >> (8 * i + 4)) & 0xF) << (16 + 4 * i)        # e_{2i+1} -> nibble i + 4
-        out = torch.where(out >= 2 ** 31, out - 2 ** 32, out).to(torch.int32)
-        wf = out.view(torch.uint8).view(w.shape[0], -1)
-        zero = (W.zero if W.zero is not None else torch.zeros_like(W.scale)) - 128.0 * W.scale
-        c = (wf, zero.contiguous())
-        W.cache["int4f"] = c
-    return c
+def split_e4m3(x2, ldx, nibbles=False, want_sum=False, src=None, rows_used=None, rows=None):
+    """Rows of x2 (or rows `src` of it) as sums of two e4m3 numbers -> (uint8 [rows, 2 * cols], scale [rows], sum [rows] or
+    None).  `nibbles`: in the order in which 4-bit codes expand.  `rows_used`: device count; later rows stay unwritten."""
+    T, K = x2.shape
+    rows = T if rows is None else rows
+    xs = torch.empty(rows, 2 * _lib().xft_split_e4m3_cols(K), dtype=torch.uint8, device=x2.device)
+    st = torch.empty(2, rows, dtype=torch.float32, device=x2.device)
+    N._check(_lib().xft_split_e4m3(N._p(x2), ldx, N._p(src), N._p(rows_used), rows, K, int(nibbles), N._p(xs), N._p(st[0]),
+                                   N._p(st[1] if want_sum else None), N._stream()), "split_e4m3")
+    N.Workspace.get(x2.device).launches += 1
+    return xs, st[0], st[1] if want_sum else None
+
+
+def gemm_e4m3(split, w, pitch, src, out, T, n_out, K, gated, dual_off, scale, zero, scale_ld, bias=None, r2=None, ldr=0, res_scale=1.0,
+              act=None, tiles=None, n_tiles=None, group_rows=0, max_tiles=0, bn=0, col_scale=None):
+    xs, xscale, xsum = split
+    ws = N.Workspace.get(xs.device)
+    rc = _lib().xft_gemm_e4m3(N._p(xs), xs.shape[0], N._p(xscale), N._p(xsum), N._p(w), w.shape[0], pitch, src, N._p(out), out.stride(0),
+                              int(out.dtype == torch.float32), T, n_out, K, int(gated), dual_off, N._p(scale), N._p(zero), scale_ld,
+                              N._p(bias), N._p(r2), ldr, C.c_float(res_scale), N._ACT[act], N._p(tiles), N._p(n_tiles), group_rows,
+                              max_tiles, bn, N._p(col_scale), N._p(ws.status), N._stream())
+    N._check(rc, "gemm_e4m3")
+    ws.launches += 1
 
 
 def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype):
@@ -57,8 +66,6 @@ def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype):
     fp32 = out_dtype == torch.float32
     out = torch.empty(T, n_out, dtype=torch.float32 if fp32 else torch.bfloat16, device=x.device)
     ws = N.Workspace.get(x.device)
-    zero = W.zero if (W.zero is not None and W.kind != "nf4") else None
-    xsum = _row_sums(x2, ldx) if zero is not None else None
     r2, ldr = (None, 0)
     if residual is not None:
         r2 = residual.reshape(-1, residual.shape[-1])
@@ -74,19 +81,22 @@ def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype):
             wp = torch.nn.functional.pad(w, (0, pad)).contiguous()[:, :cols]
             W.cache["w_pitch16"] = wp
         w = wp
-    scale_ld = W.scale.shape[1] if W.kind == "fp8" else 0
-    kind = W.kind
-    if kind == "int4":
-        cols = w.shape[1]
-        full = w if w.is_contiguous() else torch.as_strided(w, (w.shape[0], w.stride(0)), (w.stride(0), 1))
-        wq, zero = _int4_fast(W, full)
-        w = wq[:, :cols]
-        kind = "int4f"
-        if xsum is None:
-            xsum = _row_sums(x2, ldx)
-    rc = _lib().xft_qgemm(N._p(x2), ldx, N._p(w), w.shape[0], w.stride(0) * w.element_size(), _QT[kind], N._p(out),
+    zero = W.zero
+    if W.kind in _E4M3:
+        codes = W.kind == "int4"
+        if codes and zero is None:
+            zero = W.cache.get("zero0")
+            if zero is None:
+                zero = W.cache["zero0"] = torch.zeros_like(W.scale)
+        gemm_e4m3(split_e4m3(x2, ldx, codes, codes), w, w.stride(0), _E4M3[W.kind], out, T, n_out, K, gated, n_out if gated else 0,
+                  W.scale, zero if codes else None, 0 if codes else W.scale.shape[1], bias, r2, ldr, res_scale, act)
+        return out
+    if W.kind == "nf4":
+        zero = None
+    xsum = _row_sums(x2, ldx) if zero is not None else None
+    rc = _lib().xft_qgemm(N._p(x2), ldx, N._p(w), w.shape[0], w.stride(0) * w.element_size(), _QT[W.kind], N._p(out),
                           out.stride(0), int(fp32), T, n_out, K, int(gated), n_out if gated else 0, N._p(W.scale),
-                          N._p(zero), N._p(xsum), scale_ld, N._p(bias), N._p(r2), ldr, C.c_float(res_scale),
+                          N._p(zero), N._p(xsum), 0, N._p(bias), N._p(r2), ldr, C.c_float(res_scale),
                           N._ACT[act], N._p(ws.ws), C.c_size_t(ws.ws_bytes), N._p(ws.counters), ws.n_counters,
                           N._p(ws.status), N._stream())
     N._check(rc, f"qgemm[{W.kind}]")
@@ -155,7 +165,7 @@ def _w8a8(x, W, rows, bias, act, residual, res_scale, out_dtype, row0=0):
 def linear(x, W, bias=None, act=None, residual=None, res_scale=1.0, out_dtype=None):
     if W.kind == "w8a8":
         return _w8a8(x, W, W.out_features, bias, act, residual, res_scale, out_dtype)
-    if W.kind in _QT:
+    if W.kind in _QT or W.kind in _E4M3:
         return _qgemm(x, W, W.out_features, False, bias, act, residual, res_scale, out_dtype)
     raise N.KernelError(f"no sm_100a GEMM for weight kind {W.kind}")
 
@@ -163,9 +173,16 @@ def linear(x, W, bias=None, act=None, residual=None, res_scale=1.0, out_dtype=No
 def linear_gated(x, W, act="silu", bias=None):
     I = W.out_features // 2
     if W.kind == "w8a8":
-        # one int8 GEMM over both halves (activations are quantised once), then act(gate)*up
-        gu = _w8a8(x, W, 2 * I, bias, None, None, 1.0, None)
-        return N.gated_act(gu, act)
+        x2, ldx = N._rows2d(x)
+        T, K = x2.shape
+        q, sa, za, qs = quant_act(x2, ldx)
+        out = torch.empty(T, I, dtype=torch.bfloat16, device=x.device)
+        ws = N.Workspace.get(x.device)
+        N._check(_lib().xft_w8a8_gemm_gated(N._p(q), K, N._p(W.w), W.w.stride(0), N._p(out), I, T, I, K, I, N._p(sa), N._p(za), N._p(qs),
+                                            N._p(W.scale), N._p(W.zero), N._p(W.wsum), N._p(bias), N._ACT[act], N._p(ws.status),
+                                            N._stream()), "w8a8_gemm_gated")
+        ws.launches += 1
+        return out
     if W.kind == "fp8" and I % 128:
         gu = _qgemm(x, W, 2 * I, False, bias, None, None, 1.0, None)
         return N.gated_act(gu, act)
