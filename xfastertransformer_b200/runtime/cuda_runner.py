@@ -131,13 +131,14 @@ class CudaRunner:
 
     def _logits_key(self, seqs: Sequence):
         """Like `_key`, but the table is as wide as the contexts of this step, rounded up to a power of two (from 8 blocks on):
-        callers of `forward_cb` need not say how long their sequences get, and a step planned for the longest possible
-        context would cut short ones into too many parts."""
+        callers of `forward_cb` need not say how long their sequences get.  The split count of the attention is that of an
+        eager step, so that a sequence's logits do not depend on whether its steps were captured."""
         B, limit = self._key(seqs)
-        need, W = max(self.m.cache.blocks_for(s.past_len + 1) for s in seqs), 8
+        longest = max(s.past_len for s in seqs) + 1
+        need, W = self.m.cache.blocks_for(longest), 8
         while W < need:
             W *= 2
-        return B, max(min(W, limit), need), "logits"
+        return B, max(min(W, limit), need), "logits", self.m.decoder.plan_splits(len(seqs), longest, self.m.cache.int8)
 
     def worth_capturing(self, seqs: Sequence, key=None) -> bool:
         """For callers whose batch composition changes from step to step (serving): a shape is captured only when
@@ -159,7 +160,7 @@ class CudaRunner:
         o_bt = (o_bt + 3) // 4 * 4
         return o_ids, o_pos, o_slot, o_kv, o_st, o_cu, o_bt, o_bt + B * W
 
-    def _build(self, B: int, W: int, max_kv_hint: int) -> _Graph:
+    def _build(self, B: int, W: int, max_kv_hint: int, nsplit=None) -> _Graph:
         m = self.m
         g = _Graph()
         g.B, g.W = B, W
@@ -171,7 +172,7 @@ class CudaRunner:
         g.host[o_cu:o_cu + B + 1] = torch.arange(B + 1, dtype=torch.int32)
         d = g.dev
         dec = m.decoder
-        g.nsplit = dec.plan_splits(B, max_kv_hint, m.cache.int8)
+        g.nsplit = nsplit or dec.plan_splits(B, max_kv_hint, m.cache.int8)
         b = Batch(ids=d[o_ids:o_ids + B], positions=d[o_pos:o_pos + B], slots=d[o_slot:o_slot + B],
                   cu_q=list(range(B + 1)), kv_lens=[max_kv_hint] * B, block_table=d[o_bt:o_bt + B * W].view(B, W),
                   logit_rows=None, is_decode=True, max_q=1, max_kv=max_kv_hint)
@@ -344,7 +345,7 @@ class CudaRunner:
         B, W = key[:2]
         g = self.graphs.get(key)
         if g is None or g.version != m.cache.version:
-            g = self._build(B, W, W * m.cache.block)
+            g = self._build(B, W, W * m.cache.block, key[3])
             g.ring = [(g.host if i == 0 else g.host.clone().pin_memory(), torch.cuda.Event()) for i in range(self.RING)]
             g.turn = 0
             self.graphs[key] = g
