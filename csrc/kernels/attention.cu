@@ -140,6 +140,33 @@ __device__ __forceinline__ void load_tile_int8(bf16* tile, const int8_t* g, int 
   }
 }
 
+// The two halves of load_tile_int8 for one warp: the codes of a tile into registers, and from there into the tile.  A decode warp asks
+// for its next tile before it computes with this one.
+template <int HD, int KT>
+struct RawTile {
+  static constexpr int CPR = HD / 16, N = KT * CPR / 32;
+  uint4 raw[N];
+  __device__ __forceinline__ void load(const int8_t* g, int valid, int lane) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int r = (lane + 32 * i) / CPR, c = (lane + 32 * i) % CPR;
+      raw[i] = r < valid ? *reinterpret_cast<const uint4*>(g + (long long)r * HD + c * 16) : make_uint4(0, 0, 0, 0);
+    }
+  }
+  __device__ __forceinline__ void store(bf16* tile, int lane) const {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int r = (lane + 32 * i) / CPR, c = (lane + 32 * i) % CPR;
+      const int8_t* b = reinterpret_cast<const int8_t*>(&raw[i]);
+      uint32_t w[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = pack_bf16((float)b[2 * j], (float)b[2 * j + 1]);
+      *reinterpret_cast<uint4*>(tile_ptr<HD>(tile, r, 2 * c)) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(tile_ptr<HD>(tile, r, 2 * c + 1)) = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+  }
+};
+
 // One warp: 16 query rows (A fragments re-read from the swizzled Q tile) against a KT-key tile.
 // Updates the running max m[2], sum l[2] and O accumulator (two rows per thread: lane/4 and lane/4+8).
 template <int HD, int KT, bool KV_TMA = false, int TROWS = KT, bool EXT = false>
@@ -519,12 +546,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const AttnParams p) {
       if (blk < 0 || blk >= p.num_blocks) { if (lane == 0 && p.status) atomicCAS(p.status, 0, XFT_ERR_BOUNDS); blk = 0; }
       const size_t row0 = ((size_t)blk * p.hkv + kvh) * p.bs + (ti % tiles_per_block) * KT;
       const int valid = min(KT, kv_len - ti * KT);
-      if (INT8) {
-        load_tile_int8<HD, 32>(kt, reinterpret_cast<const int8_t*>(p.kc) + row0 * HD, KT, valid, lane);
-        for (int i = lane; i < KT; i += 32) ksc[i] = i < valid ? p.ks[row0 + i] : 0.f;
-      } else {
-        load_tile_bf16<HD, 32>(kt, reinterpret_cast<const bf16*>(p.kc) + row0 * HD, HD, KT, valid, lane);
-      }
+      load_tile_bf16<HD, 32>(kt, reinterpret_cast<const bf16*>(p.kc) + row0 * HD, HD, KT, valid, lane);
     }
     cp_async_commit();
   };
@@ -535,12 +557,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const AttnParams p) {
       if (blk < 0 || blk >= p.num_blocks) blk = 0;
       const size_t row0 = ((size_t)blk * p.hkv + kvh) * p.bs + (ti % tiles_per_block) * KT;
       const int valid = min(KT, kv_len - ti * KT);
-      if (INT8) {
-        load_tile_int8<HD, 32>(vt, reinterpret_cast<const int8_t*>(p.vc) + row0 * HD, KT, valid, lane);
-        for (int i = lane; i < KT; i += 32) vsc[i] = i < valid ? p.vs[row0 + i] : 0.f;
-      } else {
-        load_tile_bf16<HD, 32>(vt, reinterpret_cast<const bf16*>(p.vc) + row0 * HD, HD, KT, valid, lane);
-      }
+      load_tile_bf16<HD, 32>(vt, reinterpret_cast<const bf16*>(p.vc) + row0 * HD, HD, KT, valid, lane);
     }
     cp_async_commit();
   };
@@ -559,8 +576,43 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const AttnParams p) {
   const float slope0 = (use_alibi && r0 < nq) ? p.slopes[h_lo + r0] : 0.f;
   const float slope1 = (use_alibi && r1 < nq) ? p.slopes[h_lo + r1] : 0.f;
 
-  // Per warp: the V tile streams in while S is computed, the next K tile while P V is computed.
   int ti = t_begin + warp;
+  if constexpr (INT8) {
+    // Codes and scales of a tile are asked for one tile ahead: with the loads in front of their use a warp spent most of its time
+    // waiting (32 sequences of 2250 keys, 32 / 8 heads of 128: 164 us, 79 us so; of 256: 283 and 154 us).
+    constexpr int SC = (KT + 31) / 32;
+    RawTile<HD, KT> rk, rv;
+    float fk[SC], fv[SC];
+    auto fetch = [&](int n) {
+      if (n >= t_end) return;
+      const int t = tiles.at(n);
+      int blk = bt[t / tiles_per_block];
+      if (blk < 0 || blk >= p.num_blocks) { if (lane == 0 && p.status) atomicCAS(p.status, 0, XFT_ERR_BOUNDS); blk = 0; }
+      const size_t row0 = ((size_t)blk * p.hkv + kvh) * p.bs + (t % tiles_per_block) * KT;
+      const int valid = min(KT, kv_len - t * KT);
+      rk.load(reinterpret_cast<const int8_t*>(p.kc) + row0 * HD, valid, lane);
+      rv.load(reinterpret_cast<const int8_t*>(p.vc) + row0 * HD, valid, lane);
+#pragma unroll
+      for (int i = 0; i < SC; ++i) {
+        const int k = lane + 32 * i;
+        fk[i] = k < valid ? p.ks[row0 + k] : 0.f;
+        fv[i] = k < valid ? p.vs[row0 + k] : 0.f;
+      }
+    };
+    fetch(ti);
+    for (; ti < t_end; ti += 4) {
+      __syncwarp();                                        // the previous tile has been read
+      rk.store(kt, lane);
+      rv.store(vt, lane);
+#pragma unroll
+      for (int i = 0; i < SC; ++i)
+        if (lane + 32 * i < KT) { ksc[lane + 32 * i] = fk[i]; vsc[lane + 32 * i] = fv[i]; }
+      fetch(ti + 4);
+      __syncwarp();
+      wa.step(qs, kt, vt, tiles.at(ti) * KT, kv_len, qpos0, qpos1, p.scale, slope0, slope1, use_alibi, 0, ksc, vsc, lane, p);
+    }
+  } else {
+  // Per warp: the V tile streams in while S is computed, the next K tile while P V is computed.
   issue_k(ti);
   issue_v(ti);
   for (; ti < t_end; ti += 4) {
@@ -568,7 +620,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const AttnParams p) {
     cp_async_wait<1>();          // K(ti) landed (V(ti) may still be in flight)
     __syncwarp();
     wa.scores(s, qs, kt, tiles.at(ti) * KT, kv_len, qpos0, qpos1, p.scale, slope0, slope1, use_alibi, 0,
-              INT8 ? ksc : nullptr, INT8 ? vsc : nullptr, lane, p);
+              nullptr, nullptr, lane, p);
     __syncwarp();
     issue_k(ti + 4);             // K buffer is free again
     cp_async_wait<1>();          // V(ti) landed
@@ -576,6 +628,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const AttnParams p) {
     wa.pv(s, vt, lane);
     __syncwarp();
     issue_v(ti + 4);
+  }
   }
   cp_async_wait<0>();
   wa.reduce_l();

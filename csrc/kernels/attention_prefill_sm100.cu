@@ -45,6 +45,10 @@ struct PrefillAttnParams {
   int window, keep;           // keys within `window` positions and the first `keep` are visible (window 2^30: all)
   const float* sinks;         // [hq] or null
   int num_blocks;
+  // INT8 only: the scales of the int8 cache [num_blocks, hkv, bs]; the K / V tiles come from a copy of the codes in bf16, where
+  // block j of sequence b is at b * copy_w + j
+  const float* ks; const float* vs;
+  int copy_w;
   int* status;
 };
 
@@ -72,7 +76,10 @@ __device__ __forceinline__ float capped_log2_small(const PrefillAttnParams& p, f
   return z * p.cap_log2 * q;
 }
 
-template <bool EXT>
+// INT8: K and V are the codes of an int8 cache (exact in bf16); a key's scale multiplies its score and its weight in fp32, as in the
+// kernel for other head sizes (attention.cu).  3 prompts of 2250 tokens, 32 / 8 heads: 1308 us there, 600 us here with the
+// copy of the codes.
+template <bool EXT, bool INT8 = false>
 __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ,
                                                                  const __grid_constant__ CUtensorMap tmK,
                                                                  const __grid_constant__ CUtensorMap tmV,
@@ -151,6 +158,7 @@ __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_co
         for (int i = 0; i < 2; ++i) {
           int blk = bt[min(2 * tile_of(j) + i, n_blocks - 1)];
           if (blk < 0 || blk >= p.num_blocks) { bad = true; blk = 0; }
+          if (INT8) blk = b * p.copy_w + min(2 * tile_of(j) + i, n_blocks - 1);
           rowk[i] = (blk * p.hkv + kvh) * p.bs;
         }
         if (bad && p.status) atomicCAS(p.status, 0, XFT_ERR_BOUNDS);
@@ -234,6 +242,31 @@ __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_co
       // EXT: of these, the ones from k0 + first on and the ones below k0 + kept
       const int first = EXT ? qpos - p.window + 1 - k0 : 0, kept = EXT ? p.keep - k0 : 0;
       auto visible = [&](int i) { return i < nvalid && (!EXT || i >= first || i < kept); };
+      // scales of the tile's keys: the same 16 bytes for all threads of a warp
+      const float4 *ks_a = nullptr, *ks_b = nullptr, *vs_a = nullptr, *vs_b = nullptr;      // of the tile's two blocks
+      if constexpr (INT8) {
+        const int* bt = p.block_table + (size_t)b * p.bt_stride;
+        const int last = (kv_len + p.bs - 1) / p.bs - 1;
+        auto at = [&](int i) {
+          const int blk = bt[min(2 * tile_of(j) + i, last)];
+          return ((size_t)(blk < 0 || blk >= p.num_blocks ? 0 : blk) * p.hkv + kvh) * p.bs;      // a bad one is reported by the producer
+        };
+        const size_t a0 = at(0), a1 = at(1);
+        ks_a = reinterpret_cast<const float4*>(p.ks + a0); ks_b = reinterpret_cast<const float4*>(p.ks + a1);
+        vs_a = reinterpret_cast<const float4*>(p.vs + a0); vs_b = reinterpret_cast<const float4*>(p.vs + a1);
+      }
+      auto scaled = [&](uint32_t (&v)[32], int c) {                    // raw scores of keys [c, c + 32)
+        if constexpr (INT8) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 f = __ldg((c < 64 ? ks_a : ks_b) + ((c & 63) >> 2) + i);
+            v[4 * i] = __float_as_uint(__uint_as_float(v[4 * i]) * f.x);
+            v[4 * i + 1] = __float_as_uint(__uint_as_float(v[4 * i + 1]) * f.y);
+            v[4 * i + 2] = __float_as_uint(__uint_as_float(v[4 * i + 2]) * f.z);
+            v[4 * i + 3] = __float_as_uint(__uint_as_float(v[4 * i + 3]) * f.w);
+          }
+        }
+      };
       // pass 1: row maximum of the visible scores
       float mx = EXT ? -INFINITY : m;
       float big = 0.f;                                       // EXT: largest |raw score| of the row
@@ -252,6 +285,7 @@ __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_co
         uint32_t v[32];
         tmem_ld32(sa + c, v);
         tmem_ld_wait();
+        scaled(v, c);
         if (EXT && (whole >> (c >> 5) & 1)) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -287,6 +321,7 @@ __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_co
           uint32_t v[32];
           tmem_ld32(sa + c, v);
           tmem_ld_wait();
+          scaled(v, c);
           auto store = [&](auto seen) {
 #pragma unroll
             for (int g8 = 0; g8 < 4; ++g8) {
@@ -296,9 +331,16 @@ __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_co
                 const int e = g8 * 8 + 2 * i;
                 const float p0 = seen(c + e) ? exp2f(score(__uint_as_float(v[e])) - m) : 0.f;
                 const float p1 = seen(c + e + 1) ? exp2f(score(__uint_as_float(v[e + 1])) - m) : 0.f;
-                const __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
-                // the sum uses the rounded values, as the product does
-                sum += __low2float(pb) + __high2float(pb);
+                __nv_bfloat162 pb;
+                if constexpr (INT8) {                                  // the value's scale belongs to the product, not to the sum
+                  const float2 f = __ldg(reinterpret_cast<const float2*>(c < 64 ? vs_a : vs_b) + ((c & 63) >> 1) + g8 * 4 + i);
+                  pb = __floats2bfloat162_rn(p0 * f.x, p1 * f.y);
+                  sum += p0 + p1;
+                } else {
+                  pb = __floats2bfloat162_rn(p0, p1);
+                  // the sum uses the rounded values, as the product does
+                  sum += __low2float(pb) + __high2float(pb);
+                }
                 w[i] = *reinterpret_cast<const uint32_t*>(&pb);
               }
               *reinterpret_cast<uint4*>(prow + (((chunk0 + g8) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -359,6 +401,37 @@ __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_co
   }
 }
 
+// Codes of an int8 cache as bf16: block j, head h of sequence b -> copy[(b * w + j) * hkv + h], keys and values.
+__global__ void __launch_bounds__(256) expand_codes_kernel(const int8_t* __restrict__ kc, const int8_t* __restrict__ vc,
+                                                           __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ v,
+                                                           const int* __restrict__ block_table, int bt_stride,
+                                                           const int* __restrict__ kv_lens, int hkv, int num_blocks, int* status) {
+  const int j = blockIdx.x, h = blockIdx.y, b = blockIdx.z, w = gridDim.x;
+  grid_dep_launch();
+  grid_dep_wait();
+  if (j * 64 >= kv_lens[b]) return;
+  int blk = block_table[(size_t)b * bt_stride + j];
+  if (blk < 0 || blk >= num_blocks) { if (threadIdx.x == 0 && status) atomicCAS(status, 0, XFT_ERR_BOUNDS); blk = 0; }
+  const size_t from = ((size_t)blk * hkv + h) * 8192, to = ((size_t)(b * w + j) * hkv + h) * 8192;
+  uint4 raw[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)                                          // 16 codes each: two of K, two of V
+    raw[i] = *reinterpret_cast<const uint4*>((i < 2 ? kc : vc) + from + (threadIdx.x + 256 * (i & 1)) * 16);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int8_t* c = reinterpret_cast<const int8_t*>(&raw[i]);
+    uint32_t o[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const __nv_bfloat162 x = __floats2bfloat162_rn((float)c[2 * e], (float)c[2 * e + 1]);
+      o[e] = *reinterpret_cast<const uint32_t*>(&x);
+    }
+    uint4* dst = reinterpret_cast<uint4*>((i < 2 ? k : v) + to + (threadIdx.x + 256 * (i & 1)) * 16);
+    dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+    dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+  }
+}
+
 }  // namespace xft
 
 using namespace xft;
@@ -397,5 +470,38 @@ extern "C" int xft_attn_prefill_tc(const void* q, void* out, const void* kc, con
   dim3 grid((max_q + kPfQ - 1) / kPfQ, hq, B);
   cudaError_t e = launch_pdl(ext ? attn_prefill_tc_kernel<true> : attn_prefill_tc_kernel<false>, grid, dim3(192),
                              (size_t)kPfSmem, st, tmQ, tmK, tmV, p);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+// The same over an int8 cache with one scale per key and head; copy: bf16 [2, B * copy_w, hkv, 64, 128] for the codes, copy_w blocks
+// (at least kv_len / 64 of the longest sequence) each.
+extern "C" int xft_attn_prefill_tc_int8(const void* q, void* out, const void* kc, const void* vc, const float* ks, const float* vs,
+                                        void* copy, int copy_w, const int* block_table, int bt_stride, const int* cu_q,
+                                        const int* kv_lens, int B, int T, int max_q, int hq, int hkv, int group, int q_off, int bs,
+                                        int num_blocks, float scale, int* status, cudaStream_t st) {
+  if (B <= 0 || T <= 0 || max_q <= 0) return 0;
+  if (bs != 64 || hq <= 0 || hkv <= 0 || copy_w <= 0 || ((reinterpret_cast<uintptr_t>(ks) | reinterpret_cast<uintptr_t>(vs)) & 15)) return -1;
+  PrefillAttnParams p{};
+  p.out = (__nv_bfloat16*)out; p.block_table = block_table; p.bt_stride = bt_stride; p.cu_q = cu_q; p.kv_lens = kv_lens;
+  p.hq = hq; p.hkv = hkv; p.group = group; p.q_off = q_off; p.bs = bs; p.scale_log2 = scale * 1.4426950408889634f;
+  p.num_blocks = num_blocks; p.status = status; p.window = 1 << 30; p.ks = ks; p.vs = vs; p.copy_w = copy_w;
+  __nv_bfloat16* k = (__nv_bfloat16*)copy;
+  const uint64_t rows = (uint64_t)B * copy_w * hkv * bs;
+  __nv_bfloat16* v = k + rows * 128;
+  CUtensorMap tmQ, tmK, tmV;
+  int r = make_tensor_map(&tmQ, q, (uint64_t)T, (uint64_t)hq * 128, (uint64_t)hq * 128, 128, 2);
+  if (r) return 1000 - r;
+  if (make_tensor_map(&tmK, k, rows, 128, 128, 64, 2) || make_tensor_map(&tmV, v, rows, 128, 128, 64, 2)) return -4;
+  const auto kernel = attn_prefill_tc_kernel<false, true>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem) != cudaSuccess)
+      return 3000 + (int)cudaGetLastError();
+    attr_set = true;
+  }
+  cudaError_t e = launch_pdl(expand_codes_kernel, dim3(copy_w, hkv, B), dim3(256), 0, st, (const int8_t*)kc, (const int8_t*)vc, k, v,
+                             block_table, bt_stride, kv_lens, hkv, num_blocks, status);
+  if (e != cudaSuccess) return (int)e;
+  e = launch_pdl(kernel, dim3((max_q + kPfQ - 1) / kPfQ, hq, B), dim3(192), (size_t)kPfSmem, st, tmQ, tmK, tmV, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }

@@ -581,17 +581,25 @@ def mla_prep(q, kv, Hl, nope, rope, kvl, positions, table, kv_norm_w, eps, cache
 
 def plan_attn_splits(B, hkv, group, D, max_kv, int8=False, least=8):
     """Split-KV factor of a decode launch and the tile count it was planned on: fill the resident CTA slots (two
-    CTAs per SM for the TMA-ring kernel of bf16 caches, three for the cp.async kernel of int8 caches) while leaving
+    CTAs per SM for the TMA-ring kernel of bf16 caches and for int8 caches, three for the cp.async kernel) while leaving
     every slice at least `least` tiles."""
     tma = not int8 and _ENV().attn_tma
     kt = 64 if tma else {64: 64, 128: 32, 256: 16}[D]
-    slots = (296 if D <= 128 else 148) if tma else 444
+    slots = (296 if D <= 128 else 148) if tma else 296 if int8 else 444
     ntiles = (max_kv + kt - 1) // kt
     ctas = B * max(hkv, 1) * ((group + 15) // 16)
     nsplit = max(1, min(slots // max(ctas, 1), ntiles // least if ntiles >= 16 else 1, 32))
     if _ENV().attn_splits > 0:
         nsplit = max(1, min(_ENV().attn_splits, ntiles, 32))
     return nsplit, ntiles
+
+
+# Prompts over an int8 cache: from this many new tokens on a copy of the codes in bf16 pays for itself (it is five bytes of traffic
+# per code, the kernel without it reads each code once per 64 query rows and head), as long as the copy stays below a bound.
+# Short contexts are all launch: 100 tokens 21 us without the copy, 27 us with it; 3 x 2250 tokens 1308 and 600 us.
+INT8_TC_MIN_Q = 64
+INT8_TC_MIN_KV = 512
+INT8_TC_MAX_COPY = 1 << 30
 
 
 def paged_attention(q, kc, vc, block_table, cu_q, kv_lens, scale, ks=None, vs=None, slopes=None, causal=True,
@@ -649,6 +657,17 @@ def paged_attention(q, kc, vc, block_table, cu_q, kv_lens, scale, ks=None, vs=No
         _check(rc, "attn_prefill_tc")
         ws.launches += 1
         return out
+    if (not decode and D == 128 and bs == 64 and ks is not None and slopes is None and pl is None and softcap == 0 and window == 0
+            and sinks is None and max_q >= INT8_TC_MIN_Q and max_kv >= INT8_TC_MIN_KV):
+        w = (max_kv + 63) // 64
+        if B * w * hkv * 2 * 64 * 128 * 2 <= INT8_TC_MAX_COPY:
+            copy = torch.empty(2, B * w, hkv, 64, 128, dtype=torch.bfloat16, device=dev)
+            fn = lib().xft_attn_prefill_tc_int8
+            fn.restype = C.c_int
+            _check(fn(_p(q), _p(out), _p(kc), _p(vc), _p(ks), _p(vs), _p(copy), w, _p(block_table), block_table.stride(0), _p(cu_dev),
+                      _p(kv_dev), B, T, max_q, hq, hkv, g, q_off, bs, nb, C.c_float(scale), _p(ws.status), _stream()), "attn_prefill_tc_int8")
+            ws.launches += 2
+            return out
     rc = lib().xft_paged_attention_ext(_p(q), _p(out), _p(kc), _p(vc), _p(ks), _p(vs), _p(block_table),
                                        block_table.stride(0), _p(cu_dev), _p(kv_dev), B, max_q, hq, hkv, g, q_off, D, bs,
                                        nb, C.c_float(scale), _p(slopes), _p(pl),
