@@ -18,14 +18,14 @@ def _lib():
     lib = N.lib()
     if not _ready:
         lib.xft_mla_attention_ext.restype = C.c_int
-        lib.xft_gemm_bf16_grouped.restype = C.c_int
+        lib.xft_gemm_bf16_grouped.restype = lib.xft_gemm_bf16_grouped_tm.restype = C.c_int
         _ready = True
     return lib
 
 
 def _head_tiles(H: int, T: int, dev):
     """Static tile table of a per-head grouped GEMM: rows of head h are [h*T, (h+1)*T)."""
-    bn = 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128
+    bn = 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128 if T < 512 else 256
     key = (H, T, bn, dev.index)
     if key not in _tables:
         rows = []
@@ -43,6 +43,13 @@ def _per_head_gemm(x_ht, w_stacked, H, T, n_out, k_in):
     tiles, meta, nt, bn = _head_tiles(H, T, x_ht.device)
     out = torch.empty(H * T, n_out, dtype=torch.bfloat16, device=x_ht.device)
     ws = N.Workspace.get(x_ht.device)
+    if bn >= 128:
+        # prompts: the token-major kernel (3000 tokens, 128 heads of 512 x 128: 1980 us with the kernel of the decode steps)
+        N._check(_lib().xft_gemm_bf16_grouped_tm(N._p(x_ht), k_in, H * T, N._p(w_stacked), H * n_out, k_in, N._p(out), n_out, n_out, k_in,
+                                                 0, 0, n_out, N._p(tiles), N._p(meta), nt, bn, 0, N._p(ws.status), N._stream()),
+                 "per-head grouped gemm")
+        ws.launches += 1
+        return out
     rc = _lib().xft_gemm_bf16_grouped(N._p(x_ht), k_in, H * T, N._p(w_stacked), H * n_out, k_in, N._p(out), n_out, 0,
                                       n_out, k_in, 0, 0, n_out, N._p(tiles), N._p(meta), nt, bn, N._p(None), 0,
                                       N._p(ws.status), N._stream())

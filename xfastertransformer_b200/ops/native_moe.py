@@ -150,9 +150,11 @@ def moe_experts(x, idx, w, experts, act="silu", expert_offset=0, packed=None, ex
     ws = N.Workspace.get(dev)
     lib = _lib()
     avg = max(1, ((T * k if expected_pairs is None else min(int(expected_pairs), T * k)) + E - 1) // E)
+    # An expert with more rows than a tile reads its weights twice, so tiles are about twice the average (64 rows on 8 experts, two
+    # each: 4096 x 14336 210 us with 16 rows, 180 with 32).
     # 256 rows: two CTAs share a tile (bf16 only).  A group's last tile is half empty on average, which eats the fifth that
     # pairs gain below about 430 rows per expert
-    bn = 16 if avg <= 16 else 32 if avg <= 32 else 64 if avg <= 64 or pk.get("fp8") else 128 if avg < 512 else 256
+    bn = 16 if avg <= 8 else 32 if avg <= 20 else 64 if avg <= 64 or pk.get("fp8") else 128 if avg < 512 else 256
     max_rows = T * k
     max_tiles = (max_rows + bn - 1) // bn + E
     idx32 = idx if idx.dtype == torch.int32 else idx.int()
