@@ -794,6 +794,166 @@ __global__ void __launch_bounds__(160, (HD <= 128 ? 2 : 1)) attn_decode_tma_kern
   decode_finish<HD>(p, wa, reinterpret_cast<float*>(ring), warp < 4, warp, lane, tid, 160, nq, h_lo, b, tok, split);
 }
 
+// The same for batches whose (sequence, kv head) pairs are more than the CTAs that fit the GPU: two CTAs per SM walk the pairs, and
+// the producer goes on to the next pair's tiles while the four warps finish this one.  A CTA per pair pays its start (barriers,
+// block table, query, first tile) in every round, which short contexts feel: 32 heads of 128, 32 sequences of 130 keys 22.7 us with
+// a CTA per pair, 15.6 us so; 10 sequences 10.0 and 6.9; 8 x 4 heads, 64 sequences of 200 keys 15.4 and 11.3.  From about 800 keys on
+// the two are level (69 and 66 us), at 2000 the dealing in advance loses 2 percent, so the caller asks for this kernel only for
+// short contexts (decode = 3).  A pair's arithmetic is that of the kernel above.
+// bf16, no split, no EXT, no ALiBi; up to kDecManyRows query heads per kv head (the merge buffer beside the ring) and kDecManySeqs
+// sequences.
+constexpr int kDecManySeqs = 512, kDecManyRows = 4;
+template <int HD>
+constexpr int dec_many_smem() { return DecCfg<HD>::STAGES * DecCfg<HD>::STAGE_BYTES + 4 * kDecManyRows * (HD + 2) * 4 + 1024; }
+
+template <int HD>
+__global__ void __launch_bounds__(160, 2) attn_decode_many_kernel(const __grid_constant__ CUtensorMap tmK,
+                                                                  const __grid_constant__ CUtensorMap tmV, const AttnParams p,
+                                                                  int B, int items) {
+  constexpr int KT = kDecTile, KW = KT / 4, TILE = KT * HD, STAGES = DecCfg<HD>::STAGES, RS = HD + 2;
+  constexpr uint32_t STAGE_BYTES = DecCfg<HD>::STAGE_BYTES;
+  extern __shared__ __align__(1024) uint8_t smem_dyn[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  bf16* ring = reinterpret_cast<bf16*>(base);
+  float* mo = reinterpret_cast<float*>(base + (size_t)STAGES * STAGE_BYTES);      // [4 warps][kDecManyRows][RS]
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES];
+  __shared__ int s_kv[kDecManySeqs], s_tok[kDecManySeqs], s_abort;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 4); }
+    s_abort = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+  }
+  grid_dep_launch();
+  // lengths and the block table are inputs of the step: they may be read before the kernel in front has finished
+  for (int i = tid; i < B; i += 160) { s_kv[i] = p.kv_lens[i]; s_tok[i] = p.cu_q[i]; }
+  __syncthreads();
+  // pair `item`: sequence item % B, kv head item / B
+  auto heads = [&](int item, int& lo, int& n) {
+    const int kvh = item / B;
+    lo = max(0, kvh * p.group - p.q_off);
+    n = min(p.hq, (kvh + 1) * p.group - p.q_off) - lo;
+  };
+  auto tiles_of = [&](int item) {
+    int lo, n;
+    heads(item, lo, n);
+    return n > 0 ? (s_kv[item % B] + KT - 1) / KT : 0;
+  };
+  if (warp == 4) {
+    if (elect_one()) {
+      const int per_block = p.bs / KT;
+      Ring r = {0, 0};
+      bool waited = false, ok = true;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        const int n_tiles = tiles_of(item), kvh = item / B;
+        const int* bt = p.block_table + (size_t)(item % B) * p.bt_stride;
+        int next = n_tiles > 0 ? bt[0] : 0;
+        for (int n = 0; n < n_tiles; ++n, r.next(STAGES)) {
+          int blk = next;
+          if (n + 1 < n_tiles) next = bt[(n + 1) / per_block];
+          if (blk < 0 || blk >= p.num_blocks) { if (p.status) atomicCAS(p.status, 0, XFT_ERR_BOUNDS); blk = 0; }
+          if (!waited && n + 1 == n_tiles) { grid_dep_wait(); waited = true; }       // this tile holds the newest token
+          if (!mbar_wait(&empty_bar[r.s], r.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) { s_abort = 1; ok = false; break; }
+          const int row = (blk * p.hkv + kvh) * p.bs + (n % per_block) * KT;
+          bf16* kt = ring + (size_t)r.s * 2 * TILE;
+          mbar_expect_tx(&full_bar[r.s], STAGE_BYTES);
+#pragma unroll
+          for (int h = 0; h < HD / 64; ++h) {
+            tma_load_2d(kt + h * KT * 64, &tmK, &full_bar[r.s], h * 64, row, kEvictFirst);
+            tma_load_2d(kt + TILE + h * KT * 64, &tmV, &full_bar[r.s], h * 64, row, kEvictFirst);
+          }
+        }
+      }
+    }
+  } else {
+    grid_dep_wait();
+    const int r0 = lane >> 2, r1 = r0 + 8;
+    Ring r = {0, 0};
+    bool alive = true;
+    uint32_t qa[HD / 16][4];
+    // A fragments of the pair's query heads: rows r0 and r0 + 8, features 2 * (lane % 4) + {0, 1} and 8 further on
+    auto load_q = [&](int item) {
+      int lo, n;
+      heads(item, lo, n);
+      const bf16* q0 = p.q + ((size_t)s_tok[item % B] * p.hq + lo + r0) * HD + 2 * (lane & 3);
+#pragma unroll
+      for (int ks = 0; ks < HD / 16; ++ks) {
+        qa[ks][0] = r0 < n ? *reinterpret_cast<const uint32_t*>(q0 + ks * 16) : 0u;
+        qa[ks][2] = r0 < n ? *reinterpret_cast<const uint32_t*>(q0 + ks * 16 + 8) : 0u;
+        qa[ks][1] = r1 < n ? *reinterpret_cast<const uint32_t*>(q0 + 8 * HD + ks * 16) : 0u;
+        qa[ks][3] = r1 < n ? *reinterpret_cast<const uint32_t*>(q0 + 8 * HD + ks * 16 + 8) : 0u;
+      }
+    };
+    if ((int)blockIdx.x < items) load_q(blockIdx.x);
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+      const int kv_len = s_kv[item % B], tok = s_tok[item % B], n_tiles = tiles_of(item);
+      int h_lo, nq;
+      heads(item, h_lo, nq);
+      const int qpos0 = r0 < nq ? kv_len - 1 : -1, qpos1 = r1 < nq ? kv_len - 1 : -1;
+      WarpAttn<HD, KW, true, KT, false> wa;
+      wa.init();
+      for (int n = 0; n < n_tiles; ++n, r.next(STAGES)) {
+        if (!mbar_wait(&full_bar[r.s], r.ph, p.status, XFT_ERR_WAIT_FULL)) { s_abort = 1; alive = false; break; }
+        const bf16* kt = ring + (size_t)r.s * 2 * TILE + warp * KW * 64;
+        const int key0 = n * KT + warp * KW;
+        if (key0 < kv_len) {
+          float s[KW / 8][4];
+          wa.qk_frag(s, qa, kt, lane);
+          if (key0 + KW > kv_len) {
+            wa.mask(s, key0, kv_len, qpos0, qpos1, p.scale, 0.f, 0.f, false, 0, nullptr, lane, p);
+          } else {
+#pragma unroll
+            for (int j = 0; j < KW / 8; ++j) { s[j][0] *= p.scale; s[j][1] *= p.scale; s[j][2] *= p.scale; s[j][3] *= p.scale; }
+          }
+          wa.softmax_update(s, nullptr, lane);
+          wa.pv(s, kt + TILE, lane);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty_bar[r.s]);
+      }
+      if (item + (int)gridDim.x < items) load_q(item + gridDim.x);          // on its way while the warps merge
+      wa.reduce_l();
+#pragma unroll
+      for (int j = 0; j < HD / 8; ++j) {
+        const int d = j * 8 + 2 * (lane & 3);
+        if (r0 < nq) {
+          mo[(warp * kDecManyRows + r0) * RS + d] = wa.o[j][0];
+          mo[(warp * kDecManyRows + r0) * RS + d + 1] = wa.o[j][1];
+        }
+      }
+      if ((lane & 3) == 0 && r0 < nq) {
+        mo[(warp * kDecManyRows + r0) * RS + HD] = wa.m[0];
+        mo[(warp * kDecManyRows + r0) * RS + HD + 1] = wa.l[0];
+      }
+      if (named_bar_or(1, 128, !alive)) break;
+      for (int i = tid; i < nq * HD; i += 128) {
+        const int row = i / HD, d = i % HD;
+        float mm = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, mo[(w * kDecManyRows + row) * RS + HD]);
+        float acc = 0.f, ll = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const float mw = mo[(w * kDecManyRows + row) * RS + HD];
+          const float c = (mw == -INFINITY) ? 0.f : __expf(mw - mm);
+          acc += c * mo[(w * kDecManyRows + row) * RS + d];
+          ll += c * mo[(w * kDecManyRows + row) * RS + HD + 1];
+        }
+        p.out[((size_t)tok * p.hq + h_lo + row) * HD + d] = __float2bfloat16(ll > 0.f ? acc / ll : 0.f);
+      }
+      named_bar_sync(1, 128);                                // the merge buffer is free again
+    }
+  }
+  __syncthreads();
+  if (*reinterpret_cast<volatile int*>(&s_abort)) {
+    // a wait ran out (status holds the reason): let copies already issued land before the CTA's memory is released
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) {}
+  }
+}
+
 // merge split partials: grid (B, hq), HD threads
 __global__ void attn_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, bf16* __restrict__ out,
                                   const int* __restrict__ cu_q, int hq, int HD, int nsplit) {
@@ -849,7 +1009,7 @@ static int launch_decode(const AttnParams& p, int B, bool int8, cudaStream_t st)
 }
 
 template <int HD, bool EXT>
-static int launch_decode_tma(const AttnParams& p, int B, cudaStream_t st) {
+static int launch_decode_tma(const AttnParams& p, int B, bool brief, cudaStream_t st) {
   CUtensorMap tmK, tmV;
   const uint64_t rows = (uint64_t)p.num_blocks * p.hkv * p.bs;
   if (make_tensor_map(&tmK, p.kc, rows, HD, HD, kDecTile, 2) || make_tensor_map(&tmV, p.vc, rows, HD, HD, kDecTile, 2)) return -4;
@@ -861,6 +1021,21 @@ static int launch_decode_tma(const AttnParams& p, int B, cudaStream_t st) {
     attr_set = true;
   }
   const int qchunks = (p.group + 15) / 16;
+  if constexpr (!EXT && HD <= 128) {
+    // more pairs than resident CTAs: with fewer, every pair has a CTA at once and there is no next one to go on to
+    const int items = B * p.hkv;
+    if (brief && p.nsplit == 1 && items > 2 * 148 && p.group <= kDecManyRows && B <= kDecManySeqs && !p.slopes) {
+      static bool many_set = false;
+      if (!many_set) {
+        if (cudaFuncSetAttribute(attn_decode_many_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_many_smem<HD>()) != cudaSuccess)
+          return -5;
+        many_set = true;
+      }
+      const cudaError_t e = launch_pdl(attn_decode_many_kernel<HD>, dim3(2 * 148), dim3(160), (size_t)dec_many_smem<HD>(), st, tmK, tmV, p,
+                                       B, items);
+      return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+    }
+  }
   dim3 grid(B, p.hkv * qchunks, p.nsplit);
   cudaError_t e = launch_pdl(attn_decode_tma_kernel<HD, EXT>, grid, dim3(160), smem, st, tmK, tmV, p);
   if (e != cudaSuccess) return (int)e;
@@ -873,9 +1048,9 @@ static int launch_attention(const AttnParams& p, int B, int max_q, int HD, int d
   if (decode) {
     if (p.nsplit > 1 && (!p.part_o || !p.part_ml || !p.split_counters)) return -3;
     if (!int8 && decode != 2) {
-      if (HD == 64) return launch_decode_tma<64, EXT>(p, B, st);
-      if (HD == 128) return launch_decode_tma<128, EXT>(p, B, st);
-      if (HD == 256) return launch_decode_tma<256, EXT>(p, B, st);
+      if (HD == 64) return launch_decode_tma<64, EXT>(p, B, decode == 3, st);
+      if (HD == 128) return launch_decode_tma<128, EXT>(p, B, decode == 3, st);
+      if (HD == 256) return launch_decode_tma<256, EXT>(p, B, decode == 3, st);
       return -1;
     }
     // per-warp K+V tiles of 16 KB: a CTA stays at ~64 KB so three CTAs (12 warps) overlap loads and math per SM
@@ -890,7 +1065,8 @@ static int launch_attention(const AttnParams& p, int B, int max_q, int HD, int d
   return -1;
 }
 
-// decode != 0: every sequence has exactly one query row (2 forces the cp.async kernel for bf16 caches too).
+// decode != 0: every sequence has exactly one query row (2 forces the cp.async kernel for bf16 caches too, 3: contexts are
+// short, see attn_decode_many_kernel).
 // nsplit/part_*: split-KV scratch (decode only).  softcap > 0: scores become softcap * tanh(score / softcap).
 // window > 0: position i sees the keys j <= i with i - j < window or j < keep.  sinks [hq]: exp(sinks[h]) joins the
 // softmax denominator of head h.

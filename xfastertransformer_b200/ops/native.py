@@ -594,6 +594,8 @@ def plan_attn_splits(B, hkv, group, D, max_kv, int8=False, least=8):
     return nsplit, ntiles
 
 
+# Decode steps of contexts up to this many keys may take the kernel whose CTAs walk several (sequence, head) pairs.
+BRIEF_KV = 512
 # Prompts over an int8 cache: from this many new tokens on a copy of the codes in bf16 pays for itself (it is five bytes of traffic
 # per code, the kernel without it reads each code once per 64 query rows and head), as long as the copy stays below a bound.
 # Short contexts are all launch: 100 tokens 21 us without the copy, 27 us with it; 3 x 2250 tokens 1308 and 600 us.
@@ -671,7 +673,7 @@ def paged_attention(q, kc, vc, block_table, cu_q, kv_lens, scale, ks=None, vs=No
     rc = lib().xft_paged_attention_ext(_p(q), _p(out), _p(kc), _p(vc), _p(ks), _p(vs), _p(block_table),
                                        block_table.stride(0), _p(cu_dev), _p(kv_dev), B, max_q, hq, hkv, g, q_off, D, bs,
                                        nb, C.c_float(scale), _p(slopes), _p(pl),
-                                       (1 if _ENV().attn_tma else 2) if decode else 0, nsplit, _p(po), _p(pm),
+                                       (2 if not _ENV().attn_tma else 3 if max_kv <= BRIEF_KV else 1) if decode else 0, nsplit, _p(po), _p(pm),
                                        _p(ws.attn_counters), _p(ws.status), C.c_float(softcap), window, keep_first,
                                        _p(sinks), _stream())
     _check(rc, "paged_attention")
