@@ -18,6 +18,10 @@
 // B200, us before (expanding kernel; W8A8: its own kernel, parts through global scratch) / here, with the split of X:
 //   fp8 2 x 28672 x 8192, 16 rows 417 / 78 (6.0 TB/s); 4096 x 4096, 16 rows 21 / 8; uint4 2 x 28672 x 8192, 16 rows 165 / 82;
 //   12288 x 4096, 32 rows 29 / 19.  Error against 64 bits (12288 x 4096, relative): fp8 1.6e-3 / 1e-7, uint4 1.4e-5 / 3e-7.
+// bf16 operands (64 k per block) go the same way at decode sizes.  The kernels they had (gemm_sm100.cu, gemm_decode_sm100.cu) leave
+// parts in global scratch or finish with four warps, a dependent chain that grows with the tokens: 2 x 11008 x 4096, 32 rows 58 us
+// there, 36 here (27.6 at the copy rate); 12288 x 4096, 64 rows 40 and 27; 4096 x 4096, 32 rows 13.8 and 9.5; 8192 x 28672, 1 row
+// 70 and 69.  The fused all-reduce and the rotary epilogue stay there.
 //
 // A CTA owns 128 features x BN tokens (BN = 16, 32, 64).  Small products are cut along K over a cluster: every CTA leaves its
 // part in its own shared memory and finishes BN / cluster tokens from all parts.
@@ -27,7 +31,7 @@
 
 namespace xft {
 
-enum { kSrcFp8 = 0, kSrcU4 = 1, kSrcI8 = 2 };
+enum { kSrcFp8 = 0, kSrcU4 = 1, kSrcI8 = 2, kSrcBf16 = 3 };
 
 struct E4Params {
   int N, T, K;
@@ -46,6 +50,9 @@ struct E4Params {
   const int4* group_tiles; const int* num_group_tiles; int group_w_rows;      // see quant_gemm_sm100.cu
   const float* col_scale;
   const float* a_zero; const float* a_qsum; const float* w_sum;      // W8A8: [T], [T], [N]; x_scale, scale and zero as above
+  // bf16: a folded RMSNorm (W carries its gain): sums are multiplied with 1 / rms of the rows of rms_x, which is X
+  const __nv_bfloat16* rms_x; int rms_ldx; float rms_eps;
+  const float* rms_ssq;      // [T] their sums of squares, or null: every CTA adds them up for itself
   int* status;
 };
 
@@ -77,7 +84,7 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* v) {
 template <int BN, bool DUAL, int SRC>
 struct E4Layout {
   static constexpr int NACC = DUAL ? 2 : 1;
-  static constexpr int A_BYTES = 128 * 128 * NACC, RAW_BYTES = SRC == kSrcU4 ? 128 * 64 * NACC : 0, B_BYTES = (SRC == kSrcI8 ? 1 : 2) * BN * 128;
+  static constexpr int A_BYTES = 128 * 128 * NACC, RAW_BYTES = SRC == kSrcU4 ? 128 * 64 * NACC : 0, B_BYTES = (SRC == kSrcI8 || SRC == kSrcBf16 ? 1 : 2) * BN * 128;
   static constexpr int STAGE = (SRC == kSrcU4 ? RAW_BYTES : A_BYTES) + B_BYTES;       // what TMA fills
   static constexpr int A_RING = SRC == kSrcU4 ? 2 * A_BYTES : 0;                      // expanded codes, two buffers
   // two CTAs per SM where registers allow: one CTA's last accumulators and stores hide behind the other's stream
@@ -93,11 +100,11 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
     gemm_e4m3_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const E4Params p) {
   using L = E4Layout<BN, DUAL, SRC>;
   constexpr int NACC = L::NACC, STAGES = L::STAGES;
-  constexpr int NB = SRC == kSrcI8 ? BN : 2 * BN;                      // columns of an accumulator: hi [BN], lo [BN]
+  constexpr int NB = SRC == kSrcI8 || SRC == kSrcBf16 ? BN : 2 * BN;   // columns of an accumulator: hi [BN], lo [BN]
   constexpr int ACC = NB * NACC;
   constexpr int BUFS = SRC == kSrcFp8 ? 2 : 1;
   constexpr uint32_t TMEM_COLS = BUFS * ACC < 32 ? 32 : BUFS * ACC;
-  constexpr uint32_t IDESC = SRC == kSrcI8 ? umma_idesc(128, BN, 1, 1, 2) : umma_idesc(128, 2 * BN, 0, 0, 1);
+  constexpr uint32_t IDESC = SRC == kSrcI8 ? umma_idesc(128, BN, 1, 1, 2) : SRC == kSrcBf16 ? umma_idesc(128, BN, 1, 1, 1) : umma_idesc(128, 2 * BN, 0, 0, 1);
   constexpr int HB = BN / 2;                                           // tokens per thread: two warps share a row of the tile
   constexpr int TILE_A = 128 * 128;
 
@@ -106,6 +113,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tmem_full[2], tmem_empty[2], a_ready[2], a_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_group[4];
+  __shared__ float s_ssq[SRC == kSrcBf16 ? BN : 1];                    // bf16: sums of squares of the tokens over this CTA's k
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int tile_n, tile_t;
@@ -155,19 +163,20 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
   uint8_t* ring = smem + L::A_RING;
   if (warp == 0) {
     if (elect_one()) {
-      constexpr int W_COLS = SRC == kSrcU4 ? 64 : 128;                 // bytes of a weight row per block of 128 k
+      constexpr int W_COLS = SRC == kSrcU4 ? 64 : 128;                 // bytes of a weight row per block of 128 k (bf16: 64 k)
       constexpr int W_TILE = 128 * W_COLS;
+      constexpr int W_STEP = SRC == kSrcBf16 ? 64 : W_COLS;            // the same in elements of the tensor map
       const uint64_t hint_w = p.t_tiles == 1 || grouped ? kEvictFirst : kEvictNormal;
       auto load_w = [&](int s, int kb) {
         mbar_expect_tx(&full_bar[s], L::STAGE);
         uint8_t* st = ring + s * L::STAGE;
-        tma_load_2d(st, &tmW, &full_bar[s], kb * W_COLS, w_row0, hint_w);
-        if (DUAL) tma_load_2d(st + W_TILE, &tmW, &full_bar[s], kb * W_COLS, p.dual_off + w_row0, hint_w);
+        tma_load_2d(st, &tmW, &full_bar[s], kb * W_STEP, w_row0, hint_w);
+        if (DUAL) tma_load_2d(st + W_TILE, &tmW, &full_bar[s], kb * W_STEP, p.dual_off + w_row0, hint_w);
       };
       auto load_x = [&](int s, int kb) {
         uint8_t* st = ring + s * L::STAGE + W_TILE * NACC;
-        tma_load_2d(st, &tmX, &full_bar[s], kb * 128, x_row0, kEvictLast);
-        if (SRC != kSrcI8) tma_load_2d(st + BN * 128, &tmX, &full_bar[s], p.x_lo + kb * 128, x_row0, kEvictLast);
+        tma_load_2d(st, &tmX, &full_bar[s], SRC == kSrcBf16 ? kb * 64 : kb * 128, x_row0, kEvictLast);
+        if (SRC != kSrcI8 && SRC != kSrcBf16) tma_load_2d(st + BN * 128, &tmX, &full_bar[s], p.x_lo + kb * 128, x_row0, kEvictLast);
       };
       // weights never depend on the previous kernel: the first round is requested before the grid dependency resolves
       const int pre = min(STAGES, kend - kb0);
@@ -201,7 +210,8 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
         for (int k = 0; k < 4; ++k) {                                  // 4 x 32 k
           const uint32_t on = (SRC != kSrcFp8 && kb > kb0) || k > 0;
           auto mma = [&](uint32_t d, uint64_t a) {
-            if constexpr (SRC == kSrcI8) umma_i8(d, a, bd + 2 * k, IDESC, on);
+            if constexpr (SRC == kSrcBf16) umma_bf16(d, a, bd + 2 * k, IDESC, on);
+            else if constexpr (SRC == kSrcI8) umma_i8(d, a, bd + 2 * k, IDESC, on);
             else umma_f8(d, a, bd + 2 * k, IDESC, on);
           };
           mma(acc, ad + 2 * k);
@@ -252,10 +262,34 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
         __syncwarp();
         if (lane == 0) mbar_arrive(&tmem_empty[b.s]);
       }
-    } else if constexpr (SRC == kSrcI8) {
+    } else if constexpr (SRC == kSrcI8 || SRC == kSrcBf16) {
+      if (SRC == kSrcBf16 && p.rms_x && !p.rms_ssq) {                                // beside the main loop: 256 / BN threads per token
+        constexpr int TPT = 256 / BN;
+        const int e = threadIdx.x - 64, tok = e / TPT, sub = e % TPT;
+        grid_dep_wait();
+        float acc = 0.f;
+        if (tok < x_rows) {
+          const __nv_bfloat16* xr = p.rms_x + (size_t)(x_row0 + tok) * p.rms_ldx;
+          const int k1 = min(kb1 * 64, p.K);
+#pragma unroll 4
+          for (int k = kb0 * 64 + sub * 8; k < k1; k += TPT * 8) {
+            const uint4 v = *reinterpret_cast<const uint4*>(xr + k);
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 f = __bfloat1622float2(h[i]);
+              acc += f.x * f.x + f.y * f.y;
+            }
+          }
+        }
+#pragma unroll
+        for (int o = TPT / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (sub == 0) s_ssq[tok] = acc;
+        named_bar_sync(2, 256);
+      }
       ok = __all_sync(0xffffffffu, mbar_wait(&tmem_full[0], 0, p.status, XFT_ERR_WAIT_TMEM));
       tcgen05_fence_after();
-      if (ok) {                                                        // s32, kept as they are
+      if (ok) {                                                        // s32 (or fp32), kept as they are
         tmem_ld_cols<HB>(taddr, reinterpret_cast<uint32_t*>(g[0]));
         if constexpr (DUAL) tmem_ld_cols<HB>(taddr + NB, reinterpret_cast<uint32_t*>(g[1]));
         tmem_ld_wait();
@@ -299,6 +333,22 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
   if (warp >= 2) grid_dep_wait();                                      // outputs, residual and the row scales belong to the stream order
 
   auto finish = [&](int t, float x, float u) {                         // t: token row of X and Y
+    if constexpr (SRC == kSrcBf16) {
+      float ts = 1.f;
+      if (p.rms_x) {
+        float ssq = p.rms_ssq ? p.rms_ssq[t] : 0.f;
+        for (int s = 0; s < p.splits && !p.rms_ssq; ++s)
+          ssq += p.splits == 1 ? s_ssq[t - x_row0] : ld_dsmem(dsmem_addr(smem_u32(s_ssq + (t - x_row0)), s));
+        ts = rsqrtf(ssq / (float)p.K + p.rms_eps);
+      }
+      x = x * ts + (p.bias ? p.bias[n] : 0.f);
+      if (DUAL) x = apply_gated(x, u * ts + (p.bias ? p.bias[p.dual_off + n] : 0.f), p.act, p.res_scale);
+      else x = apply_act(x, p.act, p.res_scale);
+      if (p.residual) x = with_residual(x, __bfloat162float(p.residual[(size_t)t * p.ldr + n]), p.res_scale, p.act);
+      if (p.out_fp32) reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + n] = x;
+      else reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + n] = __float2bfloat16(x);
+      return;
+    }
     const float st = p.x_scale[t];
     if constexpr (SRC == kSrcI8) {
       const float za = p.a_zero[t], qs = p.a_qsum[t];
@@ -378,6 +428,31 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
   tcgen05_fence_before();
   __syncthreads();
   if (warp == 1) { tcgen05_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
+}
+
+// Sums of squares of rows of X, a block per row.
+__global__ void __launch_bounds__(256) row_ssq_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int K, float* __restrict__ ssq) {
+  __shared__ float s_sum[8];
+  grid_dep_launch();
+  grid_dep_wait();
+  const __nv_bfloat16* row = x + (size_t)blockIdx.x * ldx;
+  float sm = 0.f;
+  for (int k = threadIdx.x * 8; k < K; k += 2048) {
+    const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(h[i]);
+      sm += f.x * f.x + f.y * f.y;
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sm;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) sm += s_sum[w];
+    ssq[blockIdx.x] = sm;
+  }
 }
 
 // Row r of X (or row src[r]) -> [hi | lo] e4m3, its power-of-two scale and its sum.  `nibbles`: k in the order in which uint4
@@ -609,4 +684,37 @@ extern "C" int xft_w8a8_gemm_gated(const void* qx, int ldqx, const void* Wq, int
                                    const float* w_zero, const float* w_sum, const float* bias, int act, int* status, cudaStream_t st) {
   return w8a8(qx, ldqx, Wq, ldw, Y, ldo, 0, T, N, K, 1, dual_off, a_scale, a_zero, a_qsum, w_scale, w_zero, w_sum, bias, nullptr, 0, 1.f,
               act, status, st);
+}
+
+// Y = epi(X W^T) for T <= 64, bf16 operands on the same pipeline; arguments as xft_gemm_bf16 (gemm_sm100.cu), rms_eps as in xft_gemm_sk.
+// rms_ssq: room for T floats, or null.  With it the rows' sums of squares are a launch of their own (2 us); without it every CTA adds
+// them up beside its weight stream, which at 64 rows costs more than the stream hides (12288 x 4096: 10 us, at 16 rows 1 us).
+extern "C" int xft_gemm_bf16_cluster(const void* X, int ldx, const void* W, int w_rows, int ldw, void* Y, int ldo, int out_fp32, int T,
+                                     int N, int K, int gated, int dual_off, const float* bias, const void* residual, int ldr,
+                                     float res_scale, int act, const float* rms_eps, float* rms_ssq, int* status, cudaStream_t st) {
+  if (T <= 0 || N <= 0 || K <= 0) return 0;
+  if (T > 64 || (K & 7) || (ldx & 7) || (ldw & 7)) return -2;
+  E4Params p{};
+  if (rms_eps) { p.rms_x = (const __nv_bfloat16*)X; p.rms_ldx = ldx; p.rms_eps = *rms_eps; p.rms_ssq = rms_ssq; }
+  p.N = N; p.T = T; p.K = K; p.dual_off = dual_off; p.out = Y; p.ldo = ldo; p.out_fp32 = out_fp32; p.bias = bias;
+  p.residual = (const __nv_bfloat16*)residual; p.ldr = ldr; p.res_scale = res_scale; p.act = act; p.status = status;
+  const int bn = T <= 16 ? 16 : T <= 32 ? 32 : 64;
+  p.num_kb = (K + 63) / 64;
+  p.n_tiles = (N + 127) / 128;
+  p.t_tiles = (T + bn - 1) / bn;
+  p.splits = e4_splits(p.n_tiles * p.t_tiles, p.num_kb, bn);
+  CUtensorMap tmW, tmX;
+  int r = make_tensor_map(&tmW, W, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw, 128, 2);
+  if (r) return 1000 - r;
+  r = make_tensor_map(&tmX, X, (uint64_t)T, (uint64_t)K, (uint64_t)ldx, (uint32_t)bn, 2);
+  if (r) return 2000 - r;
+  if (rms_eps && rms_ssq) {
+    const cudaError_t e = launch_pdl(row_ssq_kernel, dim3(T), dim3(256), 0, st, p.rms_x, ldx, K, rms_ssq);
+    if (e != cudaSuccess) return (int)e;
+  }
+#define XFT_BF(BN_) \
+  case BN_: return gated ? launch_e4<BN_, true, kSrcBf16>(tmW, tmX, p, st) : launch_e4<BN_, false, kSrcBf16>(tmW, tmX, p, st);
+  switch (bn) { XFT_BF(16) XFT_BF(32) XFT_BF(64) }
+#undef XFT_BF
+  return -1;
 }

@@ -25,6 +25,8 @@ namespace xft {
 
 int make_tensor_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
                     uint32_t esize);
+int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes, uint32_t box_rows,
+                  uint32_t box_bytes);
 void plan_splits(int tiles, int num_kb, int bn, int nacc, size_t ws_bytes, int max_tiles, int* splits, int* kb_per_split);
 int pick_bn(int T);
 
@@ -459,27 +461,6 @@ __global__ void __launch_bounds__(256) row_sum_kernel(const __nv_bfloat16* __res
 }
 
 // ------------------------------------------------------------------------------------------ host
-typedef CUresult (*EncFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                          const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                          CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes,
-                        uint32_t box_rows, uint32_t box_bytes) {
-  static EncFn enc = nullptr;
-  if (!enc) {
-    void* fp = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fp, cudaEnableDefault, &q) != cudaSuccess) return -1;
-    enc = reinterpret_cast<EncFn>(fp);
-  }
-  if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (ld_bytes & 15)) return -2;
-  cuuint64_t dims[2] = {row_bytes, rows};
-  cuuint64_t strides[1] = {ld_bytes};
-  cuuint32_t box[2] = {box_bytes, box_rows};
-  cuuint32_t es[2] = {1, 1};
-  return enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, es,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -3;
-}
 
 template <int BN, bool DUAL, int QT>
 static int launch_q(const CUtensorMap& tmW, const CUtensorMap& tmX, QGemmParams& p, cudaStream_t st) {

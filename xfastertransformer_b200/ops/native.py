@@ -241,6 +241,9 @@ def gemm_bf16(x, w, N, gated=False, dual_off=0, bias=None, act=None, residual=No
         assert r2.stride(1) == 1 and r2.dtype == torch.bfloat16
         ldr = r2.stride(0)
     ws = Workspace.get(x.device)
+    if T <= SK_MAX_TOKENS and force_splits == 0 and row_scale is None and _use_cluster(T, N, K, gated):
+        _gemm_cluster(x2, ldx, w, out, T, N, K, gated, dual_off, bias, r2, ldr, res_scale, act)
+        return out
     if T <= SK_MAX_TOKENS and force_splits == 0 and _sk_choice(T, N, K, gated):
         _gemm_sk(x2, ldx, w, out, T, N, K, gated, dual_off, bias, r2, ldr, res_scale, act, row_scale, None, None, None)
         return out
@@ -319,6 +322,30 @@ def pick_bn(T: int) -> int:
     return 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128 if T <= 128 else 256
 
 
+def _use_cluster(T, N, K, gated) -> bool:
+    """Whether a decode-size product (T <= 64) runs on the pipeline of gemm_bf16_cluster (gemm_e4m3_sm100.cu), on B200 the faster one
+    but for two ends: above 32 rows one CTA fits an SM there, and with more tiles than SMs nothing hides its finish (32000 x 4096,
+    64 rows 68 us, the tile-per-CTA kernel 60; 12288 x 4096 27 and 40; gated products have twice the stream per tile: 2 x 28672 x
+    8192 163 and 185), and gated products of less than half a million weights a half (2 x 256 x 512, 8 rows 5.5 us and 4.8;
+    2 x 2816 x 1024 6.2 and 6.7)."""
+    if not _ENV().gemm_streamk or (gated and N * K < 1 << 19):
+        return False
+    return T <= 32 or gated or N <= 148 * 128
+
+
+def _gemm_cluster(x2, ldx, w, out, T, N, K, gated, dual_off, bias, r2, ldr, res_scale, act, rms_eps=None):
+    """One launch of the decode-size kernel of gemm_e4m3_sm100.cu (T <= 64)."""
+    ws = Workspace.get(x2.device)
+    ssq = torch.empty(T, dtype=torch.float32, device=x2.device) if rms_eps is not None and T > 32 else None
+    fn = lib().xft_gemm_bf16_cluster
+    fn.restype = C.c_int
+    rc = fn(_p(x2), ldx, _p(w), w.shape[0], w.stride(0), _p(out), out.stride(0), int(out.dtype == torch.float32), T, N, K, int(gated),
+            dual_off, _p(bias), _p(r2), ldr, C.c_float(res_scale), _ACT[act], C.byref(C.c_float(rms_eps)) if rms_eps is not None else None,
+            _p(ssq), _p(ws.status), _stream())
+    _check(rc, "gemm_bf16_cluster")
+    ws.launches += 1 + (ssq is not None)
+
+
 def _gemm_sk(x2, ldx, w, out, T, N, K, gated, dual_off, bias, r2, ldr, res_scale, act, row_scale, rms_eps, comm, qkv):
     """One launch of the decode-size weight-stream GEMM (T <= 64)."""
     ws = Workspace.get(x2.device)
@@ -335,22 +362,34 @@ def _gemm_sk(x2, ldx, w, out, T, N, K, gated, dual_off, bias, r2, ldr, res_scale
 
 
 def can_fuse_qkv_rope(W, T, D, kc, ks, q_norm_w, k_norm_w, style) -> bool:
-    """The QKV product can end in RoPE + paged cache append (one kernel instead of two): bf16 weights, head_dim 128,
+    """qkv_linear_rope_cache takes the product, RoPE and the paged cache append: bf16 weights, head_dim 128,
     a bf16 cache, no per-head q/k norm, at most SK_MAX_TOKENS rows."""
     e = _ENV()
     return (e.gemm_streamk and e.fuse_qkv_rope and W.kind == "bf16" and 0 < T <= SK_MAX_TOKENS and D == 128 and ks is None
             and kc.dtype == torch.bfloat16 and q_norm_w is None and k_norm_w is None and style in ("half", "interleaved"))
 
 
+def _qkv_one_kernel(T, NK) -> bool:
+    """Small products end in RoPE and the cache append themselves; larger ones are faster as the cluster kernel and a launch behind it.
+    us, one kernel / two: 1.6 M weights (8 + 2 x 2 heads, K 1024) 1 row 5.3 / 6.2, 32 rows 8.8 / 9.6, 64 rows 13.3 / 12.7; 4.2 M 16 rows
+    7.8 / 8.2, 32 rows 12.0 / 10.3; 12.6 M 1 row 8.2 / 9.1, 8 rows 10.5 / 10.3; 25 M 1 row 15.8 / 13.8, 32 rows 31.5 / 16.9."""
+    return NK <= (16 << 20 if T <= 4 else 5 << 20 if T <= 16 else 2 << 20 if T <= 32 else 0)
+
+
 def qkv_linear_rope_cache(x, W, bias, rms_eps, hq, hkv, positions, table, rot_dim, style, kc, vc, slots, q_scale=None,
                           rot_offset=0):
-    """q = RoPE(split(x W^T + b)) and K / V appended to the paged cache, as ONE kernel: the QKV product's epilogue
-    rotates each finished head and stores it where the attention kernel reads it.  `rms_eps` set: `x` is the
+    """q = RoPE(split(x W^T + b)) and K / V appended to the paged cache: small products as ONE kernel whose epilogue
+    rotates each finished head and stores it where the attention kernel reads it, larger ones as two (see _qkv_one_kernel).  `rms_eps` set: `x` is the
     un-normalised hidden state and W carries the norm's gain (see fold_norm_gain)."""
     x2, ldx = _rows2d(x)
     T, K = x2.shape
     N = (hq + 2 * hkv) * 128
     assert W.w.shape[0] == N and W.w.shape[1] == K and x2.dtype == torch.bfloat16
+    if not _qkv_one_kernel(T, N * K) and _use_cluster(T, N, K, False):
+        qkv = torch.empty(T, N, dtype=torch.bfloat16, device=x.device)
+        _gemm_cluster(x2, ldx, W.w, qkv, T, N, K, False, 0, bias, None, 0, 1.0, None, rms_eps)
+        return qkv_rope_cache(qkv, hq, hkv, 128, positions, table, rot_dim, style, kc, vc, None, None, slots, q_scale,
+                              rot_offset=rot_offset)
     q = torch.empty(T, hq, 128, dtype=torch.bfloat16, device=x.device)
     nb, _, bs, _ = kc.shape
     qp = SkQkv()
@@ -394,6 +433,9 @@ def linear_rms(x, W, eps, bias=None, act=None, gated=False, out_dtype=None):
     assert w.dtype == torch.bfloat16 and w.stride(1) == 1 and w.shape[1] == K and x2.dtype == torch.bfloat16
     fp32 = out_dtype == torch.float32
     out = torch.empty(T, N, dtype=torch.float32 if fp32 else torch.bfloat16, device=x.device)
+    if _use_cluster(T, N, K, gated):
+        _gemm_cluster(x2, ldx, w, out, T, N, K, gated, N if gated else 0, bias, None, 0, 1.0, act, eps)
+        return out.view(*x.shape[:-1], N)
     if _sk_choice(T, N, K, gated):
         _gemm_sk(x2, ldx, w, out, T, N, K, gated, N if gated else 0, bias, None, 0, 1.0, act, None, eps, None, None)
         return out.view(*x.shape[:-1], N)
