@@ -1,5 +1,6 @@
 // Decode-size bf16 GEMM for sm_100a (at most 64 tokens):  Y[T, N] = epilogue( X[T, K] · W[N, K]^T ), written as a
-// balanced weight stream with the layer's neighbouring work fused into its two ends.
+// balanced weight stream with the layer's neighbouring work fused into its two ends.  Plain, gated and folded-norm products
+// are faster on the cluster pipeline of gemm_e4m3_sm100.cu; what stays here: the fused all-reduce, small QKV products, small gated ones.
 //
 // The reference runs a decoder layer's linears as separate xDNN/oneDNN calls with a norm in front, a RoPE + cache
 // copy behind the QKV product and an all-reduce behind o_proj / down_proj (src/layers/attention.h, mlp_llama.h,

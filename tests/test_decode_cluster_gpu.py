@@ -62,3 +62,17 @@ def test_qkv_in_one_and_two_launches_agree(T, fold, monkeypatch):
         got.append((q.float(), k.float(), v.float()))
     for a, b in zip(*got):
         assert bool(((a - b).abs() <= 2.0 ** -6 * a.abs().amax()).all()) and float((a - b).norm() / a.norm()) < 2.0 ** -9
+
+
+@pytest.mark.parametrize("name,value", [("XFT_GEMM_STREAMK", "0"), ("XFT_GEMM_STREAMK", "2"), ("XFT_SK_CLUSTER", "4")])
+def test_a_kernel_asked_for_by_name_is_taken(name, value, monkeypatch):
+    from xfastertransformer_b200.ops import native as Nat
+    from xfastertransformer_b200.utils.flags import Env
+    assert Nat._use_cluster(16, 4096, 4096, False)
+    try:
+        monkeypatch.setenv(name, value)
+        Env.get().reload()
+        assert not Nat._use_cluster(16, 4096, 4096, False)
+    finally:
+        monkeypatch.undo()
+        Env.get().reload()

@@ -530,7 +530,7 @@ class Decoder:
                          ops.can_fuse_qkv_rope(L.qkv, xin.numel() // xin.shape[-1], self.D, cache.k[li], cache.ks[li],
                                                L.q_norm, L.k_norm, self.rope_style))
             if fused_qkv:
-                # decode sizes: RoPE and the cache append are the epilogue of the QKV product (one kernel)
+                # decode sizes: product, RoPE and cache append as one kernel (small products) or two
                 with TimeLine("QKV.linear+QKPO"):
                     q = ops.qkv_linear_rope_cache(xin, L.qkv, L.qkv_b, self.eps if L.attn_fold else None, self.hq,
                                                   self.hkv, positions, table, self.rot_dim, self.rope_style,

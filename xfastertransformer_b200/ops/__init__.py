@@ -185,7 +185,7 @@ def qkv_rope2d_cache(qkv, hq, hkv, d, positions, positions2, table, kc, vc, ks, 
 
 
 def can_fuse_qkv_rope(W, T, D, kc, ks, q_norm_w, k_norm_w, style) -> bool:
-    """True when the QKV product, RoPE and the cache append can run as one kernel (GPU, decode sizes)."""
+    """True when the QKV product, RoPE and the cache append can run as one step (GPU, decode sizes)."""
     return _cuda(kc) and _nat().can_fuse_qkv_rope(W, T, D, kc, ks, q_norm_w, k_norm_w, style)
 
 

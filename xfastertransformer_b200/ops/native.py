@@ -328,7 +328,7 @@ def _use_cluster(T, N, K, gated) -> bool:
     64 rows 68 us, the tile-per-CTA kernel 60; 12288 x 4096 27 and 40; gated products have twice the stream per tile: 2 x 28672 x
     8192 163 and 185), and gated products of less than half a million weights a half (2 x 256 x 512, 8 rows 5.5 us and 4.8;
     2 x 2816 x 1024 6.2 and 6.7)."""
-    if not _ENV().gemm_streamk or (gated and N * K < 1 << 19):
+    if not _ENV().gemm_cluster or (gated and N * K < 1 << 19):
         return False
     return T <= 32 or gated or N <= 148 * 128
 
@@ -420,8 +420,8 @@ def _ones(n: int, device) -> torch.Tensor:
 
 def linear_rms(x, W, eps, bias=None, act=None, gated=False, out_dtype=None):
     """RMSNorm(x) @ W^T where W already carries the norm's gain in its columns (see fold_norm_gain).  Up to
-    RMS_FUSE_MAX_TOKENS rows this is ONE kernel: the GEMM computes each token's 1/rms beside its main loop and
-    scales the accumulator.  Larger batches (prefill) run the gain-free norm kernel, then the GEMM."""
+    RMS_FUSE_MAX_TOKENS rows no normalised copy is written: the GEMM scales its accumulator by each token's 1/rms, from squares
+    added up beside its main loop or, above 32 rows, by a small kernel in front (see _gemm_cluster).  Larger batches (prefill) run the gain-free norm kernel, then the GEMM."""
     assert W.kind == "bf16"
     x2, ldx = _rows2d(x)
     T, K = x2.shape

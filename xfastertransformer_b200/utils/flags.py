@@ -81,6 +81,8 @@ class Env:
         self.ssd_chunk_min_q = _int("XFT_SSD_CHUNK_MIN_Q", 16)    # the same of state-space layers
         self.talking_tc = _int("XFT_TALKING_TC", 1) != 0          # attention with mixed heads on the tensor cores (0: plain kernel)
         self.gemm_streamk = _int("XFT_GEMM_STREAMK", 1) != 0
+        # products of up to 64 rows on the cluster kernel of gemm_e4m3_sm100.cu, unless one of the older ones is asked for
+        self.gemm_cluster = _int("XFT_GEMM_STREAMK", 1) == 1 and "XFT_SK_CLUSTER" not in os.environ
         self.fuse_qkv_rope = _int("XFT_FUSE_QKV_ROPE", 1) != 0
         # tensor-parallel prefill: two groups of prompts are interleaved block by block, so that the all-reduce of one
         # overlaps the compute of the other
