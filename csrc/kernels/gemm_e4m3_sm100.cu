@@ -386,6 +386,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
   } else {
     // every MMA has read its operands (the last accumulator is here), so the ring is free for this CTA's part: [column][128]
     float* part = reinterpret_cast<float*>(smem);
+    __syncwarp();                                                      // the lanes behind the elected ones of warps 0 and 1
     named_bar_sync(1, kE4Threads);                                     // the slower half may still wait for its accumulator
     if (warp >= 2) {
 #pragma unroll
