@@ -610,7 +610,9 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
     const int q = warp & 3;
     const int c_begin = warp < 6 ? 0 : FEAT / 2, c_end = c_begin + FEAT / 2;
     const int row = q * 32 + lane;
-    const bool vec = (p.N % 8 == 0) && (p.ldo % 8 == 0) && (!p.residual || p.ldr % 8 == 0);
+    // 16-byte pieces where every row of output and residual starts on one (a residual may be a slice of a wider tensor)
+    const bool vec = (p.N % 8 == 0) && (p.ldo % 8 == 0) && (!p.residual || p.ldr % 8 == 0) &&
+                     ((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.residual)) & 15) == 0;
     // 32-byte rows' pieces: every store fills a whole sector
     const bool vec32 = vec && p.ldo % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
     const bool bias16 = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;

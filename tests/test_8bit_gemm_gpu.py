@@ -110,3 +110,18 @@ def test_fp8_experts_match_64_bits(T, E, k):
     got = Nat.moe_experts(x, idx, wt, experts).double()
     Nat.Workspace.get(x.device).check_status()
     assert bool(((got - want).abs() <= tol + 1e-5).all())
+
+
+@pytest.mark.parametrize("kind", ["w8a8", "bf16"])
+@pytest.mark.parametrize("T", [40, 66, 300])
+@pytest.mark.parametrize("at", [1, 4])
+def test_residual_that_starts_between_16_bytes(kind, T, at):
+    """A slice of a wider tensor: its row pitch is a multiple of 16 bytes, its start is not.  The same bits as from a copy of it."""
+    from xfastertransformer_b200.ops import native as Nat
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, 256, generator=g, device="cuda").bfloat16()
+    W = _linear(torch.randn(512, 256, generator=g, device="cuda") * 0.05, kind)
+    res = torch.randn(T, 520, generator=g, device="cuda").bfloat16()[:, at:at + 512]
+    got, want = Nat.linear(x, W, None, None, res, 0.5), Nat.linear(x, W, None, None, res.contiguous(), 0.5)
+    Nat.Workspace.get(x.device).check_status()
+    assert torch.equal(got, want)
