@@ -334,7 +334,8 @@ __global__ void __launch_bounds__(192, 1) attn_prefill_tc_kernel(const __grid_co
                 __nv_bfloat162 pb;
                 if constexpr (INT8) {                                  // the value's scale belongs to the product, not to the sum
                   const float2 f = __ldg(reinterpret_cast<const float2*>(c < 64 ? vs_a : vs_b) + ((c & 63) >> 1) + g8 * 4 + i);
-                  pb = __floats2bfloat162_rn(p0 * f.x, p1 * f.y);
+                  // a hidden key may be a slot that no one has written since its last owner: 0 x its scale can be NaN
+                  pb = __floats2bfloat162_rn(seen(c + e) ? p0 * f.x : 0.f, seen(c + e + 1) ? p1 * f.y : 0.f);
                   sum += p0 + p1;
                 } else {
                   pb = __floats2bfloat162_rn(p0, p1);

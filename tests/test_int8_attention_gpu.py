@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 from xfastertransformer_b200.ops import reference as R
 
 
-def _run(lens, past, hq, hkv, D, seed, monkeypatch, never=False):
+def _run(lens, past, hq, hkv, D, seed, monkeypatch, never=False, stale=None):
     from xfastertransformer_b200.ops import native as N
     monkeypatch.setattr(N, "INT8_TC_MIN_KV", 1 << 30 if never else 0)
     g = torch.Generator().manual_seed(seed)
@@ -22,6 +22,12 @@ def _run(lens, past, hq, hkv, D, seed, monkeypatch, never=False):
         at += n
     kc, vc = (torch.randint(-127, 128, (nb, hkv, 64, D), generator=g, dtype=torch.int8) for _ in range(2))
     ks, vs = (torch.rand(nb, hkv, 64, generator=g) * 0.02 + 1e-4 for _ in range(2))
+    largest = float((vc.abs().amax() * vs.amax()))
+    if stale is not None:                                    # scales of slots that hold no key of these sequences
+        for i, n in enumerate(kv):
+            if n % 64:
+                for t in (ks, vs):
+                    t[int(bt[i, blocks[i] - 1]), :, n % 64:] = stale
     q = torch.randn(sum(lens), hq, D, generator=g).bfloat16()
     cu = [0]
     for n in lens:
@@ -32,7 +38,7 @@ def _run(lens, past, hq, hkv, D, seed, monkeypatch, never=False):
     got = N.paged_attention(c(q), c(kc), c(vc), c(bt), cu, kv, scale, c(ks), c(vs), None, True, None, hq // hkv, 0)
     N.Workspace.get(torch.device("cuda", 0)).check_status()
     # weights are rounded to bf16 (2^-9 each, they add up to one), the output too
-    tol = 2.0 ** -7 * float((vc.abs().amax() * vs.amax()))
+    tol = 2.0 ** -7 * largest
     err = (got.float().cpu() - want).abs().max().item()
     assert err <= tol, (err, tol)
 
@@ -53,3 +59,10 @@ def test_prompt_without_the_copy(monkeypatch):
 @pytest.mark.parametrize("kv", [[1], [16, 17, 31], [33, 64, 65, 127], [300, 900, 2049]])
 def test_steps(D, kv, monkeypatch):
     _run([1] * len(kv), [n - 1 for n in kv], 8, 2, D, D + sum(kv), monkeypatch)
+
+
+@pytest.mark.parametrize("stale", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("lens,past", [([65], [0]), ([100, 190, 64], [0, 3, 1]), ([1, 1], [99, 700])])
+def test_scales_past_the_end(stale, lens, past, monkeypatch):
+    """Slots of the last block beyond a sequence's length keep what an earlier owner left there, overflowed values too."""
+    _run(lens, past, 8, 2, 128, sum(lens), monkeypatch, stale=stale)
