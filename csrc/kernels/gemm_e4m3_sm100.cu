@@ -534,15 +534,19 @@ __global__ void __launch_bounds__(256) split_e4m3_kernel(const __nv_bfloat16* __
 int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes, uint32_t box_rows,
                   uint32_t box_bytes);                                 // quant_gemm_sm100.cu: unswizzled bytes
 
-// One round of CTAs (two per SM up to 32 tokens, see E4Layout), at least four blocks of 128 k in each.
-static int e4_splits(int tiles, int num_kb, int bn) {
-  int s = 1;
-  while (s < 8 && tiles * s * 2 <= (bn <= 32 ? 2 : 1) * 148 && num_kb / (2 * s) >= 4) s *= 2;
-  return s;
+// Parts of a tile's k: as many as one round of clusters holds, at least four blocks of k in each.  GPCs differ in their SMs, so what
+// fits is not a division: clusters of 2, 4 and 8 CTAs that B200 takes at a time, with one and with two CTAs per SM.  us, gated uint4
+// 2 x 11008 x 4096 (86 tiles, one CTA per SM), 16 rows: 31.7 with two parts, 24.3 with one; e4m3 24 rows 33.9 and 24.8; bf16 4608 x
+// 3584 (36 tiles) with its rotation behind it, 16 rows: 16.0 with eight parts, 12.4 with four, 48 rows 23.4 with four, 19.6 with two.
+static int e4_splits(int tiles, int num_kb, int per_sm) {
+  constexpr int kFit[2][3] = {{74, 33, 15}, {148, 71, 33}};
+  int i = 0;
+  while (i < 3 && tiles <= kFit[per_sm - 1][i] && num_kb >> (i + 1) >= 4) ++i;
+  return 1 << i;
 }
 
 template <int BN, bool DUAL, int SRC>
-static int launch_e4(const CUtensorMap& tmW, const CUtensorMap& tmX, const E4Params& p, cudaStream_t st) {
+static int launch_e4(const CUtensorMap& tmW, const CUtensorMap& tmX, E4Params p, cudaStream_t st) {
   using L = E4Layout<BN, DUAL, SRC>;
   const auto kernel = gemm_e4m3_kernel<BN, DUAL, SRC>;
   static bool attr_set = false;
@@ -599,6 +603,7 @@ extern "C" int xft_gemm_e4m3(const void* xs, int x_rows, const float* x_scale, c
   E4Params p{};
   p.N = N; p.T = T; p.K = K; p.dual_off = dual_off; p.out = Y; p.ldo = ldo; p.out_fp32 = out_fp32; p.bias = bias;
   p.residual = (const __nv_bfloat16*)residual; p.ldr = ldr; p.res_scale = res_scale; p.act = act; p.x_scale = x_scale;
+  p.splits = p.group_tiles ? 1 : e4_splits(p.n_tiles * p.t_tiles, p.num_kb, L::CTAS);
   p.x_sum = x_sum; p.scale = scale; p.zero = zero; p.scale_ld = scale_ld; p.status = status; p.col_scale = col_scale;
   p.group_tiles = reinterpret_cast<const int4*>(group_tiles); p.num_group_tiles = num_group_tiles; p.group_w_rows = group_w_rows;
   p.x_lo = xft_split_e4m3_cols(K);
@@ -606,8 +611,6 @@ extern "C" int xft_gemm_e4m3(const void* xs, int x_rows, const float* x_scale, c
   p.num_kb = (K + 127) / 128;
   p.n_tiles = (N + 127) / 128;
   p.t_tiles = group_tiles ? max_tiles : (T + bn - 1) / bn;
-  p.splits = 1;
-  if (!group_tiles) p.splits = e4_splits(p.n_tiles * p.t_tiles, p.num_kb, bn);
   CUtensorMap tmW, tmX;
   int r = src == kSrcU4 ? make_byte_map(&tmW, W, (uint64_t)w_rows, (uint64_t)K / 2, (uint64_t)ldw_bytes, 128, 64)
                         : make_tensor_map(&tmW, W, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw_bytes, 128, 1);
@@ -637,7 +640,6 @@ int launch_w8a8_decode(const void* qx, int ldqx, const void* Wq, int w_rows, int
   p.num_kb = (K + 127) / 128;
   p.n_tiles = (N + 127) / 128;
   p.t_tiles = (T + bn - 1) / bn;
-  p.splits = e4_splits(p.n_tiles * p.t_tiles, p.num_kb, bn);
   CUtensorMap tmW, tmX;
   int r = make_tensor_map(&tmW, Wq, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw, 128, 1);
   if (r) return 1000 - r;
@@ -703,7 +705,6 @@ extern "C" int xft_gemm_bf16_cluster(const void* X, int ldx, const void* W, int 
   p.num_kb = (K + 63) / 64;
   p.n_tiles = (N + 127) / 128;
   p.t_tiles = (T + bn - 1) / bn;
-  p.splits = e4_splits(p.n_tiles * p.t_tiles, p.num_kb, bn);
   CUtensorMap tmW, tmX;
   int r = make_tensor_map(&tmW, W, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw, 128, 2);
   if (r) return 1000 - r;
