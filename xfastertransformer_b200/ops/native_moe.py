@@ -150,11 +150,13 @@ def moe_experts(x, idx, w, experts, act="silu", expert_offset=0, packed=None, ex
     ws = N.Workspace.get(dev)
     lib = _lib()
     avg = max(1, ((T * k if expected_pairs is None else min(int(expected_pairs), T * k)) + E - 1) // E)
-    # An expert with more rows than a tile reads its weights twice, so tiles are about twice the average (64 rows on 8 experts, two
-    # each: 4096 x 14336 210 us with 16 rows, 180 with 32).
+    # An expert with more rows than a tile reads its weights twice, a larger tile costs every expert its finish.  us with tiles of 16 / 32 /
+    # 64 rows, 64 experts of 1408 x 2048 in bf16, average load 12: 220 / 235 / 262, 20: 259 / 255 / 287, 32: 315 / 264 / 320; 8 of 14336 x
+    # 4096, 12: 452 / 454 / 475, 16: 496 / 461 / 483, 32: 634 / 533 / 526, 48: 708 / 606 / 577.  fp8, 64 of 1408 x 2048, 16: 142 / 159 /
+    # 205, 32: 197 / 193 / 255; 8 of 14336 x 4096, 16: 269 / 267 / 304, 32: 349 / 333 / 336, 48: 415 / 413 / 346.
     # 256 rows: two CTAs share a tile (bf16 only).  A group's last tile is half empty on average, which eats the fifth that
     # pairs gain below about 430 rows per expert
-    bn = 16 if avg <= 8 else 32 if avg <= 20 else 64 if avg <= 64 or pk.get("fp8") else 128 if avg < 512 else 256
+    bn = 16 if avg <= (16 if pk.get("fp8") else 12) else 32 if avg <= 32 else 64 if avg <= 64 or pk.get("fp8") else 128 if avg < 512 else 256
     max_rows = T * k
     max_tiles = (max_rows + bn - 1) // bn + E
     idx32 = idx if idx.dtype == torch.int32 else idx.int()
