@@ -66,3 +66,17 @@ def test_steps(D, kv, monkeypatch):
 def test_scales_past_the_end(stale, lens, past, monkeypatch):
     """Slots of the last block beyond a sequence's length keep what an earlier owner left there, overflowed values too."""
     _run(lens, past, 8, 2, 128, sum(lens), monkeypatch, stale=stale)
+
+
+def test_prompt_on_a_full_card(monkeypatch):
+    """Where the copy of the codes has no room, the kernel that reads them where they are takes the prompt, as it did all of them."""
+    empty, refused = torch.empty, []
+
+    def short(*size, **kw):
+        if len(size) == 5 and kw.get("dtype") == torch.bfloat16:
+            refused.append(size)
+            raise torch.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+    monkeypatch.setattr(torch, "empty", short)
+    _run([130, 70], [0, 40], 8, 2, 128, 5, monkeypatch)
+    assert refused

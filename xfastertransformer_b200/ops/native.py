@@ -706,13 +706,18 @@ def paged_attention(q, kc, vc, block_table, cu_q, kv_lens, scale, ks=None, vs=No
             and sinks is None and max_q >= INT8_TC_MIN_Q and max_kv >= INT8_TC_MIN_KV):
         w = (max_kv + 63) // 64
         if B * w * hkv * 2 * 64 * 128 * 2 <= INT8_TC_MAX_COPY:
-            copy = torch.empty(2, B * w, hkv, 64, 128, dtype=torch.bfloat16, device=dev)
-            fn = lib().xft_attn_prefill_tc_int8
-            fn.restype = C.c_int
-            _check(fn(_p(q), _p(out), _p(kc), _p(vc), _p(ks), _p(vs), _p(copy), w, _p(block_table), block_table.stride(0), _p(cu_dev),
-                      _p(kv_dev), B, T, max_q, hq, hkv, g, q_off, bs, nb, C.c_float(scale), _p(ws.status), _stream()), "attn_prefill_tc_int8")
-            ws.launches += 2
-            return out
+            try:
+                copy = torch.empty(2, B * w, hkv, 64, 128, dtype=torch.bfloat16, device=dev)
+            except torch.OutOfMemoryError:
+                copy = None                                # weights and caches fill the card: the kernel below needs no copy
+            if copy is not None:
+                fn = lib().xft_attn_prefill_tc_int8
+                fn.restype = C.c_int
+                _check(fn(_p(q), _p(out), _p(kc), _p(vc), _p(ks), _p(vs), _p(copy), w, _p(block_table), block_table.stride(0), _p(cu_dev),
+                          _p(kv_dev), B, T, max_q, hq, hkv, g, q_off, bs, nb, C.c_float(scale), _p(ws.status), _stream()),
+                       "attn_prefill_tc_int8")
+                ws.launches += 2
+                return out
     rc = lib().xft_paged_attention_ext(_p(q), _p(out), _p(kc), _p(vc), _p(ks), _p(vs), _p(block_table),
                                        block_table.stride(0), _p(cu_dev), _p(kv_dev), B, max_q, hq, hkv, g, q_off, D, bs,
                                        nb, C.c_float(scale), _p(slopes), _p(pl),
