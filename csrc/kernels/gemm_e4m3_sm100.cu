@@ -5,10 +5,10 @@
 //     subnormals and the first binade are equally spaced).
 //
 // An activation becomes the sum of two e4m3 numbers: x / s_t = hi + lo / 16 with s_t a power of two per row.  A bf16 value has
-// eight significant bits, hi takes four and lo the other four, so the sum is x itself down to 2^-15 of the row's maximum and off
-// by at most 2^-23 of that maximum below.  Both halves are columns of one `kind::f8f6f4` MMA (N = 2 BN), sums are fp32.  The
-// expanding kernel (quant_gemm_sm100.cu, still used for int8 and nf4) rounds fp8 x scale to bf16 and spends about 100
-// instructions per weight byte row; here fp8 tiles go from TMA to the tensor core untouched, and uint4 costs one AND and half a
+// eight significant bits, hi takes four and lo the other four, so the sum is x itself down to 2^-13.8 of the row's maximum and off
+// by at most 2^-21.8 of that maximum below (the scaled maximum lies between 224 and 448).  Both halves are columns of one
+// `kind::f8f6f4` MMA (N = 2 BN), sums are fp32.  The expanding kernel (quant_gemm_sm100.cu, still used for int8 and nf4) rounds fp8 x
+// scale to bf16 and spends about 100 instructions per weight byte row; here fp8 tiles go from TMA to the tensor core untouched, and uint4 costs one AND and half a
 // shift per four codes.  Block scales multiply the fp32 sums of 128 k: two TMEM accumulators in turn, the epilogue warps fetch
 // one and add it to registers while the next fills.
 //
