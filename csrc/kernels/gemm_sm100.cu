@@ -547,18 +547,11 @@ int make_tensor_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t c
   return 0;
 }
 
-typedef CUresult (*EncFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                          const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                          CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes,
-                        uint32_t box_rows, uint32_t box_bytes) {
-  static EncFn enc = nullptr;
-  if (!enc) {
-    void* fp = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fp, cudaEnableDefault, &q) != cudaSuccess) return -1;
-    enc = reinterpret_cast<EncFn>(fp);
-  }
+// Bytes [rows, row_bytes] with a pitch of ld_bytes; box = box_bytes x box_rows, not swizzled.
+int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes, uint32_t box_rows,
+                  uint32_t box_bytes) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc) return -1;
   if ((reinterpret_cast<uintptr_t>(ptr) & 15) || (ld_bytes & 15)) return -2;
   cuuint64_t dims[2] = {row_bytes, rows};
   cuuint64_t strides[1] = {ld_bytes};

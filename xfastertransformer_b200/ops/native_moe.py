@@ -79,8 +79,8 @@ def _fp8_packable(gu: "object", dn: "object") -> bool:
 
 
 def _pack_fp8(experts) -> dict:
-    """fp8 experts stay fp8 on the device: the e4m3 matrices and their 128x128 block scales are stacked and the
-    grouped fp8 GEMM expands tiles to bf16 in shared memory on the way to the tensor core."""
+    """fp8 experts stay fp8 on the device: the e4m3 matrices and their 128x128 block scales are stacked; the
+    grouped product takes their tiles to the tensor core as they are (csrc/kernels/gemm_e4m3_sm100.cu)."""
     gu0, dn0 = experts[0]
     I, H = dn0.in_features, dn0.out_features
     E = len(experts)
