@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(256) split_e4m3_kernel(const __nv_bfloat16* __
 }
 
 int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes, uint32_t box_rows,
-                  uint32_t box_bytes);                                 // quant_gemm_sm100.cu: unswizzled bytes
+                  uint32_t box_bytes);                                 // gemm_sm100.cu: unswizzled bytes
 
 // Parts of a tile's k: as many as one round of clusters holds, at least four blocks of k in each.  GPCs differ in their SMs, so what
 // fits is not a division: clusters of 2, 4 and 8 CTAs that B200 takes at a time, with one and with two CTAs per SM.  us, gated uint4
@@ -555,6 +555,7 @@ static int launch_e4(const CUtensorMap& tmW, const CUtensorMap& tmX, E4Params p,
       return 3000 + (int)cudaGetLastError();
     attr_set = true;
   }
+  p.splits = p.group_tiles ? 1 : e4_splits(p.n_tiles * p.t_tiles, p.num_kb, L::CTAS);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.n_tiles * p.t_tiles, p.splits);
   cfg.blockDim = dim3(kE4Threads);
@@ -603,7 +604,6 @@ extern "C" int xft_gemm_e4m3(const void* xs, int x_rows, const float* x_scale, c
   E4Params p{};
   p.N = N; p.T = T; p.K = K; p.dual_off = dual_off; p.out = Y; p.ldo = ldo; p.out_fp32 = out_fp32; p.bias = bias;
   p.residual = (const __nv_bfloat16*)residual; p.ldr = ldr; p.res_scale = res_scale; p.act = act; p.x_scale = x_scale;
-  p.splits = p.group_tiles ? 1 : e4_splits(p.n_tiles * p.t_tiles, p.num_kb, L::CTAS);
   p.x_sum = x_sum; p.scale = scale; p.zero = zero; p.scale_ld = scale_ld; p.status = status; p.col_scale = col_scale;
   p.group_tiles = reinterpret_cast<const int4*>(group_tiles); p.num_group_tiles = num_group_tiles; p.group_w_rows = group_w_rows;
   p.x_lo = xft_split_e4m3_cols(K);
