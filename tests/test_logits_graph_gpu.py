@@ -91,3 +91,34 @@ def test_steps_on_another_stream(monkeypatch, tmp_path):
         outs.append(out)
     for x, y in zip(outs[1], outs[0]):
         _same(x, y)
+
+
+@pytest.mark.parametrize("lens", [[150], [500, 40], [700, 1100]])
+@pytest.mark.parametrize("name", ["tiny-llama", "latent"])
+def test_captured_steps_cut_attention_as_eager_ones(lens, name, monkeypatch, tmp_path):
+    """Batches that are not padded: the table of a captured step is wider, its launches are otherwise those of an eager step, so the
+    logits are the same bits."""
+    from xfastertransformer_b200.tools import synthetic
+    if name == "latent":
+        from xfastertransformer_b200.config import ModelConfig
+        cfg = ModelConfig(model_type="deepseek_moe", num_layer=2, hidden_size=512, head_num=8, kv_head_num=8, size_per_head=128, inter_size=1024,
+                          vocab_size=1024, max_pos_seq_len=4096, q_lora_rank=256, kv_lora_rank=512, qk_nope_head_dim=128, qk_rope_head_dim=64,
+                          v_head_dim=128, moe_intermediate_size=256, first_k_dense_replace=1, dense_experts=1, sparse_experts=16,
+                          routed_scaling_factor=2.5, topk_method="noaux_tc", n_group=4, topk_group=2, num_experts_per_tok=4, norm_topk_prob=True,
+                          scoring_func="sigmoid", activation_type="silu", weight_data_type="bf16", start_id=0, end_id=1)
+        write = synthetic.write_synthetic_checkpoint
+        monkeypatch.setattr(synthetic, "preset", lambda _: cfg)
+        monkeypatch.setattr(synthetic, "write_synthetic_checkpoint", lambda p, c, seed: write(p, c, seed=seed, dtype="bf16", std=0.05))
+    eager, graph = (_model(monkeypatch, tmp_path, on, name, kv_cache_dtype="bf16") for on in (False, True))
+    g = torch.Generator().manual_seed(sum(lens))
+    prompts = [torch.randint(2, 1000, (n,), generator=g).tolist() for n in lens]
+    outs = []
+    for m in (eager, graph):
+        ids, out = m.set_input_cb(prompts, None, 1300).tolist(), []
+        m.forward_cb()
+        for i in range(6):
+            m.set_input_cb([10 + i, 20 + i][:len(lens)], ids)
+            out.append(m.forward_cb())
+        outs.append(out)
+    assert graph.model.runner.graph_launches >= 3
+    assert all(torch.equal(a, b) for a, b in zip(*outs))

@@ -797,8 +797,11 @@ class Decoder:
 
     # -- sizes ------------------------------------------------------------------------------
     def plan_splits(self, B: int, max_kv: int, int8: bool) -> Optional[int]:
-        """Split-KV factor of a captured decode step, or None when every layer plans its own."""
+        """How a captured decode step cuts its attention (latent: CTAs per cluster and clusters), or None when every layer plans its own."""
         from ..ops import native as N
+        if self.spec.attention == "mla":
+            from ..ops.native_latent import mla_splits
+            return mla_splits(B * ((self.hq + 15) // 16), max_kv)
         return N.plan_attn_splits(B, max(self.hkv, 1), self.group, self.D, max_kv, int8)[0]
 
     def kv_geometry(self):

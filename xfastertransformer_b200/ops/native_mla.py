@@ -86,7 +86,7 @@ def mla_attention(q_nope, q_rope, latent_cache, block_table, cu_q, kv_lens, w_uk
     nb, _, bs, W = latent_cache.shape
     chunks = (Hl + 15) // 16
     from .native_latent import mla_scratch, mla_splits
-    nsplit, groups = mla_splits(T * chunks, max_kv)
+    nsplit, groups = (meta.meta.get("nsplit") if meta is not None else None) or mla_splits(T * chunks, max_kv)
     po, pm, cnt = mla_scratch(ws, T * chunks, nsplit, groups, L)
     q_rope = q_rope.contiguous()
     LL = C.c_longlong

@@ -131,8 +131,9 @@ class CudaRunner:
 
     def _logits_key(self, seqs: Sequence):
         """Like `_key`, but the table is as wide as the contexts of this step, rounded up to a power of two (from 8 blocks on):
-        callers of `forward_cb` need not say how long their sequences get.  The split count of the attention is that of an
-        eager step, so that a sequence's logits do not depend on whether its steps were captured."""
+        callers of `forward_cb` need not say how long their sequences get.  The attention is cut as in an eager step of the same
+        sequences (`plan_splits`), so that its sums do not depend on whether the step was captured.  Layers that plan their own cut
+        (layered models) plan on the width of the table: there a captured step may add in another order."""
         B, limit = self._key(seqs)
         longest = max(s.past_len for s in seqs) + 1
         need, W = self.m.cache.blocks_for(longest), 8
@@ -336,7 +337,8 @@ class CudaRunner:
 
     def step_logits(self, seqs: Sequence) -> torch.Tensor:
         """One decode step of `seqs` -> this rank's fp32 logits [len(seqs), vocab slice], in a tensor of the caller's.  Runs on
-        the caller's stream and waits for nothing."""
+        the caller's stream.  The host waits only for a staging buffer that is still being copied, and for the device when a shape
+        is captured."""
         m = self.m
         n = len(seqs)
         self._scratch()                                # both may grow the pools: before the version check below
