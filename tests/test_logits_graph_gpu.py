@@ -93,6 +93,46 @@ def test_steps_on_another_stream(monkeypatch, tmp_path):
         _same(x, y)
 
 
+def test_streams_that_nobody_orders(monkeypatch, tmp_path):
+    """Prompts, eager and captured steps, greedy steps and a pool that moves, each on another stream than the one before, without an
+    event between them: the engine puts its passes in order, whose scratch and caches are the same memory."""
+    eager, graph = (_model(monkeypatch, tmp_path, on) for on in (False, True))
+    streams = [torch.cuda.default_stream(), torch.cuda.Stream(), torch.cuda.Stream()]
+    outs = []
+    for m, mixed in ((eager, False), (graph, True)):
+        out, ids, turn = [], [], 0
+
+        def call(fn):
+            nonlocal turn
+            turn += 1
+            with torch.cuda.stream(streams[turn % 3 if mixed else 0]):
+                out.append(fn())
+
+        def start(prompt, room):
+            ids.extend(m.set_input_cb([prompt], None, room).tolist())
+            return m.forward_cb()
+
+        def step(tokens, greedy=False):
+            m.set_input_cb(tokens, ids, greedy=greedy)
+            return m.forward_cb_greedy() if greedy else m.forward_cb()
+        call(lambda: start(list(range(5, 400)), 600))
+        for i in range(7):
+            call(lambda: step([40 + i]))
+        call(lambda: start(list(range(300)), 6000))
+        for i in range(7):
+            call(lambda: step([60 + i, 80 + i]))
+        for i in range(4):
+            call(lambda: step([90 + i, 95 + i], greedy=True))
+        for i in range(4):
+            call(lambda: step([70 + i, 50 + i]))
+        torch.cuda.synchronize()
+        outs.append(out)
+    assert graph.model.runner.graph_launches >= 8
+    for x, y in zip(outs[1], outs[0]):
+        if x.is_floating_point():
+            _same(x, y)
+
+
 @pytest.mark.parametrize("lens", [[150], [500, 40], [700, 1100]])
 @pytest.mark.parametrize("name", ["tiny-llama", "latent"])
 def test_captured_steps_cut_attention_as_eager_ones(lens, name, monkeypatch, tmp_path):

@@ -10,6 +10,7 @@ once, so steady-state steps allocate only their outputs.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import os
 from typing import Dict, Optional
@@ -71,6 +72,21 @@ def _check(rc: int, what: str) -> None:
         raise KernelError(f"{what} failed with code {rc}")
 
 
+class _Turn:
+    """See turn."""
+    __slots__ = ("ws", "stream")
+
+    def __init__(self, ws):
+        self.ws = ws
+
+    def __enter__(self):
+        self.stream = torch.cuda.current_stream(self.ws.device)
+        self.ws.wait_turn(self.stream)
+
+    def __exit__(self, *exc):
+        self.ws.end_turn(self.stream)
+
+
 class Workspace:
     _by_dev: Dict[int, "Workspace"] = {}
 
@@ -85,6 +101,7 @@ class Workspace:
         self.part_o = None
         self.part_ml = None
         self.launches = 0
+        self.used = self.event = None          # end of the last work that used these buffers, see turn; the event that is used again
 
     @classmethod
     def get(cls, device: torch.device) -> "Workspace":
@@ -105,6 +122,17 @@ class Workspace:
             raise KernelError(f"split-KV scratch too small for {n_o} partial outputs")
         return self.part_o, self.part_ml
 
+    def turn(self):
+        return _Turn(self)
+
+    def wait_turn(self, stream) -> None:
+        if self.used is not None:
+            stream.wait_event(self.used)
+
+    def end_turn(self, stream) -> None:
+        self.used = self.event = self.event or torch.cuda.Event()
+        self.used.record(stream)
+
     def check_status(self) -> None:
         """Read the status word (synchronises).  Raises if any kernel reported a time-out or a
         bad index; the context stays usable."""
@@ -112,6 +140,12 @@ class Workspace:
         if s != 0:
             self.status.zero_()
             raise KernelError(f"kernel status {s}: {STATUS_TEXT.get(s, '?')}")
+
+
+def turn(device: torch.device):
+    """Context of a forward pass, or of anything else that touches the workspace or a model's caches: the caller's stream waits for
+    the end of the last such work, on whatever stream that ran.  The streams of successive calls need no order of the caller's."""
+    return Workspace.get(device).turn() if device.type == "cuda" else contextlib.nullcontext()
 
 
 def launches(device=None) -> int:

@@ -23,6 +23,7 @@ from typing import Dict, List, Sequence
 import torch
 
 from ..models.decoder import Batch
+from ..ops.native import Workspace, turn
 from ..utils import trace
 from . import sampler as S
 
@@ -60,7 +61,6 @@ class CudaRunner:
         self.timing = False               # record a CUDA-event pair around each step's launch
         self.step_events = []
         self._scratch_block = self._scratch_state = None
-        self._tail = None                 # end of the last logits step
         if self.enabled:
             # taken now, while the pools are empty: a block taken after a request reserved its blocks would leave that
             # request one block short and make the pools grow (and move) in the middle of its decode
@@ -267,7 +267,7 @@ class CudaRunner:
         g = self.graphs.get("idle")
         st = self.stream
         st.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(st), torch.no_grad():
+        with torch.cuda.stream(st), turn(self.dev), torch.no_grad():
             if g is None:
                 self.m.decoder.forward_idle()
                 st.synchronize()
@@ -300,14 +300,14 @@ class CudaRunner:
         self._fill(g, seqs, slots)
         st = self.stream
         st.wait_stream(torch.cuda.current_stream())
+        ws = Workspace.get(self.dev)
+        ws.wait_turn(st)
         with torch.cuda.stream(st), torch.no_grad():
             g.dev.copy_(g.host, non_blocking=True)
             if g.graph is None:
                 # eager run (allocates workspaces, JIT-free), then capture
                 self._step_body(g)
                 st.synchronize()
-                from ..ops import native as N
-                ws = N.Workspace.get(self.dev)
                 n0 = ws.launches
                 graph = torch.cuda.CUDAGraph()
                 with _capture(graph, st):
@@ -329,6 +329,7 @@ class CudaRunner:
                 self.kernel_launches += g.kernels
             g.tok_host.copy_(g.tok_dev, non_blocking=True)
         st.synchronize()
+        ws.used = None                                 # nothing is left for the next pass to wait for
         self.h2d_bytes += g.host.numel() * 4
         self.d2h_bytes += g.tok_host.numel() * 8
         return g.tok_host.tolist()[:n_real]
@@ -355,16 +356,12 @@ class CudaRunner:
         g.turn = (g.turn + 1) % self.RING
         copied.synchronize()                           # its last copy to the device is done
         self._fill(g, seqs, slots, host)
-        cur = torch.cuda.current_stream()
-        if self._tail is not None:
-            cur.wait_event(self._tail)                 # buffers of the graphs are shared by the streams of all callers
-        with torch.no_grad():
+        with turn(self.dev), torch.no_grad():          # buffers of the graphs are shared by the streams of all callers
             g.dev.copy_(host, non_blocking=True)
             copied.record()
             if g.graph is None:
                 out = m.decoder.forward(g.batch, m.cache)[:n].clone()      # eagerly: allocates workspaces; then captured
-                from ..ops import native as N
-                ws = N.Workspace.get(self.dev)
+                ws = Workspace.get(self.dev)
                 torch.cuda.synchronize(self.dev)
                 n0 = ws.launches
                 graph = torch.cuda.CUDAGraph()
@@ -375,8 +372,6 @@ class CudaRunner:
                 g.graph.replay()
                 out = g.logits[:n].clone()
                 self.graph_launches += 1
-        self._tail = self._tail or torch.cuda.Event()
-        self._tail.record()
         self.kernel_launches += g.kernels
         self.h2d_bytes += host.numel() * 4
         return out

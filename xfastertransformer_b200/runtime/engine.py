@@ -28,6 +28,7 @@ from .. import ops
 from ..config import KV_DTYPES, ModelConfig, split_hybrid_dtype
 from ..models.decoder import Batch, Decoder  # noqa: F401  (Decoder is re-exported)
 from ..models.registry import decoder_class, family_for
+from ..ops.native import turn
 from ..parallel.dist import CommError, DistContext
 from ..utils import log, trace
 from ..utils.flags import Env
@@ -822,6 +823,10 @@ class Model:
 
     def _run(self, seqs: Sequence[SequenceMeta], logits_all: bool = False) -> torch.Tensor:
         """Run the decoder over the pending inputs of `seqs`; returns this rank's logits slice."""
+        with turn(self.ctx.device):
+            return self._run_groups(seqs, logits_all)
+
+    def _run_groups(self, seqs: Sequence[SequenceMeta], logits_all: bool) -> torch.Tensor:
         if self.ctx.dp_size > 1:
             return self._dp_forward(seqs, logits_all)
         groups = self._groups(seqs)
@@ -830,7 +835,7 @@ class Model:
         if self.env.prefill_overlap and not self.decoder.spec.layered and self.ctx.tp_size > 1 and len(seqs) > 1 and all(len(s.pending) > 1 for s in seqs):
             return self._run_overlapped(seqs, groups, logits_all)
         if len(groups) > 1:
-            return torch.cat([self._run(g, logits_all) for g in groups], dim=0)
+            return torch.cat([self._run_groups(g, logits_all) for g in groups], dim=0)
         b = self.make_batch(seqs, logits_all)
         dec = self.decoder if b.is_decode else self.prefill_decoder
         name = "Next Token" if b.is_decode else "1st Token"

@@ -29,6 +29,8 @@ from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
 
+from ..ops.native import turn
+
 
 class BlockAllocator:
     def __init__(self, num_blocks: int):
@@ -187,11 +189,12 @@ class PagedKVCache:
         if self.max_states and total > self.max_states:
             raise MemoryError(f"{total} state slots needed, the pools are limited to {self.max_states}")
         pools = []
-        for i, (shape, dtype) in enumerate(self.state_geometry):
-            t = torch.zeros(total, *shape, dtype=dtype, device=self.device)
-            if old:
-                t[:old] = self.state[i]
-            pools.append(t)
+        with turn(self.device):
+            for i, (shape, dtype) in enumerate(self.state_geometry):
+                t = torch.zeros(total, *shape, dtype=dtype, device=self.device)
+                if old:
+                    t[:old] = self._leaving(self.state[i])
+                pools.append(t)
         self.state = pools
         self.state_alloc.grow(total)
         self.version += 1
@@ -209,8 +212,9 @@ class PagedKVCache:
 
     def _copy_states(self, src: Sequence[int], dst: Sequence[int]) -> None:
         a, b = (torch.tensor(list(x), dtype=torch.long, device=self.device) for x in (src, dst))
-        for t in self.state:
-            t[b] = t[a]                          # the right side is gathered first
+        with turn(self.device):
+            for t in self.state:
+                t[b] = t[a]                      # the right side is gathered first
 
     # -- capacity -------------------------------------------------------------------
     def bytes_per_block(self) -> int:
@@ -226,6 +230,18 @@ class PagedKVCache:
             return
         if self.max_blocks and total > self.max_blocks:
             raise MemoryError(f"KV cache: {total} blocks needed, the pools are limited to {self.max_blocks}")
+        with turn(self.device):
+            self._grow_pools(total)
+        self.alloc.grow(total)
+        self.version += 1
+
+    def _leaving(self, t: torch.Tensor) -> torch.Tensor:
+        """A pool that is about to be replaced: its memory waits for the stream that copies it, wherever it was allocated."""
+        if t.is_cuda:
+            t.record_stream(torch.cuda.current_stream(t.device))
+        return t
+
+    def _grow_pools(self, total: int) -> None:
         old = self.alloc.num_blocks
         mk = lambda H, d: torch.zeros(total, H, self.block, d, dtype=self.dtype, device=self.device)
         nk, nv, nks, nvs = [], [], [], []
@@ -234,17 +250,17 @@ class PagedKVCache:
             k = mk(H, kd)
             v = mk(H, vd) if vd else None
             if old:
-                k[:old] = self.k[l]
+                k[:old] = self._leaving(self.k[l])
                 if v is not None:
-                    v[:old] = self.v[l]
+                    v[:old] = self._leaving(self.v[l])
             nk.append(k)
             nv.append(v)
             if self.int8:
                 s1 = torch.zeros(total, H, self.block, dtype=torch.float32, device=self.device)
                 s2 = torch.zeros_like(s1)
                 if old:
-                    s1[:old] = self.ks[l]
-                    s2[:old] = self.vs[l]
+                    s1[:old] = self._leaving(self.ks[l])
+                    s2[:old] = self._leaving(self.vs[l])
                 nks.append(s1)
                 nvs.append(s2)
             else:
@@ -254,8 +270,6 @@ class PagedKVCache:
                 self.k[l] = None
                 self.v[l] = None
         self.k, self.v, self.ks, self.vs = nk, nv, nks, nvs
-        self.alloc.grow(total)
-        self.version += 1
 
     def blocks_for(self, n_tokens: int) -> int:
         return (n_tokens + self.block - 1) // self.block
@@ -362,13 +376,14 @@ class PagedKVCache:
             self._copy_states(*zip(*moved))
 
     def _copy_block(self, src: int, dst: int) -> None:
-        for l in range(self.L):
-            self.k[l][dst].copy_(self.k[l][src])
-            if self.v[l] is not None:
-                self.v[l][dst].copy_(self.v[l][src])
-            if self.int8:
-                self.ks[l][dst].copy_(self.ks[l][src])
-                self.vs[l][dst].copy_(self.vs[l][src])
+        with turn(self.device):
+            for l in range(self.L):
+                self.k[l][dst].copy_(self.k[l][src])
+                if self.v[l] is not None:
+                    self.v[l][dst].copy_(self.v[l][src])
+                if self.int8:
+                    self.ks[l][dst].copy_(self.ks[l][src])
+                    self.vs[l][dst].copy_(self.vs[l][src])
 
     def block_table(self, seq_ids: Sequence[int], width: Optional[int] = None) -> torch.Tensor:
         """int32 [len(seq_ids), width] on the host (unused entries 0)."""
