@@ -62,3 +62,12 @@ def test_every_pass_takes_its_turn(monkeypatch, tmp_path):
     m(torch.tensor([[1, 2, 3]]))
     m.generate(torch.tensor([[1, 2, 3]]), max_length=6)
     assert len(passes) >= 7 and min(passes) >= 1 and grown and min(grown) >= 1
+
+
+def test_shapes_leave_in_the_order_of_their_last_use():
+    from xfastertransformer_b200.runtime.cuda_runner import CudaRunner
+    r = CudaRunner.__new__(CudaRunner)
+    r.graphs = {i: object() for i in range(1, 66)}
+    assert r.worth_capturing(None, 1) and len(r.graphs) == 65
+    assert not r.worth_capturing(None, 100)                  # a new shape: the one unused for longest makes room
+    assert 1 in r.graphs and 2 not in r.graphs and len(r.graphs) == 64

@@ -29,14 +29,14 @@ from . import sampler as S
 
 
 @contextlib.contextmanager
-def _capture(graph, stream):
+def _capture(graph, stream, pool=None):
     """torch.cuda.graph without the garbage collector: a collection in the middle of a capture may destroy the graphs of a
     model that has gone out of use, which a capturing stream does not permit."""
     was = gc.isenabled()
     gc.disable()
     try:
         # thread_local: what other threads of the program do on the GPU meanwhile is no concern of this capture
-        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        with torch.cuda.graph(graph, pool=pool, stream=stream, capture_error_mode="thread_local"):
             yield
     finally:
         if was:
@@ -60,6 +60,8 @@ class CudaRunner:
         self.kernel_launches = 0          # kernels of this library launched through replayed graphs / eager steps
         self.timing = False               # record a CUDA-event pair around each step's launch
         self.step_events = []
+        # logits graphs run one after the other (`turn`) and their result is copied at once, so they share what they compute in
+        self._pool = torch.cuda.graph_pool_handle()
         self._scratch_block = self._scratch_state = None
         if self.enabled:
             # taken now, while the pools are empty: a block taken after a request reserved its blocks would leave that
@@ -147,7 +149,9 @@ class CudaRunner:
         key = key or self._key(seqs)
         hit = key in self.graphs or key == getattr(self, "_last_key", None)
         self._last_key = key
-        if len(self.graphs) > 64 and key not in self.graphs:      # bound the memory held by captured shapes
+        if key in self.graphs:
+            self.graphs[key] = self.graphs.pop(key)               # the order is that of the last use
+        elif len(self.graphs) > 64:                               # bound the memory held by captured shapes
             self.graphs.pop(next(iter(self.graphs)))
         return hit
 
@@ -365,7 +369,7 @@ class CudaRunner:
                 torch.cuda.synchronize(self.dev)
                 n0 = ws.launches
                 graph = torch.cuda.CUDAGraph()
-                with torch.cuda.stream(self.stream), _capture(graph, self.stream):
+                with torch.cuda.stream(self.stream), _capture(graph, self.stream, self._pool):
                     g.logits = m.decoder.forward(g.batch, m.cache)
                 g.graph, g.kernels = graph, ws.launches - n0
             else:
