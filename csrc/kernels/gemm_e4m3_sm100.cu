@@ -102,15 +102,23 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
   constexpr int NACC = L::NACC, STAGES = L::STAGES;
   constexpr int NB = SRC == kSrcI8 || SRC == kSrcBf16 ? BN : 2 * BN;   // columns of an accumulator: hi [BN], lo [BN]
   constexpr int ACC = NB * NACC;
-  constexpr int BUFS = SRC == kSrcFp8 ? 2 : 1;
+  // bf16: k in PARTS pieces with an accumulator each.  The tensor core drops bits below an accumulator's last one at every step, so
+  // its error grows with the k it adds up: 12288 x 4096 against 64 bits 2.1e-6 (2 CTAs per tile) and 4.4e-6 (one) of the result with
+  // one accumulator, 4.8e-7 and 1.0e-6 with four; the kernels that had these products, 1.4e-6.  It costs 0.1 to 0.3 us of a launch.
+  constexpr int PARTS = SRC == kSrcBf16 ? 4 : 1;
+  // 64 rows fetch an accumulator as soon as its k is through, beside the main loop; fewer rows all at once at the end, where a short
+  // stream pays for one wait and not for four.
+  constexpr bool EARLY = PARTS > 1 && BN == 64;
+  constexpr int BUFS = SRC == kSrcFp8 ? 2 : PARTS;
   constexpr uint32_t TMEM_COLS = BUFS * ACC < 32 ? 32 : BUFS * ACC;
+  static_assert(TMEM_COLS * L::CTAS <= 512, "accumulators of the resident CTAs");
   constexpr uint32_t IDESC = SRC == kSrcI8 ? umma_idesc(128, BN, 1, 1, 2) : SRC == kSrcBf16 ? umma_idesc(128, BN, 1, 1, 1) : umma_idesc(128, 2 * BN, 0, 0, 1);
   constexpr int HB = BN / 2;                                           // tokens per thread: two warps share a row of the tile
   constexpr int TILE_A = 128 * 128;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tmem_full[2], tmem_empty[2], a_ready[2], a_empty[2];
+  __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], tmem_full[PARTS > 2 ? PARTS : 2], tmem_empty[2], a_ready[2], a_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_group[4];
   __shared__ float s_ssq[SRC == kSrcBf16 ? BN : 1];                    // bf16: sums of squares of the tokens over this CTA's k
@@ -134,6 +142,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
       mbar_init(&a_ready[a], 256);
       mbar_init(&a_empty[a], 1);
     }
+    for (int a = 2; a < PARTS; ++a) mbar_init(&tmem_full[a], 1);
     fence_barrier_init();
     fence_proxy_async();
     tma_prefetch_desc(&tmW);
@@ -159,6 +168,9 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
   const int x_row0 = grouped ? s_group[1] : tile_t * BN;
   const int x_rows = grouped ? s_group[2] : min(BN, p.T - x_row0);
   const int kend = x_rows > 0 ? kb1 : kb0;                             // nothing to do for a tile without rows
+  // blocks per accumulator, and accumulators: up to 512 k stay in one
+  const int part_kb = max((kb1 - kb0 + PARTS - 1) / PARTS, 8);
+  const int parts = 1 + (kb1 - kb0 > part_kb) + (kb1 - kb0 > 2 * part_kb) + (kb1 - kb0 > 3 * part_kb);
 
   uint8_t* ring = smem + L::A_RING;
   if (warp == 0) {
@@ -196,6 +208,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
       const uint64_t bdesc0 = stage0 + (L::STAGE - L::B_BYTES) / 16;
       const uint64_t a0 = SRC == kSrcU4 ? umma_desc_k128(smem_u32(smem)) : stage0;
       Ring r = {0, 0}, b = {0, 0};                                     // stage; buffer of expanded codes or accumulator
+      int in_part = 0, part = 0;                                       // blocks in this accumulator; which it is
       bool ok = true;
       for (int kb = kb0; kb < kend; ++kb, r.next(STAGES), b.next(2)) {
         if (SRC == kSrcFp8) ok = mbar_wait(&tmem_empty[b.s], b.ph ^ 1, p.status, XFT_ERR_WAIT_TMEM);
@@ -205,10 +218,10 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
         tcgen05_fence_after();
         const uint64_t bd = bdesc0 + (uint64_t)(r.s * (L::STAGE / 16));
         const uint64_t ad = a0 + (uint64_t)(SRC == kSrcU4 ? b.s * (L::A_BYTES / 16) : r.s * (L::STAGE / 16));
-        const uint32_t acc = tmem_base + (SRC == kSrcFp8 ? b.s * ACC : 0);
+        const uint32_t acc = tmem_base + (SRC == kSrcFp8 ? b.s * ACC : PARTS > 1 ? part * ACC : 0);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {                                  // 4 x 32 k
-          const uint32_t on = (SRC != kSrcFp8 && kb > kb0) || k > 0;
+          const uint32_t on = (SRC != kSrcFp8 && (PARTS > 1 ? in_part > 0 : kb > kb0)) || k > 0;
           auto mma = [&](uint32_t d, uint64_t a) {
             if constexpr (SRC == kSrcBf16) umma_bf16(d, a, bd + 2 * k, IDESC, on);
             else if constexpr (SRC == kSrcI8) umma_i8(d, a, bd + 2 * k, IDESC, on);
@@ -218,10 +231,15 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
           if (DUAL) mma(acc + NB, ad + TILE_A / 16 + 2 * k);
         }
         tcgen05_commit(&empty_bar[r.s]);
+        if (PARTS > 1 && (++in_part == part_kb || kb + 1 == kend)) {
+          if (EARLY) tcgen05_commit(&tmem_full[part]);
+          ++part;
+          in_part = 0;
+        }
         if (SRC == kSrcU4) tcgen05_commit(&a_empty[b.s]);
         if (SRC == kSrcFp8) tcgen05_commit(&tmem_full[b.s]);
       }
-      if (SRC != kSrcFp8 && kend > kb0 && ok) tcgen05_commit(&tmem_full[0]);
+      if (SRC != kSrcFp8 && !EARLY && kend > kb0 && ok) tcgen05_commit(&tmem_full[0]);
     }
   }
 
@@ -289,10 +307,40 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
       }
       ok = __all_sync(0xffffffffu, mbar_wait(&tmem_full[0], 0, p.status, XFT_ERR_WAIT_TMEM));
       tcgen05_fence_after();
-      if (ok) {                                                        // s32 (or fp32), kept as they are
+      if (ok && (PARTS == 1 || EARLY)) {                               // s32 (or fp32), kept as they are
         tmem_ld_cols<HB>(taddr, reinterpret_cast<uint32_t*>(g[0]));
         if constexpr (DUAL) tmem_ld_cols<HB>(taddr + NB, reinterpret_cast<uint32_t*>(g[1]));
         tmem_ld_wait();
+      }
+      if constexpr (PARTS > 1 && !EARLY) {
+        if (ok) {
+#pragma unroll
+          for (int a = 0; a < NACC; ++a) {
+            uint32_t v[PARTS - 1][HB];
+            tmem_ld_cols<HB>(taddr + a * NB, reinterpret_cast<uint32_t*>(g[a]));
+#pragma unroll
+            for (int i = 1; i < PARTS; ++i)
+              if (i < parts) tmem_ld_cols<HB>(taddr + i * ACC + a * NB, v[i - 1]);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 1; i < PARTS; ++i)
+#pragma unroll
+              for (int j = 0; j < HB; ++j) g[a][j] += i < parts ? __uint_as_float(v[i - 1][j]) : 0.f;
+          }
+        }
+      }
+      if constexpr (EARLY) for (int i = 1; i < parts && ok; ++i) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&tmem_full[i], 0, p.status, XFT_ERR_WAIT_TMEM));
+        tcgen05_fence_after();
+        if (!ok) break;
+        uint32_t v[NACC][HB];
+        tmem_ld_cols<HB>(taddr + i * ACC, v[0]);
+        if constexpr (DUAL) tmem_ld_cols<HB>(taddr + i * ACC + NB, v[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int a = 0; a < NACC; ++a)
+#pragma unroll
+          for (int j = 0; j < HB; ++j) g[a][j] += __uint_as_float(v[a][j]);
       }
     } else {
       // codes to bytes: a 16-byte piece holds 32 of them; the even ones go to one swizzled 16-byte piece of the operand row,

@@ -76,3 +76,21 @@ def test_a_kernel_asked_for_by_name_is_taken(name, value, monkeypatch):
     finally:
         monkeypatch.undo()
         Env.get().reload()
+
+
+@pytest.mark.parametrize("T", [16, 33, 64])
+@pytest.mark.parametrize("N,K", [(12288, 4096), (4096, 4096), (896, 4864)])
+def test_sums_are_no_further_off_than_those_of_the_older_kernels(T, N, K, monkeypatch):
+    """fp32 results against 64 bits.  The sums of an accumulator are cut at its last bit, so their error grows with the k in it; a
+    quarter of room for another order of the same sums."""
+    from xfastertransformer_b200.ops import native as Nat
+    g = torch.Generator(device="cuda").manual_seed(N + T)
+    x = torch.randn(T, K, generator=g, device="cuda").bfloat16()
+    W = make_linear(torch.randn(N, K, generator=g, device="cuda") * 0.02, "bf16").to("cuda")
+    want = x.double() @ W.w.double().t()
+    errors = []
+    for use in (Nat._use_cluster, lambda *a: False):
+        monkeypatch.setattr(Nat, "_use_cluster", use)
+        errors.append(((Nat.linear(x, W, out_dtype=torch.float32).double() - want).norm() / want.norm()).item())
+    Nat.Workspace.get(x.device).check_status()
+    assert errors[0] <= 1.25 * errors[1], errors
