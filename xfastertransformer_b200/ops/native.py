@@ -356,14 +356,13 @@ def pick_bn(T: int) -> int:
     return 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128 if T <= 128 else 256
 
 
-def _use_cluster(T, N, K, gated, rms=False) -> bool:
+def _use_cluster(T, N, K, gated) -> bool:
     """Whether a decode-size product (T <= 64) runs on the pipeline of gemm_bf16_cluster (gemm_e4m3_sm100.cu), on B200 the faster one
     but for two ends: above 32 rows one CTA fits an SM there, and with more tiles than SMs nothing hides its finish (32000 x 4096,
     64 rows 68 us, the tile-per-CTA kernel 60; 12288 x 4096 27 and 40; gated products have twice the stream per tile: 2 x 28672 x
     8192 163 and 185), and gated products of less than half a million weights a half (2 x 256 x 512, 8 rows 5.5 us and 4.8;
-    2 x 2816 x 1024 6.2 and 6.7).  With a folded norm (`rms`) the sums of squares of its rows have too short a stream to hide behind up to
-    five million (2 x 4864 x 896, 4 rows 9.6 and 8.2, 24 rows 13.2 and 11.9; 2 x 5632 x 2048 12.3 and 19.1)."""
-    if not _ENV().gemm_cluster or (gated and N * K < (5 << 20 if rms and T <= 32 else 1 << 19)):
+    2 x 2816 x 1024 6.2 and 6.7)."""
+    if not _ENV().gemm_cluster or (gated and N * K < 1 << 19):
         return False
     return T <= 32 or gated or N <= 148 * 128
 
@@ -468,7 +467,7 @@ def linear_rms(x, W, eps, bias=None, act=None, gated=False, out_dtype=None):
     assert w.dtype == torch.bfloat16 and w.stride(1) == 1 and w.shape[1] == K and x2.dtype == torch.bfloat16
     fp32 = out_dtype == torch.float32
     out = torch.empty(T, N, dtype=torch.float32 if fp32 else torch.bfloat16, device=x.device)
-    if _use_cluster(T, N, K, gated, True):
+    if _use_cluster(T, N, K, gated):
         _gemm_cluster(x2, ldx, w, out, T, N, K, gated, N if gated else 0, bias, None, 0, 1.0, act, eps)
         return out.view(*x.shape[:-1], N)
     if _sk_choice(T, N, K, gated):
