@@ -14,8 +14,8 @@
 // ldmatrix by mma.sync.m16n8k16 (bf16 in, fp32 accumulate).  Decode is bandwidth-bound (every K/V byte is
 // read once): a CTA owns one kv head of one sequence and a slice of its blocks, the GQA group's query
 // heads are the 16 MMA rows, the four warps walk different tiles and merge at the end; the slice that arrives
-// last merges all slices.  bf16 caches are fed by TMA into a CTA-wide ring (attn_decode_tma_kernel); int8 caches
-// keep the cp.async path, which converts to bf16 on the way into shared memory.  Prefill gives each warp 16 query rows of one head and shares K/V tiles
+// last merges all slices.  bf16 caches, and int8 caches with heads of 128, are fed by TMA into a CTA-wide ring (attn_decode_tma_kernel,
+// attn_decode_i8_kernel); other int8 caches are converted to bf16 on the way into shared memory.  Prefill gives each warp 16 query rows of one head and shares K/V tiles
 // across the CTA.
 //
 // The EXT instantiations add, with their constants as launch parameters: a sliding window with kept first keys (position
@@ -422,7 +422,8 @@ __global__ void __launch_bounds__(128) attn_prefill_kernel(const AttnParams p) {
 // Tail of a decode CTA: merge the four consumer warps' (m, l, O) through shared memory `mo` ([4][16][HD+2] floats),
 // then either store the result (nsplit == 1) or write this slice's partial and let the slice that arrives last
 // merge all slices of the (sequence, kv head) — no second kernel, no spinning.  Every thread of the CTA calls it.
-template <int HD, class WA>
+// APART: column n of accumulator j is head feature n * HD / 8 + j (attn_decode_i8_kernel), else j * 8 + n.
+template <int HD, bool APART = false, class WA>
 __device__ __forceinline__ void decode_finish(const AttnParams& p, WA& wa, float* mo, bool consumer, int warp, int lane,
                                               int tid, int nthreads, int nq, int h_lo, int b, int tok, int split) {
   constexpr int RS = HD + 2;
@@ -430,11 +431,12 @@ __device__ __forceinline__ void decode_finish(const AttnParams& p, WA& wa, float
   if (consumer) {
 #pragma unroll
     for (int j = 0; j < HD / 8; ++j) {
-      const int d = j * 8 + 2 * (lane & 3);
+      constexpr int STEP = APART ? HD / 8 : 1;
+      const int d = APART ? 2 * (lane & 3) * STEP + j : j * 8 + 2 * (lane & 3);
       mo[(warp * 16 + r0) * RS + d] = wa.o[j][0];
-      mo[(warp * 16 + r0) * RS + d + 1] = wa.o[j][1];
+      mo[(warp * 16 + r0) * RS + d + STEP] = wa.o[j][1];
       mo[(warp * 16 + r1) * RS + d] = wa.o[j][2];
-      mo[(warp * 16 + r1) * RS + d + 1] = wa.o[j][3];
+      mo[(warp * 16 + r1) * RS + d + STEP] = wa.o[j][3];
     }
     if ((lane & 3) == 0) {
       mo[(warp * 16 + r0) * RS + HD] = wa.m[0];
@@ -794,6 +796,178 @@ __global__ void __launch_bounds__(160, (HD <= 128 ? 2 : 1)) attn_decode_tma_kern
   decode_finish<HD>(p, wa, reinterpret_cast<float*>(ring), warp < 4, warp, lane, tid, 160, nq, h_lo, b, tok, split);
 }
 
+// ------------------------------------------------------------------------------------------ decode, int8 cache
+// int8 caches with heads of 128.  The same ring, of codes and scales: a tile is 64 keys, 8 KB of K, 8 KB of V (a row of 128 codes is one
+// 128-byte swizzled row) and their scales.  Nothing is converted in shared memory: the order of the contraction is free, so a thread
+// takes 32 neighbouring codes of a key for the eight steps of S (the query's fragments are in the same order), and 16 neighbouring
+// features of four keys for the 16 column blocks of P V, in 16-byte reads without bank conflicts.  Two codes become two bf16 numbers
+// in three instructions: 128 + the low seven bits, minus 128 or 256 by the sign, all exact.
+// Bound by the instructions of a tile (about 550 per warp and 16 keys, a quarter of them conversions) and, where splits are short, by
+// start and merge.  The kernel that converts on the way into shared memory (attn_decode_kernel, still used for other head sizes) spent its
+// time on one-per-code conversions (16 per cycle and SM) and on writing and reading tiles of twice the size.  us, that / here: 8
+// sequences of 2870 keys, 32 and 8 heads 33.4 / 21.5; 32 of 2250 77.6 / 41.5; 16 of 1000, 32 heads 72.4 / 39.9; 1 of 500 12.6 / 8.2;
+// 64 of 200, 64 and 8 heads 24.9 / 17.2.
+constexpr int kI8Stage = 2 * kDecTile * 128 + 2 * kDecTile * 4;
+constexpr int kI8StageBytes = (kI8Stage + 1023) / 1024 * 1024;           // tiles start on 1024 bytes
+constexpr int kI8Stages = 5;
+constexpr int kI8Smem = kI8Stages * kI8StageBytes + 1024;
+
+// The codes in the low bytes of both halves as bf16
+__device__ __forceinline__ uint32_t codes_bf16(uint32_t w) {
+  uint32_t a, b;                                           // (w & mask) | 0x43004300 in one instruction each: left to itself the compiler takes two
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(a) : "r"(w), "r"(0x007f007fu), "r"(0x43004300u));
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(b) : "r"(w), "r"(0x00800080u), "r"(0x43004300u));
+  const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&d);
+}
+
+__global__ void __launch_bounds__(160, 2) attn_decode_i8_kernel(const __grid_constant__ CUtensorMap tmK,
+                                                                const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
+  constexpr int HD = 128, KT = kDecTile, KW = KT / 4;
+  extern __shared__ __align__(1024) uint8_t smem_dyn[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t full_bar[kI8Stages], empty_bar[kI8Stages];
+  __shared__ int s_blk[kDecMaxBlocks];
+  __shared__ int s_abort;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int i = 0; i < kI8Stages; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 4); }
+    s_abort = 0;
+    fence_barrier_init();
+  }
+  if (warp == 4 && lane == 0) { tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
+  grid_dep_launch();
+  // what may be read before grid_dep_wait(): see attn_decode_tma_kernel
+  const int b = blockIdx.x;
+  const int qchunks = (p.group + 15) / 16;
+  const int kvh = blockIdx.y / qchunks, qc = blockIdx.y % qchunks;
+  const int split = blockIdx.z;
+  const int kv_len = p.kv_lens[b];
+  const int tok = p.cu_q[b];
+  const int h_lo = max(0, kvh * p.group - p.q_off) + qc * 16;
+  const int h_hi = min(min(p.hq, (kvh + 1) * p.group - p.q_off), h_lo + 16);
+  const int nq = h_hi - h_lo;
+  if (nq <= 0) return;
+  const int ntiles = (kv_len + KT - 1) / KT;
+  const int per = (ntiles + p.nsplit - 1) / p.nsplit;
+  const int t_begin = split * per, t_end = min(ntiles, t_begin + per);
+  const int nloc = max(t_end - t_begin, 0);
+  const int* bt = p.block_table + (size_t)b * p.bt_stride;
+  const int tiles_per_block = p.bs / KT;
+  auto block_of = [&](int t) {
+    int blk = bt[t / tiles_per_block];
+    if (blk < 0 || blk >= p.num_blocks) { if (p.status) atomicCAS(p.status, 0, XFT_ERR_BOUNDS); blk = 0; }
+    return blk;
+  };
+  for (int i = tid; i < min(nloc, kDecMaxBlocks); i += 160) s_blk[i] = block_of(t_begin + i);
+  __syncthreads();
+  const int npre = max(0, min(min(kI8Stages, nloc), ntiles - 1 - t_begin));      // the newest token's tile is the last one
+  auto issue_tile = [&](int n) {
+    const int st = n % kI8Stages, t = t_begin + n;
+    const int row = ((n < kDecMaxBlocks ? s_blk[n] : block_of(t)) * p.hkv + kvh) * p.bs + (t % tiles_per_block) * KT;
+    uint8_t* to = ring + st * kI8StageBytes;
+    mbar_expect_tx(&full_bar[st], kI8Stage);
+    tma_load_2d(to, &tmK, &full_bar[st], 0, row, kEvictFirst);
+    tma_load_2d(to + KT * HD, &tmV, &full_bar[st], 0, row, kEvictFirst);
+    bulk_load(to + 2 * KT * HD, p.ks + row, KT * 4, &full_bar[st]);
+    bulk_load(to + 2 * KT * HD + KT * 4, p.vs + row, KT * 4, &full_bar[st]);
+  };
+  if (warp == 4 && elect_one())
+    for (int n = 0; n < npre; ++n) issue_tile(n);
+  grid_dep_wait();
+
+  WarpAttn<HD, KW> wa;
+  wa.init();
+  if (warp == 4) {
+    if (elect_one()) {
+      for (int n = npre; n < nloc; ++n) {
+        const int st = n % kI8Stages;
+        if (!mbar_wait(&empty_bar[st], ((n / kI8Stages) & 1) ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) { s_abort = 1; break; }
+        issue_tile(n);
+      }
+    }
+  } else {
+    const int r0 = lane >> 2, r1 = r0 + 8, t = lane & 3;
+    // step k: features 32 t + 4 k .. + 3 of both rows, the even ones and the odd ones, as a word's codes come apart
+    uint32_t qa[HD / 16][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bf16* q = p.q + ((size_t)tok * p.hq + h_lo) * HD + t * 32 + i * 8;
+      const uint4 a = r0 < nq ? *reinterpret_cast<const uint4*>(q + r0 * HD) : make_uint4(0, 0, 0, 0);
+      const uint4 c = r1 < nq ? *reinterpret_cast<const uint4*>(q + r1 * HD) : make_uint4(0, 0, 0, 0);
+      qa[2 * i][0] = __byte_perm(a.x, a.y, 0x5410); qa[2 * i][1] = __byte_perm(c.x, c.y, 0x5410);
+      qa[2 * i][2] = __byte_perm(a.x, a.y, 0x7632); qa[2 * i][3] = __byte_perm(c.x, c.y, 0x7632);
+      qa[2 * i + 1][0] = __byte_perm(a.z, a.w, 0x5410); qa[2 * i + 1][1] = __byte_perm(c.z, c.w, 0x5410);
+      qa[2 * i + 1][2] = __byte_perm(a.z, a.w, 0x7632); qa[2 * i + 1][3] = __byte_perm(c.z, c.w, 0x7632);
+    }
+    Ring r = {0, 0};
+    for (int n = 0; n < nloc; ++n, r.next(kI8Stages)) {
+      const int st = r.s;
+      if (!mbar_wait(&full_bar[st], r.ph, p.status, XFT_ERR_WAIT_FULL)) { s_abort = 1; break; }
+      const uint8_t* kt = ring + st * kI8StageBytes + warp * KW * HD;      // this warp's 16 keys
+      const uint8_t* vt = kt + KT * HD;
+      const float* scales = reinterpret_cast<const float*>(ring + st * kI8StageBytes + 2 * KT * HD) + warp * KW;
+      const int key0 = (t_begin + n) * KT + warp * KW;
+      if (key0 < kv_len) {
+        float s[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint8_t* row = kt + (j * 8 + r0) * HD;
+          const uint4 lo = *reinterpret_cast<const uint4*>(row + (((2 * t) ^ r0) << 4));
+          const uint4 hi = *reinterpret_cast<const uint4*>(row + (((2 * t + 1) ^ r0) << 4));
+          const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+          s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) mma16816(s[j], qa[k], codes_bf16(w[k]), codes_bf16(w[k] >> 8));
+        }
+        float vs[2][2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float2 ks2 = *reinterpret_cast<const float2*>(scales + j * 8 + 2 * t);
+          const float2 vs2 = *reinterpret_cast<const float2*>(scales + KT + j * 8 + 2 * t);
+          const int left = kv_len - key0 - j * 8 - 2 * t;  // slots past the end hold whatever their last owner left, scales too
+          vs[j][0] = left > 0 ? vs2.x : 0.f;
+          vs[j][1] = left > 1 ? vs2.y : 0.f;
+          s[j][0] = left > 0 ? s[j][0] * p.scale * ks2.x : -INFINITY;
+          s[j][1] = left > 1 ? s[j][1] * p.scale * ks2.y : -INFINITY;
+          s[j][2] = left > 0 ? s[j][2] * p.scale * ks2.x : -INFINITY;
+          s[j][3] = left > 1 ? s[j][3] * p.scale * ks2.y : -INFINITY;
+        }
+        wa.softmax_update(s, nullptr, lane);
+        uint32_t a[4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          a[2 * j] = pack_bf16(s[j][0] * vs[j][0], s[j][1] * vs[j][1]);
+          a[2 * j + 1] = pack_bf16(s[j][2] * vs[j][0], s[j][3] * vs[j][1]);
+        }
+        uint4 v[4];                                        // 16 features of keys 2 t, 2 t + 1 and of those 8 further on
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int key = (i >> 1) * 8 + 2 * t + (i & 1);
+          v[i] = *reinterpret_cast<const uint4*>(vt + key * HD + ((r0 ^ (key & 7)) << 4));
+        }
+#pragma unroll
+        for (int d = 0; d < 16; d += 2) {                  // features d, d + 1 of two keys in a word
+          auto pair = [&](int i) { return __byte_perm((&v[i].x)[d >> 2], (&v[i + 1].x)[d >> 2], d & 2 ? 0x7632 : 0x5410); };
+          const uint32_t x = pair(0), y = pair(2);
+          mma16816(wa.o[d], a, codes_bf16(x), codes_bf16(y));
+          mma16816(wa.o[d + 1], a, codes_bf16(x >> 8), codes_bf16(y >> 8));
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty_bar[st]);
+    }
+    wa.reduce_l();
+  }
+  __syncthreads();
+  if (s_abort) {
+    const long long t0 = clock64();                        // as in attn_decode_tma_kernel
+    while (clock64() - t0 < 2000000LL) {}
+    return;
+  }
+  decode_finish<HD, true>(p, wa, reinterpret_cast<float*>(ring), warp < 4, warp, lane, tid, 160, nq, h_lo, b, tok, split);
+}
+
 // The same for batches whose (sequence, kv head) pairs are more than the CTAs that fit the GPU: two CTAs per SM walk the pairs, and
 // the producer goes on to the next pair's tiles while the four warps finish this one.  A CTA per pair pays its start (barriers,
 // block table, query, first tile) in every round, which short contexts feel: 32 heads of 128, 32 sequences of 130 keys 22.7 us with
@@ -1042,6 +1216,20 @@ static int launch_decode_tma(const AttnParams& p, int B, bool brief, cudaStream_
   return (int)cudaGetLastError();
 }
 
+static int launch_decode_i8(const AttnParams& p, int B, cudaStream_t st) {
+  CUtensorMap tmK, tmV;
+  const uint64_t rows = (uint64_t)p.num_blocks * p.hkv * p.bs;
+  if (make_tensor_map(&tmK, p.kc, rows, 128, 128, kDecTile, 1) || make_tensor_map(&tmV, p.vc, rows, 128, 128, kDecTile, 1)) return -4;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(attn_decode_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kI8Smem) != cudaSuccess) return -5;
+    attr_set = true;
+  }
+  const cudaError_t e = launch_pdl(attn_decode_i8_kernel, dim3(B, p.hkv * ((p.group + 15) / 16), p.nsplit), dim3(160), (size_t)kI8Smem, st,
+                                   tmK, tmV, p);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
 template <bool EXT>
 static int launch_attention(const AttnParams& p, int B, int max_q, int HD, int decode, cudaStream_t st) {
   const bool int8 = p.ks != nullptr;
@@ -1053,6 +1241,10 @@ static int launch_attention(const AttnParams& p, int B, int max_q, int HD, int d
       if (HD == 256) return launch_decode_tma<256, EXT>(p, B, decode == 3, st);
       return -1;
     }
+    // codes through the ring: plain heads of 128 whose scales a bulk copy and whose queries 16-byte loads can start at
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p.kc) | reinterpret_cast<uintptr_t>(p.vc) | reinterpret_cast<uintptr_t>(p.ks) |
+                         reinterpret_cast<uintptr_t>(p.vs) | reinterpret_cast<uintptr_t>(p.q);
+    if (!EXT && int8 && HD == 128 && !p.slopes && decode != 2 && !(at & 15)) return launch_decode_i8(p, B, st);
     // per-warp K+V tiles of 16 KB: a CTA stays at ~64 KB so three CTAs (12 warps) overlap loads and math per SM
     if (HD == 64) return launch_decode<64, 64, EXT>(p, B, int8, st);
     if (HD == 128) return launch_decode<128, 32, EXT>(p, B, int8, st);
