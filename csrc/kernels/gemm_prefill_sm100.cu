@@ -67,6 +67,8 @@ struct PrefillParams {
   // W8A8: int8 X and W, see xft_w8a8_gemm (all per token or per weight row)
   const float* a_scale; const float* a_zero; const float* a_qsum; const float* w_scale; const float* w_zero; const float* w_sum;
   int dual_rows;                         // weight rows between a gate feature and its up feature (ungated: all)
+  // weights of codes in bf16: w_scale and w_zero per weight row, and the rows' sums of X
+  const float* x_sum;
   BulkArParams ar;
 };
 
@@ -445,10 +447,13 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_kernel(const __grid_const
 // up rows.  Both producers signal the first CTA's full barrier; a commit frees the stage in both.
 //
 // NCOL: accumulator columns of a tile (gated: half of them gate, half up).
+// SRC: bf16 operands; int8 operands of W8A8; bf16 activations and codes (int8 or uint4, exact in bf16, see xft_gemm_codes_tm), whose
+// scale and zero point per weight row come in with the epilogue.
+enum { kTmBf16 = 0, kTmI8 = 1, kTmCodes = 2 };
 constexpr int kPrefillTmThreads = 320;      // producer, MMA, two epilogue warps per quarter of the accumulator's rows
 __host__ __device__ constexpr int prefill_tm_stages(int stage_bytes) { return 196 * 1024 / stage_bytes < kPrefillMaxStages ? 196 * 1024 / stage_bytes : kPrefillMaxStages; }
 
-template <int NCOL, bool DUAL, int CG, bool I8 = false>
+template <int NCOL, bool DUAL, int CG, int SRC = kTmBf16>
 __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(const __grid_constant__ CUtensorMap tmX,
                                                                  const __grid_constant__ CUtensorMap tmW,
                                                                  const PrefillParams p) {
@@ -459,9 +464,10 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int STAGES = prefill_tm_stages(STAGE_BYTES);
   constexpr uint32_t TMEM_COLS = 2 * NCOL;               // double-buffered accumulators
+  constexpr bool I8 = SRC == kTmI8, CODES = SRC == kTmCodes;
   constexpr int KEL = I8 ? 128 : 64;                     // k of a step: 128 bytes of a row
   constexpr uint32_t IDESC = umma_idesc(TOK, NCOL, 1, 1, I8 ? 2 : 1);
-  constexpr int CW = DUAL || I8 ? 16 : 32;               // columns of an epilogue step: registers for what it holds at once
+  constexpr int CW = DUAL || SRC != kTmBf16 ? 16 : 32;               // columns of an epilogue step: registers for what it holds at once
   static_assert((NCOL == 256 || NCOL == 128) && (CG == 1 || CG == 2), "tile of the token-major kernel");
 
   extern __shared__ uint8_t smem_raw[];
@@ -638,7 +644,20 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
       if constexpr (I8) {
         if (t_ok) { sa = __ldg(p.a_scale + t); za = __ldg(p.a_zero + t); qs = __ldg(p.a_qsum + t); }
       }
+      float xs = 0.f;
+      if constexpr (CODES) {
+        if (t_ok && p.w_zero) xs = __ldg(p.x_sum + t);
+      }
       auto dequant = [&](const uint32_t* acc, int nn, bool whole, float* to) {
+        if constexpr (CODES) {
+#pragma unroll
+          for (int j = 0; j < CW; ++j) {
+            const int m = whole || nn % p.dual_rows + j < p.N ? nn + j : nn;
+            const float b = p.bias ? __ldg(p.bias + m) : 0.f;
+            to[j] = fmaf(__uint_as_float(acc[j]), __ldg(p.w_scale + m), p.w_zero ? fmaf(__ldg(p.w_zero + m), xs, b) : b);
+          }
+          return;
+        }
 #pragma unroll
         for (int j = 0; j < CW; ++j) {
           const int m = whole || nn % p.dual_rows + j < p.N ? nn + j : nn;
@@ -672,13 +691,13 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
         }
         if (!t_ok || n0 >= p.N) continue;
         float x[CW];
-        if constexpr (I8) {
+        if constexpr (I8 || CODES) {
           dequant(v, n0, full, x);
         } else {
 #pragma unroll
           for (int j = 0; j < CW; ++j) x[j] = __uint_as_float(v[j]);
         }
-        if (I8) {                                  // the bias is in already
+        if (I8 || CODES) {                         // the bias is in already
         } else if (p.bias && full && bias16) {
 #pragma unroll
           for (int j = 0; j < CW / 4; ++j) {
@@ -720,7 +739,7 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
         }
         if constexpr (DUAL) {
           float up[CW];
-          if constexpr (I8) {
+          if constexpr (I8 || CODES) {
             dequant(vu, p.dual_off + n0, full, up);
           } else {
 #pragma unroll
@@ -729,7 +748,7 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
 #pragma unroll
           for (int j = 0; j < CW; ++j) {
             float u = up[j];
-            if (!I8 && p.bias && (full || n0 + j < p.N)) u += __ldg(p.bias + p.dual_off + n0 + j);
+            if (!I8 && !CODES && p.bias && (full || n0 + j < p.N)) u += __ldg(p.bias + p.dual_off + n0 + j);
             x[j] = p.act == kActClamped ? clamped_glu(x[j], u, p.res_scale) : x[j] * u;
           }
         }
@@ -801,9 +820,10 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
   }
 }
 
-template <int NCOL, bool DUAL, int CG, bool I8 = false>
+template <int NCOL, bool DUAL, int CG, int SRC = kTmBf16>
 static int launch_prefill_tm(const void* X, int ldx, const void* W, int w_rows, int ldw, PrefillParams& p, int num_ctas,
                              cudaStream_t st) {
+  constexpr bool I8 = SRC == kTmI8;
   constexpr int STAGE_BYTES = 128 * 64 * 2 + NCOL / CG * 64 * 2;
   constexpr int FEAT = DUAL ? NCOL / 2 : NCOL;
   p.n_tiles = (p.N + FEAT - 1) / FEAT;
@@ -816,7 +836,7 @@ static int launch_prefill_tm(const void* X, int ldx, const void* W, int w_rows, 
   const size_t smem = (size_t)prefill_tm_stages(STAGE_BYTES) * STAGE_BYTES + 1024;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_prefill_tm_kernel<NCOL, DUAL, CG, I8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    if (cudaFuncSetAttribute(gemm_prefill_tm_kernel<NCOL, DUAL, CG, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
       return 3000 + (int)cudaGetLastError();
     attr_set = true;
@@ -833,7 +853,7 @@ static int launch_prefill_tm(const void* X, int ldx, const void* W, int w_rows, 
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = CG > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_prefill_tm_kernel<NCOL, DUAL, CG, I8>, tmX, tmW, (const PrefillParams)p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_prefill_tm_kernel<NCOL, DUAL, CG, SRC>, tmX, tmW, (const PrefillParams)p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -990,12 +1010,13 @@ static int prefill_tm(const void* X, int ldx, const void* W, int w_rows, int ldw
   };
   const float wide = rounds(256, 256, pairs) + 8.f, pair = 0.6f * rounds(256, 128, pairs) + 9.f,
               single = 0.65f * rounds(128, 128, num_ctas) + 3.f;
-  if (i8) {                          // pairs only: the same line between wide and narrow tiles
-    if (wide <= pair) return gated ? launch_prefill_tm<256, true, 2, true>(X, ldx, W, w_rows, ldw, p, num_ctas, st)
-                                   : launch_prefill_tm<256, false, 2, true>(X, ldx, W, w_rows, ldw, p, num_ctas, st);
-    return gated ? launch_prefill_tm<128, true, 2, true>(X, ldx, W, w_rows, ldw, p, num_ctas, st)
-                 : launch_prefill_tm<128, false, 2, true>(X, ldx, W, w_rows, ldw, p, num_ctas, st);
-  }
+  // W8A8 and codes: pairs only, the same line between wide and narrow tiles
+#define XFT_TM_SRC(NCOL, SRC)                                                                       \
+  (gated ? launch_prefill_tm<NCOL, true, 2, SRC>(X, ldx, W, w_rows, ldw, p, num_ctas, st)           \
+         : launch_prefill_tm<NCOL, false, 2, SRC>(X, ldx, W, w_rows, ldw, p, num_ctas, st))
+  if (i8) return wide <= pair ? XFT_TM_SRC(256, kTmI8) : XFT_TM_SRC(128, kTmI8);
+  if (p.w_scale) return wide <= pair ? XFT_TM_SRC(256, kTmCodes) : XFT_TM_SRC(128, kTmCodes);
+#undef XFT_TM_SRC
   if (wide <= pair && wide <= single) return XFT_TM(256, 2);
   return pair < single ? XFT_TM(128, 2) : XFT_TM(128, 1);
 #undef XFT_TM
@@ -1037,6 +1058,84 @@ extern "C" int xft_gemm_bf16_grouped_tm(const void* X, int ldx, int x_rows, cons
   p.group_tiles = reinterpret_cast<const int4*>(group_tiles); p.num_group_tiles = num_group_tiles; p.group_w_rows = group_w_rows;
   p.t_tiles = max_tiles; p.group_rows = tile_rows;
   return prefill_tm(X, ldx, W, w_rows, ldw, p, gated, 0, st);
+}
+
+namespace xft {
+// Codes of weights as bf16, four rows per block, 16 codes of each per thread.  uint4: the even one of a byte's two in its low half.
+// Bound by the stores.
+constexpr int kCodeRows = 4;
+template <bool U4>
+__global__ void __launch_bounds__(256) codes_bf16_kernel(const uint8_t* __restrict__ w, long long ldw, int rows, int K,
+                                                         __nv_bfloat16* __restrict__ out) {
+  grid_dep_launch();
+  const int k = (blockIdx.y * 256 + threadIdx.x) * 16, r0 = blockIdx.x * kCodeRows;
+  uint4 raw[kCodeRows];
+#pragma unroll
+  for (int i = 0; i < kCodeRows; ++i) {
+    const uint8_t* src = w + (size_t)(r0 + i) * ldw;
+    if (k < K && r0 + i < rows) {
+      if constexpr (U4) {
+        const uint2 h = *reinterpret_cast<const uint2*>(src + k / 2);
+        raw[i].x = h.x; raw[i].y = h.y;
+      } else {
+        raw[i] = *reinterpret_cast<const uint4*>(src + k);
+      }
+    }
+  }
+  grid_dep_wait();                                                     // the buffer may still be read by the product before
+#pragma unroll
+  for (int i = 0; i < kCodeRows; ++i) {
+    if (k >= K || r0 + i >= rows) return;
+    uint32_t o[8];
+    if constexpr (U4) {
+      const uint32_t q[2] = {raw[i].x, raw[i].y};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {                                    // byte j & 3: 128 + code in bf16, minus 128
+        const uint32_t c = (q[j >> 2] >> (8 * (j & 3))) & 0xff, pair = ((c & 15) | (c >> 4) << 16) | 0x43004300u;
+        const uint32_t base = 0x43004300u;
+        const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&pair), *reinterpret_cast<const __nv_bfloat162*>(&base));
+        o[j] = *reinterpret_cast<const uint32_t*>(&d);
+      }
+    } else {
+      const int8_t* c = reinterpret_cast<const int8_t*>(&raw[i]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const __nv_bfloat162 x = __floats2bfloat162_rn((float)c[2 * j], (float)c[2 * j + 1]);
+        o[j] = *reinterpret_cast<const uint32_t*>(&x);
+      }
+    }
+    __nv_bfloat16* dst = out + (size_t)(r0 + i) * K + k;
+    if ((reinterpret_cast<uintptr_t>(dst) & 31) == 0 && k + 8 < K) {
+      st_global_256(dst, o);
+    } else {
+      reinterpret_cast<uint4*>(dst)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+      if (k + 8 < K) reinterpret_cast<uint4*>(dst)[1] = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+  }
+}
+}  // namespace xft
+
+// Prompts over int8 (u4 = 0) or uint4 weights: the codes of all w_rows rows as bf16 into `codes` [w_rows, K], which holds them exactly,
+// then the token-major product; y = scale (X codes^T) + zero sum(X) per weight row, then bias, activation, residual as in
+// xft_gemm_bf16_prefill_tm.  x_sum: the rows' sums of X, where zero is given.  K a multiple of 8, rows of W on 16 bytes.
+extern "C" int xft_gemm_codes_tm(const void* X, int ldx, const void* W, int w_rows, int ldw_bytes, int u4, void* codes, void* Y, int ldo,
+                                 int out_fp32, int T, int N, int K, int gated, int dual_off, const float* scale, const float* zero,
+                                 const float* x_sum, const float* bias, const void* residual, int ldr, float res_scale, int act,
+                                 int* status, cudaStream_t st) {
+  if (T <= 0 || N <= 0 || K <= 0) return 0;
+  if ((K & 7) || (ldx & 7) || (ldw_bytes & 15) || ldw_bytes < (u4 ? K / 2 : K) || !scale || (zero && !x_sum) ||
+      ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(codes)) & 15))
+    return -2;
+  const cudaError_t e = launch_pdl(u4 ? codes_bf16_kernel<true> : codes_bf16_kernel<false>,
+                                   dim3((w_rows + kCodeRows - 1) / kCodeRows, (K + 4095) / 4096), dim3(256), 0, st, (const uint8_t*)W,
+                                   (long long)ldw_bytes, w_rows, K, (__nv_bfloat16*)codes);
+  if (e != cudaSuccess) return (int)e;
+  PrefillParams p{};
+  p.N = N; p.T = T; p.K = K; p.out = reinterpret_cast<__nv_bfloat16*>(Y); p.ldo = ldo; p.out_fp32 = out_fp32; p.bias = bias;
+  p.residual = reinterpret_cast<const __nv_bfloat16*>(residual); p.ldr = ldr; p.res_scale = res_scale; p.act = act;
+  p.status = status; p.dual_off = dual_off; p.dual_rows = gated ? dual_off : 0x7fffffff;
+  p.w_scale = scale; p.w_zero = zero; p.x_sum = x_sum;
+  return prefill_tm(X, ldx, codes, w_rows, K, p, gated, 0, st);
 }
 
 // W8A8 above 64 tokens, see xft_w8a8_gemm (gemm_e4m3_sm100.cu)

@@ -1,6 +1,6 @@
 """Bindings of the quantised GEMM kernels: weight-only int8 / nf4 dequant-GEMM and W8A8 (dynamic int8 activations x int8 weights
 on the int8 tensor path) in csrc/kernels/quant_gemm_sm100.cu, fp8-e4m3 and uint4 weights on the fp8 tensor path in
-csrc/kernels/gemm_e4m3_sm100.cu."""
+csrc/kernels/gemm_e4m3_sm100.cu, prompts over int8 and uint4 weights in csrc/kernels/gemm_prefill_sm100.cu (CODES_ROWS)."""
 from __future__ import annotations
 
 import ctypes as C
@@ -58,6 +58,26 @@ def gemm_e4m3(split, w, pitch, src, out, T, n_out, K, gated, dual_off, scale, ze
     ws.launches += 1
 
 
+# Prompts over int8 or uint4 weights: above so many rows (ungated, gated) a product's codes are written out as bf16, which holds them
+# exactly, for the kernel of bf16 prompts (gemm_prefill_sm100.cu), as long as that copy stays below a bound.  The kernels that expand
+# per tile do it once for every 128 (int8) or 64 (uint4) rows.  B200, us there / here: int8 2 x 11008 x 4096 128 rows 112 / 119, 192
+# rows 199 / 118, 1210 rows 592 / 225; 12288 x 4096 128 rows 74 / 71, 192 rows 128 / 71; uint4 2 x 11008 x 4096 320 rows 111 / 138,
+# 384 rows 139 / 138, 1210 rows 392 / 212; 2 x 28672 x 8192 384 rows 510 / 495; 12288 x 4096 192 rows 62 / 68, 256 rows 85 / 68, 1210
+# rows 329 / 139; 4096 x 11008 256 rows 64 / 70, 320 rows 102 / 71.
+CODES_ROWS = {"int8": (128, 128), "int4": (256, 320)}
+CODES_MAX_COPY = 1 << 30
+
+
+def _codes_copy(W, rows, K, T, gated, dev):
+    """Room for a product's codes in bf16, or None where it does not pay or has no room."""
+    if W.kind not in CODES_ROWS or T <= CODES_ROWS[W.kind][gated] or rows * K * 2 > CODES_MAX_COPY or not N._ENV().gemm_prefill_tm:
+        return None
+    try:
+        return torch.empty(rows, K, dtype=torch.bfloat16, device=dev)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype):
     x2, ldx = N._rows2d(x)
     T, K = x2.shape
@@ -82,6 +102,16 @@ def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype):
             W.cache["w_pitch16"] = wp
         w = wp
     zero = W.zero
+    copy = _codes_copy(W, w.shape[0], K, T, gated, x.device)
+    if copy is not None:
+        fn = _lib().xft_gemm_codes_tm
+        fn.restype = C.c_int
+        N._check(fn(N._p(x2), ldx, N._p(w), w.shape[0], w.stride(0) * w.element_size(), int(W.kind == "int4"), N._p(copy), N._p(out),
+                    out.stride(0), int(fp32), T, n_out, K, int(gated), n_out if gated else 0, N._p(W.scale), N._p(zero),
+                    N._p(_row_sums(x2, ldx) if zero is not None else None), N._p(bias), N._p(r2), ldr, C.c_float(res_scale), N._ACT[act],
+                    N._p(ws.status), N._stream()), "gemm_codes_tm")
+        ws.launches += 2
+        return out
     if W.kind in _E4M3:
         codes = W.kind == "int4"
         if codes and zero is None:
