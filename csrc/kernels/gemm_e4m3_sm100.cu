@@ -81,6 +81,17 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* v) {
   else tmem_ld32(taddr, *reinterpret_cast<uint32_t (*)[32]>(v));
 }
 
+// act(x) and act(x) * u, out of line but for what is common: every activation at every place makes code that a launch of a few
+// microseconds waits for
+__device__ __noinline__ float other_act(float x, int act, float param) { return apply_act(x, act, param); }
+__device__ __noinline__ float other_gated(float x, float u, int act, float param) { return apply_gated(x, u, act, param); }
+__device__ __forceinline__ float act_of(float x, int act, float param) {
+  return act == 0 ? x : act == 2 ? apply_act(x, 2) : other_act(x, act, param);
+}
+__device__ __forceinline__ float gated_of(float x, float u, int act, float param) {
+  return act == 2 ? apply_act(x, 2) * u : other_gated(x, u, act, param);
+}
+
 template <int BN, bool DUAL, int SRC>
 struct E4Layout {
   static constexpr int NACC = DUAL ? 2 : 1;
@@ -89,7 +100,7 @@ struct E4Layout {
   static constexpr int A_RING = SRC == kSrcU4 ? 2 * A_BYTES : 0;                      // expanded codes, two buffers
   // two CTAs per SM where registers allow: one CTA's last accumulators and stores hide behind the other's stream
   static constexpr int CTAS = BN <= 32 && A_RING + 3 * STAGE <= 110 * 1024 ? 2 : 1;
-  static constexpr int FIT = ((CTAS == 2 ? 110 : 224) * 1024 - A_RING) / STAGE;
+  static constexpr int FIT = ((CTAS == 2 ? 110 : 222) * 1024 - A_RING) / STAGE;
   static constexpr int STAGES = FIT > 8 ? 8 : FIT;
   static constexpr int SMEM = A_RING + STAGES * STAGE + 1024;
   static_assert(STAGES >= 3 && BN * NACC * 512 <= A_RING + STAGES * STAGE, "ring, and room for this CTA's part of the sums");
@@ -122,6 +133,11 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_group[4];
   __shared__ float s_ssq[SRC == kSrcBf16 ? BN : 1];                    // bf16: sums of squares of the tokens over this CTA's k
+  // what the finish needs per feature (gate rows, then up rows) and per token, fetched beside the main loop.  uint4: scale, zero; W8A8:
+  // scale, zero, sum of codes
+  constexpr int NCOL = SRC == kSrcI8 ? 3 : SRC == kSrcU4 ? 2 : 0, NROW = SRC == kSrcI8 ? 3 : SRC == kSrcBf16 ? 1 : 2;
+  __shared__ alignas(16) float s_col[NCOL ? NCOL : 1][NACC][NCOL ? 128 : 4];
+  __shared__ float s_row[NROW][BN];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int tile_n, tile_t;
@@ -245,8 +261,52 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
 
   // ---- warps 2..9: row = feature of the tile, tokens [c0, c0 + HB) of it
   const int q = warp & 3, row = q * 32 + lane, half = warp >= 6, c0 = half * HB;
-  const int n = tile_n * 128 + row;
-  const bool n_ok = n < p.N;
+  // the finish: warp w takes tokens w, w + 8, .. of this CTA's share of the tile, a lane four features of each
+  const int per = BN / p.splits, f0 = lane * 4, n = tile_n * 128 + f0;
+  const bool vec = n + 4 <= p.N && (p.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & (p.out_fp32 ? 15 : 7)) == 0;
+  const bool vec_res = n + 4 <= p.N && (p.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 7) == 0;
+  constexpr int MINE = BN / 8;
+  uint2 res[MINE];                                                     // residuals of those tokens
+  if (NCOL && warp >= 2) {                                             // weights' numbers depend on no earlier kernel
+    const int e = threadIdx.x - 64, nn = tile_n * 128 + (e & 127);
+    if (e < 128 * NACC) {
+      const int at = (e >= 128 ? p.dual_off : 0) + nn;
+      const float* from[3] = {p.scale, p.zero, p.w_sum};
+#pragma unroll
+      for (int i = 0; i < NCOL; ++i) s_col[i][e >> 7][e & 127] = nn < p.N && from[i] ? __ldg(from[i] + at) : 0.f;
+    }
+  }
+  auto fetch_rows = [&]() {                                            // what earlier kernels leave per token
+    const int e = threadIdx.x - 64;
+    if (e < BN) {
+      const int t = x_row0 + e;
+      const bool in = e < x_rows;
+      if constexpr (SRC == kSrcBf16) {
+        s_row[0][e] = in && p.rms_ssq ? p.rms_ssq[t] : 0.f;
+      } else {
+        s_row[0][e] = in ? p.x_scale[t] : 0.f;
+        if constexpr (SRC == kSrcI8) { s_row[1][e] = in ? p.a_zero[t] : 0.f; s_row[2][e] = in ? p.a_qsum[t] : 0.f; }
+        if constexpr (SRC == kSrcU4) s_row[1][e] = in ? p.x_sum[t] : 0.f;
+        if constexpr (SRC == kSrcFp8) s_row[1][e] = in && p.col_scale ? p.col_scale[t] : 1.f;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) {
+      const int c = rank * per + warp - 2 + 8 * i;
+      res[i] = make_uint2(0, 0);
+      if (p.residual && warp - 2 + 8 * i < per && c < x_rows) {
+        const __nv_bfloat16* r = p.residual + (size_t)(x_row0 + c) * p.ldr + n;
+        if (vec_res) {
+          res[i] = *reinterpret_cast<const uint2*>(r);
+        } else {
+          __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(&res[i]);
+#pragma unroll
+          for (int f = 0; f < 4; ++f)
+            if (n + f < p.N) to[f] = r[f];
+        }
+      }
+    }
+  };
   float g[NACC][HB];
 #pragma unroll
   for (int i = 0; i < NACC; ++i)
@@ -265,6 +325,8 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
         to[j] = fmaf(factor, fmaf(__uint_as_float(lo[j]), 0.0625f, __uint_as_float(hi[j])), to[j]);
     };
     if constexpr (SRC == kSrcFp8) {
+      grid_dep_wait();
+      fetch_rows();
       const float* sc = p.scale + (size_t)(w_row0 >> 7) * p.scale_ld;
       const float* sc_up = sc + (size_t)(p.dual_off >> 7) * p.scale_ld;
       Ring b = {0, 0};
@@ -281,10 +343,11 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
         if (lane == 0) mbar_arrive(&tmem_empty[b.s]);
       }
     } else if constexpr (SRC == kSrcI8 || SRC == kSrcBf16) {
+      grid_dep_wait();
+      fetch_rows();
       if (SRC == kSrcBf16 && p.rms_x && !p.rms_ssq) {                                // beside the main loop: 256 / BN threads per token
         constexpr int TPT = 256 / BN;
         const int e = threadIdx.x - 64, tok = e / TPT, sub = e % TPT;
-        grid_dep_wait();
         float acc = 0.f;
         if (tok < x_rows) {
           const __nv_bfloat16* xr = p.rms_x + (size_t)(x_row0 + tok) * p.rms_ldx;
@@ -303,7 +366,6 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
 #pragma unroll
         for (int o = TPT / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (sub == 0) s_ssq[tok] = acc;
-        named_bar_sync(2, 256);
       }
       ok = __all_sync(0xffffffffu, mbar_wait(&tmem_full[0], 0, p.status, XFT_ERR_WAIT_TMEM));
       tcgen05_fence_after();
@@ -368,6 +430,8 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
         }
         mbar_arrive(&a_ready[b.s]);
       }
+      grid_dep_wait();
+      fetch_rows();
       if (kend > kb0) {
         ok = __all_sync(0xffffffffu, mbar_wait(&tmem_full[0], 0, p.status, XFT_ERR_WAIT_TMEM));
         tcgen05_fence_after();
@@ -378,97 +442,140 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
       }
     }
   }
-  if (warp >= 2) grid_dep_wait();                                      // outputs, residual and the row scales belong to the stream order
-
-  auto finish = [&](int t, float x, float u) {                         // t: token row of X and Y
-    if constexpr (SRC == kSrcBf16) {
-      float ts = 1.f;
-      if (p.rms_x) {
-        float ssq = p.rms_ssq ? p.rms_ssq[t] : 0.f;
-        for (int s = 0; s < p.splits && !p.rms_ssq; ++s)
-          ssq += p.splits == 1 ? s_ssq[t - x_row0] : ld_dsmem(dsmem_addr(smem_u32(s_ssq + (t - x_row0)), s));
-        ts = rsqrtf(ssq / (float)p.K + p.rms_eps);
-      }
-      x = x * ts + (p.bias ? p.bias[n] : 0.f);
-      if (DUAL) x = apply_gated(x, u * ts + (p.bias ? p.bias[p.dual_off + n] : 0.f), p.act, p.res_scale);
-      else x = apply_act(x, p.act, p.res_scale);
-      if (p.residual) x = with_residual(x, __bfloat162float(p.residual[(size_t)t * p.ldr + n]), p.res_scale, p.act);
-      if (p.out_fp32) reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + n] = x;
-      else reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + n] = __float2bfloat16(x);
-      return;
-    }
-    const float st = p.x_scale[t];
-    if constexpr (SRC == kSrcI8) {
-      const float za = p.a_zero[t], qs = p.a_qsum[t];
-      auto value = [&](float acc, int nn) {
-        return w8a8_value((float)__float_as_int(acc), st, za, qs, p.scale[nn], p.zero ? p.zero[nn] : 0.f, p.w_sum ? p.w_sum[nn] : 0.f,
-                          p.K, p.bias ? p.bias[nn] : 0.f);
-      };
-      if (DUAL) x = apply_act(bf16_round(value(x, n)), p.act) * bf16_round(value(u, p.dual_off + n));
-      else x = apply_act(value(x, n), p.act);
-      if (p.residual) x += p.res_scale * __bfloat162float(p.residual[(size_t)t * p.ldr + n]);
-      if (p.out_fp32) reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + n] = x;
-      else reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + n] = __float2bfloat16(x);
-      return;
-    }
-    float s0 = st, s1 = st, b0 = p.bias ? p.bias[n] : 0.f, b1 = DUAL && p.bias ? p.bias[p.dual_off + n] : 0.f;
-    if (SRC == kSrcU4) {
-      const float xs = p.x_sum[t];
-      s0 *= p.scale[n];
-      b0 += p.zero[n] * xs;
-      if (DUAL) { s1 *= p.scale[p.dual_off + n]; b1 += p.zero[p.dual_off + n] * xs; }
-    }
-    x = apply_act(fmaf(x, s0, b0), p.act);
-    if (DUAL) x *= fmaf(u, s1, b1);
-    if (p.col_scale) x *= p.col_scale[t];
-    if (p.residual) x += p.res_scale * __bfloat162float(p.residual[(size_t)t * p.ldr + n]);
-    if (p.out_fp32) reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + n] = x;
-    else reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + n] = __float2bfloat16(x);
-  };
-  if (p.splits == 1) {
-    if (warp >= 2 && ok && n_ok) {
+  // Every MMA has read its operands (the last accumulator is here), so the ring is free for this CTA's part of the sums, [column][128].
+  // From there a lane takes four features of a token at once: residual and output move in 8-byte pieces, what the finish needs is
+  // already here, and no load waits for the one before.  A thread per feature that walked its tokens waited for a global load in each:
+  // us, so / now: bf16 12288 x 4096 with a folded norm 16 rows 21.8 / 20.1, 64 rows 36.8 / 23.6; 2 x 11008 x 4096 32 rows 38.3 / 34.3, 64
+  // rows 52.3 / 37.2; 896 x 896 16 rows 5.8 / 4.1, 64 rows 12.0 / 6.0; W8A8 12288 x 4096 32 rows 15.9 / 13.8; one row is level (2 x 11008
+  // x 4096 31.5 / 32.0, 4096 x 4096 8.4 / 8.5).
+  float* part = reinterpret_cast<float*>(smem);
+  if (warp >= 2) {
 #pragma unroll
-      for (int j = 0; j < HB; ++j)
-        if (c0 + j < x_rows) finish(x_row0 + c0 + j, g[0][j], DUAL ? g[NACC - 1][j] : 0.f);
-    }
-  } else {
-    // every MMA has read its operands (the last accumulator is here), so the ring is free for this CTA's part: [column][128]
-    float* part = reinterpret_cast<float*>(smem);
-    __syncwarp();                                                      // the lanes behind the elected ones of warps 0 and 1
-    named_bar_sync(1, kE4Threads);                                     // the slower half may still wait for its accumulator
-    if (warp >= 2) {
+    for (int i = 0; i < NACC; ++i)
 #pragma unroll
-      for (int i = 0; i < NACC; ++i)
-#pragma unroll
-        for (int j = 0; j < HB; ++j) part[(i * BN + c0 + j) * 128 + row] = g[i][j];
-    }
-    __syncwarp();
+      for (int j = 0; j < HB; ++j) part[(i * BN + c0 + j) * 128 + row] = g[i][j];
+  }
+  __syncwarp();                                                        // the lanes behind the elected ones of warps 0 and 1
+  if (p.splits > 1) {
     cluster_arrive();
     cluster_wait();
-    const int per = BN / p.splits;                                     // tokens of this CTA, half of them per warp of a row
-    if (warp >= 2 && n_ok) {
-      const int lo = rank * per + (half ? (per + 1) / 2 : 0), hi = half ? (rank + 1) * per : rank * per + (per + 1) / 2;
-      for (int c = lo; c < hi && c < x_rows; ++c) {
-        float v[8], w[8];
+  } else if (warp >= 2) {
+    named_bar_sync(1, 256);
+  }
+  if (warp >= 2 && n < p.N && (ok || p.splits > 1)) {
+    float4 bias[NACC];
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          const uint32_t a = smem_u32(part + c * 128 + row);
-          v[s] = s < p.splits ? ld_dsmem(dsmem_addr(a, s)) : 0.f;
-          w[s] = DUAL && s < p.splits ? ld_dsmem(dsmem_addr(a + BN * 512, s)) : 0.f;
-        }
-        float x = 0.f, u = 0.f;
-        if constexpr (SRC == kSrcI8) {
-          int xi = 0, ui = 0;
+    for (int a = 0; a < NACC; ++a) {
+      bias[a] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.bias) {
 #pragma unroll
-          for (int s = 0; s < 8; ++s) { xi += __float_as_int(v[s]); ui += __float_as_int(w[s]); }
-          x = __int_as_float(xi); u = __int_as_float(ui);
-        } else {
-#pragma unroll
-          for (int s = 0; s < 8; ++s) { x += v[s]; u += w[s]; }
-        }
-        finish(x_row0 + c, x, u);
+        for (int f = 0; f < 4; ++f)
+          if (n + f < p.N) (&bias[a].x)[f] = __ldg(p.bias + a * p.dual_off + n + f);
       }
     }
+#pragma unroll 1
+    for (int i = 0; i < MINE; ++i) {
+      const int mine = warp - 2 + 8 * i, c = rank * per + mine;
+      if (mine >= per || c >= x_rows) break;
+      float4 y[NACC];
+      float ssq = SRC == kSrcBf16 ? s_row[0][c] : 0.f;
+      const bool own_ssq = SRC == kSrcBf16 && p.rms_x && !p.rms_ssq;
+      const uint32_t at = smem_u32(part + c * 128 + f0), at_ssq = smem_u32(s_ssq + (SRC == kSrcBf16 ? c : 0));
+      if (p.splits == 1) {
+#pragma unroll
+        for (int a = 0; a < NACC; ++a) y[a] = *reinterpret_cast<const float4*>(part + (a * BN + c) * 128 + f0);
+        if (own_ssq) ssq += s_ssq[SRC == kSrcBf16 ? c : 0];
+      } else {
+        float q[8];
+        if (own_ssq) {
+#pragma unroll
+          for (int r = 0; r < 8; ++r) q[r] = r < p.splits ? ld_dsmem(dsmem_addr(at_ssq, r)) : 0.f;
+        }
+#pragma unroll
+        for (int a = 0; a < NACC; ++a) {
+          float4 v[8];
+#pragma unroll
+          for (int r = 0; r < 8; ++r) v[r] = r < p.splits ? ld_dsmem4(dsmem_addr(at + a * BN * 512, r)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int f = 0; f < 4; ++f) {
+            if constexpr (SRC == kSrcI8) {
+              int sum = 0;
+#pragma unroll
+              for (int r = 0; r < 8; ++r) sum += __float_as_int((&v[r].x)[f]);
+              (&y[a].x)[f] = __int_as_float(sum);
+            } else {
+              float sum = 0.f;
+#pragma unroll
+              for (int r = 0; r < 8; ++r) sum += (&v[r].x)[f];
+              (&y[a].x)[f] = sum;
+            }
+          }
+        }
+        if (own_ssq) {
+#pragma unroll
+          for (int r = 0; r < 8; ++r) if (r < p.splits) ssq += q[r];
+        }
+      }
+      const size_t t = x_row0 + c;
+      const __nv_bfloat16* rv = reinterpret_cast<const __nv_bfloat16*>(&res[i]);
+      float ts = 1.f;
+      if (SRC == kSrcBf16 && p.rms_x) ts = rsqrtf(ssq / (float)p.K + p.rms_eps);
+      float out[4];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        float x = (&y[0].x)[f], u = DUAL ? (&y[NACC - 1].x)[f] : 0.f;
+        const float b = (&bias[0].x)[f], bu = (&bias[NACC - 1].x)[f], r = __bfloat162float(rv[f]);
+        if constexpr (SRC == kSrcBf16) {
+          x = x * ts + b;
+          if (DUAL) x = gated_of(x, u * ts + bu, p.act, p.res_scale);
+          else x = act_of(x, p.act, p.res_scale);
+          if (p.residual) x = with_residual(x, r, p.res_scale, p.act);
+        } else if constexpr (SRC == kSrcI8) {
+          auto value = [&](float acc, int a, float to) {
+            return w8a8_value((float)__float_as_int(acc), s_row[0][c], s_row[1][c], s_row[2][c], s_col[0][a][f0 + f], s_col[1][a][f0 + f],
+                              s_col[2][a][f0 + f], p.K, to);
+          };
+          if (DUAL) x = act_of(bf16_round(value(x, 0, b)), p.act, 1.f) * bf16_round(value(u, NACC - 1, bu));
+          else x = act_of(value(x, 0, b), p.act, 1.f);
+          if (p.residual) x += p.res_scale * r;
+        } else {
+          const float st = s_row[0][c];
+          if constexpr (SRC == kSrcU4) {
+            const float xs = s_row[1][c];
+            x = act_of(fmaf(x, st * s_col[0][0][f0 + f], b + s_col[1][0][f0 + f] * xs), p.act, 1.f);
+            if (DUAL) x *= fmaf(u, st * s_col[0][NACC - 1][f0 + f], bu + s_col[1][NACC - 1][f0 + f] * xs);
+          } else {
+            x = act_of(fmaf(x, st, b), p.act, 1.f);
+            if (DUAL) x *= fmaf(u, st, bu);
+            if (p.col_scale) x *= s_row[1][c];
+          }
+          if (p.residual) x += p.res_scale * r;
+        }
+        out[f] = x;
+      }
+      if (p.out_fp32) {
+        float* to = reinterpret_cast<float*>(p.out) + t * p.ldo + n;
+        if (vec) {
+          *reinterpret_cast<float4*>(to) = make_float4(out[0], out[1], out[2], out[3]);
+        } else {
+#pragma unroll
+          for (int f = 0; f < 4; ++f)
+            if (n + f < p.N) to[f] = out[f];
+        }
+      } else {
+        __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(p.out) + t * p.ldo + n;
+        if (vec) {
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(out[0], out[1]), hi = __floats2bfloat162_rn(out[2], out[3]);
+          *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        } else {
+#pragma unroll
+          for (int f = 0; f < 4; ++f)
+            if (n + f < p.N) to[f] = __float2bfloat16(out[f]);
+        }
+      }
+    }
+  }
+  if (p.splits > 1) {
     __syncwarp();
     cluster_arrive();                                                  // nobody leaves while its part is being read
     cluster_wait();

@@ -305,6 +305,11 @@ __device__ __forceinline__ float ld_dsmem(uint32_t addr) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ float4 ld_dsmem4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 
 // Two CTAs of a cluster on one MMA (cta_group::2).  Accumulators are allocated and freed by one warp of each CTA; the MMA is
 // issued by one thread of the first CTA; TMA loads of both may complete on a barrier of the first (`bar`: its address in the
