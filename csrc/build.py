@@ -29,7 +29,7 @@ ACCURATE = {"plain.cu", "latent.cu", "head_prep.cu", "gla.cu", "ssd.cu", "talkin
 # what a layered model calls: GEMMs, attention, norms, rotary + cache append, experts, arg-max, and what these link against
 LAYERED = ["attention.cu", "attention_prefill_sm100.cu", "elementwise.cu", "gemm_decode_sm100.cu", "gemm_e4m3_sm100.cu",
            "gemm_prefill_sm100.cu",
-           "gemm_sm100.cu", "gla.cu", "head_prep.cu", "latent.cu", "latent_prefill_sm100.cu", "mla.cu", "moe.cu", "plain.cu", "residual_norm.cu",
+           "gemm_sm100.cu", "gla.cu", "head_prep.cu", "latent.cu", "latent_prefill_sm100.cu", "mla.cu", "moe.cu", "plain.cu", "quant_rows.cu", "residual_norm.cu",
            "ssd.cu", "talking.cu", "talking_mma.cu"]
 
 

@@ -612,7 +612,8 @@ __global__ void __launch_bounds__(256) row_ssq_kernel(const __nv_bfloat16* __res
 }
 
 // Row r of X (or row src[r]) -> [hi | lo] e4m3, its power-of-two scale and its sum.  `nibbles`: k in the order in which uint4
-// codes expand, 16 even ones and 16 odd ones of every 32.  Rows from *rows_used on are left alone.
+// codes expand, 16 even ones and 16 odd ones of every 32.  Rows from *rows_used on are left alone.  (Rows of more than 32768; others
+// in quant_rows.cu.)
 __global__ void __launch_bounds__(256) split_e4m3_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int* __restrict__ src,
                                                          const int* __restrict__ rows_used, int K, int Kp, int nibbles,
                                                          uint8_t* __restrict__ out, float* __restrict__ scale, float* __restrict__ sum) {
@@ -686,6 +687,8 @@ __global__ void __launch_bounds__(256) split_e4m3_kernel(const __nv_bfloat16* __
   }
 }
 
+int launch_split(const void* x, int ldx, const int* src, const int* rows_used, const float* gain, float eps, int rows, int K, int Kp,
+                 int nibbles, void* out, float* scale, float* sum, cudaStream_t st);      // quant_rows.cu
 int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row_bytes, uint64_t ld_bytes, uint32_t box_rows,
                   uint32_t box_bytes);                                 // gemm_sm100.cu: unswizzled bytes
 
@@ -740,6 +743,8 @@ extern "C" int xft_split_e4m3(const void* x, int ldx, const int* src, const int*
                               float* scale, float* sum, cudaStream_t st) {
   if (rows <= 0) return 0;
   if ((K & 7) || (ldx & 7) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15)) return -2;
+  const int rc = launch_split(x, ldx, src, rows_used, nullptr, 0.f, rows, K, xft_split_e4m3_cols(K), nibbles, out, scale, sum, st);
+  if (rc != -1) return rc;
   const cudaError_t e = launch_pdl(split_e4m3_kernel, dim3(rows), dim3(256), 0, st, (const __nv_bfloat16*)x, ldx, src, rows_used, K,
                                    xft_split_e4m3_cols(K), nibbles, (uint8_t*)out, scale, sum);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();

@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(192) qgemm_kernel(const __grid_constant__ CUte
   }
 }
 
-// Per-row dynamic int8 quantisation of activations (+ the sums the W8A8 epilogue needs) and plain row sums.
+// Per-row dynamic int8 quantisation of activations (+ the sums the W8A8 epilogue needs) for rows that quant_rows.cu does not take.
 __global__ void __launch_bounds__(256) quant_act_kernel(const __nv_bfloat16* __restrict__ x, int ldx, int8_t* __restrict__ q,
                                                         int ldq, float* __restrict__ scale, float* __restrict__ zero,
                                                         float* __restrict__ qsum, int K) {
@@ -570,9 +570,16 @@ extern "C" int xft_qgemm_grouped(const void* X, int ldx, int x_rows, const void*
   return -1;
 }
 
+namespace xft {
+int launch_quant_act(const void* x, int ldx, const float* gain, float eps, void* q, int ldq, float* scale, float* zero, float* sum,
+                     int rows, int K, cudaStream_t st);                // quant_rows.cu
+}
+
 extern "C" int xft_quant_act(const void* x, int ldx, void* q, int ldq, float* scale, float* zero, float* qsum, int T, int K,
                              cudaStream_t st) {
   if (T <= 0) return 0;
+  const int rc = launch_quant_act(x, ldx, nullptr, 0.f, q, ldq, scale, zero, qsum, T, K, st);
+  if (rc != -1) return rc;
   cudaError_t e = launch_pdl(quant_act_kernel, dim3(T), dim3(256), 0, st, (const __nv_bfloat16*)x, ldx, (int8_t*)q, ldq, scale,
                              zero, qsum, K);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();

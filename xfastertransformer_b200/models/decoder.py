@@ -466,6 +466,10 @@ class Decoder:
     # ------------------------------------------------------------------------------------
     # forward
     # ------------------------------------------------------------------------------------
+    def _quantises(self, W) -> bool:
+        """Whether the product behind an RMSNorm rewrites its rows as codes, with nothing else reading the normalised state."""
+        return W is not None and W.kind in ("w8a8", "int4", "fp8") and self.spec.norm == "rms" and not self.spec.resid_from_norm
+
     def _norm(self, x, w, b):
         if self.spec.norm == "rms":
             return ops.rmsnorm(x, w, self.eps)
@@ -512,11 +516,13 @@ class Decoder:
     def _attention(self, L: Layer, x, b: Batch, cache: PagedKVCache, li: int):
         c, s = self.cfg, self.spec
         h = None
-        if not L.attn_fold:
+        # the norm in front of a product that quantises its rows goes with that (ops.norm_linear), unless something else reads it
+        norm_later = not L.attn_fold and self._quantises(L.qkv_a if s.attention == "mla" else L.qkv)
+        if not L.attn_fold and not norm_later:
             with TimeLine("Attention.norm"):
                 h = self._norm(x, L.attn_norm_w, L.attn_norm_b)
         if s.attention == "mla":
-            a = self._mla(L, h, b, cache, li)
+            a = self._mla(L, x if norm_later else h, b, cache, li, norm_later)
         else:
             table, q_scale, positions = self.rope_table, None, b.positions
             if s.logn_ntk and table is not None:
@@ -525,8 +531,8 @@ class Decoder:
                     q_scale = torch.clamp(torch.log(b.positions.float() + 1) / math.log(seq_len), min=1.0)
             if s.telechat_ntk and table is not None:
                 table = self._telechat_rope(b.max_kv, b.max_q)
-            xin = x if L.attn_fold else h
-            fused_qkv = (xin.is_cuda and s.rope != "2d" and
+            xin = x if L.attn_fold or norm_later else h
+            fused_qkv = (xin.is_cuda and s.rope != "2d" and not norm_later and
                          ops.can_fuse_qkv_rope(L.qkv, xin.numel() // xin.shape[-1], self.D, cache.k[li], cache.ks[li],
                                                L.q_norm, L.k_norm, self.rope_style))
             if fused_qkv:
@@ -537,7 +543,10 @@ class Decoder:
                                                   cache.k[li], cache.v[li], b.slots, q_scale)
             else:
                 with TimeLine("QKV.linear"):
-                    qkv = ops.linear_rms(x, L.qkv, self.eps, L.qkv_b) if L.attn_fold else ops.linear(h, L.qkv, L.qkv_b)
+                    if norm_later:
+                        qkv = ops.norm_linear(x, L.attn_norm_w, self.eps, L.qkv, L.qkv_b)
+                    else:
+                        qkv = ops.linear_rms(x, L.qkv, self.eps, L.qkv_b) if L.attn_fold else ops.linear(h, L.qkv, L.qkv_b)
             with TimeLine("QKPO"):
                 if fused_qkv:
                     pass
@@ -564,18 +573,20 @@ class Decoder:
         return ops.qkv_rope2d_cache(qkv, self.hq, self.hkv, self.D, b.positions, b.positions2, self.rope_table,
                                     cache.k[li], cache.v[li], cache.ks[li], cache.vs[li], b.slots)
 
-    def _mla(self, L: Layer, h, b: Batch, cache: PagedKVCache, li: int):
+    def _mla(self, L: Layer, h, b: Batch, cache: PagedKVCache, li: int, norm_first: bool = False):
+        """`norm_first`: h is the state before the layer's norm."""
         c = self.cfg
+        down = lambda W: ops.norm_linear(h, L.attn_norm_w, self.eps, W) if norm_first else ops.linear(h, W)
         nope, rope, vd, kvl, ql = c.qk_nope_head_dim, c.qk_rope_head_dim, c.v_head_dim, c.kv_lora_rank, c.q_lora_rank
         T = h.shape[0]
         Hl = self.hq
         if ql > 0:
-            qa_kv = ops.linear(h, L.qkv_a)                       # [T, ql + kvl + rope]
+            qa_kv = down(L.qkv_a)                                # [T, ql + kvl + rope]
             qa = ops.rmsnorm(qa_kv[:, :ql], L.q_a_norm, self.eps)
             q = ops.linear(qa, L.q_b)
             kv = qa_kv[:, ql:]
         elif L.qkv_a is not None:
-            both = ops.linear(h, L.qkv_a)
+            both = down(L.qkv_a)
             q, kv = both[:, : Hl * (nope + rope)], both[:, Hl * (nope + rope):]
         else:
             q, kv = ops.linear(h, L.q_direct), ops.linear(h, L.kv_a)
@@ -591,6 +602,10 @@ class Decoder:
         if L.mlp_fold:
             with TimeLine("LlamaMLP"):
                 g = ops.linear_rms(x, L.gate_up, self.eps, None, L.act, gated=True)
+                return self._row_parallel(g, L.down, None, x, 1.0)
+        if k == "llama" and self._quantises(L.gate_up):
+            with TimeLine("LlamaMLP"):
+                g = ops.norm_linear(x, L.mlp_norm_w, self.eps, L.gate_up, None, L.act, gated=True)
                 return self._row_parallel(g, L.down, None, x, 1.0)
         with TimeLine("MLP.norm"):
             h = self._norm(x, L.mlp_norm_w, L.mlp_norm_b)

@@ -119,6 +119,14 @@ def linear_rms(x, W, eps, bias=None, act=None, gated=False, out_dtype=None):
     return _linear_rms(x, W, eps, bias, act, gated, out_dtype)
 
 
+def norm_linear(x, gain, eps, W, bias=None, act=None, gated=False):
+    """RMSNorm(x; gain) @ W^T: as rmsnorm and linear (or linear_gated) after each other, in fewer launches where the rows are quantised."""
+    if _verbose() or not _cuda(x):
+        h = rmsnorm(x, gain, eps)
+        return linear_gated(h, W, act, bias) if gated else linear(h, W, bias, act)
+    return _nat().norm_linear(x, gain, eps, W, bias, act, gated)
+
+
 def linear_gated(x, W, act="silu", bias=None, limit=0.0):
     """act(g) * u with (g | u) = x W^T + bias; act "clamped": g = min(g, limit), u = u clamped to +-limit, and the result is
     g sigmoid(1.702 g) (u + 1)."""

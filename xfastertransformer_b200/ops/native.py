@@ -482,6 +482,19 @@ def linear_rms(x, W, eps, bias=None, act=None, gated=False, out_dtype=None):
     return out.view(*x.shape[:-1], N)
 
 
+def norm_linear(x, gain, eps, W, bias=None, act=None, gated=False):
+    """RMSNorm(x; gain) @ W^T of weights that do not carry the gain: the norm goes with the launch that quantises the rows where there is
+    one that takes it."""
+    if W.kind not in ("bf16", "fp32"):
+        from . import native_quant as Q
+        x2, _ = _rows2d(x)
+        if Q.norm_fits(W, *x2.shape, gated, gain):
+            y = Q.linear_gated(x2, W, act, bias, (gain, eps)) if gated else Q.linear(x2, W, bias, act, norm=(gain, eps))
+            return y.view(*x.shape[:-1], y.shape[-1])
+    h = rmsnorm(x, gain, eps)
+    return linear_gated(h, W, act, bias) if gated else linear(h, W, bias, act)
+
+
 def linear(x, W, bias=None, act=None, residual=None, res_scale=1.0, out_dtype=None):
     lead = x.shape[:-1]
     if W.kind == "bf16":

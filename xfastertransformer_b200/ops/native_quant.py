@@ -19,7 +19,7 @@ def _lib():
     lib = N.lib()
     if not _ready:
         for fn in ("xft_qgemm", "xft_quant_act", "xft_row_sum", "xft_w8a8_gemm", "xft_split_e4m3", "xft_split_e4m3_cols",
-                   "xft_gemm_e4m3", "xft_w8a8_gemm_gated"):
+                   "xft_gemm_e4m3", "xft_w8a8_gemm_gated", "xft_rms_quant_act", "xft_rms_split_e4m3"):
             getattr(lib, fn).restype = C.c_int
         _ready = True
     return lib
@@ -33,15 +33,20 @@ def _row_sums(x2, ldx):
     return out
 
 
-def split_e4m3(x2, ldx, nibbles=False, want_sum=False, src=None, rows_used=None, rows=None):
+def split_e4m3(x2, ldx, nibbles=False, want_sum=False, src=None, rows_used=None, rows=None, norm=None):
     """Rows of x2 (or rows `src` of it) as sums of two e4m3 numbers -> (uint8 [rows, 2 * cols], scale [rows], sum [rows] or
-    None).  `nibbles`: in the order in which 4-bit codes expand.  `rows_used`: device count; later rows stay unwritten."""
+    None).  `nibbles`: in the order in which 4-bit codes expand.  `rows_used`: device count; later rows stay unwritten.  `norm`:
+    (gain, eps) of an RMSNorm in front (norm_fits)."""
     T, K = x2.shape
     rows = T if rows is None else rows
     xs = torch.empty(rows, 2 * _lib().xft_split_e4m3_cols(K), dtype=torch.uint8, device=x2.device)
     st = torch.empty(2, rows, dtype=torch.float32, device=x2.device)
-    N._check(_lib().xft_split_e4m3(N._p(x2), ldx, N._p(src), N._p(rows_used), rows, K, int(nibbles), N._p(xs), N._p(st[0]),
-                                   N._p(st[1] if want_sum else None), N._stream()), "split_e4m3")
+    if norm is not None:
+        N._check(_lib().xft_rms_split_e4m3(N._p(x2), ldx, N._p(norm[0]), C.c_float(norm[1]), rows, K, int(nibbles), N._p(xs), N._p(st[0]),
+                                           N._p(st[1] if want_sum else None), N._stream()), "rms_split_e4m3")
+    else:
+        N._check(_lib().xft_split_e4m3(N._p(x2), ldx, N._p(src), N._p(rows_used), rows, K, int(nibbles), N._p(xs), N._p(st[0]),
+                                       N._p(st[1] if want_sum else None), N._stream()), "split_e4m3")
     N.Workspace.get(x2.device).launches += 1
     return xs, st[0], st[1] if want_sum else None
 
@@ -78,7 +83,14 @@ def _codes_copy(W, rows, K, T, gated, dev):
         return None
 
 
-def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype):
+def norm_fits(W, T, K, gated, gain) -> bool:
+    """Whether a product of W takes (gain, eps) of an RMSNorm of its rows (csrc/kernels/quant_rows.cu): kinds that rewrite the rows in any
+    case, at the sizes at which that adds a row's squares as xft_rmsnorm does."""
+    return (W.kind == "w8a8" or W.kind in _E4M3 and not (W.kind in CODES_ROWS and T > CODES_ROWS[W.kind][gated])) and 2048 <= K <= 8192 \
+        and K % 8 == 0 and gain.dtype == torch.float32 and gain.data_ptr() % 16 == 0 and not (gated and W.kind == "fp8" and W.out_features % 256)
+
+
+def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype, norm=None):
     x2, ldx = N._rows2d(x)
     T, K = x2.shape
     if K % 8:
@@ -118,7 +130,7 @@ def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype):
             zero = W.cache.get("zero0")
             if zero is None:
                 zero = W.cache["zero0"] = torch.zeros_like(W.scale)
-        gemm_e4m3(split_e4m3(x2, ldx, codes, codes), w, w.stride(0), _E4M3[W.kind], out, T, n_out, K, gated, n_out if gated else 0,
+        gemm_e4m3(split_e4m3(x2, ldx, codes, codes, norm=norm), w, w.stride(0), _E4M3[W.kind], out, T, n_out, K, gated, n_out if gated else 0,
                   W.scale, zero if codes else None, 0 if codes else W.scale.shape[1], bias, r2, ldr, res_scale, act)
         return out
     if W.kind == "nf4":
@@ -159,21 +171,25 @@ def quantize_rows(w, kind):
     return q, sz[0], sz[1], wsum
 
 
-def quant_act(x2, ldx):
-    """bf16 [T,K] -> (int8 [T,K], scale[T], zero[T], qsum[T]) per-row dynamic asymmetric."""
+def quant_act(x2, ldx, norm=None):
+    """bf16 [T,K] -> (int8 [T,K], scale[T], zero[T], qsum[T]) per-row dynamic asymmetric.  `norm`: as in split_e4m3."""
     T, K = x2.shape
     q = torch.empty(T, K, dtype=torch.int8, device=x2.device)
     s = torch.empty(3, T, dtype=torch.float32, device=x2.device)
-    N._check(_lib().xft_quant_act(N._p(x2), ldx, N._p(q), K, N._p(s[0]), N._p(s[1]), N._p(s[2]), T, K, N._stream()),
-             "quant_act")
+    if norm is not None:
+        N._check(_lib().xft_rms_quant_act(N._p(x2), ldx, N._p(norm[0]), C.c_float(norm[1]), N._p(q), K, N._p(s[0]), N._p(s[1]), N._p(s[2]), T, K,
+                                          N._stream()), "rms_quant_act")
+    else:
+        N._check(_lib().xft_quant_act(N._p(x2), ldx, N._p(q), K, N._p(s[0]), N._p(s[1]), N._p(s[2]), T, K, N._stream()),
+                 "quant_act")
     N.Workspace.get(x2.device).launches += 1
     return q, s[0], s[1], s[2]
 
 
-def _w8a8(x, W, rows, bias, act, residual, res_scale, out_dtype, row0=0):
+def _w8a8(x, W, rows, bias, act, residual, res_scale, out_dtype, row0=0, norm=None):
     x2, ldx = N._rows2d(x)
     T, K = x2.shape
-    q, sa, za, qs = quant_act(x2, ldx)
+    q, sa, za, qs = quant_act(x2, ldx, norm)
     fp32 = out_dtype == torch.float32
     out = torch.empty(T, rows, dtype=torch.float32 if fp32 else torch.bfloat16, device=x.device)
     ws = N.Workspace.get(x.device)
@@ -192,20 +208,20 @@ def _w8a8(x, W, rows, bias, act, residual, res_scale, out_dtype, row0=0):
     return out
 
 
-def linear(x, W, bias=None, act=None, residual=None, res_scale=1.0, out_dtype=None):
+def linear(x, W, bias=None, act=None, residual=None, res_scale=1.0, out_dtype=None, norm=None):
     if W.kind == "w8a8":
-        return _w8a8(x, W, W.out_features, bias, act, residual, res_scale, out_dtype)
+        return _w8a8(x, W, W.out_features, bias, act, residual, res_scale, out_dtype, norm=norm)
     if W.kind in _QT or W.kind in _E4M3:
-        return _qgemm(x, W, W.out_features, False, bias, act, residual, res_scale, out_dtype)
+        return _qgemm(x, W, W.out_features, False, bias, act, residual, res_scale, out_dtype, norm)
     raise N.KernelError(f"no sm_100a GEMM for weight kind {W.kind}")
 
 
-def linear_gated(x, W, act="silu", bias=None):
+def linear_gated(x, W, act="silu", bias=None, norm=None):
     I = W.out_features // 2
     if W.kind == "w8a8":
         x2, ldx = N._rows2d(x)
         T, K = x2.shape
-        q, sa, za, qs = quant_act(x2, ldx)
+        q, sa, za, qs = quant_act(x2, ldx, norm)
         out = torch.empty(T, I, dtype=torch.bfloat16, device=x.device)
         ws = N.Workspace.get(x.device)
         N._check(_lib().xft_w8a8_gemm_gated(N._p(q), K, N._p(W.w), W.w.stride(0), N._p(out), I, T, I, K, I, N._p(sa), N._p(za), N._p(qs),
@@ -216,4 +232,4 @@ def linear_gated(x, W, act="silu", bias=None):
     if W.kind == "fp8" and I % 128:
         gu = _qgemm(x, W, 2 * I, False, bias, None, None, 1.0, None)
         return N.gated_act(gu, act)
-    return _qgemm(x, W, I, True, bias, act, None, 1.0, None)
+    return _qgemm(x, W, I, True, bias, act, None, 1.0, None, norm)
