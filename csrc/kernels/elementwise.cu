@@ -491,10 +491,12 @@ __global__ void __launch_bounds__(128) mla_prep_kernel(const MlaPrepParams p) {
   const int half = p.rope / 2;
   if (h < p.Hl) {
     const bf16* src = p.q + (size_t)t * p.ldq + (size_t)h * (p.nope + p.rope);
-    bf16* dn = p.q_nope + (p.nope_head_major ? (size_t)h * p.T + t : (size_t)t * p.Hl + h) * p.nope;
+    const bool packed = p.nope_head_major == 2;            // both parts of a head behind each other, as in q
+    bf16* dn = p.q_nope + (packed ? ((size_t)t * p.Hl + h) * (p.nope + p.rope)
+                                  : (p.nope_head_major ? (size_t)h * p.T + t : (size_t)t * p.Hl + h) * p.nope);
     for (int d = lane * 2; d < p.nope; d += 64)
       *reinterpret_cast<__nv_bfloat162*>(dn + d) = *reinterpret_cast<const __nv_bfloat162*>(src + d);
-    bf16* dr = p.q_rope + ((size_t)t * p.Hl + h) * p.rope;
+    bf16* dr = packed ? dn + p.nope : p.q_rope + ((size_t)t * p.Hl + h) * p.rope;
     for (int i = lane; i < half; i += 32) {
       const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(src + p.nope + 2 * i);
       const float x1 = __low2float(x), x2 = __high2float(x), c = cs[i], s = cs[half + i];

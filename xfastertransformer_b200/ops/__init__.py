@@ -238,13 +238,16 @@ def latent_cache_write(latent, cache, slots):
     cache[(slots // blk).long(), 0, (slots % blk).long()] = latent.to(cache.dtype)
 
 
-def mla_prep(q, kv, Hl, nope, rope, kvl, positions, table, kv_norm_w, eps, cache, slots):
+def mla_prep(q, kv, Hl, nope, rope, kvl, positions, table, kv_norm_w, eps, cache, slots, cu_q=None, vd=0):
     """What sits between the MLA projections and the MLA attention: split every query head of q [T, Hl*(nope+rope)]
     into its no-position part and its rotated part (interleaved pairs), RMS-normalise the compressed KV kv[:, :kvl],
     rotate the shared key part kv[:, kvl:], and append (normalised KV ‖ rotated key) to the latent cache at `slots`.
-    Returns (q_nope [T,Hl,nope], q_rope [T,Hl,rope]).  One kernel on the GPU."""
+    Returns (q_nope [T,Hl,nope], q_rope [T,Hl,rope]).  One kernel on the GPU.  `cu_q` (prompts) and `vd`, the values' size: what the
+    attention behind it is asked for, so that the queries come in the layout that it reads."""
     if _cuda(q) and cache.dtype == torch.bfloat16:
-        return _nat().mla_prep(q, kv, Hl, nope, rope, kvl, positions, table, kv_norm_w, eps, cache, slots)
+        from .native_mla import expands
+        return _nat().mla_prep(q, kv, Hl, nope, rope, kvl, positions, table, kv_norm_w, eps, cache, slots,
+                               cu_q is not None and expands(cu_q, nope, rope, kvl, vd))
     T = q.shape[0]
     q3 = q.reshape(T, Hl, nope + rope)
     ckv = R.rmsnorm(kv[:, :kvl], kv_norm_w, eps)

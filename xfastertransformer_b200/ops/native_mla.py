@@ -1,5 +1,7 @@
-"""DeepSeek MLA on the GPU: absorb GEMMs as grouped tcgen05 GEMMs (one group per head) around the latent-cache
-attention kernel (csrc/kernels/mla.cu).  The absorbed form is used for prefill and decode alike."""
+"""DeepSeek MLA on the GPU.  Decode steps and portions of a few tokens take the absorbed form: grouped tcgen05 GEMMs (one group per head)
+around the latent-cache attention kernel (csrc/kernels/mla.cu), which works per token.  Longer portions take the expanded form
+(csrc/kernels/latent_prefill_sm100.cu, see native_latent): the latents that they see times W_uk and W_uv once, then attention in tiles
+of 128 queries."""
 from __future__ import annotations
 
 import ctypes as C
@@ -58,12 +60,88 @@ def _per_head_gemm(x_ht, w_stacked, H, T, n_out, k_in):
     return out
 
 
+def expands(cu_q, nope, rope, kvl, vd) -> bool:
+    """Whether a batch's portions of at least XFT_LATENT_EXPAND_MIN_Q new tokens take the expanded form: sizes that attn_flat_tc_kernel has,
+    and 64 tokens that take it, or 256 where shorter portions beside them need a launch of the other form.  us of a layer's attention
+    with its per-head products, 128 heads, absorbed / expanded (error against 64 bits): 32 prompts of about 97 tokens 2087 / 339 (2.682e-3
+    and 2.680e-3 of the result), 32 of 16 355 / 218, 8 of 8 115 / 84, one of 200 169 / 78, of 2000 3866 / 344 (2.84e-3, 2.76e-3), 64 tokens
+    behind 4000 508 / 238; one of 16 tokens 58 / 78; 140 tokens in two portions beside two short ones 128 / 174."""
+    if nope % 64 or rope % 64 or nope + rope > 256 or kvl % 8 or vd % 64 or vd > 128:
+        return False
+    least = N._ENV().latent_expand_min_q
+    n = [cu_q[i + 1] - cu_q[i] for i in range(len(cu_q) - 1)]
+    return sum(q for q in n if q >= least) >= (64 if min(n) >= least else 256)
+
+
+class _Heads:
+    """What native_latent.flat_attention asks of packed rows."""
+
+    def __init__(self, heads, nope, rope, vd, rank):
+        self.heads, self.dim, self.rot, self.vdim, self.rank = heads, nope, rope, vd, rank
+        self.q_width, self.gate, self.head_gate = heads * (nope + rope), False, False
+
+
+def _expanded(q_nope, q_rope, cache, block_table, sp, w_uk, w_uv, scale, out) -> bool:
+    """Portions `sp.long` into `out`; False where keys and values have no room."""
+    from . import native_latent as NL
+    T, Hl, nope = q_nope.shape
+    rope, L, vd = q_rope.shape[2], w_uk.shape[2], w_uv.shape[1]
+    step = (Hl * (nope + rope), nope + rope, 1)
+    if q_nope.stride() == step and q_rope.stride() == step and q_rope.data_ptr() == q_nope.data_ptr() + 2 * nope:
+        q = q_nope.as_strided((T, step[0]), (step[0], 1))                # the packed heads of mla_prep
+    else:
+        q = torch.cat([q_nope, q_rope], -1).view(T, -1)
+    nb, _, bs, W = cache.shape
+    per = max(1, min(Hl, NL.EXPAND_BYTES // (2 * sp.rows * (nope + vd))))
+    try:
+        flat = torch.empty(sp.rows, W, dtype=q.dtype, device=q.device)
+        kv = torch.empty(sp.rows * per * (nope + vd), dtype=q.dtype, device=q.device)
+    except torch.OutOfMemoryError:
+        return False
+    ws, d = N.Workspace.get(q.device), _Heads(Hl, nope, rope, vd, L)
+    N._check(NL._fn("xft_latent_gather")(N._p(cache), W, bs, nb, N._p(block_table), block_table.stride(0), N._p(sp.seq), N._p(sp.lo),
+                                         N._p(sp.row), len(sp.long), sp.rows, N._p(flat), N._p(ws.status), N._stream()), "latent_gather")
+    ws.launches += 1
+    wk, wv = w_uk.reshape(Hl * nope, L), w_uv.reshape(Hl * vd, L)
+    for h0 in range(0, Hl, per):
+        n = min(per, Hl - h0)
+        part = kv[:sp.rows * n * (nope + vd)].view(sp.rows, n * (nope + vd))
+        N.gemm_bf16(flat[:, :L], wk[h0 * nope:(h0 + n) * nope], n * nope, out=part[:, :n * nope])
+        N.gemm_bf16(flat[:, :L], wv[h0 * vd:(h0 + n) * vd], n * vd, out=part[:, n * nope:])
+        NL.flat_attention(q, d, part, flat, sp, h0, n, scale, 0, out)
+    return True
+
+
 def mla_attention(q_nope, q_rope, latent_cache, block_table, cu_q, kv_lens, w_uk, w_uv, scale, absorbed=True, meta=None):
     T, Hl, nope = q_nope.shape
     L = w_uk.shape[2]
     vd = w_uv.shape[1]
     rope = q_rope.shape[2]
     assert L == 512 and rope == 64, "MLA kernel is specialised for kv_lora_rank 512 + rope 64"
+    dev = q_nope.device
+    cu_dev, kv_dev, B, decode, max_kv = N.batch_arrays(cu_q, kv_lens, meta, dev)
+    if not decode and scale > 0 and expands(cu_q, nope, rope, L, vd):
+        from .native_latent import _Spans
+        kept = meta.meta if meta is not None else {}
+        key = ("latent spans", 0, N._ENV().latent_expand_min_q)
+        sp = kept.get(key)
+        if sp is None:
+            sp = kept[key] = _Spans(cu_q, kv_lens, 0, key[2], dev)
+        out = torch.empty(T, Hl * vd, dtype=torch.bfloat16, device=dev)
+        if _expanded(q_nope, q_rope, latent_cache, block_table, sp, w_uk, w_uv, scale, out):
+            if sp.part is not None:
+                rows, seqs, cu, kv, n, most = sp.part
+                out.index_copy_(0, rows.long(), _absorbed(q_nope.index_select(0, rows), q_rope.index_select(0, rows), latent_cache,
+                                                          block_table.index_select(0, seqs), cu, kv, n, most, w_uk, w_uv, scale,
+                                                          None).view(rows.shape[0], Hl * vd))
+            return out.view(T, Hl, vd)
+    return _absorbed(q_nope, q_rope, latent_cache, block_table, cu_dev, kv_dev, B, max_kv, w_uk, w_uv, scale,
+                     meta.meta.get("nsplit") if meta is not None else None)
+
+
+def _absorbed(q_nope, q_rope, latent_cache, block_table, cu_dev, kv_dev, B, max_kv, w_uk, w_uv, scale, splits):
+    T, Hl, nope = q_nope.shape
+    L, vd, rope = w_uk.shape[2], w_uv.shape[1], q_rope.shape[2]
     dev = q_nope.device
     ws = N.Workspace.get(dev)
     # W_uk^T stacked per head: [Hl*L, nope] (linear weight [out=L, in=nope])
@@ -76,17 +154,11 @@ def mla_attention(q_nope, q_rope, latent_cache, block_table, cu_q, kv_lens, w_uk
     wv = w_uv.reshape(Hl * vd, L)
     q_ht = q_nope.transpose(0, 1).contiguous().view(Hl * T, nope)
     q_abs = _per_head_gemm(q_ht, wk, Hl, T, L, nope)                 # [Hl*T, L]
-    if meta is not None and getattr(meta, "cu_q_dev", None) is not None:
-        cu_dev, kv_dev, max_kv, B = meta.cu_q_dev, meta.kv_lens_dev, meta.max_kv, len(kv_lens)
-    else:
-        cu_dev = torch.tensor(list(cu_q), dtype=torch.int32, device=dev)
-        kv_dev = torch.tensor(list(kv_lens), dtype=torch.int32, device=dev)
-        max_kv, B = max(kv_lens), len(kv_lens)
     o_lat = torch.empty(Hl * T, L, dtype=torch.bfloat16, device=dev)
     nb, _, bs, W = latent_cache.shape
     chunks = (Hl + 15) // 16
     from .native_latent import mla_scratch, mla_splits
-    nsplit, groups = (meta.meta.get("nsplit") if meta is not None else None) or mla_splits(T * chunks, max_kv)
+    nsplit, groups = splits or mla_splits(T * chunks, max_kv)
     po, pm, cnt = mla_scratch(ws, T * chunks, nsplit, groups, L)
     q_rope = q_rope.contiguous()
     LL = C.c_longlong
