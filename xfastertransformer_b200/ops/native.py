@@ -64,7 +64,8 @@ def _p(t: Optional[torch.Tensor]):
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the raw handle of torch.cuda.current_stream(), which takes several us to make an object around it
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _check(rc: int, what: str) -> None:
