@@ -358,14 +358,14 @@ def pick_bn(T: int) -> int:
 
 
 def _use_cluster(T, N, K, gated) -> bool:
-    """Whether a decode-size product (T <= 64) runs on the pipeline of gemm_bf16_cluster (gemm_e4m3_sm100.cu), on B200 the faster one
-    but for two ends: above 32 rows one CTA fits an SM there, and with more tiles than SMs nothing hides its finish (32000 x 4096,
-    64 rows 68 us, the tile-per-CTA kernel 60; 12288 x 4096 27 and 40; gated products have twice the stream per tile: 2 x 28672 x
-    8192 163 and 185), and gated products of less than half a million weights a half (2 x 256 x 512, 8 rows 5.5 us and 4.8;
-    2 x 2816 x 1024 6.2 and 6.7)."""
+    """Whether a decode-size product (T <= 64) runs on the pipeline of gemm_bf16_cluster (gemm_e4m3_sm100.cu), on B200 the faster one.
+    us, there and the other kernel: 32000 x 4096 32 rows 44 and 54, 64 rows 50 and 70; 151936 x 896 64 rows 76 and 155; 12288 x 4096 64
+    rows 24 and 40.  But for two ends where its sums are further off (against 64 bits, of the result): gated products of less than half
+    a million weights a half (2 x 256 x 512, 8 rows 4.3 us and 5.2, 4.7e-7 and 2.7e-7), and above 32 rows with more tiles than SMs
+    reductions of up to 512 (32000 x 512 4.7e-7 and 4.1e-7; 32000 x 4096 1.0e-6 and 4.5e-6)."""
     if not _ENV().gemm_cluster or (gated and N * K < 1 << 19):
         return False
-    return T <= 32 or gated or N <= 148 * 128
+    return T <= 32 or gated or N <= 148 * 128 or K > 512
 
 
 def _gemm_cluster(x2, ldx, w, out, T, N, K, gated, dual_off, bias, r2, ldr, res_scale, act, rms_eps=None):
