@@ -100,6 +100,10 @@ struct E4Layout {
   static constexpr int A_RING = SRC == kSrcU4 ? 2 * A_BYTES : 0;                      // expanded codes, two buffers
   // two CTAs per SM where registers allow: one CTA's last accumulators and stores hide behind the other's stream
   static constexpr int CTAS = BN <= 32 && A_RING + 3 * STAGE <= 110 * 1024 ? 2 : 1;
+  // Registers are left for the CTAs of the kernels behind: with programmatic launches those sit beside this one, their first weights
+  // under way.  At 90 registers (16 rows, bf16) instead of 64 the products of a 7B layer were as fast one behind the other, but 31 steps
+  // of one row over 16 layers took 48.3 ms instead of 46.3.
+  static constexpr int MIN_CTAS = CTAS == 2 && (BN == 16 || SRC == kSrcI8) ? 3 : CTAS;
   static constexpr int FIT = ((CTAS == 2 ? 110 : 222) * 1024 - A_RING) / STAGE;
   static constexpr int STAGES = FIT > 8 ? 8 : FIT;
   static constexpr int SMEM = A_RING + STAGES * STAGE + 1024;
@@ -107,7 +111,7 @@ struct E4Layout {
 };
 
 template <int BN, bool DUAL, int SRC>
-__global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
+__global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
     gemm_e4m3_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const E4Params p) {
   using L = E4Layout<BN, DUAL, SRC>;
   constexpr int NACC = L::NACC, STAGES = L::STAGES;
@@ -266,7 +270,22 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
   const bool vec = n + 4 <= p.N && (p.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & (p.out_fp32 ? 15 : 7)) == 0;
   const bool vec_res = n + 4 <= p.N && (p.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 7) == 0;
   constexpr int MINE = BN / 8;
-  uint2 res[MINE];                                                     // residuals of those tokens
+  auto residual_of = [&](int i) {                                      // of this thread's i-th token
+    uint2 v = make_uint2(0, 0);
+    const int c = rank * per + warp - 2 + 8 * i;
+    if (p.residual && warp - 2 + 8 * i < per && c < x_rows) {
+      const __nv_bfloat16* r = p.residual + (size_t)(x_row0 + c) * p.ldr + n;
+      if (vec_res) {
+        v = *reinterpret_cast<const uint2*>(r);
+      } else {
+        __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(&v);
+#pragma unroll
+        for (int f = 0; f < 4; ++f)
+          if (n + f < p.N) to[f] = r[f];
+      }
+    }
+    return v;
+  };
   if (NCOL && warp >= 2) {                                             // weights' numbers depend on no earlier kernel
     const int e = threadIdx.x - 64, nn = tile_n * 128 + (e & 127);
     if (e < 128 * NACC) {
@@ -276,7 +295,10 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
       for (int i = 0; i < NCOL; ++i) s_col[i][e >> 7][e & 127] = nn < p.N && from[i] ? __ldg(from[i] + at) : 0.f;
     }
   }
+  // residuals are asked for a token ahead, the first beside the main loop (all of them there cost every launch 0.4 us)
+  uint2 next_res = make_uint2(0, 0);
   auto fetch_rows = [&]() {                                            // what earlier kernels leave per token
+    next_res = residual_of(0);
     const int e = threadIdx.x - 64;
     if (e < BN) {
       const int t = x_row0 + e;
@@ -288,22 +310,6 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
         if constexpr (SRC == kSrcI8) { s_row[1][e] = in ? p.a_zero[t] : 0.f; s_row[2][e] = in ? p.a_qsum[t] : 0.f; }
         if constexpr (SRC == kSrcU4) s_row[1][e] = in ? p.x_sum[t] : 0.f;
         if constexpr (SRC == kSrcFp8) s_row[1][e] = in && p.col_scale ? p.col_scale[t] : 1.f;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < MINE; ++i) {
-      const int c = rank * per + warp - 2 + 8 * i;
-      res[i] = make_uint2(0, 0);
-      if (p.residual && warp - 2 + 8 * i < per && c < x_rows) {
-        const __nv_bfloat16* r = p.residual + (size_t)(x_row0 + c) * p.ldr + n;
-        if (vec_res) {
-          res[i] = *reinterpret_cast<const uint2*>(r);
-        } else {
-          __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(&res[i]);
-#pragma unroll
-          for (int f = 0; f < 4; ++f)
-            if (n + f < p.N) to[f] = r[f];
-        }
       }
     }
   };
@@ -443,8 +449,8 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
     }
   }
   // Every MMA has read its operands (the last accumulator is here), so the ring is free for this CTA's part of the sums, [column][128].
-  // From there a lane takes four features of a token at once: residual and output move in 8-byte pieces, what the finish needs is
-  // already here, and no load waits for the one before.  A thread per feature that walked its tokens waited for a global load in each:
+  // From there a lane takes four features of a token at once: residual and output move in 8-byte pieces, scales are already here, and
+  // no load waits for the one before.  A thread per feature that walked its tokens waited for a global load in each:
   // us, so / now: bf16 12288 x 4096 with a folded norm 16 rows 21.8 / 20.1, 64 rows 36.8 / 23.6; 2 x 11008 x 4096 32 rows 38.3 / 34.3, 64
   // rows 52.3 / 37.2; 896 x 896 16 rows 5.8 / 4.1, 64 rows 12.0 / 6.0; W8A8 12288 x 4096 32 rows 15.9 / 13.8; one row is level (2 x 11008
   // x 4096 31.5 / 32.0, 4096 x 4096 8.4 / 8.5).
@@ -477,6 +483,8 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
     for (int i = 0; i < MINE; ++i) {
       const int mine = warp - 2 + 8 * i, c = rank * per + mine;
       if (mine >= per || c >= x_rows) break;
+      const uint2 res = next_res;
+      next_res = residual_of(i + 1);
       float4 y[NACC];
       float ssq = SRC == kSrcBf16 ? s_row[0][c] : 0.f;
       const bool own_ssq = SRC == kSrcBf16 && p.rms_x && !p.rms_ssq;
@@ -517,7 +525,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::CTAS)
         }
       }
       const size_t t = x_row0 + c;
-      const __nv_bfloat16* rv = reinterpret_cast<const __nv_bfloat16*>(&res[i]);
+      const __nv_bfloat16* rv = reinterpret_cast<const __nv_bfloat16*>(&res);
       float ts = 1.f;
       if (SRC == kSrcBf16 && p.rms_x) ts = rsqrtf(ssq / (float)p.K + p.rms_eps);
       float out[4];
