@@ -436,8 +436,9 @@ __device__ __forceinline__ void leave_cluster(const AttnParams& p) {
 // global scratch and the slice that arrives last merges all — no second kernel, no spinning.  Every thread of the CTA calls it.
 // The sums are the same.  us by scratch / in clusters: bf16 cache, one sequence of 3000 keys, 32 and 8 heads, five slices 14.5 / 9.6;
 // 8 of 2870 in four 21.0 / 18.7; 2 of 3000, 64 and 8 heads, five 20.0 / 12.4; int8 cache, 8 of 2870 in four 21.5 / 19.4.
-// APART: column n of accumulator j is head feature n * HD / 8 + j (attn_decode_i8_kernel), else j * 8 + n.
-template <int HD, bool APART = false, class WA>
+// RING: a kernel that may be launched in clusters.  APART: column n of accumulator j is head feature n * HD / 8 + j
+// (attn_decode_i8_kernel), else j * 8 + n.
+template <int HD, bool RING, bool APART = false, class WA>
 __device__ __forceinline__ void decode_finish(const AttnParams& p, WA& wa, float* mo, bool consumer, int warp, int lane,
                                               int tid, int nthreads, int nq, int h_lo, int b, int tok, int split) {
   constexpr int RS = HD + 2;
@@ -476,7 +477,7 @@ __device__ __forceinline__ void decode_finish(const AttnParams& p, WA& wa, float
     const int h = h_lo + r;
     if (p.nsplit == 1) {
       p.out[((size_t)tok * p.hq + h) * HD + d] = __float2bfloat16(ll > 0.f ? acc / ll : 0.f);
-    } else if (p.cluster) {
+    } else if (RING && p.cluster) {
       float* part = mo + 4 * 16 * RS + r * RS;
       part[d] = acc;
       if (d == 0) { part[HD] = mm; part[HD + 1] = ll; }
@@ -486,7 +487,7 @@ __device__ __forceinline__ void decode_finish(const AttnParams& p, WA& wa, float
       if (d == 0) { p.part_ml[pi * 2] = mm; p.part_ml[pi * 2 + 1] = ll; }
     }
   }
-  if (p.nsplit > 1 && p.cluster) {
+  if (RING && p.nsplit > 1 && p.cluster) {
     __syncwarp();
     cluster_arrive();
     cluster_wait();
@@ -685,7 +686,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const AttnParams p) {
   cp_async_wait<0>();
   wa.reduce_l();
   __syncthreads();
-  decode_finish<HD>(p, wa, reinterpret_cast<float*>(kv), true, warp, lane, tid, 128, nq, h_lo, b, tok, split);
+  decode_finish<HD, false>(p, wa, reinterpret_cast<float*>(kv), true, warp, lane, tid, 128, nq, h_lo, b, tok, split);
 }
 
 // ------------------------------------------------------------------------------------------ decode, TMA ring
@@ -845,7 +846,7 @@ __global__ void __launch_bounds__(160, (HD <= 128 ? 2 : 1)) attn_decode_tma_kern
     return;
   }
   // every issued tile was consumed, so the ring is idle and can carry the merge
-  decode_finish<HD>(p, wa, reinterpret_cast<float*>(ring), warp < 4, warp, lane, tid, 160, nq, h_lo, b, tok, split);
+  decode_finish<HD, true>(p, wa, reinterpret_cast<float*>(ring), warp < 4, warp, lane, tid, 160, nq, h_lo, b, tok, split);
 }
 
 // ------------------------------------------------------------------------------------------ decode, int8 cache
@@ -1019,7 +1020,7 @@ __global__ void __launch_bounds__(160, 2) attn_decode_i8_kernel(const __grid_con
     leave_cluster(p);
     return;
   }
-  decode_finish<HD, true>(p, wa, reinterpret_cast<float*>(ring), warp < 4, warp, lane, tid, 160, nq, h_lo, b, tok, split);
+  decode_finish<HD, true, true>(p, wa, reinterpret_cast<float*>(ring), warp < 4, warp, lane, tid, 160, nq, h_lo, b, tok, split);
 }
 
 // The same for batches whose (sequence, kv head) pairs are more than the CTAs that fit the GPU: two CTAs per SM walk the pairs, and

@@ -468,7 +468,8 @@ class Decoder:
     # ------------------------------------------------------------------------------------
     def _quantises(self, W) -> bool:
         """Whether the product behind an RMSNorm rewrites its rows as codes, with nothing else reading the normalised state."""
-        return W is not None and W.kind in ("w8a8", "int4", "fp8") and self.spec.norm == "rms" and not self.spec.resid_from_norm
+        return (W is not None and W.kind in ("w8a8", "int4", "fp8") and self.spec.norm == "rms" and not self.spec.resid_from_norm
+                and Env.get().fuse_norm)
 
     def _norm(self, x, w, b):
         if self.spec.norm == "rms":
