@@ -94,7 +94,13 @@ __device__ __forceinline__ float gated_of(float x, float u, int act, float param
 
 template <int BN, bool DUAL, int SRC>
 struct E4Layout {
-  static constexpr int NACC = DUAL ? 2 : 1;
+  // Gated uint4, up to 32 rows: 64 gate and 64 up rows stacked in one tile.  With a tile of each, the expanded codes left room for one
+  // CTA per SM, and 2 x 11008 x 4096 kept 86 SMs busy.  us, so / stacked: 2 x 11008 x 4096 16 rows 20.9 / 19.5, 32 rows 23.0 / 22.0; 2 x
+  // 4864 x 896 7.0 / 5.3, 8.4 / 6.5; 2 x 28672 x 8192 75.0 / 69.3, 80.4 / 77.2.  64 rows leave one CTA per SM in either form, and stacked
+  // tiles read the rows twice as often: 26.9 / 35.6, 90.7 / 120.7.
+  static constexpr bool STACK = DUAL && SRC == kSrcU4 && BN <= 32;
+  static constexpr int FEAT = STACK ? 64 : 128;
+  static constexpr int NACC = DUAL && !STACK ? 2 : 1;
   static constexpr int A_BYTES = 128 * 128 * NACC, RAW_BYTES = SRC == kSrcU4 ? 128 * 64 * NACC : 0, B_BYTES = (SRC == kSrcI8 || SRC == kSrcBf16 ? 1 : 2) * BN * 128;
   static constexpr int STAGE = (SRC == kSrcU4 ? RAW_BYTES : A_BYTES) + B_BYTES;       // what TMA fills
   static constexpr int A_RING = SRC == kSrcU4 ? 2 * A_BYTES : 0;                      // expanded codes, two buffers
@@ -114,7 +120,8 @@ template <int BN, bool DUAL, int SRC>
 __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
     gemm_e4m3_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const E4Params p) {
   using L = E4Layout<BN, DUAL, SRC>;
-  constexpr int NACC = L::NACC, STAGES = L::STAGES;
+  constexpr int NACC = L::NACC, STAGES = L::STAGES, FEAT = L::FEAT, HALVES = DUAL ? 2 : 1;
+  constexpr bool STACK = L::STACK;
   constexpr int NB = SRC == kSrcI8 || SRC == kSrcBf16 ? BN : 2 * BN;   // columns of an accumulator: hi [BN], lo [BN]
   constexpr int ACC = NB * NACC;
   // bf16: k in PARTS pieces with an accumulator each.  The tensor core drops bits below an accumulator's last one at every step, so
@@ -159,7 +166,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
       mbar_init(&tmem_empty[a], 8);
-      mbar_init(&a_ready[a], 256);
+      mbar_init(&a_ready[a], 8);
       mbar_init(&a_empty[a], 1);
     }
     for (int a = 2; a < PARTS; ++a) mbar_init(&tmem_full[a], 1);
@@ -184,7 +191,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
     }
     __syncthreads();
   }
-  const int w_row0 = (grouped ? s_group[0] * p.group_w_rows : 0) + tile_n * 128;
+  const int w_row0 = (grouped ? s_group[0] * p.group_w_rows : 0) + tile_n * FEAT;
   const int x_row0 = grouped ? s_group[1] : tile_t * BN;
   const int x_rows = grouped ? s_group[2] : min(BN, p.T - x_row0);
   const int kend = x_rows > 0 ? kb1 : kb0;                             // nothing to do for a tile without rows
@@ -203,7 +210,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
         mbar_expect_tx(&full_bar[s], L::STAGE);
         uint8_t* st = ring + s * L::STAGE;
         tma_load_2d(st, &tmW, &full_bar[s], kb * W_STEP, w_row0, hint_w);
-        if (DUAL) tma_load_2d(st + W_TILE, &tmW, &full_bar[s], kb * W_STEP, p.dual_off + w_row0, hint_w);
+        if (DUAL) tma_load_2d(st + FEAT * W_COLS, &tmW, &full_bar[s], kb * W_STEP, p.dual_off + w_row0, hint_w);
       };
       auto load_x = [&](int s, int kb) {
         uint8_t* st = ring + s * L::STAGE + W_TILE * NACC;
@@ -248,7 +255,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
             else umma_f8(d, a, bd + 2 * k, IDESC, on);
           };
           mma(acc, ad + 2 * k);
-          if (DUAL) mma(acc + NB, ad + TILE_A / 16 + 2 * k);
+          if (NACC == 2) mma(acc + NB, ad + TILE_A / 16 + 2 * k);
         }
         tcgen05_commit(&empty_bar[r.s]);
         if (PARTS > 1 && (++in_part == part_kb || kb + 1 == kend)) {
@@ -265,15 +272,18 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
 
   // ---- warps 2..9: row = feature of the tile, tokens [c0, c0 + HB) of it
   const int q = warp & 3, row = q * 32 + lane, half = warp >= 6, c0 = half * HB;
-  // the finish: warp w takes tokens w, w + 8, .. of this CTA's share of the tile, a lane four features of each
-  const int per = BN / p.splits, f0 = lane * 4, n = tile_n * 128 + f0;
+  // the finish: warp w takes tokens w, w + 8, .. of this CTA's share of the tile, a lane four features of each (stacked tiles: half a
+  // warp a token)
+  constexpr int AT_ONCE = STACK ? 16 : 8;
+  const int per = BN / p.splits, f0 = (STACK ? lane & 15 : lane) * 4, n = tile_n * FEAT + f0;
+  const int tok0 = STACK ? 2 * (warp - 2) + (lane >> 4) : warp - 2;
   const bool vec = n + 4 <= p.N && (p.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & (p.out_fp32 ? 15 : 7)) == 0;
   const bool vec_res = n + 4 <= p.N && (p.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 7) == 0;
-  constexpr int MINE = BN / 8;
+  constexpr int MINE = BN / AT_ONCE;
   auto residual_of = [&](int i) {                                      // of this thread's i-th token
     uint2 v = make_uint2(0, 0);
-    const int c = rank * per + warp - 2 + 8 * i;
-    if (p.residual && warp - 2 + 8 * i < per && c < x_rows) {
+    const int c = rank * per + tok0 + AT_ONCE * i;
+    if (p.residual && tok0 + AT_ONCE * i < per && c < x_rows) {
       const __nv_bfloat16* r = p.residual + (size_t)(x_row0 + c) * p.ldr + n;
       if (vec_res) {
         v = *reinterpret_cast<const uint2*>(r);
@@ -287,9 +297,9 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
     return v;
   };
   if (NCOL && warp >= 2) {                                             // weights' numbers depend on no earlier kernel
-    const int e = threadIdx.x - 64, nn = tile_n * 128 + (e & 127);
+    const int e = threadIdx.x - 64, nn = tile_n * FEAT + (e & (FEAT - 1));
     if (e < 128 * NACC) {
-      const int at = (e >= 128 ? p.dual_off : 0) + nn;
+      const int at = (e >= FEAT ? p.dual_off : 0) + nn;
       const float* from[3] = {p.scale, p.zero, p.w_sum};
 #pragma unroll
       for (int i = 0; i < NCOL; ++i) s_col[i][e >> 7][e & 127] = nn < p.N && from[i] ? __ldg(from[i] + at) : 0.f;
@@ -417,15 +427,19 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
       Ring r = {0, 0}, b = {0, 0};
       bool alive = true;
       for (int kb = kb0; kb < kend; ++kb, r.next(STAGES), b.next(2)) {
-        alive = alive && mbar_wait(&full_bar[r.s], r.ph, p.status, XFT_ERR_WAIT_FULL) &&
-                mbar_wait(&a_empty[b.s], b.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY);
+        uint4 codes[2 * NACC];
+        alive = alive && mbar_wait(&full_bar[r.s], r.ph, p.status, XFT_ERR_WAIT_FULL);
         if (alive) {
-          const uint8_t* raw = ring + r.s * L::STAGE;
+#pragma unroll
+          for (int i = 0; i < 2 * NACC; ++i) codes[i] = *reinterpret_cast<const uint4*>(ring + r.s * L::STAGE + (e + 256 * i) * 16);
+        }
+        alive = alive && mbar_wait(&a_empty[b.s], b.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY);
+        if (alive) {
           uint8_t* a = smem + b.s * L::A_BYTES;
 #pragma unroll
           for (int i = 0; i < 2 * NACC; ++i) {
             const int ci = e + 256 * i, tr = ci >> 2, part = ci & 3;   // row of the stacked tiles, 32 codes of it
-            const uint4 w = *reinterpret_cast<const uint4*>(raw + ci * 16);
+            const uint4 w = codes[i];
             constexpr uint32_t M = 0x0F0F0F0Fu;
             uint8_t* dst = a + tr * 128;
             *reinterpret_cast<uint4*>(dst + (((2 * part) ^ (tr & 7)) << 4)) = make_uint4(w.x & M, w.y & M, w.z & M, w.w & M);
@@ -434,7 +448,8 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
           }
           fence_proxy_async();
         }
-        mbar_arrive(&a_ready[b.s]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&a_ready[b.s]);                     // per warp: with 256 arrivals a block 2 x 28672 x 8192 64 rows took 90.7 us, so 86
       }
       grid_dep_wait();
       fetch_rows();
@@ -443,7 +458,7 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
         tcgen05_fence_after();
         if (ok) {
           fetch(0, g[0], 512.f);
-          if constexpr (DUAL) fetch(NB, g[1], 512.f);
+          if constexpr (NACC == 2) fetch(NB, g[1], 512.f);
         }
       }
     }
@@ -469,9 +484,9 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
     named_bar_sync(1, 256);
   }
   if (warp >= 2 && n < p.N && (ok || p.splits > 1)) {
-    float4 bias[NACC];
+    float4 bias[HALVES];
 #pragma unroll
-    for (int a = 0; a < NACC; ++a) {
+    for (int a = 0; a < HALVES; ++a) {
       bias[a] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (p.bias) {
 #pragma unroll
@@ -481,17 +496,18 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
     }
 #pragma unroll 1
     for (int i = 0; i < MINE; ++i) {
-      const int mine = warp - 2 + 8 * i, c = rank * per + mine;
+      const int mine = tok0 + AT_ONCE * i, c = rank * per + mine;
       if (mine >= per || c >= x_rows) break;
       const uint2 res = next_res;
       next_res = residual_of(i + 1);
-      float4 y[NACC];
+      float4 y[HALVES];
       float ssq = SRC == kSrcBf16 ? s_row[0][c] : 0.f;
       const bool own_ssq = SRC == kSrcBf16 && p.rms_x && !p.rms_ssq;
+      constexpr int UP = STACK ? 64 : BN * 128;                        // from a gate feature to its up feature
       const uint32_t at = smem_u32(part + c * 128 + f0), at_ssq = smem_u32(s_ssq + (SRC == kSrcBf16 ? c : 0));
       if (p.splits == 1) {
 #pragma unroll
-        for (int a = 0; a < NACC; ++a) y[a] = *reinterpret_cast<const float4*>(part + (a * BN + c) * 128 + f0);
+        for (int a = 0; a < HALVES; ++a) y[a] = *reinterpret_cast<const float4*>(part + c * 128 + f0 + a * UP);
         if (own_ssq) ssq += s_ssq[SRC == kSrcBf16 ? c : 0];
       } else {
         float q[8];
@@ -500,10 +516,10 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
           for (int r = 0; r < 8; ++r) q[r] = r < p.splits ? ld_dsmem(dsmem_addr(at_ssq, r)) : 0.f;
         }
 #pragma unroll
-        for (int a = 0; a < NACC; ++a) {
+        for (int a = 0; a < HALVES; ++a) {
           float4 v[8];
 #pragma unroll
-          for (int r = 0; r < 8; ++r) v[r] = r < p.splits ? ld_dsmem4(dsmem_addr(at + a * BN * 512, r)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int r = 0; r < 8; ++r) v[r] = r < p.splits ? ld_dsmem4(dsmem_addr(at + a * UP * 4, r)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
           for (int f = 0; f < 4; ++f) {
             if constexpr (SRC == kSrcI8) {
@@ -531,8 +547,8 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
       float out[4];
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
-        float x = (&y[0].x)[f], u = DUAL ? (&y[NACC - 1].x)[f] : 0.f;
-        const float b = (&bias[0].x)[f], bu = (&bias[NACC - 1].x)[f], r = __bfloat162float(rv[f]);
+        float x = (&y[0].x)[f], u = DUAL ? (&y[HALVES - 1].x)[f] : 0.f;
+        const float b = (&bias[0].x)[f], bu = (&bias[HALVES - 1].x)[f], r = __bfloat162float(rv[f]);
         if constexpr (SRC == kSrcBf16) {
           x = x * ts + b;
           if (DUAL) x = gated_of(x, u * ts + bu, p.act, p.res_scale);
@@ -551,7 +567,8 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
           if constexpr (SRC == kSrcU4) {
             const float xs = s_row[1][c];
             x = act_of(fmaf(x, st * s_col[0][0][f0 + f], b + s_col[1][0][f0 + f] * xs), p.act, 1.f);
-            if (DUAL) x *= fmaf(u, st * s_col[0][NACC - 1][f0 + f], bu + s_col[1][NACC - 1][f0 + f] * xs);
+            constexpr int AT = STACK ? 64 : 0;                         // up features of a stacked tile
+            if (DUAL) x *= fmaf(u, st * s_col[0][NACC - 1][AT + f0 + f], bu + s_col[1][NACC - 1][AT + f0 + f] * xs);
           } else {
             x = act_of(fmaf(x, st, b), p.act, 1.f);
             if (DUAL) x *= fmaf(u, st, bu);
@@ -702,7 +719,7 @@ int make_byte_map(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t row
 
 // Parts of a tile's k: as many as one round of clusters holds, at least four blocks of k in each.  GPCs differ in their SMs, so what
 // fits is not a division: clusters of 2, 4 and 8 CTAs that B200 takes at a time, with one and with two CTAs per SM.  us, gated uint4
-// 2 x 11008 x 4096 (86 tiles, one CTA per SM), 16 rows: 31.7 with two parts, 24.3 with one; e4m3 24 rows 33.9 and 24.8; bf16 4608 x
+// 2 x 11008 x 4096 (86 tiles of each half, one CTA per SM), 16 rows: 31.7 with two parts, 24.3 with one; e4m3 24 rows 33.9 and 24.8; bf16 4608 x
 // 3584 (36 tiles) with its rotation behind it, 16 rows: 16.0 with eight parts, 12.4 with four, 48 rows 23.4 with four, 19.6 with two.
 static int e4_splits(int tiles, int num_kb, int per_sm) {
   constexpr int kFit[2][3] = {{74, 33, 15}, {148, 71, 33}};
@@ -776,11 +793,12 @@ extern "C" int xft_gemm_e4m3(const void* xs, int x_rows, const float* x_scale, c
   p.group_tiles = reinterpret_cast<const int4*>(group_tiles); p.num_group_tiles = num_group_tiles; p.group_w_rows = group_w_rows;
   p.x_lo = xft_split_e4m3_cols(K);
   if (!group_tiles) bn = T <= 16 ? 16 : T <= 32 ? 32 : 64;
+  const int feat = src == kSrcU4 && gated && bn <= 32 ? 64 : 128;                  // E4Layout::FEAT
   p.num_kb = (K + 127) / 128;
-  p.n_tiles = (N + 127) / 128;
+  p.n_tiles = (N + feat - 1) / feat;
   p.t_tiles = group_tiles ? max_tiles : (T + bn - 1) / bn;
   CUtensorMap tmW, tmX;
-  int r = src == kSrcU4 ? make_byte_map(&tmW, W, (uint64_t)w_rows, (uint64_t)K / 2, (uint64_t)ldw_bytes, 128, 64)
+  int r = src == kSrcU4 ? make_byte_map(&tmW, W, (uint64_t)w_rows, (uint64_t)K / 2, (uint64_t)ldw_bytes, (uint32_t)feat, 64)
                         : make_tensor_map(&tmW, W, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw_bytes, 128, 1);
   if (r) return 1000 - r;
   r = make_tensor_map(&tmX, xs, (uint64_t)x_rows, (uint64_t)2 * p.x_lo, (uint64_t)2 * p.x_lo, (uint32_t)bn, 1);

@@ -56,6 +56,26 @@ def test_gated_matches_its_parts(kind, T, I, K):
     assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16 * gu.abs().amax()).all())
 
 
+@pytest.mark.parametrize("T,I,K", [(1, 8, 64), (2, 72, 528), (16, 1096, 1040), (17, 200, 4096), (33, 136, 528), (64, 64, 2048), (100, 584, 272)])
+def test_gated_uint4_ragged_features_match_64_bits(T, I, K):
+    """Features that do not fill a tile of 64 gate and 64 up rows, one feature tile and many, with and without parts of k.  The products
+    of either half are within the bound of `test_split_activations_match_64_bits`; |silu'| <= 1.1 and |silu(g)| <= |g| carry it on,
+    and the result rounds to bf16."""
+    from xfastertransformer_b200.ops import native as Nat
+    g = torch.Generator(device="cuda").manual_seed(T + I + K)
+    x = torch.randn(T, K, generator=g, device="cuda").bfloat16()
+    W = _linear(torch.randn(2 * I, K, generator=g, device="cuda") * 0.05, "int4")
+    w = R.dequant_weight(W).double()
+    gu = x.double() @ w.t()
+    tol = 2.0 ** -18 * (x.double().abs() @ (w.abs().t() + W.zero.double().abs()[None] * 2)) + \
+        2.0 ** -21 * x.double().abs().amax(1, keepdim=True) * w.abs().sum(1)[None]
+    want = torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]
+    got = Nat.linear_gated(x, W, "silu").double()
+    Nat.Workspace.get(x.device).check_status()
+    bound = 1.1 * tol[:, :I] * gu[:, I:].abs() + (gu[:, :I].abs() + 1.1 * tol[:, :I]) * tol[:, I:] + 2.0 ** -8 * want.abs() + 2.0 ** -20
+    assert bool(((got - want).abs() <= bound).all()), ((got - want).abs() / bound).max().item()
+
+
 @pytest.mark.parametrize("T,N,K", [s for s in SHAPES if s[2] % 16 == 0] + [(300, 136, 144), (2300, 4104, 1024)])
 def test_w8a8_sums_are_exact(T, N, K):
     """The integers that the tensor path sums, from the same codes: only the fp32 formula around the sum rounds."""
