@@ -550,8 +550,9 @@ __global__ void __launch_bounds__(kE4Threads, E4Layout<BN, DUAL, SRC>::MIN_CTAS)
         float x = (&y[0].x)[f], u = DUAL ? (&y[HALVES - 1].x)[f] : 0.f;
         const float b = (&bias[0].x)[f], bu = (&bias[HALVES - 1].x)[f], r = __bfloat162float(rv[f]);
         if constexpr (SRC == kSrcBf16) {
-          x = x * ts + b;
-          if (DUAL) x = gated_of(x, u * ts + bu, p.act, p.res_scale);
+          // Which multiply-adds are fused is spelled out: a last bit here moves every logit of a model with biases behind folded norms
+          x = DUAL ? __fmaf_rn(x, ts, b) : __fadd_rn(__fmul_rn(x, ts), b);
+          if (DUAL) x = gated_of(x, __fadd_rn(__fmul_rn(u, ts), bu), p.act, p.res_scale);
           else x = act_of(x, p.act, p.res_scale);
           if (p.residual) x = with_residual(x, r, p.res_scale, p.act);
         } else if constexpr (SRC == kSrcI8) {
