@@ -453,20 +453,7 @@ __global__ void __launch_bounds__(256) row_sum_kernel(const __nv_bfloat16* __res
   grid_dep_wait();
   const int t = blockIdx.x;
   float acc = 0.f;
-  const __nv_bfloat16* row = x + (size_t)t * ldx;
-  if (((K | ldx) & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-    for (int i = threadIdx.x * 8; i < K; i += 2048) {
-      const uint4 v = *reinterpret_cast<const uint4*>(row + i);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = __bfloat1622float2(h[j]);
-        acc += f.x + f.y;
-      }
-    }
-  } else {
-    for (int i = threadIdx.x; i < K; i += 256) acc += __bfloat162float(row[i]);
-  }
+  for (int i = threadIdx.x; i < K; i += 256) acc += __bfloat162float(x[(size_t)t * ldx + i]);
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) ssum[threadIdx.x >> 5] = acc;
   __syncthreads();
