@@ -739,7 +739,10 @@ static int launch_e4(const CUtensorMap& tmW, const CUtensorMap& tmX, E4Params p,
       return 3000 + (int)cudaGetLastError();
     attr_set = true;
   }
-  p.splits = p.group_tiles ? 1 : e4_splits(p.n_tiles * p.t_tiles, p.num_kb, L::CTAS);
+  // stacked tiles: as many parts as tiles of 128 features on an SM each would have (64 rows have those), so a row's sums do not depend on
+  // how many rows stand beside it
+  p.splits = p.group_tiles ? 1 : L::STACK ? e4_splits((p.n_tiles + 1) / 2 * p.t_tiles, p.num_kb, 1)
+                                          : e4_splits(p.n_tiles * p.t_tiles, p.num_kb, L::CTAS);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.n_tiles * p.t_tiles, p.splits);
   cfg.blockDim = dim3(kE4Threads);
