@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(192, 1) gemm_prefill_kernel(const __grid_const
 // up rows.  Both producers signal the first CTA's full barrier; a commit frees the stage in both.
 //
 // NCOL: accumulator columns of a tile (gated: half of them gate, half up).
-// SRC: bf16 operands; int8 operands of W8A8; bf16 activations and codes (int8 or uint4, exact in bf16, see xft_gemm_codes_tm), whose
+// SRC: bf16 operands; int8 operands of W8A8; bf16 activations and int8 codes (exact in bf16, see xft_gemm_codes_tm), whose
 // scale and zero point per weight row come in with the epilogue.
 enum { kTmBf16 = 0, kTmI8 = 1, kTmCodes = 2 };
 constexpr int kPrefillTmThreads = 320;      // producer, MMA, two epilogue warps per quarter of the accumulator's rows
@@ -653,8 +653,9 @@ __global__ void __launch_bounds__(kPrefillTmThreads, 1) gemm_prefill_tm_kernel(c
 #pragma unroll
           for (int j = 0; j < CW; ++j) {
             const int m = whole || nn % p.dual_rows + j < p.N ? nn + j : nn;
-            const float b = p.bias ? __ldg(p.bias + m) : 0.f;
-            to[j] = fmaf(__uint_as_float(acc[j]), __ldg(p.w_scale + m), p.w_zero ? fmaf(__ldg(p.w_zero + m), xs, b) : b);
+            // the roundings of qgemm_kernel (quant_gemm_sm100.cu), spelled out
+            const float y = __fmul_rn(__uint_as_float(acc[j]), __ldg(p.w_scale + m));
+            to[j] = __fadd_rn(p.w_zero ? __fmaf_rn(__ldg(p.w_zero + m), xs, y) : y, p.bias ? __ldg(p.bias + m) : 0.f);
           }
           return;
         }
@@ -1061,48 +1062,26 @@ extern "C" int xft_gemm_bf16_grouped_tm(const void* X, int ldx, int x_rows, cons
 }
 
 namespace xft {
-// Codes of weights as bf16, four rows per block, 16 codes of each per thread.  uint4: the even one of a byte's two in its low half.
-// Bound by the stores.
+// int8 codes of weights as bf16, four rows per block, 16 codes of each per thread.  Bound by the stores.
 constexpr int kCodeRows = 4;
-template <bool U4>
 __global__ void __launch_bounds__(256) codes_bf16_kernel(const uint8_t* __restrict__ w, long long ldw, int rows, int K,
                                                          __nv_bfloat16* __restrict__ out) {
   grid_dep_launch();
   const int k = (blockIdx.y * 256 + threadIdx.x) * 16, r0 = blockIdx.x * kCodeRows;
   uint4 raw[kCodeRows];
 #pragma unroll
-  for (int i = 0; i < kCodeRows; ++i) {
-    const uint8_t* src = w + (size_t)(r0 + i) * ldw;
-    if (k < K && r0 + i < rows) {
-      if constexpr (U4) {
-        const uint2 h = *reinterpret_cast<const uint2*>(src + k / 2);
-        raw[i].x = h.x; raw[i].y = h.y;
-      } else {
-        raw[i] = *reinterpret_cast<const uint4*>(src + k);
-      }
-    }
-  }
+  for (int i = 0; i < kCodeRows; ++i)
+    if (k < K && r0 + i < rows) raw[i] = *reinterpret_cast<const uint4*>(w + (size_t)(r0 + i) * ldw + k);
   grid_dep_wait();                                                     // the buffer may still be read by the product before
 #pragma unroll
   for (int i = 0; i < kCodeRows; ++i) {
     if (k >= K || r0 + i >= rows) return;
+    const int8_t* c = reinterpret_cast<const int8_t*>(&raw[i]);
     uint32_t o[8];
-    if constexpr (U4) {
-      const uint32_t q[2] = {raw[i].x, raw[i].y};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {                                    // byte j & 3: 128 + code in bf16, minus 128
-        const uint32_t c = (q[j >> 2] >> (8 * (j & 3))) & 0xff, pair = ((c & 15) | (c >> 4) << 16) | 0x43004300u;
-        const uint32_t base = 0x43004300u;
-        const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&pair), *reinterpret_cast<const __nv_bfloat162*>(&base));
-        o[j] = *reinterpret_cast<const uint32_t*>(&d);
-      }
-    } else {
-      const int8_t* c = reinterpret_cast<const int8_t*>(&raw[i]);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const __nv_bfloat162 x = __floats2bfloat162_rn((float)c[2 * j], (float)c[2 * j + 1]);
-        o[j] = *reinterpret_cast<const uint32_t*>(&x);
-      }
+    for (int j = 0; j < 8; ++j) {
+      const __nv_bfloat162 x = __floats2bfloat162_rn((float)c[2 * j], (float)c[2 * j + 1]);
+      o[j] = *reinterpret_cast<const uint32_t*>(&x);
     }
     __nv_bfloat16* dst = out + (size_t)(r0 + i) * K + k;
     if ((reinterpret_cast<uintptr_t>(dst) & 31) == 0 && k + 8 < K) {
@@ -1115,20 +1094,19 @@ __global__ void __launch_bounds__(256) codes_bf16_kernel(const uint8_t* __restri
 }
 }  // namespace xft
 
-// Prompts over int8 (u4 = 0) or uint4 weights: the codes of all w_rows rows as bf16 into `codes` [w_rows, K], which holds them exactly,
-// then the token-major product; y = scale (X codes^T) + zero sum(X) per weight row, then bias, activation, residual as in
+// Prompts over int8 weights: the codes of all w_rows rows as bf16 into `codes` [w_rows, K], which holds them exactly, then the
+// token-major product; y = scale (X codes^T) + zero sum(X) per weight row, then bias, activation, residual as in
 // xft_gemm_bf16_prefill_tm.  x_sum: the rows' sums of X, where zero is given.  K a multiple of 8, rows of W on 16 bytes.
-extern "C" int xft_gemm_codes_tm(const void* X, int ldx, const void* W, int w_rows, int ldw_bytes, int u4, void* codes, void* Y, int ldo,
+extern "C" int xft_gemm_codes_tm(const void* X, int ldx, const void* W, int w_rows, int ldw_bytes, void* codes, void* Y, int ldo,
                                  int out_fp32, int T, int N, int K, int gated, int dual_off, const float* scale, const float* zero,
                                  const float* x_sum, const float* bias, const void* residual, int ldr, float res_scale, int act,
                                  int* status, cudaStream_t st) {
   if (T <= 0 || N <= 0 || K <= 0) return 0;
-  if ((K & 7) || (ldx & 7) || (ldw_bytes & 15) || ldw_bytes < (u4 ? K / 2 : K) || !scale || (zero && !x_sum) ||
+  if ((K & 7) || (ldx & 7) || (ldw_bytes & 15) || ldw_bytes < K || !scale || (zero && !x_sum) ||
       ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(codes)) & 15))
     return -2;
-  const cudaError_t e = launch_pdl(u4 ? codes_bf16_kernel<true> : codes_bf16_kernel<false>,
-                                   dim3((w_rows + kCodeRows - 1) / kCodeRows, (K + 4095) / 4096), dim3(256), 0, st, (const uint8_t*)W,
-                                   (long long)ldw_bytes, w_rows, K, (__nv_bfloat16*)codes);
+  const cudaError_t e = launch_pdl(codes_bf16_kernel, dim3((w_rows + kCodeRows - 1) / kCodeRows, (K + 4095) / 4096), dim3(256), 0, st,
+                                   (const uint8_t*)W, (long long)ldw_bytes, w_rows, K, (__nv_bfloat16*)codes);
   if (e != cudaSuccess) return (int)e;
   PrefillParams p{};
   p.N = N; p.T = T; p.K = K; p.out = reinterpret_cast<__nv_bfloat16*>(Y); p.ldo = ldo; p.out_fp32 = out_fp32; p.bias = bias;

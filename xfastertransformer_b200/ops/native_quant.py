@@ -1,6 +1,6 @@
 """Bindings of the quantised GEMM kernels: weight-only int8 / nf4 dequant-GEMM and W8A8 (dynamic int8 activations x int8 weights
 on the int8 tensor path) in csrc/kernels/quant_gemm_sm100.cu, fp8-e4m3 and uint4 weights on the fp8 tensor path in
-csrc/kernels/gemm_e4m3_sm100.cu, prompts over int8 and uint4 weights in csrc/kernels/gemm_prefill_sm100.cu (CODES_ROWS)."""
+csrc/kernels/gemm_e4m3_sm100.cu, prompts over int8 weights in csrc/kernels/gemm_prefill_sm100.cu (CODES_ROWS)."""
 from __future__ import annotations
 
 import ctypes as C
@@ -63,19 +63,23 @@ def gemm_e4m3(split, w, pitch, src, out, T, n_out, K, gated, dual_off, scale, ze
     ws.launches += 1
 
 
-# Prompts over int8 or uint4 weights: above so many rows (ungated, gated) a product's codes are written out as bf16, which holds them
-# exactly, for the kernel of bf16 prompts (gemm_prefill_sm100.cu), as long as that copy stays below a bound.  The kernels that expand
-# per tile do it once for every 128 (int8) or 64 (uint4) rows.  B200, us there / here: int8 2 x 11008 x 4096 128 rows 112 / 119, 192
-# rows 199 / 118, 1210 rows 592 / 225; 12288 x 4096 128 rows 74 / 71, 192 rows 128 / 71; uint4 2 x 11008 x 4096 320 rows 111 / 138,
-# 384 rows 139 / 138, 1210 rows 392 / 212; 2 x 28672 x 8192 384 rows 510 / 495; 12288 x 4096 192 rows 62 / 68, 256 rows 85 / 68, 1210
-# rows 329 / 139; 4096 x 11008 256 rows 64 / 70, 320 rows 102 / 71.
-CODES_ROWS = {"int8": (128, 128), "int4": (256, 320)}
+# Prompts over int8 weights: above so many rows a product's codes are written out as bf16, which holds them exactly, for the kernel of
+# bf16 prompts (gemm_prefill_sm100.cu), as long as that copy stays below a bound.  qgemm_kernel, which expands them once for every 128
+# rows, keeps what it cuts into parts of k: those sums have another order.  B200, us there / here: 2 x 11008 x 4096 128 rows 112 / 119, 192
+# rows 199 / 118, 1210 rows 592 / 225; 12288 x 4096 128 rows 74 / 71, 192 rows 128 / 71.  uint4 weights stay with the halves in e4m3
+# (gemm_e4m3_sm100.cu) at any size: their sums are others too, 0.9 % of the logits after eight layers.
+CODES_ROWS = 128
 CODES_MAX_COPY = 1 << 30
 
 
-def _codes_copy(W, rows, K, T, gated, dev):
-    """Room for a product's codes in bf16, or None where it does not pay or has no room."""
-    if W.kind not in CODES_ROWS or T <= CODES_ROWS[W.kind][gated] or rows * K * 2 > CODES_MAX_COPY or not N._ENV().gemm_prefill_tm:
+def _codes_copy(W, n_out, rows, K, T, gated, ws, dev):
+    """Room for a product's codes in bf16, or None where it does not pay, would change sums or has no room."""
+    if W.kind != "int8" or T <= CODES_ROWS or rows * K * 2 > CODES_MAX_COPY or not N._ENV().gemm_prefill_tm:
+        return None
+    parts, per = C.c_int(), C.c_int()
+    _lib().xft_plan_splits((n_out + 127) // 128 * ((T + 127) // 128), (K + 63) // 64, 128, 1 + gated, C.c_size_t(ws.ws_bytes), ws.n_counters,
+                           C.byref(parts), C.byref(per))
+    if parts.value > 1:
         return None
     try:
         return torch.empty(rows, K, dtype=torch.bfloat16, device=dev)
@@ -86,8 +90,8 @@ def _codes_copy(W, rows, K, T, gated, dev):
 def norm_fits(W, T, K, gated, gain) -> bool:
     """Whether a product of W takes (gain, eps) of an RMSNorm of its rows (csrc/kernels/quant_rows.cu): kinds that rewrite the rows in any
     case, at the sizes at which that adds a row's squares as xft_rmsnorm does."""
-    return (W.kind == "w8a8" or W.kind in _E4M3 and not (W.kind in CODES_ROWS and T > CODES_ROWS[W.kind][gated])) and 2048 <= K <= 8192 \
-        and K % 8 == 0 and gain.dtype == torch.float32 and gain.data_ptr() % 16 == 0 and not (gated and W.kind == "fp8" and W.out_features % 256)
+    return (W.kind == "w8a8" or W.kind in _E4M3) and 2048 <= K <= 8192 and K % 8 == 0 and gain.dtype == torch.float32 \
+        and gain.data_ptr() % 16 == 0 and not (gated and W.kind == "fp8" and W.out_features % 256)
 
 
 def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype, norm=None):
@@ -114,11 +118,11 @@ def _qgemm(x, W, n_out, gated, bias, act, residual, res_scale, out_dtype, norm=N
             W.cache["w_pitch16"] = wp
         w = wp
     zero = W.zero
-    copy = _codes_copy(W, w.shape[0], K, T, gated, x.device)
+    copy = _codes_copy(W, n_out, w.shape[0], K, T, gated, ws, x.device)
     if copy is not None:
         fn = _lib().xft_gemm_codes_tm
         fn.restype = C.c_int
-        N._check(fn(N._p(x2), ldx, N._p(w), w.shape[0], w.stride(0) * w.element_size(), int(W.kind == "int4"), N._p(copy), N._p(out),
+        N._check(fn(N._p(x2), ldx, N._p(w), w.shape[0], w.stride(0) * w.element_size(), N._p(copy), N._p(out),
                     out.stride(0), int(fp32), T, n_out, K, int(gated), n_out if gated else 0, N._p(W.scale), N._p(zero),
                     N._p(_row_sums(x2, ldx) if zero is not None else None), N._p(bias), N._p(r2), ldr, C.c_float(res_scale), N._ACT[act],
                     N._p(ws.status), N._stream()), "gemm_codes_tm")
