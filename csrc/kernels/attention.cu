@@ -850,21 +850,21 @@ __global__ void __launch_bounds__(160, (HD <= 128 ? 2 : 1)) attn_decode_tma_kern
 }
 
 // ------------------------------------------------------------------------------------------ decode, int8 cache
-// int8 caches with heads of 128.  The same ring, of codes and scales: a tile is 64 keys, 8 KB of K, 8 KB of V (a row of 128 codes is one
-// 128-byte swizzled row) and their scales.  Nothing is converted in shared memory: the order of the contraction is free, so a thread
-// takes 32 neighbouring codes of a key for the eight steps of S (the query's fragments are in the same order), and 16 neighbouring
-// features of four keys for the 16 column blocks of P V, in 16-byte reads without bank conflicts.  Two codes become two bf16 numbers
-// in three instructions: 128 + the low seven bits, minus 128 or 256 by the sign, all exact.
-// Bound by the instructions of a tile (about 550 per warp and 16 keys, a quarter of them conversions) and, where splits are short, by
-// start and merge.  The kernel that converts on the way into shared memory (attn_decode_kernel, still used for other head sizes) spent its
-// time on one-per-code conversions (16 per cycle and SM) and on writing and reading tiles of twice the size.  us, that / here: 8
-// sequences of 2870 keys, 32 and 8 heads 33.4 / 21.5; 32 of 2250 77.6 / 41.5; 16 of 1000, 32 heads 72.4 / 39.9; 1 of 500 12.6 / 8.2;
-// 64 of 200, 64 and 8 heads 24.9 / 17.2.
-constexpr int kI8Stage = 2 * kDecTile * 128 + 2 * kDecTile * 4;
-constexpr int kI8StageBytes = (kI8Stage + 1023) / 1024 * 1024;           // tiles start on 1024 bytes
-constexpr int kI8Stages = 5;
-constexpr int kI8Smem = kI8Stages * kI8StageBytes + 1024;
-static_assert(5 * 16 * (128 + 2) * 4 <= kI8Stages * kI8StageBytes, "the warps' and the CTA's partial results");
+// int8 caches with heads of 128: a ring of codes and scales, a slot of which is a tile of 32 keys (4 KB of K, 4 KB of V, where a row of 128
+// codes is one 128-byte swizzled row, and their scales) for one of four warps.  Tiles, slices and the order of every sum are those of
+// attn_decode_kernel, so both give the same bits.  Nothing is converted in shared memory: a step of the contraction takes the 16 codes of a
+// key that it takes there, four neighbours per thread (ldmatrix; the sum of an mma step does not depend on the order inside it), and P V
+// takes 16 neighbouring features of four keys per thread, in 16-byte reads without bank conflicts.  Two codes become two bf16 numbers in
+// three instructions: 128 + the low seven bits, minus 128 or 256 by the sign, all exact.
+// Bound by the instructions of a tile and, where splits are short, by start and merge.  The kernel that converts on the way into shared
+// memory (attn_decode_kernel, still used for other head sizes, ALiBi, caps and sinks) spends its time on one-per-code conversions (16 per
+// cycle and SM) and on writing and reading tiles of twice the size.  us, that / here: 8 sequences of 2870 keys, 32 and 8 heads 33.4 / 19.4; 32
+// of 2250 78.5 / 40.5; 16 of 1000, 32 heads 72.0 / 38.5; 1 of 500 14.5 / 7.5; 64 of 200, 64 and 8 heads 25.1 / 17.1; 2 of 32000 75.8 / 46.0.
+constexpr int kI8Tile = 32, kI8Slots = 12;
+constexpr int kI8SlotBytes = 2 * kI8Tile * 128, kI8ScaleBytes = 2 * kI8Tile * 4;
+constexpr int kI8Smem = kI8Slots * (kI8SlotBytes + kI8ScaleBytes) + 1024;
+static_assert(kI8Slots % 4 == 0, "a warp's slots");
+static_assert(5 * 16 * (128 + 2) * 4 <= kI8Slots * kI8SlotBytes, "the warps' and the CTA's partial results");
 
 // The codes in the low bytes of both halves as bf16
 __device__ __forceinline__ uint32_t codes_bf16(uint32_t w) {
@@ -877,15 +877,16 @@ __device__ __forceinline__ uint32_t codes_bf16(uint32_t w) {
 
 __global__ void __launch_bounds__(160, 2) attn_decode_i8_kernel(const __grid_constant__ CUtensorMap tmK,
                                                                 const __grid_constant__ CUtensorMap tmV, const AttnParams p) {
-  constexpr int HD = 128, KT = kDecTile, KW = KT / 4;
+  constexpr int HD = 128, KT = kI8Tile;
   extern __shared__ __align__(1024) uint8_t smem_dyn[];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t full_bar[kI8Stages], empty_bar[kI8Stages];
+  float* scale_ring = reinterpret_cast<float*>(ring + kI8Slots * kI8SlotBytes);
+  __shared__ uint64_t full_bar[kI8Slots], empty_bar[kI8Slots];
   __shared__ int s_blk[kDecMaxBlocks];
   __shared__ int s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int i = 0; i < kI8Stages; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 4); }
+    for (int i = 0; i < kI8Slots; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
     s_abort = 0;
     fence_barrier_init();
   }
@@ -915,89 +916,88 @@ __global__ void __launch_bounds__(160, 2) attn_decode_i8_kernel(const __grid_con
   };
   for (int i = tid; i < min(nloc, kDecMaxBlocks); i += 160) s_blk[i] = block_of(t_begin + i);
   __syncthreads();
-  const int npre = max(0, min(min(kI8Stages, nloc), ntiles - 1 - t_begin));      // the newest token's tile is the last one
-  auto issue_tile = [&](int n) {
-    const int st = n % kI8Stages, t = t_begin + n;
+  const int npre = max(0, min(min(kI8Slots, nloc), ntiles - 1 - t_begin));       // the newest token's tile is the last one
+  auto issue_tile = [&](int n, int slot) {
+    const int t = t_begin + n;
     const int row = ((n < kDecMaxBlocks ? s_blk[n] : block_of(t)) * p.hkv + kvh) * p.bs + (t % tiles_per_block) * KT;
-    uint8_t* to = ring + st * kI8StageBytes;
-    mbar_expect_tx(&full_bar[st], kI8Stage);
-    tma_load_2d(to, &tmK, &full_bar[st], 0, row, kEvictFirst);
-    tma_load_2d(to + KT * HD, &tmV, &full_bar[st], 0, row, kEvictFirst);
-    bulk_load(to + 2 * KT * HD, p.ks + row, KT * 4, &full_bar[st]);
-    bulk_load(to + 2 * KT * HD + KT * 4, p.vs + row, KT * 4, &full_bar[st]);
+    uint8_t* to = ring + slot * kI8SlotBytes;
+    float* sc = scale_ring + slot * 2 * KT;
+    mbar_expect_tx(&full_bar[slot], kI8SlotBytes + kI8ScaleBytes);
+    tma_load_2d(to, &tmK, &full_bar[slot], 0, row, kEvictFirst);
+    bulk_load(sc, p.ks + row, KT * 4, &full_bar[slot]);
+    tma_load_2d(to + KT * HD, &tmV, &full_bar[slot], 0, row, kEvictFirst);
+    bulk_load(sc + KT, p.vs + row, KT * 4, &full_bar[slot]);
   };
   if (warp == 4 && elect_one())
-    for (int n = 0; n < npre; ++n) issue_tile(n);
+    for (int n = 0; n < npre; ++n) issue_tile(n, n);
   grid_dep_wait();
 
-  WarpAttn<HD, KW> wa;
+  WarpAttn<HD, KT> wa;
   wa.init();
   if (warp == 4) {
     if (elect_one()) {
-      for (int n = npre; n < nloc; ++n) {
-        const int st = n % kI8Stages;
-        if (!mbar_wait(&empty_bar[st], ((n / kI8Stages) & 1) ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) { s_abort = 1; break; }
-        issue_tile(n);
+      Ring r = {npre % kI8Slots, npre == kI8Slots ? 1u : 0u};
+      for (int n = npre; n < nloc; ++n, r.next(kI8Slots)) {
+        if (!mbar_wait(&empty_bar[r.s], r.ph ^ 1, p.status, XFT_ERR_WAIT_EMPTY)) { s_abort = 1; break; }
+        issue_tile(n, r.s);
       }
     }
   } else {
     const int r0 = lane >> 2, r1 = r0 + 8, t = lane & 3;
-    // step k: features 32 t + 4 k .. + 3 of both rows, the even ones and the odd ones, as a word's codes come apart
+    // step k: features 16 k + 4 t .. + 3 of both rows, the even ones and the odd ones, as a word's codes come apart
     uint32_t qa[HD / 16][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const bf16* q = p.q + ((size_t)tok * p.hq + h_lo) * HD + t * 32 + i * 8;
-      const uint4 a = r0 < nq ? *reinterpret_cast<const uint4*>(q + r0 * HD) : make_uint4(0, 0, 0, 0);
-      const uint4 c = r1 < nq ? *reinterpret_cast<const uint4*>(q + r1 * HD) : make_uint4(0, 0, 0, 0);
-      qa[2 * i][0] = __byte_perm(a.x, a.y, 0x5410); qa[2 * i][1] = __byte_perm(c.x, c.y, 0x5410);
-      qa[2 * i][2] = __byte_perm(a.x, a.y, 0x7632); qa[2 * i][3] = __byte_perm(c.x, c.y, 0x7632);
-      qa[2 * i + 1][0] = __byte_perm(a.z, a.w, 0x5410); qa[2 * i + 1][1] = __byte_perm(c.z, c.w, 0x5410);
-      qa[2 * i + 1][2] = __byte_perm(a.z, a.w, 0x7632); qa[2 * i + 1][3] = __byte_perm(c.z, c.w, 0x7632);
+    for (int k = 0; k < HD / 16; ++k) {
+      const bf16* q = p.q + ((size_t)tok * p.hq + h_lo) * HD + k * 16 + t * 4;
+      const uint2 a = r0 < nq ? *reinterpret_cast<const uint2*>(q + r0 * HD) : make_uint2(0, 0);
+      const uint2 c = r1 < nq ? *reinterpret_cast<const uint2*>(q + r1 * HD) : make_uint2(0, 0);
+      qa[k][0] = __byte_perm(a.x, a.y, 0x5410); qa[k][1] = __byte_perm(c.x, c.y, 0x5410);
+      qa[k][2] = __byte_perm(a.x, a.y, 0x7632); qa[k][3] = __byte_perm(c.x, c.y, 0x7632);
     }
-    Ring r = {0, 0};
-    for (int n = 0; n < nloc; ++n, r.next(kI8Stages)) {
-      const int st = r.s;
-      if (!mbar_wait(&full_bar[st], r.ph, p.status, XFT_ERR_WAIT_FULL)) { s_abort = 1; break; }
-      const uint8_t* kt = ring + st * kI8StageBytes + warp * KW * HD;      // this warp's 16 keys
+    Ring r = {0, 0};                                       // over this warp's slots: warp, warp + 4, ..
+    for (int n = warp; n < nloc; n += 4, r.next(kI8Slots / 4)) {
+      const int slot = warp + 4 * r.s;
+      if (!mbar_wait(&full_bar[slot], r.ph, p.status, XFT_ERR_WAIT_FULL)) { s_abort = 1; break; }
+      const uint8_t* kt = ring + slot * kI8SlotBytes;
       const uint8_t* vt = kt + KT * HD;
-      const float* scales = reinterpret_cast<const float*>(ring + st * kI8StageBytes + 2 * KT * HD) + warp * KW;
-      const int key0 = (t_begin + n) * KT + warp * KW;
-      if (key0 < kv_len) {
-        float s[2][4];
+      const float* scales = scale_ring + slot * 2 * KT;
+      const int key0 = (t_begin + n) * KT;
+      float s[KT / 8][4];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const uint8_t* row = kt + (j * 8 + r0) * HD;
-          const uint4 lo = *reinterpret_cast<const uint4*>(row + (((2 * t) ^ r0) << 4));
-          const uint4 hi = *reinterpret_cast<const uint4*>(row + (((2 * t + 1) ^ r0) << 4));
-          const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-          s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+      for (int j = 0; j < KT / 8; ++j) {                   // row lane & 7 of the eight keys, 16-byte chunks lane >> 3 and four further on
+        const uint8_t* row = kt + (j * 8 + (lane & 7)) * HD;
+        uint32_t w[2][4];
+        ldsm_x4(w[0], row + (((lane >> 3) ^ (lane & 7)) << 4));
+        ldsm_x4(w[1], row + (((4 + (lane >> 3)) ^ (lane & 7)) << 4));
+        s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
 #pragma unroll
-          for (int k = 0; k < 8; ++k) mma16816(s[j], qa[k], codes_bf16(w[k]), codes_bf16(w[k] >> 8));
-        }
-        float vs[2][2];
+        for (int k = 0; k < HD / 16; ++k) mma16816(s[j], qa[k], codes_bf16(w[k >> 2][k & 3]), codes_bf16(w[k >> 2][k & 3] >> 8));
+      }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const float2 ks2 = *reinterpret_cast<const float2*>(scales + j * 8 + 2 * t);
-          const float2 vs2 = *reinterpret_cast<const float2*>(scales + KT + j * 8 + 2 * t);
-          const int left = kv_len - key0 - j * 8 - 2 * t;  // slots past the end hold whatever their last owner left, scales too
-          vs[j][0] = left > 0 ? vs2.x : 0.f;
-          vs[j][1] = left > 1 ? vs2.y : 0.f;
-          s[j][0] = left > 0 ? s[j][0] * p.scale * ks2.x : -INFINITY;
-          s[j][1] = left > 1 ? s[j][1] * p.scale * ks2.y : -INFINITY;
-          s[j][2] = left > 0 ? s[j][2] * p.scale * ks2.x : -INFINITY;
-          s[j][3] = left > 1 ? s[j][3] * p.scale * ks2.y : -INFINITY;
-        }
-        wa.softmax_update(s, nullptr, lane);
+      for (int j = 0; j < KT / 8; ++j) {
+        const float2 ks2 = *reinterpret_cast<const float2*>(scales + j * 8 + 2 * t);
+        const int left = kv_len - key0 - j * 8 - 2 * t;    // slots past the end hold whatever their last owner left, scales too
+        s[j][0] = left > 0 ? s[j][0] * p.scale * ks2.x : -INFINITY;
+        s[j][1] = left > 1 ? s[j][1] * p.scale * ks2.y : -INFINITY;
+        s[j][2] = left > 0 ? s[j][2] * p.scale * ks2.x : -INFINITY;
+        s[j][3] = left > 1 ? s[j][3] * p.scale * ks2.y : -INFINITY;
+      }
+      wa.softmax_update(s, nullptr, lane);
+#pragma unroll
+      for (int k = 0; k < KT / 16; ++k) {
         uint32_t a[4];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          a[2 * j] = pack_bf16(s[j][0] * vs[j][0], s[j][1] * vs[j][1]);
-          a[2 * j + 1] = pack_bf16(s[j][2] * vs[j][0], s[j][3] * vs[j][1]);
+        for (int i = 0; i < 2; ++i) {
+          const int j = 2 * k + i, left = kv_len - key0 - j * 8 - 2 * t;
+          const float2 vs2 = *reinterpret_cast<const float2*>(scales + KT + j * 8 + 2 * t);
+          const float x = left > 0 ? vs2.x : 0.f, y = left > 1 ? vs2.y : 0.f;
+          a[2 * i] = pack_bf16(s[j][0] * x, s[j][1] * y);
+          a[2 * i + 1] = pack_bf16(s[j][2] * x, s[j][3] * y);
         }
         uint4 v[4];                                        // 16 features of keys 2 t, 2 t + 1 and of those 8 further on
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int key = (i >> 1) * 8 + 2 * t + (i & 1);
+          const int key = k * 16 + (i >> 1) * 8 + 2 * t + (i & 1);
           v[i] = *reinterpret_cast<const uint4*>(vt + key * HD + ((r0 ^ (key & 7)) << 4));
         }
 #pragma unroll
@@ -1009,7 +1009,7 @@ __global__ void __launch_bounds__(160, 2) attn_decode_i8_kernel(const __grid_con
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty_bar[st]);
+      if (lane == 0) mbar_arrive(&empty_bar[slot]);
     }
     wa.reduce_l();
   }
@@ -1297,7 +1297,7 @@ static int launch_decode_tma(const AttnParams& p, int B, bool brief, cudaStream_
 static int launch_decode_i8(const AttnParams& p, int B, cudaStream_t st) {
   CUtensorMap tmK, tmV;
   const uint64_t rows = (uint64_t)p.num_blocks * p.hkv * p.bs;
-  if (make_tensor_map(&tmK, p.kc, rows, 128, 128, kDecTile, 1) || make_tensor_map(&tmV, p.vc, rows, 128, 128, kDecTile, 1)) return -4;
+  if (make_tensor_map(&tmK, p.kc, rows, 128, 128, kI8Tile, 1) || make_tensor_map(&tmV, p.vc, rows, 128, 128, kI8Tile, 1)) return -4;
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(attn_decode_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kI8Smem) != cudaSuccess) return -5;

@@ -678,20 +678,11 @@ def plan_attn_splits(B, hkv, group, D, max_kv, int8=False, least=8):
     """Split-KV factor of a decode launch and the tile count it was planned on: fill the resident CTA slots (two
     CTAs per SM for the TMA-ring kernel of bf16 caches and for int8 caches, three for the cp.async kernel) while leaving
     every slice at least `least` tiles."""
-    ctas = B * max(hkv, 1) * ((group + 15) // 16)
-    if int8 and D == 128 and least == 8 and _ENV().attn_splits <= 0:
-        # the ring of codes merges in clusters: as many slices as one round of clusters holds (two CTAs per SM), with two 64-key tiles
-        # each.  us for 1, 2, 4, 8 slices: 1 sequence of 3000 keys, 8 kv heads 38.5, 22.7, 13.1, 9.1; 8 of 2870 46, 30, 19.4, 26; 8 of 600
-        # 11.5, 10.1, 9.1, 15.9; 4 of 1500, 32 kv heads 27, 18, 24, 34; 16 of 200, 8 kv heads 7.9, 9.8, 15.3
-        ntiles = (max_kv + 63) // 64
-        fit = 8 if ctas <= 33 else 4 if ctas <= 71 else 2 if ctas <= 148 else 1
-        while fit > 1 and (ntiles < 8 or 2 * fit > ntiles):
-            fit //= 2
-        return fit, ntiles
     tma = not int8 and _ENV().attn_tma
     kt = 64 if tma else {64: 64, 128: 32, 256: 16}[D]
     slots = (296 if D <= 128 else 148) if tma else 296 if int8 else 444
     ntiles = (max_kv + kt - 1) // kt
+    ctas = B * max(hkv, 1) * ((group + 15) // 16)
     nsplit = max(1, min(slots // max(ctas, 1), ntiles // least if ntiles >= 16 else 1, 32))
     if _ENV().attn_splits > 0:
         nsplit = max(1, min(_ENV().attn_splits, ntiles, 32))
