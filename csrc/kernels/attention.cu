@@ -532,20 +532,43 @@ __device__ __forceinline__ void decode_finish(const AttnParams& p, WA& wa, float
     __syncthreads();
     if (s_last) {
       __threadfence();
-      for (int i = tid; i < nq * HD; i += nthreads) {
-        const int r = i / HD, d = i % HD;
-        const int h = h_lo + r;
-        const size_t base = ((size_t)b * p.hq + h) * p.nsplit;
+      // four features and eight slices with their loads under way together: a thread that walked the slices one by one waited for each
+      // (us, so / now: 32 and 8 heads, one sequence, int8 cache 3000 keys in 11 slices 18.9 / 12.3, 8000 in 31 28.1 / 15.0, 32000 in 32 36.4 /
+      // 26.8; bf16 cache 32000 in 32 35.9 / 27.3)
+      for (int i = tid; i < nq * (HD / 4); i += nthreads) {
+        const int r = i / (HD / 4), d = i % (HD / 4);
+        const size_t base = ((size_t)b * p.hq + h_lo + r) * p.nsplit;
         float mm = -INFINITY;
-        for (int s = 0; s < p.nsplit; ++s) mm = fmaxf(mm, __ldcg(p.part_ml + (base + s) * 2));
-        float acc = 0.f, ll = 0.f;
-        for (int s = 0; s < p.nsplit; ++s) {
-          const float ms = __ldcg(p.part_ml + (base + s) * 2);
-          const float c = (ms == -INFINITY) ? 0.f : __expf(ms - mm);
-          acc += c * __ldcg(p.part_o + (base + s) * HD + d);
-          ll += c * __ldcg(p.part_ml + (base + s) * 2 + 1);
+        for (int s0 = 0; s0 < p.nsplit; s0 += 8) {
+          float ms[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) ms[k] = s0 + k < p.nsplit ? __ldcg(p.part_ml + (base + s0 + k) * 2) : -INFINITY;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) mm = fmaxf(mm, ms[k]);
         }
-        p.out[((size_t)tok * p.hq + h) * HD + d] = __float2bfloat16(ll > 0.f ? acc / ll : 0.f);
+        float acc[4] = {0.f, 0.f, 0.f, 0.f}, ll = 0.f;
+        for (int s0 = 0; s0 < p.nsplit; s0 += 8) {
+          float ms[8], ls[8], as[8][4];
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (s0 + k < p.nsplit) {
+              ms[k] = __ldcg(p.part_ml + (base + s0 + k) * 2);
+              ls[k] = __ldcg(p.part_ml + (base + s0 + k) * 2 + 1);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) as[k][e] = __ldcg(p.part_o + (base + s0 + k) * HD + d + e * (HD / 4));
+            }
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (s0 + k < p.nsplit) {
+              const float c = (ms[k] == -INFINITY) ? 0.f : __expf(ms[k] - mm);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) acc[e] += c * as[k][e];
+              ll += c * ls[k];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          p.out[((size_t)tok * p.hq + h_lo + r) * HD + d + e * (HD / 4)] = __float2bfloat16(ll > 0.f ? acc[e] / ll : 0.f);
       }
     }
   }
