@@ -23,6 +23,8 @@
 // scores, and one sink per query head (a term of the softmax denominator that has no key and no value).
 #include "ptx.cuh"
 
+#include <atomic>
+
 namespace xft {
 
 typedef __nv_bfloat16 bf16;
@@ -46,7 +48,7 @@ struct AttnParams {
   // decode split
   int nsplit; float* part_o; float* part_ml;   // [B, hq, nsplit, HD], [B, hq, nsplit, 2]
   int* split_counters;      // [B * gridDim.y] arrival counters (zero between launches)
-  int cluster;              // != 0: the slices of a (sequence, kv head) are the CTAs of a cluster
+  int cluster;              // != 0: the slices of a (sequence, kv head) are the CTAs of a cluster (launch_slices)
   int* status;
   // EXT only
   float softcap, inv_cap2;  // cap and 2 / cap (softcap 0: none)
@@ -434,8 +436,8 @@ __device__ __forceinline__ void leave_cluster(const AttnParams& p) {
 // then either store the result (nsplit == 1), or merge the slices of the (sequence, kv head): in a cluster each CTA leaves its
 // partial behind the warps' in its own shared memory and stores a share of the result from all of them; otherwise it goes to
 // global scratch and the slice that arrives last merges all — no second kernel, no spinning.  Every thread of the CTA calls it.
-// The sums are the same.  us by scratch / in clusters: bf16 cache, one sequence of 3000 keys, 32 and 8 heads, five slices 14.5 / 9.6;
-// 8 of 2870 in four 21.0 / 18.7; 2 of 3000, 64 and 8 heads, five 20.0 / 12.4; int8 cache, 8 of 2870 in four 21.5 / 19.4.
+// The sums are the same.  us by scratch (its loads still one behind the other) / in clusters, bf16 cache: one sequence of 3000 keys, 32 and
+// 8 heads, five slices 14.5 / 9.6; 8 of 2870 in four 21.0 / 18.7; 2 of 3000, 64 and 8 heads, five 20.0 / 12.4.
 // RING: a kernel that may be launched in clusters.  APART: column n of accumulator j is head feature n * HD / 8 + j
 // (attn_decode_i8_kernel), else j * 8 + n.
 template <int HD, bool RING, bool APART = false, class WA>
@@ -1260,29 +1262,44 @@ static int launch_decode(const AttnParams& p, int B, bool int8, cudaStream_t st)
   return (int)cudaGetLastError();
 }
 
-// Launch of a ring kernel; up to eight slices of a (sequence, kv head) share a cluster.
-template <typename K>
-static int launch_slices(K kernel, dim3 grid, size_t smem, const CUtensorMap& tmK, const CUtensorMap& tmV, AttnParams p, cudaStream_t st) {
-  p.cluster = p.nsplit > 1 && p.nsplit <= 8;
+// Launch of a ring kernel; up to eight slices of a (sequence, kv head) share a cluster, where the GPU takes all of the clusters at a time
+// (GPCs differ in their SMs, so that is asked for).  Where it does not, a second round costs more than the merge through scratch.
+// us, clusters in two rounds / scratch, 32 and 8 heads, bf16 cache: 9 x 4000 keys in four slices 36.7 / 27.1, 12 x 3000 in three 38.5 / 26.8,
+// 6 x 5000 in six 33.4 / 23.7; 8 and 1 heads: 36 x 4500 in eight 26.8 / 20.6; int8 cache 9 x 4000 in four 36.6 / 24.8.
+template <auto KERNEL>
+static int launch_slices(dim3 grid, size_t smem, const CUtensorMap& tmK, const CUtensorMap& tmV, AttnParams p, cudaStream_t st) {
+  static std::atomic<int> fit[9];                          // clusters of so many CTAs, plus one; 0: not asked yet
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(160);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
   int n = 0;
+  p.cluster = 0;
+  if (p.nsplit > 1 && p.nsplit <= 8) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = p.nsplit;
+    cfg.numAttrs = 1;
+    int most = fit[p.nsplit].load(std::memory_order_relaxed) - 1;
+    if (most < 0) {
+      if (cudaOccupancyMaxActiveClusters(&most, KERNEL, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        most = 0;
+      }
+      fit[p.nsplit].store(most + 1, std::memory_order_relaxed);
+    }
+    p.cluster = (long long)grid.x * grid.y <= most;
+    n = p.cluster;
+  }
   if (g_xft_pdl) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
-  if (p.cluster) {
-    attr[n].id = cudaLaunchAttributeClusterDimension;
-    attr[n].val.clusterDim.x = attr[n].val.clusterDim.y = 1;
-    attr[n++].val.clusterDim.z = p.nsplit;
-  }
-  cfg.attrs = attr;
   cfg.numAttrs = n;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tmK, tmV, (const AttnParams)p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, KERNEL, tmK, tmV, (const AttnParams)p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -1314,7 +1331,7 @@ static int launch_decode_tma(const AttnParams& p, int B, bool brief, cudaStream_
       return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
     }
   }
-  return launch_slices(attn_decode_tma_kernel<HD, EXT>, dim3(B, p.hkv * qchunks, p.nsplit), smem, tmK, tmV, p, st);
+  return launch_slices<attn_decode_tma_kernel<HD, EXT>>(dim3(B, p.hkv * qchunks, p.nsplit), smem, tmK, tmV, p, st);
 }
 
 static int launch_decode_i8(const AttnParams& p, int B, cudaStream_t st) {
@@ -1326,7 +1343,7 @@ static int launch_decode_i8(const AttnParams& p, int B, cudaStream_t st) {
     if (cudaFuncSetAttribute(attn_decode_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kI8Smem) != cudaSuccess) return -5;
     attr_set = true;
   }
-  return launch_slices(attn_decode_i8_kernel, dim3(B, p.hkv * ((p.group + 15) / 16), p.nsplit), kI8Smem, tmK, tmV, p, st);
+  return launch_slices<attn_decode_i8_kernel>(dim3(B, p.hkv * ((p.group + 15) / 16), p.nsplit), kI8Smem, tmK, tmV, p, st);
 }
 
 template <bool EXT>
