@@ -592,7 +592,7 @@ class Decoder:
         else:
             q, kv = ops.linear(h, L.q_direct), ops.linear(h, L.kv_a)
         q_nope, q_rope = ops.mla_prep(q, kv, Hl, nope, rope, kvl, b.positions, self.rope_table, L.kv_a_norm, self.eps,
-                                      cache.k[li], b.slots, None if b.is_decode else b.cu_q, vd)
+                                      cache.k[li], b.slots, None if b.is_decode else b.cu_q, vd, b.kv_lens)
         a = ops.mla_attention(q_nope, q_rope, cache.k[li], b.block_table, b.cu_q, b.kv_lens, L.w_uk, L.w_uv,
                               self.scale, absorbed=b.is_decode, meta=b)
         return a.reshape(T, Hl * vd)

@@ -238,16 +238,17 @@ def latent_cache_write(latent, cache, slots):
     cache[(slots // blk).long(), 0, (slots % blk).long()] = latent.to(cache.dtype)
 
 
-def mla_prep(q, kv, Hl, nope, rope, kvl, positions, table, kv_norm_w, eps, cache, slots, cu_q=None, vd=0):
+def mla_prep(q, kv, Hl, nope, rope, kvl, positions, table, kv_norm_w, eps, cache, slots, cu_q=None, vd=0, kv_lens=None):
     """What sits between the MLA projections and the MLA attention: split every query head of q [T, Hl*(nope+rope)]
     into its no-position part and its rotated part (interleaved pairs), RMS-normalise the compressed KV kv[:, :kvl],
     rotate the shared key part kv[:, kvl:], and append (normalised KV ‖ rotated key) to the latent cache at `slots`.
-    Returns (q_nope [T,Hl,nope], q_rope [T,Hl,rope]).  One kernel on the GPU.  `cu_q` (prompts) and `vd`, the values' size: what the
-    attention behind it is asked for, so that the queries come in the layout that it reads."""
+    Returns (q_nope [T,Hl,nope], q_rope [T,Hl,rope]).  One kernel on the GPU.  `cu_q` and `kv_lens` (prompts) and `vd`, the values' size:
+    what the attention behind it is asked for, so that the queries come in the layout that it reads."""
     if _cuda(q) and cache.dtype == torch.bfloat16:
+        from ..utils.flags import Env
         from .native_mla import expands
         return _nat().mla_prep(q, kv, Hl, nope, rope, kvl, positions, table, kv_norm_w, eps, cache, slots,
-                               cu_q is not None and expands(cu_q, nope, rope, kvl, vd))
+                               cu_q is not None and Env.get().mla_expand and expands(cu_q, nope, rope, kvl, vd, kv_lens))
     T = q.shape[0]
     q3 = q.reshape(T, Hl, nope + rope)
     ckv = R.rmsnorm(kv[:, :kvl], kv_norm_w, eps)

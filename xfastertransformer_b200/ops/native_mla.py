@@ -1,7 +1,8 @@
-"""DeepSeek MLA on the GPU.  Decode steps and portions of a few tokens take the absorbed form: grouped tcgen05 GEMMs (one group per head)
-around the latent-cache attention kernel (csrc/kernels/mla.cu), which works per token.  Longer portions take the expanded form
-(csrc/kernels/latent_prefill_sm100.cu, see native_latent): the latents that they see times W_uk and W_uv once, then attention in tiles
-of 128 queries."""
+"""DeepSeek MLA on the GPU.  The absorbed form is used for prefill and decode alike: grouped tcgen05 GEMMs (one group per head) around the
+latent-cache attention kernel (csrc/kernels/mla.cu), which works per token.  With XFT_MLA_EXPAND=1 longer portions of prompts take the
+expanded form (csrc/kernels/latent_prefill_sm100.cu, see native_latent): the latents that they see times W_uk and W_uv once, then
+attention in tiles of 128 queries.  It is faster, but rounds keys and values of each head to bf16 where the absorbed form rounds its query
+and its latent result, so a model's logits differ by as much as either differs from 64 bits."""
 from __future__ import annotations
 
 import ctypes as C
@@ -60,17 +61,25 @@ def _per_head_gemm(x_ht, w_stacked, H, T, n_out, k_in):
     return out
 
 
-def expands(cu_q, nope, rope, kvl, vd) -> bool:
-    """Whether a batch's portions of at least XFT_LATENT_EXPAND_MIN_Q new tokens take the expanded form: sizes that attn_flat_tc_kernel has,
-    and 64 tokens that take it, or 256 where shorter portions beside them need a launch of the other form.  us of a layer's attention
-    with its per-head products, 128 heads, absorbed / expanded (error against 64 bits): 32 prompts of about 97 tokens 2087 / 339 (2.682e-3
-    and 2.680e-3 of the result), 32 of 16 355 / 218, 8 of 8 115 / 84, one of 200 169 / 78, of 2000 3866 / 344 (2.84e-3, 2.76e-3), 64 tokens
-    behind 4000 508 / 238; one of 16 tokens 58 / 78; 140 tokens in two portions beside two short ones 128 / 174."""
+def expands(cu_q, nope, rope, kvl, vd, kv_lens=None) -> bool:
+    """Whether a batch's portions of at least XFT_LATENT_EXPAND_MIN_Q new tokens pay for the expanded form: sizes that attn_flat_tc_kernel
+    has, 64 tokens that take it, or 256 where shorter portions beside them need a launch of the other form, and, as it works per visible key
+    and the absorbed form per key and token, 40 tokens per visible key or 256 keys per portion.  us of a layer's attention with its
+    per-head products, 128 heads, absorbed / expanded (error against 64 bits): 32 prompts of about 97 tokens 2087 / 339 (2.682e-3 and
+    2.680e-3 of the result), 32 of 16 351 / 212, one of 200 169 / 78, of 2000 3866 / 344 (2.84e-3, 2.76e-3); 4 x 16 tokens behind 300 keys
+    141 / 116, 4000 511 / 840, 32000 3345 / 6757; 32 x 16 behind 300 529 / 648; 8 x 32 behind 1000 574 / 509, 16000 5690 / 6534; 4 x 64
+    behind 4000 1566 / 853, 32000 11339 / 6909; one of 16 tokens 58 / 78; 140 tokens in two portions beside two short ones 128 / 174."""
     if nope % 64 or rope % 64 or nope + rope > 256 or kvl % 8 or vd % 64 or vd > 128:
         return False
     least = N._ENV().latent_expand_min_q
     n = [cu_q[i + 1] - cu_q[i] for i in range(len(cu_q) - 1)]
-    return sum(q for q in n if q >= least) >= (64 if min(n) >= least else 256)
+    long = [i for i, q in enumerate(n) if q >= least]
+    if sum(n[i] for i in long) < (64 if min(n) >= least else 256):
+        return False
+    if kv_lens is None:
+        return True
+    keys = sum(kv_lens[i] for i in long)
+    return keys <= 256 * len(long) or sum(n[i] * kv_lens[i] for i in long) >= 40 * keys
 
 
 class _Heads:
@@ -120,7 +129,7 @@ def mla_attention(q_nope, q_rope, latent_cache, block_table, cu_q, kv_lens, w_uk
     assert L == 512 and rope == 64, "MLA kernel is specialised for kv_lora_rank 512 + rope 64"
     dev = q_nope.device
     cu_dev, kv_dev, B, decode, max_kv = N.batch_arrays(cu_q, kv_lens, meta, dev)
-    if not decode and scale > 0 and expands(cu_q, nope, rope, L, vd):
+    if N._ENV().mla_expand and not decode and scale > 0 and expands(cu_q, nope, rope, L, vd, kv_lens):
         from .native_latent import _Spans
         kept = meta.meta if meta is not None else {}
         key = ("latent spans", 0, N._ENV().latent_expand_min_q)

@@ -77,6 +77,7 @@ class Env:
         # a very large value switches it off
         self.attn_tc_min_q = _int("XFT_ATTN_TC_MIN_Q", 2)
         self.latent_expand_min_q = _int("XFT_LATENT_EXPAND_MIN_Q", 16)   # prompt portions from this size on expand their latents
+        self.mla_expand = _int("XFT_MLA_EXPAND", 0) != 0          # DeepSeek's prompts: such portions in the expanded form
         self.gla_chunk_min_q = _int("XFT_GLA_CHUNK_MIN_Q", 16)    # gated linear attention: portions from this size on go in chunks
         self.ssd_chunk_min_q = _int("XFT_SSD_CHUNK_MIN_Q", 16)    # the same of state-space layers
         self.talking_tc = _int("XFT_TALKING_TC", 1) != 0          # attention with mixed heads on the tensor cores (0: plain kernel)
