@@ -796,6 +796,13 @@ static int launch_prefill(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
 
 using namespace xft;
 
+extern "C" int xft_paged_attention_ext(const void* q, void* out, const void* kc, const void* vc, const float* ks, const float* vs,
+                                       const int* block_table, int bt_stride, const int* cu_q, const int* kv_lens, int B, int max_q,
+                                       int hq, int hkv, int group, int q_off, int HD, int bs, int num_blocks, float scale,
+                                       const float* slopes, const int* prefix_lens, int decode, int nsplit, float* part_o,
+                                       float* part_ml, int* split_counters, int* status, float softcap, int window, int keep,
+                                       const float* sinks, cudaStream_t st);      // attention.cu
+
 // Causal prefill attention over the paged bf16 cache, head_dim 128 (see the file comment).  q, out: [T, hq, 128];
 // caches [num_blocks, hkv, bs, 128] with bs = 64; cu_q [B + 1], kv_lens [B] (keys visible after this call's append).
 // softcap > 0: scores become softcap * tanh(score / softcap).  window > 0: position i sees the keys j <= i with
@@ -807,11 +814,15 @@ extern "C" int xft_attn_prefill_tc(const void* q, void* out, const void* kc, con
                                    int window, int keep, const float* sinks, int* status, cudaStream_t st) {
   if (B <= 0 || T <= 0 || max_q <= 0) return 0;
   if (bs != 64 || hq <= 0 || hkv <= 0 || softcap < 0.f || window < 0 || keep < 0) return -1;
+  const bool ext = softcap > 0.f || window > 0 || sinks;
+  if (!ext && !(scale > 0.f))                  // attn_prefill_tc_kernel takes the maximum before scores are scaled, and hides keys there
+    return xft_paged_attention_ext(q, out, kc, vc, nullptr, nullptr, block_table, bt_stride, cu_q, kv_lens, B, max_q, hq, hkv, group, q_off,
+                                   128, bs, num_blocks, scale, nullptr, nullptr, 0, 1, nullptr, nullptr, nullptr, status, 0.f, 0, 0, nullptr,
+                                   st);
   PrefillAttnParams p{};
   p.out = (__nv_bfloat16*)out; p.block_table = block_table; p.bt_stride = bt_stride; p.cu_q = cu_q; p.kv_lens = kv_lens;
   p.hq = hq; p.hkv = hkv; p.group = group; p.q_off = q_off; p.bs = bs; p.scale_log2 = scale * 1.4426950408889634f;
   p.num_blocks = num_blocks; p.status = status;
-  const bool ext = softcap > 0.f || window > 0 || sinks;
   p.window = window > 0 ? min(window, 1 << 30) : 1 << 30; p.keep = window > 0 ? keep : 0; p.sinks = sinks;
   p.cap_log2 = softcap * 1.4426950408889634f;
   p.inv_cap = softcap > 0.f ? scale / softcap : 0.f;
@@ -840,6 +851,9 @@ extern "C" int xft_attn_prefill_tc_int8(const void* q, void* out, const void* kc
                                         int num_blocks, float scale, int* status, cudaStream_t st) {
   if (B <= 0 || T <= 0 || max_q <= 0) return 0;
   if (bs != 64 || hq <= 0 || hkv <= 0 || copy_w <= 0 || ((reinterpret_cast<uintptr_t>(ks) | reinterpret_cast<uintptr_t>(vs)) & 15)) return -1;
+  if (!(scale > 0.f))
+    return xft_paged_attention_ext(q, out, kc, vc, ks, vs, block_table, bt_stride, cu_q, kv_lens, B, max_q, hq, hkv, group, q_off, 128, bs,
+                                   num_blocks, scale, nullptr, nullptr, 0, 1, nullptr, nullptr, nullptr, status, 0.f, 0, 0, nullptr, st);
   PrefillAttnParams p{};
   p.out = (__nv_bfloat16*)out; p.block_table = block_table; p.bt_stride = bt_stride; p.cu_q = cu_q; p.kv_lens = kv_lens;
   p.hq = hq; p.hkv = hkv; p.group = group; p.q_off = q_off; p.bs = bs; p.scale_log2 = scale * 1.4426950408889634f;
