@@ -190,8 +190,13 @@ __global__ void __launch_bounds__(kRowThreads) quant_rows_kernel(const RowsParam
 template <bool NORM, int MODE>
 static int launch_rows(const RowsParams& p, int rows, cudaStream_t st) {
   const int span = MODE == kRowsInt8 ? p.K : p.Kp;
-  const auto kernel = span <= 4096 ? quant_rows_kernel<2, NORM, MODE> : span <= 8192 ? quant_rows_kernel<4, NORM, MODE>
-                      : span <= 16384 ? quant_rows_kernel<8, NORM, MODE> : quant_rows_kernel<16, NORM, MODE>;
+  const auto kernel = [&] {
+    if constexpr (!NORM) {                                             // with a norm up to 8192, see xft_rms_quant_act
+      if (span > 16384) return quant_rows_kernel<16, NORM, MODE>;
+      if (span > 8192) return quant_rows_kernel<8, NORM, MODE>;
+    }
+    return span > 4096 ? quant_rows_kernel<4, NORM, MODE> : quant_rows_kernel<2, NORM, MODE>;
+  }();
   const cudaError_t e = launch_pdl(kernel, dim3(rows), dim3(kRowThreads), 0, st, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
